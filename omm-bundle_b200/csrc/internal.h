@@ -65,6 +65,37 @@ struct __align__(16) zdbl {
     double x, y;
 };
 
+// ----------------------------------------------------------------- elementwise kernels
+// The elementwise kernels walk the matrix in column-major element order, thread t taking elements
+// t, t + T, t + 2T, ... (T threads).  (row, column) advance by (T % rows, T / rows) with one carry, so
+// that an element costs an add and a compare instead of a 64-bit division and remainder (about 70
+// instructions, which made these kernels issue-bound: 2049 x 1537 complex C = B took 22 us, the bytes
+// need 15).
+struct Walk {
+    size_t e, total, step;
+    int i, j, di, dj, rows;
+    __device__ Walk(int rows_, int cols) : rows(rows_) {
+        e = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+        total = (size_t)rows * cols;
+        step = (size_t)gridDim.x * blockDim.x;
+        // the launches cover at most 148 * 32 * 256 threads: the first element and the step fit 32 bits
+        const unsigned r = rows > 0 ? (unsigned)rows : 1u, e0 = (unsigned)e, st = (unsigned)step;
+        i = (int)(e0 % r);
+        j = (int)(e0 / r);
+        di = (int)(st % r);
+        dj = (int)(st / r);
+    }
+    __device__ void next() {
+        e += step;
+        i += di;
+        j += dj;
+        if (i >= rows) {
+            i -= rows;
+            ++j;
+        }
+    }
+};
+
 // ----------------------------------------------------------------- device memory
 struct DevBuf {
     void* p = nullptr;

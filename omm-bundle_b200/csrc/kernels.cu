@@ -5,6 +5,7 @@
 // Real matrices are double, complex ones zdbl (interleaved re, im).
 #include "internal.h"
 
+#include <algorithm>
 #include <cmath>
 
 namespace ommgpu {
@@ -43,40 +44,88 @@ inline int grid_for(size_t elems, int per_thread = 4) {
     return (int)b;
 }
 
-// C = beta*C + alpha*op(A)  (MatrixSwitch_m_add.F90:95-175: C=beta*C first, then += alpha*op(A))
+constexpr int kAhead = 4;  // elements whose loads a thread issues before it uses the first
+
+// C = beta*C + alpha*A  (MatrixSwitch_m_add.F90:95-175: C=beta*C first, then += alpha*op(A)).
+// Bound by memory: two reads and a write per element.
 template <typename T>
-__global__ void axpby_kernel(int rows, int cols, const T* __restrict__ A, int lda, int op, T* __restrict__ C, int ldc,
+__global__ void axpby_kernel(int rows, int cols, const T* __restrict__ A, int lda, T* __restrict__ C, int ldc,
                              zdbl alpha, zdbl beta, int beta_zero) {
-    size_t total = (size_t)rows * cols;
-    for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (size_t)gridDim.x * blockDim.x) {
-        int i = (int)(e % rows), j = (int)(e / rows);
-        T a;
-        if (op == 0) a = A[i + (size_t)j * lda];
-        else if (op == 1) a = A[j + (size_t)i * lda];
-        else a = Sc<T>::conj(A[j + (size_t)i * lda]);
-        T c = beta_zero ? T{} : Sc<T>::mul(beta, C[i + (size_t)j * ldc]);
-        C[i + (size_t)j * ldc] = Sc<T>::add(c, Sc<T>::mul(alpha, a));
+    Walk w(rows, cols);
+    while (w.e < w.total) {
+        T a[kAhead], cin[kAhead];
+        T* at[kAhead];
+        int cnt = 0;
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u) {
+            at[u] = nullptr;
+            if (w.e < w.total) {
+                a[u] = A[w.i + (size_t)w.j * lda];
+                at[u] = C + w.i + (size_t)w.j * ldc;
+                cin[u] = *at[u];
+                ++cnt;
+                w.next();
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u)
+            if (u < cnt) {
+                T c = beta_zero ? T{} : Sc<T>::mul(beta, cin[u]);
+                *at[u] = Sc<T>::add(c, Sc<T>::mul(alpha, a[u]));
+            }
+    }
+}
+
+// C = beta*C + alpha*A^T or alpha*A^H: one 32 x 32 tile per block turn, A's tile staged through shared
+// memory so that its reads run down its columns.  2049 x 1537 complex: 23 us where the element walk,
+// one 32-byte sector per element of A, took 45.
+template <typename T>
+__global__ void axpby_trans_kernel(int rows, int cols, const T* __restrict__ A, int lda, int conj, T* __restrict__ C,
+                                   int ldc, zdbl alpha, zdbl beta, int beta_zero) {
+    __shared__ T tile[32][33];
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;  // 32 x 8
+    const int tr = (rows + 31) / 32, tc = (cols + 31) / 32;
+    for (long long t = blockIdx.x; t < (long long)tr * tc; t += gridDim.x) {
+        const int r0 = (int)(t % tr) * 32, c0 = (int)(t / tr) * 32;
+        T cin[4];
+        __syncthreads();
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int yy = ty + 8 * q;
+            const int j = c0 + tx, i = r0 + yy;  // A(j, i)
+            if (i < rows && j < cols) tile[yy][tx] = A[j + (size_t)i * lda];
+            const int ci = r0 + tx, cj = c0 + yy;
+            if (ci < rows && cj < cols) cin[q] = C[ci + (size_t)cj * ldc];
+        }
+        __syncthreads();
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int yy = ty + 8 * q, i = r0 + tx, j = c0 + yy;
+            if (i < rows && j < cols) {
+                T a = tile[tx][yy];
+                if (conj) a = Sc<T>::conj(a);
+                T c = beta_zero ? T{} : Sc<T>::mul(beta, cin[q]);
+                C[i + (size_t)j * ldc] = Sc<T>::add(c, Sc<T>::mul(alpha, a));
+            }
+        }
     }
 }
 
 template <typename T>
 __global__ void scale_kernel(int rows, int cols, T* C, int ldc, zdbl beta) {
-    size_t total = (size_t)rows * cols;
-    for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (size_t)gridDim.x * blockDim.x) {
-        int i = (int)(e % rows), j = (int)(e / rows);
-        C[i + (size_t)j * ldc] = Sc<T>::mul(beta, C[i + (size_t)j * ldc]);
+    for (Walk w(rows, cols); w.e < w.total; w.next()) {
+        T* c = C + w.i + (size_t)w.j * ldc;
+        *c = Sc<T>::mul(beta, *c);
     }
 }
 
 // m_set (MatrixSwitch_m_set.F90:19-75): lu 0 all, 1 upper (j>=i), 2 lower (j<=i)
 template <typename T>
 __global__ void set_kernel(int rows, int cols, T* C, int ldc, int lu, zdbl alpha, zdbl beta) {
-    size_t total = (size_t)rows * cols;
-    for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (size_t)gridDim.x * blockDim.x) {
-        int i = (int)(e % rows), j = (int)(e / rows);
-        if (lu == 1 && j < i) continue;
-        if (lu == 2 && j > i) continue;
-        C[i + (size_t)j * ldc] = Sc<T>::from(i == j ? beta : alpha);
+    for (Walk w(rows, cols); w.e < w.total; w.next()) {
+        if (lu == 1 && w.j < w.i) continue;
+        if (lu == 2 && w.j > w.i) continue;
+        C[w.i + (size_t)w.j * ldc] = Sc<T>::from(w.i == w.j ? beta : alpha);
     }
 }
 
@@ -106,18 +155,42 @@ __global__ void fill_lower_kernel(int n, T* C, int ldc) {
 }
 
 // W += x*(Wd^H + Wd) + x^2*Wdd  (omm.F90:499-501, :514-516, :168-170), applied as the
-// reference's three m_add calls in order.
+// reference's three m_add calls in order.  One 32 x 32 tile per block turn, Wd's mirror tile staged
+// through shared memory (read element by element it cost a 32-byte sector per element).
 template <typename T>
-__global__ void w_update_kernel(int n, T* W, int ldw, const T* Wd, int ldd, const T* Wdd, int lddd, double x) {
-    size_t total = (size_t)n * n;
+__global__ void w_update_kernel(int n, T* W, int ldw, const T* __restrict__ Wd, int ldd, const T* __restrict__ Wdd,
+                                int lddd, double x) {
+    __shared__ T tile[32][33];
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;  // 32 x 8
+    const int tiles = (n + 31) / 32;
     zdbl xz{x, 0.0}, x2{x * x, 0.0};
-    for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (size_t)gridDim.x * blockDim.x) {
-        int i = (int)(e % n), j = (int)(e / n);
-        T w = W[i + (size_t)j * ldw];
-        w = Sc<T>::add(w, Sc<T>::mul(xz, Sc<T>::conj(Wd[j + (size_t)i * ldd])));
-        w = Sc<T>::add(w, Sc<T>::mul(xz, Wd[i + (size_t)j * ldd]));
-        w = Sc<T>::add(w, Sc<T>::mul(x2, Wdd[i + (size_t)j * lddd]));
-        W[i + (size_t)j * ldw] = w;
+    for (long long t = blockIdx.x; t < (long long)tiles * tiles; t += gridDim.x) {
+        const int r0 = (int)(t % tiles) * 32, c0 = (int)(t / tiles) * 32;
+        T w[4], d[4], dd[4];
+        __syncthreads();
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int yy = ty + 8 * q;
+            if (c0 + tx < n && r0 + yy < n) tile[yy][tx] = Wd[c0 + tx + (size_t)(r0 + yy) * ldd];
+            const int i = r0 + tx, j = c0 + yy;
+            if (i < n && j < n) {
+                w[q] = W[i + (size_t)j * ldw];
+                d[q] = Wd[i + (size_t)j * ldd];
+                dd[q] = Wdd[i + (size_t)j * lddd];
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int yy = ty + 8 * q, i = r0 + tx, j = c0 + yy;
+            if (i < n && j < n) {
+                T v = w[q];
+                v = Sc<T>::add(v, Sc<T>::mul(xz, Sc<T>::conj(tile[tx][yy])));
+                v = Sc<T>::add(v, Sc<T>::mul(xz, d[q]));
+                v = Sc<T>::add(v, Sc<T>::mul(x2, dd[q]));
+                W[i + (size_t)j * ldw] = v;
+            }
+        }
     }
 }
 
@@ -143,28 +216,51 @@ __device__ inline void lcg_jump(unsigned long long t, unsigned long long& A, uns
 }
 template <typename T>
 __global__ void lcg_kernel(int n, int m, T* C, int ldc, double scale) {
-    size_t total = (size_t)n * m;
+    // a thread's elements are a fixed number of draws apart: the jump to its first one and the jump
+    // from one to the next are formed once each
+    Walk w(n, m);
+    if (w.e >= w.total) return;
     const unsigned long long M = (1ull << 31) - 1;
-    for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (size_t)gridDim.x * blockDim.x) {
-        unsigned long long A, Cc;
-        lcg_jump(2ull * e + 1ull, A, Cc);
-        unsigned long long x1 = (A * 123456ull + Cc) & M;
+    unsigned long long A, Cc, As, Cs;
+    lcg_jump(2ull * w.e + 1ull, A, Cc);
+    lcg_jump(2ull * w.step, As, Cs);
+    unsigned long long x1 = (A * 123456ull + Cc) & M;
+    for (; w.e < w.total; w.next()) {
         unsigned long long x2 = (1103515245ull * x1 + 12345ull) & M;
         double r1 = (double)x1 / 2147483648.0, r2 = (double)x2 / 2147483648.0;
         double h = 0.5 * r1;
         double el = (r2 - 0.5 >= 0.0) ? fabs(h) : -fabs(h);
         el = el * scale;
-        int j = (int)(e % n), i = (int)(e / n);
         zdbl v{el, 0.0};
-        C[j + (size_t)i * ldc] = Sc<T>::from(v);
+        C[w.i + (size_t)w.j * ldc] = Sc<T>::from(v);
+        x1 = (As * x1 + Cs) & M;
     }
 }
 
 // ---- reductions ------------------------------------------------------------------
+// (s, c) + (s2, c2) for compensated sums: s + s2 split exactly into t + e (Knuth's TwoSum),
+// the rounding errors carried in c
+__device__ inline void comp_add(double& s, double& c, double s2, double c2) {
+    const double t = s + s2, z = t - s;
+    const double e = (s - (t - z)) + (s2 - z);
+    s = t;
+    c += c2 + e;
+}
+
+// blocks of the running reduction that have stored their partial sums; the last one sets it back to
+// zero (reductions follow each other on the library's one stream)
+__device__ unsigned g_reduce_done;
+
+// Every block stores its K partial sums; the block that arrives last adds the nb records up with
+// compensation, in a fixed order (each thread a strided share, then a tree over the warp's lanes,
+// then the warps in turn), so the result does not depend on timing, and writes it to `out` in pinned
+// host memory.  (A second kernel for the sum and a copy of its result cost 4 + 3 us and their gaps
+// in each of a CG step's two reductions.)
 template <int K>
-__device__ inline void block_reduce_store(double (&v)[K], double* out) {
-    __shared__ double sm[K][kThreads / 32];
-    int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+__device__ inline void block_reduce_finish(double (&v)[K], double* part, double* out) {
+    __shared__ double sm[K][kThreads / 32], s_cmp[K][kThreads / 32];
+    __shared__ bool last;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nb = (int)gridDim.x;
 #pragma unroll
     for (int k = 0; k < K; ++k) {
         double a = v[k];
@@ -175,32 +271,20 @@ __device__ inline void block_reduce_store(double (&v)[K], double* out) {
     if (threadIdx.x < K) {
         double s = 0.0;
         for (int i = 0; i < (int)(blockDim.x / 32); ++i) s += sm[threadIdx.x][i];
-        out[(size_t)blockIdx.x * K + threadIdx.x] = s;
+        part[(size_t)blockIdx.x * K + threadIdx.x] = s;
+        __threadfence();
     }
-}
-
-// (s, c) + (s2, c2) for compensated sums: s + s2 split exactly into t + e (Knuth's TwoSum),
-// the rounding errors carried in c
-__device__ inline void comp_add(double& s, double& c, double s2, double c2) {
-    const double t = s + s2, z = t - s;
-    const double e = (s - (t - z)) + (s2 - z);
-    s = t;
-    c += c2 + e;
-}
-
-// Final pass: one block sums nb partial records of K values with compensation, in a fixed order
-// (each thread a strided share, then a tree over the warp's lanes, then the warps in turn), so
-// the result does not depend on timing.
-template <int K>
-__global__ void final_reduce_kernel(const double* part, int nb, double* out) {
-    __shared__ double s_sum[K][kThreads / 32], s_cmp[K][kThreads / 32];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicInc(&g_reduce_done, (unsigned)nb - 1u) == (unsigned)nb - 1u;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
     double s[K], c[K];
 #pragma unroll
     for (int k = 0; k < K; ++k) s[k] = c[k] = 0.0;
     for (int b = threadIdx.x; b < nb; b += blockDim.x)
 #pragma unroll
-        for (int k = 0; k < K; ++k) comp_add(s[k], c[k], part[(size_t)b * K + k], 0.0);
+        for (int k = 0; k < K; ++k) comp_add(s[k], c[k], __ldcg(part + (size_t)b * K + k), 0.0);
 #pragma unroll
     for (int k = 0; k < K; ++k) {
         for (int o = 16; o > 0; o >>= 1) {
@@ -208,7 +292,7 @@ __global__ void final_reduce_kernel(const double* part, int nb, double* out) {
             comp_add(s[k], c[k], s2, c2);
         }
         if (lane == 0) {
-            s_sum[k][w] = s[k];
+            sm[k][w] = s[k];
             s_cmp[k][w] = c[k];
         }
     }
@@ -216,7 +300,7 @@ __global__ void final_reduce_kernel(const double* part, int nb, double* out) {
     if (threadIdx.x < K) {
         const int k = threadIdx.x;
         double S = 0.0, C = 0.0;
-        for (int i = 0; i < (int)(blockDim.x / 32); ++i) comp_add(S, C, s_sum[k][i], s_cmp[k][i]);
+        for (int i = 0; i < (int)(blockDim.x / 32); ++i) comp_add(S, C, sm[k][i], s_cmp[k][i]);
         out[k] = S + C;
     }
 }
@@ -231,19 +315,32 @@ __device__ inline void dot_acc<zdbl>(zdbl a, zdbl b, double& re, double& im) {
     im += a.x * b.y - a.y * b.x;
 }
 
+// Bound by memory (two reads per element); kAhead pairs of loads in flight per thread.
 template <typename T>
-__global__ void dot_kernel(int rows, int cols, const T* A, int lda, const T* B, int ldb, double* part) {
+__global__ void dot_kernel(int rows, int cols, const T* __restrict__ A, int lda, const T* __restrict__ B, int ldb,
+                           double* part, double* out) {
     double v[2] = {0.0, 0.0};
-    size_t total = (size_t)rows * cols;
-    for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (size_t)gridDim.x * blockDim.x) {
-        int i = (int)(e % rows), j = (int)(e / rows);
-        dot_acc<T>(A[i + (size_t)j * lda], B[i + (size_t)j * ldb], v[0], v[1]);
+    Walk w(rows, cols);
+    while (w.e < w.total) {
+        T a[kAhead], b[kAhead];
+        int cnt = 0;
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u)
+            if (w.e < w.total) {
+                a[u] = A[w.i + (size_t)w.j * lda];
+                b[u] = B[w.i + (size_t)w.j * ldb];
+                ++cnt;
+                w.next();
+            }
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u)
+            if (u < cnt) dot_acc<T>(a[u], b[u], v[0], v[1]);
     }
-    block_reduce_store<2>(v, part);
+    block_reduce_finish<2>(v, part, out);
 }
 
 template <typename T>
-__global__ void trace_kernel(int n, const T* A, int lda, double* part) {
+__global__ void trace_kernel(int n, const T* A, int lda, double* part, double* out) {
     double v[2] = {0.0, 0.0};
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         T a = A[i + (size_t)i * lda];
@@ -253,7 +350,7 @@ __global__ void trace_kernel(int n, const T* A, int lda, double* part) {
         v[0] += z.x;
         v[1] += z.y;
     }
-    block_reduce_store<2>(v, part);
+    block_reduce_finish<2>(v, part, out);
 }
 
 // The 13 traces of calc_coeff (omm_ops.F90:194-211) in one pass over the six n x n
@@ -272,8 +369,10 @@ __device__ inline double re_of(T a) {
     else return ((const zdbl*)&a)->x;
 }
 template <typename T>
-__global__ void coeff_kernel(int n, const T* HW, int l0, const T* SW, int l1, const T* HWd, int l2, const T* SWd,
-                             int l3, const T* HWdd, int l4, const T* SWdd, int l5, double* part) {
+__global__ void coeff_kernel(int n, const T* __restrict__ HW, int l0, const T* __restrict__ SW, int l1,
+                             const T* __restrict__ HWd, int l2, const T* __restrict__ SWd, int l3,
+                             const T* __restrict__ HWdd, int l4, const T* __restrict__ SWdd, int l5, double* part,
+                             double* out) {
     __shared__ T tileT[32][33];
     double v[13];
 #pragma unroll
@@ -284,54 +383,94 @@ __global__ void coeff_kernel(int n, const T* HW, int l0, const T* SW, int l1, co
         int bi = t % tiles, bj = t / tiles;
         // load SWd tile (rows bj*32.., cols bi*32..) so that tileT[c][r] = SWd(bj*32+r, bi*32+c)
         __syncthreads();
-        for (int yy = ty; yy < 32; yy += 8) {
-            int r = bj * 32 + tx, c = bi * 32 + yy;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            int yy = ty + 8 * q, r = bj * 32 + tx, c = bi * 32 + yy;
             T val{};
             if (r < n && c < n) val = SWd[r + (size_t)c * l3];
             tileT[yy][tx] = val;
         }
-        __syncthreads();
-        for (int yy = ty; yy < 32; yy += 8) {
-            int i = bi * 32 + tx, j = bj * 32 + yy;
-            if (i >= n || j >= n) continue;
-            T hw = HW[i + (size_t)j * l0], sw = SW[i + (size_t)j * l1], hwd = HWd[i + (size_t)j * l2];
-            T swd = SWd[i + (size_t)j * l3], hwdd = HWdd[i + (size_t)j * l4], swdd = SWdd[i + (size_t)j * l5];
-            T swdT = tileT[tx][yy];  // SWd(j, i)
-            if (i == j) {
-                v[0] += re_of(hw);
-                v[2] += re_of(hwd);
-                v[5] += re_of(hwdd);
+        // two rounds of two elements each, the loads of a round (twelve) before its sums
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            T hw[2], sw[2], hwd[2], swd[2], hwdd[2], swdd[2];
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                const int i = bi * 32 + tx, j = bj * 32 + ty + 8 * (2 * h + q);
+                if (i < n && j < n) {
+                    hw[q] = HW[i + (size_t)j * l0];
+                    sw[q] = SW[i + (size_t)j * l1];
+                    hwd[q] = HWd[i + (size_t)j * l2];
+                    swd[q] = SWd[i + (size_t)j * l3];
+                    hwdd[q] = HWdd[i + (size_t)j * l4];
+                    swdd[q] = SWdd[i + (size_t)j * l5];
+                }
             }
-            v[1] += re_dot(hw, sw);
-            v[3] += re_dot(sw, hwd);
-            v[4] += re_dot(hw, swd);
-            v[6] += re_dot(hwdd, sw);
-            v[7] += re_dot(hw, swdd);
-            v[8] += re_dot(Sc<T>::conj(swdT), hwd);  // mm_trace(SWd^H, HWd): conj((SWd^H)_ij) = SWd_ji
-            v[9] += re_dot(swd, hwd);
-            v[10] += re_dot(hwdd, swd);
-            v[11] += re_dot(swdd, hwd);
-            v[12] += re_dot(hwdd, swdd);
+            if (h == 0) __syncthreads();  // tileT is complete
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                const int yy = ty + 8 * (2 * h + q), i = bi * 32 + tx, j = bj * 32 + yy;
+                if (i >= n || j >= n) continue;
+                T swdT = tileT[tx][yy];  // SWd(j, i)
+                if (i == j) {
+                    v[0] += re_of(hw[q]);
+                    v[2] += re_of(hwd[q]);
+                    v[5] += re_of(hwdd[q]);
+                }
+                v[1] += re_dot(hw[q], sw[q]);
+                v[3] += re_dot(sw[q], hwd[q]);
+                v[4] += re_dot(hw[q], swd[q]);
+                v[6] += re_dot(hwdd[q], sw[q]);
+                v[7] += re_dot(hw[q], swdd[q]);
+                v[8] += re_dot(Sc<T>::conj(swdT), hwd[q]);  // mm_trace(SWd^H, HWd): conj((SWd^H)_ij) = SWd_ji
+                v[9] += re_dot(swd[q], hwd[q]);
+                v[10] += re_dot(hwdd[q], swd[q]);
+                v[11] += re_dot(swdd[q], hwd[q]);
+                v[12] += re_dot(hwdd[q], swdd[q]);
+            }
         }
     }
-    block_reduce_store<13>(v, part);
+    block_reduce_finish<13>(v, part, out);
 }
 
-template <typename T>
-__global__ void lambda_kernel(int rows, int cols, const T* PG, int l0, const T* G, int l1, const T* Gp, int l2,
-                              const T* PGp, int l3, double* part) {
+// SAME: no preconditioner, PG is G and PG_p is G_p (two reads per element instead of four)
+template <typename T, bool SAME>
+__global__ void lambda_kernel(int rows, int cols, const T* __restrict__ PG, int l0, const T* __restrict__ G, int l1,
+                              const T* __restrict__ Gp, int l2, const T* __restrict__ PGp, int l3, double* part,
+                              double* out) {
     double v[2] = {0.0, 0.0};
-    size_t total = (size_t)rows * cols;
-    for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (size_t)gridDim.x * blockDim.x) {
-        int i = (int)(e % rows), j = (int)(e / rows);
-        T g = G[i + (size_t)j * l1], gp = Gp[i + (size_t)j * l2];
-        T w2;
-        if constexpr (sizeof(T) == 8) w2 = g - gp;
-        else w2 = zdbl{((zdbl*)&g)->x - ((zdbl*)&gp)->x, ((zdbl*)&g)->y - ((zdbl*)&gp)->y};
-        v[0] += re_dot(PG[i + (size_t)j * l0], w2);  // mm_trace(PG, work2), work2 = G - G_p
-        v[1] += re_dot(PGp[i + (size_t)j * l3], gp); // mm_trace(PG_p, G_p)
+    Walk w(rows, cols);
+    while (w.e < w.total) {
+        T g[kAhead], gp[kAhead], pg[SAME ? 1 : kAhead], pgp[SAME ? 1 : kAhead];
+        int cnt = 0;
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u)
+            if (w.e < w.total) {
+                g[u] = G[w.i + (size_t)w.j * l1];
+                gp[u] = Gp[w.i + (size_t)w.j * l2];
+                if constexpr (!SAME) {
+                    pg[u] = PG[w.i + (size_t)w.j * l0];
+                    pgp[u] = PGp[w.i + (size_t)w.j * l3];
+                }
+                ++cnt;
+                w.next();
+            }
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u)
+            if (u < cnt) {
+                T w2;
+                if constexpr (sizeof(T) == 8) w2 = g[u] - gp[u];
+                else w2 = zdbl{((zdbl*)&g[u])->x - ((zdbl*)&gp[u])->x, ((zdbl*)&g[u])->y - ((zdbl*)&gp[u])->y};
+                if constexpr (SAME) {
+                    v[0] += re_dot(g[u], w2);
+                    v[1] += re_dot(gp[u], gp[u]);
+                } else {
+                    v[0] += re_dot(pg[u], w2);    // mm_trace(PG, work2), work2 = G - G_p
+                    v[1] += re_dot(pgp[u], gp[u]);  // mm_trace(PG_p, G_p)
+                }
+            }
     }
-    block_reduce_store<2>(v, part);
+    block_reduce_finish<2>(v, part, out);
 }
 
 template <typename T>
@@ -366,14 +505,16 @@ double* scratch_partials(size_t nrec, int K) {
     return rt().scratch.as<double>();
 }
 
-template <int K>
-void finish_reduce(double* part, int nb, double* out) {
-    double* res = part + (size_t)nb * K;  // result slot right after the partials
-    final_reduce_kernel<K><<<1, kThreads, 0, rt().stream>>>(part, nb, res);
-    OMM_KCHECK();
-    OMM_CK(cudaMemcpyAsync(rt().host_pinned, res, K * sizeof(double), cudaMemcpyDeviceToHost, rt().stream));
+// the reduction's result, which its last block wrote to the pinned buffer
+void finish_reduce(int K, double* out) {
     sync();
     for (int k = 0; k < K; ++k) out[k] = rt().host_pinned[k];
+}
+
+// blocks of a kernel that takes 32 x 32 tiles in turn
+inline int tile_grid(int rows, int cols) {
+    const long long t = (long long)((rows + 31) / 32) * ((cols + 31) / 32);
+    return (int)std::max<long long>(1, std::min<long long>(t, 148 * 8));
 }
 
 }  // namespace
@@ -386,12 +527,22 @@ void k_axpby(const DView& A, char op, DView& C, const double alpha[2], const dou
     if (tot == 0) return;
     zdbl a{alpha[0], alpha[1]}, b{beta[0], beta[1]};
     int bz = 0;  // the reference multiplies C by beta even when beta == 0 (NaN propagates); keep that
-    if (C.is_real)
-        axpby_kernel<double><<<grid_for(tot), kThreads, 0, rt().stream>>>(C.rows, C.cols, A.as<double>(), A.ld, oc,
-                                                                            C.as<double>(), C.ld, a, b, bz);
-    else
-        axpby_kernel<zdbl><<<grid_for(tot), kThreads, 0, rt().stream>>>(C.rows, C.cols, A.as<zdbl>(), A.ld, oc,
-                                                                          C.as<zdbl>(), C.ld, a, b, bz);
+    if (oc == 0) {
+        if (C.is_real)
+            axpby_kernel<double><<<grid_for(tot), kThreads, 0, rt().stream>>>(C.rows, C.cols, A.as<double>(), A.ld,
+                                                                                C.as<double>(), C.ld, a, b, bz);
+        else
+            axpby_kernel<zdbl><<<grid_for(tot), kThreads, 0, rt().stream>>>(C.rows, C.cols, A.as<zdbl>(), A.ld,
+                                                                              C.as<zdbl>(), C.ld, a, b, bz);
+    } else {
+        const int grid = tile_grid(C.rows, C.cols);
+        if (C.is_real)
+            axpby_trans_kernel<double><<<grid, kThreads, 0, rt().stream>>>(C.rows, C.cols, A.as<double>(), A.ld, 0,
+                                                                             C.as<double>(), C.ld, a, b, bz);
+        else
+            axpby_trans_kernel<zdbl><<<grid, kThreads, 0, rt().stream>>>(C.rows, C.cols, A.as<zdbl>(), A.ld, oc == 2,
+                                                                           C.as<zdbl>(), C.ld, a, b, bz);
+    }
     OMM_KCHECK();
 }
 
@@ -432,13 +583,13 @@ void k_fill_lower_from_upper(DView& C) {
 }
 
 void k_w_update(DView& W, const DView& Wd, const DView& Wdd, double x) {
-    size_t tot = (size_t)W.rows * W.rows;
+    const int grid = tile_grid(W.rows, W.rows);
     if (W.is_real)
-        w_update_kernel<double><<<grid_for(tot), kThreads, 0, rt().stream>>>(W.rows, W.as<double>(), W.ld,
+        w_update_kernel<double><<<grid, kThreads, 0, rt().stream>>>(W.rows, W.as<double>(), W.ld,
                                                                                Wd.as<double>(), Wd.ld,
                                                                                Wdd.as<double>(), Wdd.ld, x);
     else
-        w_update_kernel<zdbl><<<grid_for(tot), kThreads, 0, rt().stream>>>(W.rows, W.as<zdbl>(), W.ld, Wd.as<zdbl>(),
+        w_update_kernel<zdbl><<<grid, kThreads, 0, rt().stream>>>(W.rows, W.as<zdbl>(), W.ld, Wd.as<zdbl>(),
                                                                              Wd.ld, Wdd.as<zdbl>(), Wdd.ld, x);
     OMM_KCHECK();
 }
@@ -454,10 +605,11 @@ void k_lcg_init(DView& C) {
 void r_trace(const DView& A, double out[2]) {
     int nb = 64;
     double* part = scratch_partials(nb + 1, 2);
-    if (A.is_real) trace_kernel<double><<<nb, kThreads, 0, rt().stream>>>(A.rows, A.as<double>(), A.ld, part);
-    else trace_kernel<zdbl><<<nb, kThreads, 0, rt().stream>>>(A.rows, A.as<zdbl>(), A.ld, part);
+    if (A.is_real) trace_kernel<double><<<nb, kThreads, 0, rt().stream>>>(A.rows, A.as<double>(), A.ld, part,
+                                                                          rt().host_pinned);
+    else trace_kernel<zdbl><<<nb, kThreads, 0, rt().stream>>>(A.rows, A.as<zdbl>(), A.ld, part, rt().host_pinned);
     OMM_KCHECK();
-    finish_reduce<2>(part, nb, out);
+    finish_reduce(2, out);
 }
 
 void r_dot(const DView& A, const DView& B, double out[2]) {
@@ -465,11 +617,13 @@ void r_dot(const DView& A, const DView& B, double out[2]) {
     int nb = grid_for(tot, 8);
     double* part = scratch_partials(nb + 1, 2);
     if (A.is_real)
-        dot_kernel<double><<<nb, kThreads, 0, rt().stream>>>(A.rows, A.cols, A.as<double>(), A.ld, B.as<double>(), B.ld, part);
+        dot_kernel<double><<<nb, kThreads, 0, rt().stream>>>(A.rows, A.cols, A.as<double>(), A.ld, B.as<double>(), B.ld, part,
+                                                            rt().host_pinned);
     else
-        dot_kernel<zdbl><<<nb, kThreads, 0, rt().stream>>>(A.rows, A.cols, A.as<zdbl>(), A.ld, B.as<zdbl>(), B.ld, part);
+        dot_kernel<zdbl><<<nb, kThreads, 0, rt().stream>>>(A.rows, A.cols, A.as<zdbl>(), A.ld, B.as<zdbl>(), B.ld, part,
+                                                          rt().host_pinned);
     OMM_KCHECK();
-    finish_reduce<2>(part, nb, out);
+    finish_reduce(2, out);
 }
 
 void r_coeff(const DView& HW, const DView& SW, const DView& HWd, const DView& SWd, const DView& HWdd, const DView& SWdd,
@@ -483,15 +637,15 @@ void r_coeff(const DView& HW, const DView& SW, const DView& HWd, const DView& SW
         coeff_kernel<double><<<nb, kThreads, 0, rt().stream>>>(n, HW.as<double>(), HW.ld, SW.as<double>(), SW.ld,
                                                                  HWd.as<double>(), HWd.ld, SWd.as<double>(), SWd.ld,
                                                                  HWdd.as<double>(), HWdd.ld, SWdd.as<double>(),
-                                                                 SWdd.ld, part);
+                                                                 SWdd.ld, part, rt().host_pinned);
     else
         coeff_kernel<zdbl><<<nb, kThreads, 0, rt().stream>>>(n, HW.as<zdbl>(), HW.ld, SW.as<zdbl>(), SW.ld,
                                                                HWd.as<zdbl>(), HWd.ld, SWd.as<zdbl>(), SWd.ld,
                                                                HWdd.as<zdbl>(), HWdd.ld, SWdd.as<zdbl>(), SWdd.ld,
-                                                               part);
+                                                               part, rt().host_pinned);
     OMM_KCHECK();
     double t[13];
-    finish_reduce<13>(part, nb, t);
+    finish_reduce(13, t);
     // omm_ops.F90:213-217
     coeff[0] = 2.0 * t[0] - t[1];
     coeff[1] = 2.0 * (2.0 * t[2] - t[3] - t[4]);
@@ -504,15 +658,16 @@ void r_lambda(const DView& PG, const DView& G, const DView& Gp, const DView& PGp
     size_t tot = (size_t)G.rows * G.cols;
     int nb = grid_for(tot, 8);
     double* part = scratch_partials(nb + 1, 2);
-    if (G.is_real)
-        lambda_kernel<double><<<nb, kThreads, 0, rt().stream>>>(G.rows, G.cols, PG.as<double>(), PG.ld, G.as<double>(),
-                                                                  G.ld, Gp.as<double>(), Gp.ld, PGp.as<double>(),
-                                                                  PGp.ld, part);
-    else
-        lambda_kernel<zdbl><<<nb, kThreads, 0, rt().stream>>>(G.rows, G.cols, PG.as<zdbl>(), PG.ld, G.as<zdbl>(), G.ld,
-                                                                Gp.as<zdbl>(), Gp.ld, PGp.as<zdbl>(), PGp.ld, part);
+    const bool same = PG.p == G.p && PG.ld == G.ld && PGp.p == Gp.p && PGp.ld == Gp.ld;
+    auto launch = [&](auto tag, auto kernel) {
+        using T = decltype(tag);
+        kernel<<<nb, kThreads, 0, rt().stream>>>(G.rows, G.cols, PG.as<T>(), PG.ld, G.as<T>(), G.ld, Gp.as<T>(), Gp.ld,
+                                                 PGp.as<T>(), PGp.ld, part, rt().host_pinned);
+    };
+    if (G.is_real) launch(double{}, same ? lambda_kernel<double, true> : lambda_kernel<double, false>);
+    else launch(zdbl{}, same ? lambda_kernel<zdbl, true> : lambda_kernel<zdbl, false>);
     OMM_KCHECK();
-    finish_reduce<2>(part, nb, out);
+    finish_reduce(2, out);
 }
 
 void gemm(char opA, char opB, int M, int N, int K, const double alpha[2], const DView& A, const DView& B,

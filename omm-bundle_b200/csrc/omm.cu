@@ -643,29 +643,26 @@ void eval_direction(OmmCall& c, const DView& Dir, double coeff[5]) {
             view(s.Wdd, n, n, 2 * n, c.real, n), coeff);
 }
 
-__global__ void calcG_left_real(int n, const double* SW, const double* HW, double* L) {
-    size_t tot = (size_t)n * 2 * n;
-    for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < tot; e += (size_t)gridDim.x * blockDim.x) {
-        int i = (int)(e % n), j = (int)(e / n);
+__global__ void calcG_left_real(int n, const double* __restrict__ SW, const double* __restrict__ HW,
+                                double* __restrict__ L) {
+    for (Walk w(n, 2 * n); w.e < w.total; w.next()) {
         double v;
-        if (j < n) v = (i == j ? 4.0 : 0.0) - 2.0 * SW[i + (size_t)j * n];
-        else v = -2.0 * HW[i + (size_t)(j - n) * n];
-        L[e] = v;
+        if (w.j < n) v = (w.i == w.j ? 4.0 : 0.0) - 2.0 * SW[w.e];
+        else v = -2.0 * HW[w.e - (size_t)n * n];
+        L[w.e] = v;
     }
 }
-__global__ void calcG_left_cplx(int n, const zdbl* SW, const zdbl* HW, zdbl* L) {
-    size_t tot = (size_t)n * 2 * n;
-    for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < tot; e += (size_t)gridDim.x * blockDim.x) {
-        int i = (int)(e % n), j = (int)(e / n);
+__global__ void calcG_left_cplx(int n, const zdbl* __restrict__ SW, const zdbl* __restrict__ HW, zdbl* __restrict__ L) {
+    for (Walk w(n, 2 * n); w.e < w.total; w.next()) {
         zdbl v;
-        if (j < n) {
-            zdbl s = SW[i + (size_t)j * n];
-            v = {(i == j ? 4.0 : 0.0) - 2.0 * s.x, -2.0 * s.y};
+        if (w.j < n) {
+            zdbl s = SW[w.e];
+            v = {(w.i == w.j ? 4.0 : 0.0) - 2.0 * s.x, -2.0 * s.y};
         } else {
-            zdbl h = HW[i + (size_t)(j - n) * n];
+            zdbl h = HW[w.e - (size_t)n * n];
             v = {-2.0 * h.x, -2.0 * h.y};
         }
-        L[e] = v;
+        L[w.e] = v;
     }
 }
 
