@@ -14,7 +14,9 @@
 #include <atomic>
 #include <chrono>
 #include <map>
+#include <functional>
 #include <mutex>
+#include <thread>
 
 namespace ommgpu {
 
@@ -259,6 +261,7 @@ static void invalidate_csc(msw_matrix* M) {
     M->d_rowind.release();
     M->d_val.release();
     M->plan.reset();
+    M->no_groups = -1;
     M->tc_plan.reset();
     M->tc2_plan.reset();
     M->tc2_plan_split.reset();
@@ -278,20 +281,43 @@ const msw_matrix* csc_transpose(const msw_matrix* A) {
     T->fmt = Fmt::CSC;
     T->loc = Loc::Device;
     T->nnz = A->nnz;
-    T->h_colptr.assign(T->dim2 + 1, 0);
-    for (int l = 0; l < A->nnz; ++l) T->h_colptr[A->h_rowind[l] + 1]++;
-    for (int j = 0; j < T->dim2; ++j) T->h_colptr[j + 1] += T->h_colptr[j];
-    std::vector<int> pos(T->h_colptr.begin(), T->h_colptr.end() - 1);
-    T->h_rowind.assign(A->nnz, 0);
-    int w = A->is_real ? 1 : 2;
-    T->h_val.assign((size_t)A->nnz * w, 0.0);
-    for (int c = 0; c < A->dim2; ++c)
-        for (int l = A->h_colptr[c]; l < A->h_colptr[c + 1]; ++l) {
-            int r = A->h_rowind[l];
-            int d = pos[r]++;
-            T->h_rowind[d] = c;
-            for (int q = 0; q < w; ++q) T->h_val[(size_t)d * w + q] = A->h_val[(size_t)l * w + q];
+    // counting sort by row on host threads: each takes a range of A's columns and counts its rows; the
+    // counts' prefix over (row, thread) gives every thread its places, so the entries of a row keep
+    // their column order whatever the number of threads
+    const int w = A->is_real ? 1 : 2, rows = T->dim2;
+    const int nt = A->nnz < (1 << 16) ? 1 : (int)std::min(8u, std::max(1u, std::thread::hardware_concurrency()));
+    T->h_colptr.assign(rows + 1, 0);
+    T->h_rowind.resize(A->nnz);
+    T->h_val.resize((size_t)A->nnz * w);
+    std::vector<std::vector<int>> pos(nt, std::vector<int>(rows, 0));
+    auto run = [&](const std::function<void(int, int, int)>& f) {  // f(thread, first column, last column)
+        std::vector<std::thread> th;
+        for (int t = 1; t < nt; ++t)
+            th.emplace_back(f, t, (int)((long long)A->dim2 * t / nt), (int)((long long)A->dim2 * (t + 1) / nt));
+        f(0, 0, A->dim2 / nt);
+        for (auto& t : th) t.join();
+    };
+    run([&](int t, int c0, int c1) {
+        for (int l = A->h_colptr[c0]; l < A->h_colptr[c1]; ++l) pos[t][A->h_rowind[l]]++;
+    });
+    int at = 0;
+    for (int r = 0; r < rows; ++r) {
+        T->h_colptr[r] = at;
+        for (int t = 0; t < nt; ++t) {
+            const int n = pos[t][r];
+            pos[t][r] = at;
+            at += n;
         }
+    }
+    T->h_colptr[rows] = at;
+    run([&](int t, int c0, int c1) {
+        for (int c = c0; c < c1; ++c)
+            for (int l = A->h_colptr[c]; l < A->h_colptr[c + 1]; ++l) {
+                const int d = pos[t][A->h_rowind[l]]++;
+                T->h_rowind[d] = c;
+                for (int q = 0; q < w; ++q) T->h_val[(size_t)d * w + q] = A->h_val[(size_t)l * w + q];
+            }
+    });
     M->transposed = T;
     return T.get();
 }

@@ -203,6 +203,7 @@ struct msw_matrix {
     ommgpu::DevBuf d_colptr, d_rowind, d_val;
     unsigned long long pattern_id = ommgpu::next_pattern_id();
     std::shared_ptr<ommgpu::SpmmPlan> plan;       // lazily built
+    int no_groups = -1;  // 1: the pattern has no column groups, 0: a plan decides, -1: not looked at (spmm.cu)
     std::shared_ptr<ommgpu::SpmmTcPlan> tc_plan;  // lazily built (empty plan = not eligible)
     std::shared_ptr<ommgpu::SpmmTc2Plan> tc2_plan, tc2_plan_split;  // group-block forms (bf16, split)
     std::shared_ptr<ommgpu::OzSpmmPlan> oz_plan;  // int8 form (with the S of the same pattern), lazily built

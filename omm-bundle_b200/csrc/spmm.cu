@@ -7,7 +7,7 @@
 //
 // Two kernels:
 //  * gather  : one CTA per (row chunk, output column); generic CSC.
-//  * cgu     : "column-group union".  Output columns are cut into groups of G
+//  * cgu     : "column-group union", on the FP64 tensor cores (complex ones as two value sets).  Output columns are cut into groups of G
 //              consecutive columns; a group's nonzeros live in the union U_g
 //              of their row indices, and the group is the dense product
 //              A(:, U_g) * B_g with B_g the |U_g| x G block of B (zero filled).
@@ -68,13 +68,16 @@ template <> struct Ar<zdbl> {
     __device__ static zdbl zero() { return {0.0, 0.0}; }
 };
 
-// C(r, j) = beta*C(r,j) + alpha*sum_l val_l*A(r, row_l); blockIdx.y = column j.
+// C(r, j) = beta*C(r,j) + alpha*sum_l val_l*A(r, row_l); blockIdx.y = column j.  With only_if, nothing
+// unless that flag is set.
 template <typename T>
 __global__ void __launch_bounds__(kGatherThreads) gather_kernel(int n, const T* __restrict__ A, int lda,
                                                                   const int* __restrict__ colptr,
                                                                   const int* __restrict__ rowind,
                                                                   const T* __restrict__ val, T* __restrict__ C,
-                                                                  int ldc, zdbl alpha, zdbl beta, int beta_zero) {
+                                                                  int ldc, zdbl alpha, zdbl beta, int beta_zero,
+                                                                  const int* __restrict__ only_if) {
+    if (only_if && *only_if == 0) return;
     constexpr int R = 4;  // rows per thread
     int j = blockIdx.y;
     int r0 = blockIdx.x * (kGatherThreads * R) + threadIdx.x;
@@ -114,293 +117,291 @@ __global__ void __launch_bounds__(kGatherThreads) gather_kernel(int n, const T* 
     }
 }
 
-// Column-group union kernel.  CTA = (row tile of BM = 16*TM rows, group g).
-// 64 threads: tm in [0,16) covers rows tm + 16*i (i < TM), tn in [0,4) covers
-// group columns tn*TN + q (q < TN).  NM = 1 or 2 value sets (fused H and S).
-// The next K-chunk (BK union rows) is fetched into registers while the current
-// one is multiplied out of shared memory.
-template <typename T, int TM, int TN, int NM>
-__global__ void __launch_bounds__(64) cgu_kernel(int n, int N, const T* __restrict__ A, int lda,
-                                                 const int* __restrict__ gptr, const int* __restrict__ urows,
-                                                 const T* __restrict__ B0, const T* __restrict__ B1,
-                                                 T* __restrict__ C0, int ldc0, T* __restrict__ C1, int ldc1,
-                                                 zdbl alpha, zdbl beta, int beta_zero) {
-    constexpr int BM = 16 * TM;
-    constexpr int G = 4 * TN;
-    constexpr int BK = 8;
-    constexpr int A_PER = BK * BM / 64;          // A elements per thread per chunk
-    constexpr int B_PER = (BK * G + 63) / 64;    // B elements per thread per chunk and value set
-    __shared__ T As[BK][BM];
-    __shared__ T Bs[NM][BK][G];
-    const int g = blockIdx.y;
-    const int r0 = blockIdx.x * BM;
-    const int tid = threadIdx.x;
-    const int tm = tid & 15, tn = tid >> 4;
-    const int k_begin = gptr[g], K = gptr[g + 1] - k_begin;
-    const T* Bg[2] = {B0 + (size_t)k_begin * G, (NM == 2) ? B1 + (size_t)k_begin * G : nullptr};
-
-    T acc[NM][TM][TN];
-#pragma unroll
-    for (int s = 0; s < NM; ++s)
-#pragma unroll
-        for (int i = 0; i < TM; ++i)
-#pragma unroll
-            for (int q = 0; q < TN; ++q) acc[s][i][q] = Ar<T>::zero();
-
-    T ra[A_PER];
-    T rb[NM][B_PER];
-    auto fetch = [&](int k0) {
-#pragma unroll
-        for (int u = 0; u < A_PER; ++u) {
-            int e = tid + 64 * u;
-            int kk = e / BM, mm = e % BM;
-            int r = r0 + mm;
-            ra[u] = Ar<T>::zero();
-            if (k0 + kk < K && r < n) ra[u] = A[(size_t)__ldg(urows + k_begin + k0 + kk) * lda + r];
-        }
-#pragma unroll
-        for (int s = 0; s < NM; ++s)
-#pragma unroll
-            for (int u = 0; u < B_PER; ++u) {
-                int e = tid + 64 * u;
-                int kk = e / G;
-                rb[s][u] = Ar<T>::zero();
-                if (e < BK * G && k0 + kk < K) rb[s][u] = Bg[s][(size_t)k0 * G + e];
-            }
-    };
-    auto stash = [&]() {
-#pragma unroll
-        for (int u = 0; u < A_PER; ++u) {
-            int e = tid + 64 * u;
-            As[e / BM][e % BM] = ra[u];
-        }
-#pragma unroll
-        for (int s = 0; s < NM; ++s)
-#pragma unroll
-            for (int u = 0; u < B_PER; ++u) {
-                int e = tid + 64 * u;
-                if (e < BK * G) Bs[s][e / G][e % G] = rb[s][u];
-            }
-    };
-
-    const int nk = (K + BK - 1) / BK;
-    if (nk > 0) {
-        fetch(0);
-        stash();
-        __syncthreads();
-    }
-    for (int t = 0; t < nk; ++t) {
-        if (t + 1 < nk) fetch((t + 1) * BK);
-#pragma unroll
-        for (int kk = 0; kk < BK; ++kk) {
-            T a[TM];
-#pragma unroll
-            for (int i = 0; i < TM; ++i) a[i] = As[kk][tm + 16 * i];
-#pragma unroll
-            for (int s = 0; s < NM; ++s) {
-                T b[TN];
-#pragma unroll
-                for (int q = 0; q < TN; ++q) b[q] = Bs[s][kk][tn * TN + q];
-#pragma unroll
-                for (int i = 0; i < TM; ++i)
-#pragma unroll
-                    for (int q = 0; q < TN; ++q) acc[s][i][q] = Ar<T>::fmaa(a[i], b[q], acc[s][i][q]);
-            }
-        }
-        __syncthreads();
-        if (t + 1 < nk) {
-            stash();
-            __syncthreads();
-        }
-    }
-#pragma unroll
-    for (int s = 0; s < NM; ++s) {
-        T* Cs = (s == 0) ? C0 : C1;
-        int ldc = (s == 0) ? ldc0 : ldc1;
-#pragma unroll
-        for (int q = 0; q < TN; ++q) {
-            int col = g * G + tn * TN + q;
-            if (col >= N) continue;
-#pragma unroll
-            for (int i = 0; i < TM; ++i) {
-                int r = r0 + tm + 16 * i;
-                if (r >= n) continue;
-                T* c = Cs + r + (size_t)col * ldc;
-                T out = Ar<T>::mulz(alpha, acc[s][i][q]);
-                if (!beta_zero) out = Ar<T>::add(Ar<T>::mulz(beta, *c), out);
-                *c = out;
-            }
-        }
-    }
-}
-
 // ---- FP64 column-group kernel on the FP64 tensor cores (mma.sync m8n8k4 f64; tcgen05 has no
-// FP64 kind).  Per CTA 128 rows of A (4 warps x 32) x one column group (G = 8..32 columns, NM
-// value sets).  K (the group's union rows) runs in 16-row chunks, double buffered with cp.async
-// gathers of the union rows' column segments of A.  Per 4-k step a warp issues
-// 4 (row tiles) x G/8 (column tiles) x NM DMMAs; the A fragments serve both value sets.
+// FP64 kind).  Per CTA 32 MT rows of A (4 warps x 8 MT) x one column group (G = 8..32 columns, NM
+// value sets).  K (the group's union rows) runs in 8-row chunks through a ring of four stages: the
+// chunk's column segments of A and rows of B come by cp.async (16 bytes where the source allows),
+// three chunks ahead of the one being multiplied, one barrier per chunk.  Per 4-k step a warp issues
+// MT (row tiles) x G/8 (column tiles) x NM DMMAs; the A fragments serve both value sets.
 // Fragment layouts (m8n8k4, f64): A(r, k) at lane 4r + k, B(k, c) at lane 4c + k,
 // D(r, 2q + i) at lane 4r + q, element i.
-__device__ __forceinline__ void cp_async8(double* dst, const double* src) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
+// The rows of both shared tiles are padded to 4 (mod 16) doubles -- or 12, its mirror -- so that the
+// 16 lanes of a half-warp's fragment load (4 rows x 4 k) fall in 32 distinct banks.  With the padding
+// of 8 doubles used before, every fragment load took two passes and the L1 path (85 % busy)
+// held the DMMA pipe at 64 %.
+// lattice_8x8x8 (n = 1,536): H alone 1.30 -> 1.10 ms (27 TFLOP/s; the gathers then move about
+// 5.5 TB/s from L2), H and S fused 2.21 -> 1.89 ms (31.7 TFLOP/s, near cuBLAS DGEMM's 36).  Within 3 %:
+// three or five stages, 16-row chunks in two stages, 64-row tiles; 16-row chunks in four stages
+// (two CTAs per SM) 17 % slower.
+//
+// Complex matrices (CPLX) take the same kernel: A, interleaved, is a real matrix of 2n rows; B_re
+// and B_im are the two value sets; and with P = A [B_re | B_im], Re C(r, c) = P(2r, c) - P(2r+1, G+c),
+// Im C(r, c) = P(2r, G+c) + P(2r+1, c): one lane exchange in the epilogue.
+__device__ __forceinline__ void cp_async8(double* dst, const double* src, int bytes) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)),
+                 "l"(src), "r"(bytes)
+                 : "memory");
+}
+__device__ __forceinline__ void cp_async16(double* dst, const double* src, int bytes) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)),
+                 "l"(src), "r"(bytes)
                  : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait1() { asm volatile("cp.async.wait_group 1;" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait0() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() {
+    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
 __device__ __forceinline__ void dmma(double (&d)[2], double a, double b) {
     asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
                  : "+d"(d[0]), "+d"(d[1])
                  : "d"(a), "d"(b));
 }
 
-constexpr int kDmmaBM = 128, kDmmaBK = 16, kDmmaAS = kDmmaBM + 8;  // A rows padded: fragment loads in 2 wavefronts
-template <int G>
-constexpr int dmma_gs() {
-    return (G % 16 == 8) ? G : G + 8;  // B row stride with 2 * stride = 16 (mod 32) banks
-}
-template <int G, int NM>
-constexpr int dmma_smem() {
-    return 2 * (kDmmaBK * kDmmaAS + NM * kDmmaBK * dmma_gs<G>()) * (int)sizeof(double);
+constexpr int kDmmaBK = 8, kDmmaStages = 4;
+template <int G, int NM, int MT>
+constexpr int dmma_stage() {  // doubles of one stage
+    return kDmmaBK * ((32 * MT + 4) + NM * (G + 4));
 }
 
-// stage_k: the group's union rows are staged in shared memory (after the operand buffers) once,
-// so the gathers of every chunk index shared memory instead of waiting on global loads.
-template <int G, int NM>
-__global__ void __launch_bounds__(128) cgu_dmma_kernel(int n, int N, const double* __restrict__ A, int lda,
-                                                       const int* __restrict__ gptr, const int* __restrict__ urows,
-                                                       const double* __restrict__ B0, const double* __restrict__ B1,
-                                                       double* __restrict__ C0, int ldc0, double* __restrict__ C1,
-                                                       int ldc1, double alpha, double beta, int beta_zero,
-                                                       int stage_k) {
-    constexpr int BM = kDmmaBM, BK = kDmmaBK, AS = kDmmaAS, GS = dmma_gs<G>(), NT = G / 8;
-    extern __shared__ double dsm[];
-    double* As = dsm;                       // [2][BK][AS]
-    double* Bs = dsm + 2 * BK * AS;         // [2][NM][BK][GS]
-    int* s_ur = (int*)(dsm + dmma_smem<G, NM>() / (int)sizeof(double));  // [K] when stage_k
+struct DmmaArgs {
+    int n, N;  // rows of A and C in doubles (2 x the matrix rows for complex matrices), columns
+    const double* A;
+    long long lda;  // doubles between A's columns
+    const int *gptr, *urows;
+    const double *B0, *B1;  // value sets (B1 unused for complex ones: B0 holds re, im pairs)
+    double *C0, *C1;
+    long long rs, cs, cs1;  // strides of C in doubles: row (of the complex matrix), column of C0 and of C1
+    double alpha, alpha_im, beta, beta_im;
+    int beta_zero;
+    int stage_k;  // the group's union rows are staged in shared memory once (else read from global)
+    int vec;      // A's column segments are 16-byte aligned
+};
+
+template <int G, int NM, int MT, bool CPLX>
+__global__ void __launch_bounds__(128) cgu_dmma_kernel(const __grid_constant__ DmmaArgs p) {
+    constexpr int BM = 32 * MT, BK = kDmmaBK, AS = BM + 4, GS = G + 4, NT = G / 8, ST = kDmmaStages;
+    constexpr int STAGE = dmma_stage<G, NM, MT>();
+    extern __shared__ __align__(16) double dsm[];  // [ST] stages: A [BK][AS], B [NM][BK][GS]
+    int* s_ur = (int*)(dsm + ST * STAGE);          // [K] when stage_k
     const int g = blockIdx.y, r0 = blockIdx.x * BM;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int kb = gptr[g], K = gptr[g + 1] - kb;
-    if (stage_k) {
-        for (int i = threadIdx.x; i < K; i += blockDim.x) s_ur[i] = urows[kb + i];
+    const int kb = p.gptr[g], K = p.gptr[g + 1] - kb;
+    if (p.stage_k) {
+        for (int i = threadIdx.x; i < K; i += 128) s_ur[i] = p.urows[kb + i];
         __syncthreads();
     }
-    const int* ur = stage_k ? s_ur : urows + kb;
-    const double* Bg[2] = {B0 + (size_t)kb * G, NM == 2 ? B1 + (size_t)kb * G : nullptr};
+    const int* ur = p.stage_k ? s_ur : p.urows + kb;
 
-    double acc[NM][4][NT][2];
+    double acc[NM][MT][NT][2];
 #pragma unroll
     for (int s = 0; s < NM; ++s)
 #pragma unroll
-        for (int mt = 0; mt < 4; ++mt)
+        for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
             for (int nt = 0; nt < NT; ++nt) acc[s][mt][nt][0] = acc[s][mt][nt][1] = 0.0;
 
-    auto load = [&](int stage, int k0) {
-        double* as = As + stage * BK * AS;
+    auto load = [&](int t) {
+        double* as = dsm + (t % ST) * STAGE;
+        const int k0 = t * BK;
+        if (p.vec) {
+            constexpr int VR = BM / 2;  // 16-byte vectors of a row of the tile
 #pragma unroll
-        for (int u = 0; u < BK * BM / 128; ++u) {  // 16 column-segment elements per thread
-            const int e = threadIdx.x + 128 * u;
-            const int kk = e / BM, mm = e % BM;
-            const int k = k0 + kk, r = r0 + mm;
-            double* dst = as + kk * AS + mm;
-            if (k < K && r < n) cp_async8(dst, A + (size_t)ur[k] * lda + r);
-            else *dst = 0.0;
-        }
-        double* bs = Bs + stage * NM * BK * GS;
-#pragma unroll
-        for (int s = 0; s < NM; ++s)
-            for (int e = threadIdx.x; e < BK * G; e += 128) {
-                const int kk = e / G, c = e % G;
-                double* dst = bs + (s * BK + kk) * GS + c;
-                if (k0 + kk < K) cp_async8(dst, Bg[s] + (size_t)(k0 + kk) * G + c);
-                else *dst = 0.0;
+            for (int u = 0; u < BK * VR / 128; ++u) {
+                const int e = threadIdx.x + 128 * u;
+                const int kk = e / VR, mm = 2 * (e % VR), k = k0 + kk, r = r0 + mm;
+                const int bytes = k < K ? 8 * max(0, min(2, p.n - r)) : 0;
+                cp_async16(as + kk * AS + mm, bytes ? p.A + (size_t)ur[k] * p.lda + r : p.A, bytes);
             }
+        } else {
+#pragma unroll
+            for (int u = 0; u < BK * BM / 128; ++u) {
+                const int e = threadIdx.x + 128 * u;
+                const int kk = e / BM, mm = e % BM, k = k0 + kk, r = r0 + mm;
+                const int bytes = k < K && r < p.n ? 8 : 0;
+                cp_async8(as + kk * AS + mm, bytes ? p.A + (size_t)ur[k] * p.lda + r : p.A, bytes);
+            }
+        }
+        double* bs = as + BK * AS;
+        if constexpr (CPLX) {
+            const double* B = p.B0 + (size_t)(kb + k0) * G * 2;
+            for (int e = threadIdx.x; e < 2 * BK * G; e += 128) {
+                const int kk = e / (2 * G), c = (e % (2 * G)) / 2, s = e & 1;
+                const int bytes = k0 + kk < K ? 8 : 0;
+                cp_async8(bs + (s * BK + kk) * GS + c, bytes ? B + e : p.B0, bytes);
+            }
+        } else {
+#pragma unroll
+            for (int s = 0; s < NM; ++s) {
+                const double* Bp = s == 0 ? p.B0 : p.B1;
+                const double* B = Bp + (size_t)(kb + k0) * G;
+                for (int e = threadIdx.x; e < BK * G / 2; e += 128) {
+                    const int kk = e / (G / 2), c = 2 * (e % (G / 2));
+                    const int bytes = k0 + kk < K ? 16 : 0;
+                    cp_async16(bs + (s * BK + kk) * GS + c, bytes ? B + 2 * e : Bp, bytes);
+                }
+            }
+        }
     };
 
     const int nk = (K + BK - 1) / BK;
-    if (nk > 0) load(0, 0);
-    cp_async_commit();
-    for (int t = 0; t < nk; ++t) {
-        if (t + 1 < nk) load((t + 1) & 1, (t + 1) * BK);
+#pragma unroll
+    for (int t = 0; t < ST - 1; ++t) {
+        if (t < nk) load(t);
         cp_async_commit();
-        cp_async_wait1();  // chunk t has landed
-        __syncthreads();
-        const double* as = As + (t & 1) * BK * AS;
-        const double* bs = Bs + (t & 1) * NM * BK * GS;
+    }
+    for (int t = 0; t < nk; ++t) {
+        cp_async_wait<ST - 2>();  // chunk t has landed (this thread's part)
+        __syncthreads();          // everyone's part, and the slot of chunk t - 1 is free
+        if (t + ST - 1 < nk) load(t + ST - 1);
+        cp_async_commit();
+        const double* as = dsm + (t % ST) * STAGE;
+        const double* bs = as + BK * AS;
 #pragma unroll
         for (int k4 = 0; k4 < BK; k4 += 4) {
             const int ka = k4 + (lane & 3);
-            double af[4];
+            double af[MT];
 #pragma unroll
-            for (int mt = 0; mt < 4; ++mt) af[mt] = as[ka * AS + warp * 32 + mt * 8 + (lane >> 2)];
+            for (int mt = 0; mt < MT; ++mt) af[mt] = as[ka * AS + warp * 8 * MT + mt * 8 + (lane >> 2)];
 #pragma unroll
             for (int s = 0; s < NM; ++s)
 #pragma unroll
                 for (int nt = 0; nt < NT; ++nt) {
                     const double bf = bs[(s * BK + ka) * GS + nt * 8 + (lane >> 2)];
 #pragma unroll
-                    for (int mt = 0; mt < 4; ++mt) dmma(acc[s][mt][nt], af[mt], bf);
+                    for (int mt = 0; mt < MT; ++mt) dmma(acc[s][mt][nt], af[mt], bf);
                 }
         }
-        __syncthreads();  // the buffer is refilled by the next iteration's load
     }
-    cp_async_wait0();
+    cp_async_wait<0>();
 #pragma unroll
-    for (int s = 0; s < NM; ++s) {
-        double* Cs = s == 0 ? C0 : C1;
-        const int ldc = s == 0 ? ldc0 : ldc1;
-#pragma unroll
-        for (int mt = 0; mt < 4; ++mt) {
-            const int r = r0 + warp * 32 + mt * 8 + (lane >> 2);
-            if (r >= n) continue;
+    for (int mt = 0; mt < MT; ++mt) {
+        const int r = r0 + warp * 8 * MT + mt * 8 + (lane >> 2);
+        if constexpr (CPLX) {
 #pragma unroll
             for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
                 for (int i = 0; i < 2; ++i) {
+                    // lane's row 2r' (+1) holds A_re (A_im) times B_re in set 0 and B_im in set 1; the
+                    // row of the other parity is four lanes away
+                    const double re = acc[0][mt][nt][i], im = acc[1][mt][nt][i];
+                    const double ore = __shfl_xor_sync(0xffffffffu, re, 4), oim = __shfl_xor_sync(0xffffffffu, im, 4);
+                    const bool odd = (lane >> 2) & 1;
+                    const double zr = odd ? ore - im : re - oim;  // Re C = P(2r', c) - P(2r'+1, G+c)
+                    const double zi = odd ? oim + re : im + ore;  // Im C = P(2r', G+c) + P(2r'+1, c)
                     const int col = g * G + nt * 8 + (lane & 3) * 2 + i;
-                    if (col >= N) continue;
-                    double* c = Cs + r + (size_t)col * ldc;
-                    double out = alpha * acc[s][mt][nt][i];
-                    if (!beta_zero) out += beta * *c;
-                    *c = out;
+                    const bool in = r < p.n && col < p.N;  // the same for both lanes of a row (n is even)
+                    // the even lane writes the real part, the odd one the imaginary part
+                    double out = odd ? p.alpha * zi + p.alpha_im * zr : p.alpha * zr - p.alpha_im * zi;
+                    double* c = p.C0 + (size_t)(r >> 1) * p.rs + (size_t)col * p.cs;
+                    if (in && !p.beta_zero) {
+                        const double cr = c[0], ci = c[1];
+                        out += odd ? p.beta * ci + p.beta_im * cr : p.beta * cr - p.beta_im * ci;
+                    }
+                    __syncwarp();  // both parts are read before either is written
+                    if (in) c[odd ? 1 : 0] = out;
                 }
+        } else {
+            if (r >= p.n) continue;
+#pragma unroll
+            for (int s = 0; s < NM; ++s)
+#pragma unroll
+                for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+                    for (int i = 0; i < 2; ++i) {
+                        const int col = g * G + nt * 8 + (lane & 3) * 2 + i;
+                        if (col >= p.N) continue;
+                        double* c = (s == 0 ? p.C0 : p.C1) + (size_t)r * p.rs + (size_t)col * (s == 0 ? p.cs : p.cs1);
+                        double out = p.alpha * acc[s][mt][nt][i];
+                        if (!p.beta_zero) out += p.beta * *c;
+                        *c = out;
+                    }
         }
     }
 }
 
+template <int G, int NM, int MT, bool CPLX>
+void launch_cgu_dmma_t(const DmmaArgs& a, int ngroups, int extra) {
+    const int SM = kDmmaStages * dmma_stage<G, NM, MT>() * (int)sizeof(double) + extra;
+    static int attr = 0;
+    if (SM > attr) {
+        OMM_CK(cudaFuncSetAttribute(cgu_dmma_kernel<G, NM, MT, CPLX>, cudaFuncAttributeMaxDynamicSharedMemorySize, SM));
+        attr = SM;
+    }
+    dim3 grid((a.n + 32 * MT - 1) / (32 * MT), ngroups);
+    cgu_dmma_kernel<G, NM, MT, CPLX><<<grid, 128, SM, rt().stream>>>(a);
+}
+template <int G, int NM, bool CPLX>
+void launch_cgu_dmma_m(const DmmaArgs& a, int ngroups, int extra, int mt) {
+    if (mt == 4) launch_cgu_dmma_t<G, NM, 4, CPLX>(a, ngroups, extra);
+    else if (mt == 2) launch_cgu_dmma_t<G, NM, 2, CPLX>(a, ngroups, extra);
+    else launch_cgu_dmma_t<G, NM, 1, CPLX>(a, ngroups, extra);
+}
 template <int G>
-void launch_cgu_dmma(const DView& A, const SpmmPlan& P, const SpmmPlan* P2, DView& C, DView* C2, double al,
-                     double be, int bz, int N) {
-    dim3 grid((A.rows + kDmmaBM - 1) / kDmmaBM, P.ngroups);
-    const int stage_k = (P.maxK > 0 && P.maxK <= 4096) ? 1 : 0;  // at most 16 KB of indices beside the buffers
+void launch_cgu_dmma_g(const DmmaArgs& a, int ngroups, int extra, int mt, bool two, bool cplx) {
+    if (cplx) launch_cgu_dmma_m<G, 2, true>(a, ngroups, extra, mt);
+    else if (two) launch_cgu_dmma_m<G, 2, false>(a, ngroups, extra, mt);
+    else launch_cgu_dmma_m<G, 1, false>(a, ngroups, extra, mt);
+}
+
+// Rows of A per CTA: 128 (MT = 4) read each B row once per 128 rows and have the most DMMAs per
+// fragment load; 64 and 32 pay where they leave less of the last row block empty, or where the
+// grid of 128-row blocks would not give every SM its CTAs (all at the same k order, so the
+// results are the same bits).
+int dmma_row_tiles(int n, int ngroups) {
+    int best = 4;
+    double cost = 0.0;
+    for (int mt : {4, 2, 1}) {
+        const long long blocks = (long long)((n + 32 * mt - 1) / (32 * mt)) * ngroups;
+        const double waves = std::max(1.0, std::ceil((double)blocks / 148.0) / 1.0);
+        const double c = waves * mt * (mt == 4 ? 1.0 : mt == 2 ? 1.1 : 1.35);
+        if (mt == 4 || c < 0.95 * cost) {
+            best = mt;
+            cost = c;
+        }
+    }
+    return best;
+}
+
+// C (+ C2 for the second value set) = alpha A B + beta C; with trans, C is the transpose of the
+// product's layout: element (r, j) at C[j + r ldc]
+void launch_cgu_dmma(const DView& A, const SpmmPlan& P, const SpmmPlan* P2, DView& C, DView* C2, const double al[2],
+                     const double be[2], int bz, int N, bool trans) {
+    const bool cplx = !A.is_real;
+    const int w = cplx ? 2 : 1;
+    DmmaArgs a{};
+    a.n = A.rows * w;
+    a.N = N;
+    a.A = A.as<double>();
+    a.lda = (long long)A.ld * w;
+    a.gptr = P.gptr.as<int>();
+    a.urows = P.urows.as<int>();
+    a.B0 = P.bvals.as<double>();
+    a.B1 = P2 ? P2->bvals.as<double>() : nullptr;
+    a.C0 = C.as<double>();
+    a.C1 = P2 ? C2->as<double>() : nullptr;
+    a.rs = trans ? (long long)C.ld * w : w;
+    a.cs = trans ? w : (long long)C.ld * w;
+    a.cs1 = P2 ? (trans ? w : (long long)C2->ld * w) : 0;
+    a.alpha = al[0];
+    a.alpha_im = cplx ? al[1] : 0.0;
+    a.beta = be[0];
+    a.beta_im = cplx ? be[1] : 0.0;
+    a.beta_zero = bz;
+    a.stage_k = (P.maxK > 0 && P.maxK <= 4096) ? 1 : 0;  // at most 16 KB of indices beside the ring
+    a.vec = (a.lda % 2 == 0 && (reinterpret_cast<uintptr_t>(a.A) & 15) == 0) ? 1 : 0;
+    const int extra = a.stage_k ? (P.maxK * (int)sizeof(int) + 15) / 16 * 16 : 0;
+    const int mt = dmma_row_tiles(a.n, P.ngroups);
     ktime_begin();
-    const int extra = stage_k ? (P.maxK * (int)sizeof(int) + 15) / 16 * 16 : 0;
-    if (P2) {
-        const int SM = dmma_smem<G, 2>() + extra;
-        static int attr = 0;
-        if (SM > attr) {
-            OMM_CK(cudaFuncSetAttribute(cgu_dmma_kernel<G, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, SM));
-            attr = SM;
-        }
-        cgu_dmma_kernel<G, 2><<<grid, 128, SM, rt().stream>>>(A.rows, N, A.as<double>(), A.ld, P.gptr.as<int>(),
-                                                                P.urows.as<int>(), P.bvals.as<double>(),
-                                                                P2->bvals.as<double>(), C.as<double>(), C.ld,
-                                                                C2->as<double>(), C2->ld, al, be, bz, stage_k);
-    } else {
-        const int SM = dmma_smem<G, 1>() + extra;
-        static int attr = 0;
-        if (SM > attr) {
-            OMM_CK(cudaFuncSetAttribute(cgu_dmma_kernel<G, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, SM));
-            attr = SM;
-        }
-        cgu_dmma_kernel<G, 1><<<grid, 128, SM, rt().stream>>>(A.rows, N, A.as<double>(), A.ld, P.gptr.as<int>(),
-                                                                P.urows.as<int>(), P.bvals.as<double>(), nullptr,
-                                                                C.as<double>(), C.ld, nullptr, 0, al, be, bz, stage_k);
+    switch (P.G) {
+        case 8: launch_cgu_dmma_g<8>(a, P.ngroups, extra, mt, P2 != nullptr, cplx); break;
+        case 16: launch_cgu_dmma_g<16>(a, P.ngroups, extra, mt, P2 != nullptr, cplx); break;
+        case 24: launch_cgu_dmma_g<24>(a, P.ngroups, extra, mt, P2 != nullptr, cplx); break;
+        default: launch_cgu_dmma_g<32>(a, P.ngroups, extra, mt, P2 != nullptr, cplx); break;
     }
     OMM_KCHECK();
     // FP64 flops of the dense group blocks (= 2 nnz n per product for atom-block patterns)
-    ktime_end("cgu_dmma_kernel", 2.0 * A.rows * (double)P.h_urows.size() * P.G * (P2 ? 2 : 1));
+    ktime_end("cgu_dmma_kernel", 2.0 * a.n * (double)P.h_urows.size() * P.G * (P2 || cplx ? 2 : 1));
 }
 
 // FP32 variant of the column-group kernel for the reduced-precision solver stages:
@@ -510,6 +511,13 @@ __global__ void __launch_bounds__(64) cgu32_kernel(int n, int N, const float* __
             }
         }
     }
+}
+
+// *flag = 1 when a (rows x cols, column stride lda) holds an Inf or NaN
+__global__ void nonfinite_kernel(int rows, int cols, const double* __restrict__ a, long long lda, int* flag) {
+    bool bad = false;
+    for (Walk w(rows, cols); w.e < w.total; w.next()) bad |= !(fabs(a[w.i + (size_t)w.j * lda]) <= 1.7976931348623157e308);
+    if (bad) *flag = 1;
 }
 
 __global__ void f64_to_f32_kernel(size_t n, const double* __restrict__ a, float* __restrict__ b) {
@@ -752,33 +760,6 @@ void finish_plan(const msw_matrix* B, SpmmPlan& Pl) {
     }
 }
 
-template <typename T, int TM, int TN>
-void launch_cgu(const DView& A, const SpmmPlan& P, const SpmmPlan* P2, DView& C, DView* C2, zdbl al, zdbl be,
-                int bz, int N) {
-    constexpr int BM = 16 * TM;
-    dim3 grid((A.rows + BM - 1) / BM, P.ngroups);
-    if (P2)
-        cgu_kernel<T, TM, TN, 2><<<grid, 64, 0, rt().stream>>>(A.rows, N, A.as<T>(), A.ld, P.gptr.as<int>(),
-                                                               P.urows.as<int>(), P.bvals.as<T>(), P2->bvals.as<T>(),
-                                                               C.as<T>(), C.ld, C2->as<T>(), C2->ld, al, be, bz);
-    else
-        cgu_kernel<T, TM, TN, 1><<<grid, 64, 0, rt().stream>>>(A.rows, N, A.as<T>(), A.ld, P.gptr.as<int>(),
-                                                               P.urows.as<int>(), P.bvals.as<T>(), nullptr,
-                                                               C.as<T>(), C.ld, nullptr, 0, al, be, bz);
-    OMM_KCHECK();
-}
-
-template <typename T, int TM>
-void dispatch_cgu(int G, const DView& A, const SpmmPlan& P, const SpmmPlan* P2, DView& C, DView* C2, zdbl al,
-                  zdbl be, int bz, int N) {
-    switch (G) {
-        case 8: launch_cgu<T, TM, 2>(A, P, P2, C, C2, al, be, bz, N); break;
-        case 16: launch_cgu<T, TM, 4>(A, P, P2, C, C2, al, be, bz, N); break;
-        case 24: launch_cgu<T, TM, 6>(A, P, P2, C, C2, al, be, bz, N); break;
-        default: launch_cgu<T, TM, 8>(A, P, P2, C, C2, al, be, bz, N); break;
-    }
-}
-
 }  // namespace
 
 void spmm_plan_cache_clear() { clear_kept_groups(); }
@@ -811,8 +792,8 @@ bool same_pattern(const msw_matrix* A, const msw_matrix* B) {
     return eq;
 }
 
-void spmm_dense_csc_gather(const DView& A, const msw_matrix* B, DView& C, const double alpha[2],
-                           const double beta[2]) {
+static void launch_gather(const DView& A, const msw_matrix* B, DView& C, const double alpha[2], const double beta[2],
+                          const int* only_if) {
     ensure_csc_device(B);
     int n = A.rows, N = B->dim2;
     if (n == 0 || N == 0) return;
@@ -822,17 +803,51 @@ void spmm_dense_csc_gather(const DView& A, const msw_matrix* B, DView& C, const 
     if (A.is_real)
         gather_kernel<double><<<grid, kGatherThreads, 0, rt().stream>>>(n, A.as<double>(), A.ld, B->d_colptr.as<int>(),
                                                                         B->d_rowind.as<int>(), B->d_val.as<double>(),
-                                                                        C.as<double>(), C.ld, al, be, bz);
+                                                                        C.as<double>(), C.ld, al, be, bz, only_if);
     else
         gather_kernel<zdbl><<<grid, kGatherThreads, 0, rt().stream>>>(n, A.as<zdbl>(), A.ld, B->d_colptr.as<int>(),
                                                                       B->d_rowind.as<int>(), B->d_val.as<zdbl>(),
-                                                                      C.as<zdbl>(), C.ld, al, be, bz);
+                                                                      C.as<zdbl>(), C.ld, al, be, bz, only_if);
     OMM_KCHECK();
+}
+void spmm_dense_csc_gather(const DView& A, const msw_matrix* B, DView& C, const double alpha[2],
+                           const double beta[2]) {
+    launch_gather(A, B, C, alpha, beta, nullptr);
+}
+
+// Whether a look at 16 of the matrix's 8-column groups, evenly spaced, already rules the column-group
+// kernels out: their fill is below half of what a plan needs (a wider group of the same columns is
+// emptier still).  Saves a matrix with an irregular pattern the search over group widths, which takes
+// the host milliseconds per 10^5 nonzeros; a sample near the limit leaves the decision to the plan.
+bool rules_out_groups(const msw_matrix* B) {
+    msw_matrix* Bm = const_cast<msw_matrix*>(B);
+    if (Bm->plan) return false;
+    if (Bm->no_groups < 0) {
+        const int ng = B->dim2 / 8, take = std::min(ng, 16);
+        long long nnz = 0, cells = 0;
+        std::vector<int> seen(B->dim1, -1);
+        for (int s = 0; s < take; ++s) {
+            const int j = (int)((long long)s * ng / take) * 8;
+            for (int l = B->h_colptr[j]; l < B->h_colptr[j + 8]; ++l) {
+                int& mark = seen[B->h_rowind[l]];
+                cells += mark != s ? 8 : 0;
+                mark = s;
+            }
+            nnz += B->h_colptr[j + 8] - B->h_colptr[j];
+        }
+        Bm->no_groups = take == 16 && nnz * 4 < cells ? 1 : 0;
+    }
+    return Bm->no_groups == 1;
 }
 
 void spmm_dense_csc(const DView& A, const msw_matrix* B, DView& C, const double alpha[2], const double beta[2],
                     const msw_matrix* B2, DView* C2) {
     if (A.rows == 0 || B->dim2 == 0) return;
+    if (rules_out_groups(B)) {
+        spmm_dense_csc_gather(A, B, C, alpha, beta);
+        if (B2 && C2) spmm_dense_csc(A, B2, *C2, alpha, beta);
+        return;
+    }
     SpmmPlan& P = get_plan(B);
     bool fuse = B2 && C2 && same_pattern(B, B2);
     if (!P.cgu) {
@@ -854,23 +869,9 @@ void spmm_dense_csc(const DView& A, const msw_matrix* B, DView& C, const double 
         P2 = B2m->plan.get();
         if (P2->G != P.G || P2->h_gptr != P.h_gptr) fuse = false, P2 = nullptr;
     }
-    zdbl al{alpha[0], alpha[1]}, be{beta[0], beta[1]};
-    int bz = (beta[0] == 0.0 && beta[1] == 0.0) ? 1 : 0;
-    if (A.is_real) {
-        // FP64 tensor cores (DMMA)
-        const SpmmPlan* Q = fuse ? P2 : nullptr;
-        DView* C2f = fuse ? C2 : nullptr;
-        switch (P.G) {
-            case 8: launch_cgu_dmma<8>(A, P, Q, C, C2f, alpha[0], beta[0], bz, B->dim2); break;
-            case 16: launch_cgu_dmma<16>(A, P, Q, C, C2f, alpha[0], beta[0], bz, B->dim2); break;
-            case 24: launch_cgu_dmma<24>(A, P, Q, C, C2f, alpha[0], beta[0], bz, B->dim2); break;
-            default: launch_cgu_dmma<32>(A, P, Q, C, C2f, alpha[0], beta[0], bz, B->dim2); break;
-        }
-    } else {
-        // rows per thread chosen so that the accumulators of one or two value sets fit in registers
-        if (fuse) dispatch_cgu<zdbl, 2>(P.G, A, P, P2, C, C2, al, be, bz, B->dim2);
-        else dispatch_cgu<zdbl, 4>(P.G, A, P, nullptr, C, nullptr, al, be, bz, B->dim2);
-    }
+    const int bz = (beta[0] == 0.0 && beta[1] == 0.0) ? 1 : 0;
+    fuse = fuse && A.is_real;  // a complex matrix's two parts take both value sets of the kernel
+    launch_cgu_dmma(A, P, fuse ? P2 : nullptr, C, fuse ? C2 : nullptr, alpha, beta, bz, B->dim2, false);
     if (B2 && C2 && !fuse) spmm_dense_csc(A, B2, *C2, alpha, beta);
 }
 
@@ -989,8 +990,8 @@ void gemspm(char opA, const DView& A, char opB, const msw_matrix* B, DView& C, c
     if (trA) {
         Aop.rows = A.cols;
         Aop.cols = A.rows;
-        Aop.ld = A.cols;
-        tA.alloc((size_t)Aop.rows * Aop.cols * (A.is_real ? 8 : 16));
+        Aop.ld = (A.cols + 1) & ~1;  // even: 16-byte column segments for the column-group kernel
+        tA.alloc(std::max<size_t>(1, (size_t)Aop.ld * Aop.cols) * (A.is_real ? 8 : 16));
         Aop.p = tA.p;
         transpose_into(A, opA, Aop);
     }
@@ -1014,58 +1015,73 @@ void gemspm(char opA, const DView& A, char opB, const msw_matrix* B, DView& C, c
     spmm_dense_csc(Aop, Bop, C, alpha, beta);
 }
 
-// psp_gespmm (pspSpmm.F90:61-123): C = alpha*op(A)*op(B) + beta*C with A CSC.
-// Evaluated as C^T = op(B)^T op(A)^T with the dense x CSC kernel, then transposed back.
+// psp_gespmm (pspSpmm.F90:61-123): C = alpha*op(A)*op(B) + beta*C with A CSC, evaluated as
+// C^T = op(B)^T op(A)^T with the dense x CSC kernels.  op(A)^T is A^T's CSC for 'n' and A itself
+// otherwise; where 'c' asks for conj(A), the dense operand is conjugated instead and so is the
+// product: conj(conj(X) A) = X conj(A).  The column-group kernel writes the product transposed, in
+// place of a second matrix and a transposing add (5 x 5 x 5 atoms of 24 orbitals, 375 columns: 114 us
+// with the transposed copy of B; the gather kernel, which took every pattern before, 500 us).
 void gespmm(char opA, const msw_matrix* A, char opB, const DView& B, DView& C, const double alpha[2],
             const double beta[2]) {
-    // X = op(B)^T as a dense (N x K) matrix; for complex the conjugation rule
-    // (op(B)^T)_{jk} = op(B)_{kj} is carried into a per-op choice below.
-    bool real = B.is_real;
-    int M = C.rows, N = C.cols;
-    // op(B)^T: 'n' -> B^T, 't' -> B, 'c' -> conj(B)
-    DevBuf tX, tY;
-    DView X;
-    X.is_real = real;
-    bool bN = (opB == 'n' || opB == 'N'), bT = (opB == 't' || opB == 'T');
+    const bool real = B.is_real;
+    const int M = C.rows, N = C.cols;
+    const bool aN = (opA == 'n' || opA == 'N'), aC = !real && (opA == 'c' || opA == 'C');
+    const bool bN = (opB == 'n' || opB == 'N'), bC = !real && (opB == 'c' || opB == 'C');
+    const bool conj = aC != bC;  // X = op(B)^T, conjugated once more when op(A) is 'c'
+    const size_t es = real ? 8 : 16;
+    DevBuf tX, tmp;
+    DView X = B;
     if (bN) {
-        X.rows = B.cols; X.cols = B.rows; X.ld = B.cols;
-        tX.alloc((size_t)X.rows * X.cols * (real ? 8 : 16));
+        X.rows = B.cols; X.cols = B.rows;
+        X.ld = std::max(2, (B.cols + 1) & ~1);  // even: 16-byte column segments for the column-group kernel
+        tX.alloc((size_t)X.ld * std::max(1, X.cols) * es);
         X.p = tX.p;
-        transpose_into(B, 't', X);
-    } else if (bT || real) {
-        X = B;
-    } else {
-        X.rows = B.rows; X.cols = B.cols; X.ld = B.rows;
-        tX.alloc((size_t)X.rows * X.cols * 16);
-        X.p = tX.p;
+        transpose_into(B, conj ? 'c' : 't', X);
+    } else if (conj) {
         // conj(B) = (B^H)^T: two transposes keep this on existing kernels
-        DevBuf tmp;
-        DView Th{nullptr, B.cols, B.rows, B.cols, false};
-        tmp.alloc((size_t)B.rows * B.cols * 16);
+        DView Th{nullptr, B.cols, B.rows, std::max(1, B.cols), false};
+        tmp.alloc(std::max<size_t>(1, (size_t)B.rows * B.cols) * 16);
         Th.p = tmp.p;
         transpose_into(B, 'c', Th);
+        X.ld = std::max(1, B.rows);
+        tX.alloc(std::max<size_t>(1, (size_t)X.rows * X.cols) * 16);
+        X.p = tX.p;
         transpose_into(Th, 't', X);
     }
-    // Y = op(A)^T as CSC: 'n' -> A^T, 't' -> A, 'c' -> conj(A)
-    const msw_matrix* Y = A;
-    std::shared_ptr<msw_matrix> conjA;
-    bool aN = (opA == 'n' || opA == 'N'), aT = (opA == 't' || opA == 'T');
-    if (aN) Y = csc_transpose(A);
-    else if (!aT && !A->is_real) {
-        conjA = std::make_shared<msw_matrix>();
-        *conjA = msw_matrix();
-        conjA->dim1 = A->dim1; conjA->dim2 = A->dim2; conjA->is_real = false; conjA->fmt = Fmt::CSC;
-        conjA->nnz = A->nnz; conjA->h_colptr = A->h_colptr; conjA->h_rowind = A->h_rowind; conjA->h_val = A->h_val;
-        for (int l = 0; l < conjA->nnz; ++l) conjA->h_val[2 * l + 1] = -conjA->h_val[2 * l + 1];
-        Y = conjA.get();
+    const msw_matrix* Y = aN ? csc_transpose(A) : A;
+    if (N == 0 || M == 0) return;
+    const double one[2] = {1.0, 0.0}, zero[2] = {0.0, 0.0};
+    const SpmmPlan* P = rules_out_groups(Y) ? nullptr : &get_plan(Y);
+    if (P && !P->cgu) P = nullptr;
+    // every cell of the groups' blocks is a nonzero (atom blocks): nothing is multiplied that the sparse
+    // product leaves out
+    const bool full = P && P->efficiency == 1.0;
+    if (full && !aC) {
+        const int bz = (beta[0] == 0.0 && beta[1] == 0.0) ? 1 : 0;
+        launch_cgu_dmma(X, *P, nullptr, C, nullptr, alpha, beta, bz, M, true);
+        return;
     }
-    // Z = X * Y  (N x M), then C = alpha*Z^T + beta*C
+    // Z = X * Y  (N x M), then C = alpha*Z^T (or Z^H) + beta*C
+    DevBuf tZ, flag;
     DView Z{nullptr, N, M, N, real};
-    tY.alloc((size_t)N * M * (real ? 8 : 16));
-    Z.p = tY.p;
-    double one[2] = {1.0, 0.0}, zero[2] = {0.0, 0.0};
-    spmm_dense_csc_gather(X, Y, Z, one, zero);
-    k_axpby(Z, 't', C, alpha, beta);
+    tZ.alloc((size_t)N * M * es);
+    Z.p = tZ.p;
+    if (P) {
+        launch_cgu_dmma(X, *P, nullptr, Z, nullptr, one, zero, 1, M, false);
+        if (!full) {
+            // a zero cell times an Inf or NaN of X is a NaN that the sparse product does not have: when X
+            // holds any, the gather kernel forms the product again from the nonzeros alone
+            flag.alloc_zero(sizeof(int));
+            nonfinite_kernel<<<(int)std::min<size_t>(((size_t)X.rows * X.cols + 255) / 256, 148 * 8), 256, 0,
+                               rt().stream>>>(X.rows * (real ? 1 : 2), X.cols, X.as<double>(),
+                                              (long long)X.ld * (real ? 1 : 2), flag.as<int>());
+            OMM_KCHECK();
+            launch_gather(X, Y, Z, one, zero, flag.as<int>());
+        }
+    } else {
+        spmm_dense_csc_gather(X, Y, Z, one, zero);
+    }
+    k_axpby(Z, aC ? 'c' : 't', C, alpha, beta);
 }
 
 }  // namespace ommgpu

@@ -1,0 +1,83 @@
+"""The FP64 column-group kernel at the edges of its tiles: rows around the 32, 64 and 128 row blocks,
+group widths with and without zero cells, complex matrices as two value sets, transposed output
+(psp_gespmm) and odd leading dimensions, against dense products in numpy."""
+import numpy as np
+import pytest
+
+import ommgpu as G
+from ommgpu import synth
+
+pytestmark = pytest.mark.gpu
+
+
+def _case(norb, cplx, seed):
+    p = synth.lattice((5, 5, 5), seed=seed, norb=norb, nocc=1, compute_mu=False)
+    H = p.H
+    if cplx:
+        rng = np.random.default_rng(seed)
+        H = synth.CSCMatrix(H.dim1, H.dim2, H.colptr, H.rowind, H.val * np.exp(1j * rng.uniform(0, 6, H.nnz)))
+    return H
+
+
+def _rnd(rng, shape, cplx):
+    a = rng.standard_normal(shape)
+    return np.asfortranarray(a + 1j * rng.standard_normal(shape) if cplx else a)
+
+
+def _op(a, op):
+    return a if op == "n" else a.T if op == "t" else a.conj().T
+
+
+def _check(got, ref, mag):
+    # a sum of at most 33 * norb products in FP64, in any order: n eps sum|a||b|, with a margin of 4
+    bound = 4 * (33 * 32 + 8) * np.finfo(float).eps * (mag + np.abs(ref))
+    assert np.all(np.abs(got - ref) <= bound), float(np.max(np.abs(got - ref) / np.maximum(bound, 1e-300)))
+
+
+@pytest.mark.parametrize("cplx", [False, True])
+@pytest.mark.parametrize("norb", [8, 13, 16, 24, 32])
+@pytest.mark.parametrize("n", [1, 31, 33, 65, 129, 300])
+def test_gemspm_rows_and_widths(norb, n, cplx):
+    H = _case(norb, cplx, 50 + norb)
+    rng = np.random.default_rng(n)
+    m, Hd = H.dim1, H.to_dense()
+    A, C0 = _rnd(rng, (n, m), cplx), _rnd(rng, (n, m), cplx)
+    al, be = (0.7 - 0.2j, 0.3 + 0.1j) if cplx else (0.7, 0.3)
+    C = G.Matrix.from_numpy(C0)
+    G.psp_gemspm(n, m, m, G.Matrix.from_numpy(A), "n", G.Matrix.from_csc(H), "n", C, al, be)
+    _check(C.numpy(), al * (A @ Hd) + be * C0, np.abs(A) @ np.abs(Hd) + np.abs(C0))
+
+
+@pytest.mark.parametrize("cplx", [False, True])
+@pytest.mark.parametrize("opA", ["n", "t", "c"])
+@pytest.mark.parametrize("opB", ["n", "t", "c"])
+@pytest.mark.parametrize("norb,n", [(8, 65), (13, 33), (24, 130)])
+def test_gespmm_ops_and_widths(norb, n, opA, opB, cplx):
+    H = _case(norb, cplx, 70 + norb)
+    rng = np.random.default_rng(n)
+    m, Hd = H.dim1, H.to_dense()
+    B = _rnd(rng, (m, n) if opB == "n" else (n, m), cplx)
+    C0 = _rnd(rng, (m, n), cplx)
+    al, be = (0.7 - 0.2j, 0.3 + 0.1j) if cplx else (0.7, 0.3)
+    C = G.Matrix.from_numpy(C0)
+    G.psp_gespmm(m, n, m, G.Matrix.from_csc(H), opA, G.Matrix.from_numpy(B), opB, C, al, be)
+    a, b = _op(Hd, opA), _op(B, opB)
+    _check(C.numpy(), al * (a @ b) + be * C0, np.abs(a) @ np.abs(b) + np.abs(C0))
+
+
+@pytest.mark.parametrize("norb", [13, 24])
+@pytest.mark.parametrize("bad", [np.inf, np.nan])
+def test_gespmm_nonfinite_stays_in_its_rows(norb, bad):
+    """A row of the dense operand that holds an Inf or NaN reaches the rows of the product whose sparse
+    rows hold that column, and no others."""
+    H = _case(norb, False, 90)
+    rng = np.random.default_rng(4)
+    m, n, k = H.dim1, 40, 77
+    B = _rnd(rng, (m, n), False)
+    B[k, 3] = bad
+    C = G.Matrix.allocate(m, n)
+    G.psp_gespmm(m, n, m, G.Matrix.from_csc(H), "n", G.Matrix.from_numpy(B), "n", C, 1.0, 0.0)
+    got = C.numpy()
+    touched = np.zeros((m, n), bool)
+    touched[:, 3] = H.to_dense()[:, k] != 0.0
+    assert np.array_equal(~np.isfinite(got), touched)
