@@ -479,7 +479,8 @@ int omm_gpu_gemm_f64(char opA, char opB, int M, int N, int K, double alpha, cons
  * its pipeline errors are read with omm_gpu_tc_errors. */
 int omm_gpu_gemm_f64_async(char opA, char opB, int M, int N, int K, double alpha, const double* A, int lda,
                            const double* B, int ldb, double beta, double* C, int ldc);
-/* FP64 SpMM on the int8 tensor cores, as the FP64 CG step forms [HG; SG] = D [H, S]
+/* FP64 SpMM on the int8 tensor cores: [HG; SG] = D [H, S] exactly to 53-bit operands (omm's own
+ * step takes the FP64 tensor-core SpMM, which is faster and closer to the exact sums)
  * (psp_gemspm's local product, pspBLAS/src/pspLevel3/pspMspm_nn.F90:191-198, with
  * both matrices at once): Y(0:n-1, :) = A H and, when S is given (same pattern as H),
  * Y(n:2n-1, :) = A S.  A (n x m) and Y (ldy >= n, or 2n with S) are device FP64
@@ -489,7 +490,7 @@ int omm_gpu_gemm_f64_async(char opA, char opB, int M, int N, int K, double alpha
  * exactly (16 moduli, as omm_gpu_gemm_f64).  OMM_ERR_UNSUPPORTED when the matrices
  * do not fit.  Synchronous.  No reference counterpart. */
 int omm_gpu_spmm_f64(const double* A, int lda, int n, const msw_matrix* H, const msw_matrix* S, double* Y, int ldy);
-/* Form of that int8 SpMM kernel (and of the FP64 CG step's): 0 = one column group per CTA,
+/* Form of that int8 SpMM kernel: 0 = one column group per CTA,
  * four pipeline stages of one chunk pair; 1 (default) = one group per CTA, two stages of three
  * chunk pairs, chunks adjacent in memory fetched as one copy of up to 24 KB; 2 = two
  * consecutive column groups per CTA walking the union of their rows once, with two-pair

@@ -330,7 +330,8 @@ bool oz_spmm_kb_halves(bool with_s);
 // Y = beta Y + alpha X (real, R x K, rows contiguous) with the exponents oz_prepare would form of
 // Y's rows (erow, R ints) and of its columns (ecol, K ints: the rows of Y^T); either may be null
 void oz_axpby_exps(int R, int K, double alpha, const DView& X, double beta, DView& Y, int* erow, int* ecol);
-// out (A.rows x B.rows) = alpha * A B^T + beta * out; herm as for gemm_bf16_tn
+// out (A.rows x B.rows) = alpha * A B^T + beta * out; herm > 0 (any divisor of A.rows): out is a stack of
+// Hermitian herm x herm blocks and only the tiles reaching their upper triangles are formed
 // out_part 0 / 1: C is complex and the product goes to its real / imaginary part
 void oz_gemm(const OzOperand& A, const OzOperand& B, double alpha, double beta, DView& C, int herm = 0,
              int out_part = -1);

@@ -475,7 +475,7 @@ std::shared_ptr<BlockPtrs> block_ptrs(const DView& A, const DView& B, DView& W, 
 // where a staircase of shrinking row blocks does not), then the lower triangles mirrored.
 // False when n does not split into equal blocks of at least 128.
 bool hermitian_blocks_batched(const DView& A, const DView& B, DView& W, int n, int k, int halves) {
-    if (A.is_real && n % 128 == 0 && fp64_emu_enabled() && fp64_emu_worth(halves * n, n, k)) {
+    if (A.is_real && fp64_emu_enabled() && fp64_emu_worth(halves * n, n, k)) {
         // one FP64 product on the int8 tensor cores over the stacked halves, forming only the
         // tiles that reach each half's upper triangle, then the mirror
         gemm_f64_emu('n', 't', halves * n, n, k, 1.0, A, B, 0.0, W, n);
@@ -555,7 +555,7 @@ void hermitian_pair_nt(const DView& Y, const DView& Dir, DView& Wdd, int n, int 
 // the FP64 step's products of a real problem run on the int8 tensor cores (eval_direction's
 // Gram products and SpMM from shared residues, calc_G through gemm_f64_emu)
 bool fp64_step_emu(const OmmCall& c) {
-    return c.real && c.n % 128 == 0 && fp64_emu_enabled() && fp64_emu_worth(2 * c.n, c.n, c.m);
+    return c.real && fp64_emu_enabled() && fp64_emu_worth(2 * c.n, c.n, c.m);
 }
 
 // D = G + lambda D (omm.F90:444-446) for the FP64 step; on the int8 path the same pass forms the
@@ -603,30 +603,22 @@ void eval_direction(OmmCall& c, const DView& Dir, double coeff[5]) {
     DView Y = view(s.Y, 2 * n, m, 2 * n, c.real);
     DView Wdd = view(s.Wdd, 2 * n, n, 2 * n, c.real);
     if (fp64_step_emu(c)) {
-        // both Gram products on the int8 tensor cores, sharing the residues of Dir, and -- for
-        // atom-block CSC H (and S) -- the SpMM too, from the same residues
+        // both Gram products on the int8 tensor cores, sharing the residues of Dir
         OzOperand* od = &oz_scratch(OZS_DIR);
         OzOperand* oa = &oz_scratch(OZS_X);
         const int bits = oz_bits(m, OZ_NMOD);
-        const msw_matrix* S2 = c.s_identity ? nullptr : c.Sm;
-        const bool sp = c.H_csc && !c.hcb && (c.s_identity || (c.S_csc && same_pattern(c.Hm, c.Sm))) &&
-                        oz_spmm_available(c.Hm, S2);
         // the exponents the last D / X update formed, when Dir is that D and X is unchanged since
         const int* de = (s.de_ok && s.de_src == Dir.p) ? s.De.as<int>() : nullptr;
         const int* xe = s.xr_ok ? s.Xe_r.as<int>() : nullptr;
         s.de_ok = s.xr_ok = false;
-        oz_prepare(Dir, false, n, m, OZ_NMOD, bits, *od, sp, -1, de, sp && oz_spmm_kb_halves(S2 != nullptr));
+        oz_prepare(Dir, false, n, m, OZ_NMOD, bits, *od, false, -1, de);
         oz_prepare(X, false, 2 * n, m, OZ_NMOD, bits, *oa, false, -1, xe);
         oz_gemm(*oa, *od, 1.0, 0.0, Wd);                   // [HWd; SWd] = [HC; SC] Dir^T
-        DView Yv = view(s.Y, S2 ? 2 * n : n, m, 2 * n, true);
-        if (sp && oz_spmm(c.Hm, S2, *od, Yv)) {            // [HG; SG] = Dir [H, S]
-            if (!S2) {
-                DView bot = view(s.Y, n, m, 2 * n, true, n);
-                copy_view(Dir, bot);
-            }
-        } else {
-            apply_HS(c, Dir, s.Y);
-        }
+        // [HG; SG] = Dir [H, S] on the FP64 tensor cores: 1.89 ms at lattice_8x8x8.  The int8 SpMM
+        // (omm_gpu_spmm_f64) takes 1.71 + 0.25 ms for its reconstructions and 0.07 for the k-blocked
+        // residues, needs its plan per registered H (7 ms), loses more where groups straddle atoms (13
+        // orbitals: 45.4 against 33.5 ms a solve), and is a third further from the exact sums.
+        apply_HS(c, Dir, s.Y);
         oz_prepare(Y, false, 2 * n, m, OZ_NMOD, bits, *oa);
         oz_gemm(*oa, *od, 1.0, 0.0, Wdd, n);               // [HWdd; SWdd]: upper tiles of each half
         DView top = view(s.Wdd, n, n, 2 * n, true), bot = view(s.Wdd, n, n, 2 * n, true, n);
@@ -899,8 +891,8 @@ void density_product(const DView& C, const DView& CD, DView& D) {
     int m = C.cols, n = C.rows;
     if (C.is_real && fp64_emu_enabled() && fp64_emu_worth(m, m, n)) {
         // FP64-accurate D = C^T CD on the int8 tensor cores: only the tiles reaching the upper
-        // triangle when m splits into 128-row tiles, then the mirror
-        gemm_f64_emu('t', 'n', m, m, n, 1.0, C, CD, 0.0, D, m % 128 == 0 ? m : 0);
+        // triangle, then the mirror
+        gemm_f64_emu('t', 'n', m, m, n, 1.0, C, CD, 0.0, D, m);
         k_fill_lower_from_upper(D);
         return;
     }

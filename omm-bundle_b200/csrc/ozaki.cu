@@ -849,6 +849,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
 }
 
 // ------------------------------------------------------------------ reconstruction
+// Whether the tile of rows m0 .. m0 + bm - 1 (of M) and columns up to cmax reaches the upper triangle of
+// one of the stacked herm x herm Hermitian blocks: a tile that holds a block's first row does
+__host__ __device__ inline bool oz_tile_needed(int m0, int bm, int M, int herm, int cmax) {
+    if (herm == 0) return true;
+    const int last = (m0 + bm < M ? m0 + bm : M) - 1;
+    return m0 / herm != last / herm || m0 % herm <= cmax;
+}
+
 struct RecParams {
     int M, N, nmod;
     const uint8_t* R;
@@ -938,7 +946,7 @@ __global__ void __launch_bounds__(256) oz_reconstruct_kernel(const __grid_consta
     for (int jj = 0; jj < 8; ++jj) {
         const int j = blockIdx.y * 8 + jj;
         if (j >= p.N) return;
-        if (p.herm > 0 && ((i0 / BM) * BM) % p.herm > ((p.n_off + j) / BN) * BN + BN - 1) continue;
+        if (!oz_tile_needed(i0 / BM * BM, BM, p.M, p.herm, ((p.n_off + j) / BN) * BN + BN - 1)) continue;
         const int eb = p.eB[j];
         const uint8_t* r = p.R + (size_t)i0 + (size_t)j * p.ldr;
         uint32_t res[MAXMOD];
@@ -961,8 +969,8 @@ __global__ void __launch_bounds__(256) oz_reconstruct_kernel(const __grid_consta
 }
 
 // ------------------------------------------------------------------ FP64 SpMM on the int8 tensor cores
-// Y = A [H, S] for atom-block CSC H and S (the FP64 CG step's [HG; SG] = D [H, S]) by the same
-// modular method: A's rows and H's / S's columns are rounded to 53-bit integers, and every modulus
+// Y = A [H, S] for atom-block CSC H and S (omm_gpu_spmm_f64; the CG step's [HG; SG] = D [H, S] takes the
+// FP64 tensor-core kernel of spmm.cu) by the same modular method: A's rows and H's / S's columns are rounded to 53-bit integers, and every modulus
 // is one int8 SpMM over the column-group plan of spmm.cu -- output columns in groups of G whose
 // nonzero rows form a union U_g -- with U_g covered by 16-row chunks.  A's residues come
 // k-blocked (per block of 256 rows, chunk c holds A(:, 16 c .. 16 c + 15) as 256 rows x 16 B,
@@ -1660,7 +1668,7 @@ const DevBuf& tile_list(int M, int nc, int herm, int c0, int bm, int bn) {
     for (int L = 0; L < nM * nN; ++L) {
         const int per = GROUP * nN, g = L / per, first = g * GROUP, size = std::min(GROUP, nM - first), r = L - g * per;
         const int m0 = (first + r % size) * bm, n0 = (r / size) * bn;
-        if (herm == 0 || m0 % herm <= c0 + n0 + bn - 1) v.push_back(make_int2(m0, n0));
+        if (oz::oz_tile_needed(m0, bm, M, herm, c0 + n0 + bn - 1)) v.push_back(make_int2(m0, n0));
     }
     auto b = std::make_unique<DevBuf>();
     b->alloc(std::max<size_t>(1, v.size()) * sizeof(int2));
@@ -1684,7 +1692,7 @@ void oz_gemm(const OzOperand& A, const OzOperand& B, double alpha, double beta, 
     const int M = A.rows, N = B.rows, K = A.K;
     if (B.K != K || A.nmod != B.nmod) fail(OMM_ERR_ARG, "oz_gemm: operands differ in K or moduli");
     if (K > MAX_K) fail(OMM_ERR_ARG, "oz_gemm: K must be below 2^17");
-    if (herm < 0 || (herm > 0 && (herm % BM || M % herm))) fail(OMM_ERR_ARG, "oz_gemm: bad Hermitian block size");
+    if (herm < 0 || (herm > 0 && M % herm)) fail(OMM_ERR_ARG, "oz_gemm: bad Hermitian block size");
     const Table& tb = table(A.nmod);
     if ((double)(A.bits + B.bits) > tb.log2P - 2.0 - std::log2((double)std::max(K, 1)))
         fail(OMM_ERR_ARG, "oz_gemm: operand bits exceed the moduli's range");
@@ -1701,8 +1709,7 @@ void oz_gemm(const OzOperand& A, const OzOperand& B, double alpha, double beta, 
         OMM_CK(cudaFuncSetAttribute(oz_gemm_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM2_BYTES));
         attr = true;
     }
-    // SM pairs (256 x 256 tiles) unless a Hermitian block would split a pair's rows
-    const bool pairs = tc_pairs_enabled() && M > BM && (herm == 0 || herm % BM2 == 0);
+    const bool pairs = tc_pairs_enabled() && M > BM;  // 256 x 256 tiles on SM pairs
     const int tbm_ = pairs ? BM2 : BM, tbn_ = pairs ? BN2 : BN;
     const CUtensorMap ta = map_planes(A.planes.p, M, K, A.ldk, A.nmod, BM);
     const CUtensorMap tbm = map_planes(B.planes.p, N, K, B.ldk, B.nmod, pairs ? 128 : BN);
@@ -1767,7 +1774,7 @@ void oz_gemm(const OzOperand& A, const OzOperand& B, double alpha, double beta, 
             double cells = 0.0;
             for (int m0 = 0; m0 < M; m0 += tbm_)
                 for (int n0 = 0; n0 < nc; n0 += tbn_)
-                    if (herm == 0 || m0 % herm <= c0 + n0 + tbn_ - 1)
+                    if (oz_tile_needed(m0, tbm_, M, herm, c0 + n0 + tbn_ - 1))
                         cells += (double)std::min(tbm_, M - m0) * std::min(tbn_, nc - n0);
             ktime_end(pairs ? "oz_gemm_pair_kernel" : "oz_gemm_kernel", 2.0 * K * cells * A.nmod);
         }
