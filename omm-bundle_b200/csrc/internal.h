@@ -253,6 +253,7 @@ void k_set(DView& C, char seC, const double alpha[2], const double beta[2]);
 void k_set_element(DView& C, int i, int j, const double alpha[2], const double beta[2]);
 void k_fill_lower_from_upper(DView& C);      // C(j,i) = conj(C(i,j)) for j > i
 void k_w_update(DView& W, const DView& Wd, const DView& Wdd, double x);  // W += x (Wd^H + Wd) + x^2 Wdd
+void k_calcG_left(const DView& SW, const DView& HW, DView& L);  // L = [4I - 2 SW, -2 HW], n x 2n
 void k_lcg_init(DView& C);                   // reference C0 (NORAND LCG), unscaled
 // reductions (deterministic two-pass); results copied to host
 void r_trace(const DView& A, double out[2]);                          // sum of diagonal
@@ -344,9 +345,10 @@ bool oz_spmm(const msw_matrix* H, const msw_matrix* S, const OzOperand& A, DView
 // b_exps: the exponents of op(B)'s columns already formed (oz_axpby_exps)
 void gemm_f64_emu(char opA, char opB, int M, int N, int K, double alpha, const DView& A, const DView& B, double beta,
                   DView& C, int herm = 0, const int* b_exps = nullptr);
-// complex op(A) op(B) (ops 'n', 't', 'c'; real alpha, beta) as four real FP64-accurate products
+// complex op(A) op(B) (ops 'n', 't', 'c'; real alpha, beta) as four real FP64-accurate products;
+// herm as for oz_gemm
 void gemm_z_emu(char opA, char opB, int M, int N, int K, double alpha, const DView& A, const DView& B, double beta,
-                DView& C);
+                DView& C, int herm = 0);
 bool fp64_emu_enabled();  // real FP64 GEMMs of the solver on the int8 tensor cores (default on)
 void set_fp64_emu(int mode, long long panel_bytes);
 size_t oz_panel_bytes();

@@ -473,6 +473,19 @@ __global__ void lambda_kernel(int rows, int cols, const T* __restrict__ PG, int 
     block_reduce_finish<2>(v, part, out);
 }
 
+// L = [4I - 2 SW, -2 HW] (n x 2n), the left factor of calc_G as one product
+template <typename T>
+__global__ void calcG_left_kernel(int n, const T* __restrict__ SW, int lds, const T* __restrict__ HW, int ldh,
+                                  T* __restrict__ L, int ldl) {
+    for (Walk w(n, 2 * n); w.e < w.total; w.next()) {
+        const bool left = w.j < n;
+        T v = left ? SW[w.i + (size_t)w.j * lds] : HW[w.i + (size_t)(w.j - n) * ldh];
+        v = Sc<T>::mul(zdbl{-2.0, 0.0}, v);
+        if (left && w.i == w.j) v = Sc<T>::add(Sc<T>::from(zdbl{4.0, 0.0}), v);
+        L[w.i + (size_t)w.j * ldl] = v;
+    }
+}
+
 template <typename T>
 __global__ void transpose_kernel(int rows, int cols, const T* A, int lda, int conj, T* Tm, int ldt) {
     // Tm (cols x rows) = op(A), A rows x cols
@@ -591,6 +604,19 @@ void k_w_update(DView& W, const DView& Wd, const DView& Wdd, double x) {
     else
         w_update_kernel<zdbl><<<grid, kThreads, 0, rt().stream>>>(W.rows, W.as<zdbl>(), W.ld, Wd.as<zdbl>(),
                                                                              Wd.ld, Wdd.as<zdbl>(), Wdd.ld, x);
+    OMM_KCHECK();
+}
+
+void k_calcG_left(const DView& SW, const DView& HW, DView& L) {
+    const int n = L.rows;
+    const size_t tot = (size_t)n * 2 * n;
+    if (L.is_real)
+        calcG_left_kernel<double><<<grid_for(tot), kThreads, 0, rt().stream>>>(n, SW.as<double>(), SW.ld,
+                                                                                 HW.as<double>(), HW.ld, L.as<double>(),
+                                                                                 L.ld);
+    else
+        calcG_left_kernel<zdbl><<<grid_for(tot), kThreads, 0, rt().stream>>>(n, SW.as<zdbl>(), SW.ld, HW.as<zdbl>(),
+                                                                               HW.ld, L.as<zdbl>(), L.ld);
     OMM_KCHECK();
 }
 

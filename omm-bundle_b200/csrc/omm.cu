@@ -635,39 +635,12 @@ void eval_direction(OmmCall& c, const DView& Dir, double coeff[5]) {
             view(s.Wdd, n, n, 2 * n, c.real, n), coeff);
 }
 
-__global__ void calcG_left_real(int n, const double* __restrict__ SW, const double* __restrict__ HW,
-                                double* __restrict__ L) {
-    for (Walk w(n, 2 * n); w.e < w.total; w.next()) {
-        double v;
-        if (w.j < n) v = (w.i == w.j ? 4.0 : 0.0) - 2.0 * SW[w.e];
-        else v = -2.0 * HW[w.e - (size_t)n * n];
-        L[w.e] = v;
-    }
-}
-__global__ void calcG_left_cplx(int n, const zdbl* __restrict__ SW, const zdbl* __restrict__ HW, zdbl* __restrict__ L) {
-    for (Walk w(n, 2 * n); w.e < w.total; w.next()) {
-        zdbl v;
-        if (w.j < n) {
-            zdbl s = SW[w.e];
-            v = {(w.i == w.j ? 4.0 : 0.0) - 2.0 * s.x, -2.0 * s.y};
-        } else {
-            zdbl h = HW[w.e - (size_t)n * n];
-            v = {-2.0 * h.x, -2.0 * h.y};
-        }
-        L[w.e] = v;
-    }
-}
-
 // calc_G (omm_ops.F90:17-39): G = 4 HC - 2 SW HC - 2 HW SC = [4I - 2SW, -2HW] [HC; SC]
 void calc_G(OmmCall& c, DView& G) {
     IpState& s = *c.s;
     int n = c.n, m = c.m;
-    size_t tot = (size_t)n * 2 * n;
-    int grid = (int)std::min<size_t>((tot + 255) / 256, 148 * 16);
-    if (c.real) calcG_left_real<<<grid, 256, 0, rt().stream>>>(n, s.SW.as<double>(), s.HW.as<double>(), s.Lg.as<double>());
-    else calcG_left_cplx<<<grid, 256, 0, rt().stream>>>(n, s.SW.as<zdbl>(), s.HW.as<zdbl>(), s.Lg.as<zdbl>());
-    OMM_KCHECK();
     DView L = view(s.Lg, n, 2 * n, n, c.real);
+    k_calcG_left(view(s.SW, n, n, n, c.real), view(s.HW, n, n, n, c.real), L);
     DView X = view(s.X, 2 * n, m, 2 * n, c.real);
     if (s.xc_ok && c.real && fp64_emu_enabled() && fp64_emu_worth(n, m, 2 * n)) {
         // X's column exponents from the update that just wrote X (fp64_x_update)

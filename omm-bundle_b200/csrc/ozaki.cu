@@ -2139,7 +2139,7 @@ void gemm_f64_emu(char opA, char opB, int M, int N, int K, double alpha, const D
 // FP64-accurate products of the parts: with op(A) = Ar + i sA Ai and op(B) = Br + i sB Bi
 // (s = -1 for 'c'),  Re C = Ar Br - sA sB Ai Bi,  Im C = sB Ar Bi + sA Ai Br
 void gemm_z_emu(char opA, char opB, int M, int N, int K, double alpha, const DView& A, const DView& B, double beta,
-                DView& C) {
+                DView& C, int herm) {
     const int bits = oz_bits(K, OZ_NMOD);
     const double sA = opA == 'c' ? -1.0 : 1.0, sB = opB == 'c' ? -1.0 : 1.0;
     OzOperand& ar = oz_scratch(OZS_GEMM_A);
@@ -2150,10 +2150,10 @@ void gemm_z_emu(char opA, char opB, int M, int N, int K, double alpha, const DVi
     oz_prepare(A, opA != 'n', M, K, OZ_NMOD, bits, ai, false, 1);
     oz_prepare(B, opB == 'n', N, K, OZ_NMOD, bits, br, false, 0);
     oz_prepare(B, opB == 'n', N, K, OZ_NMOD, bits, bi, false, 1);
-    oz_gemm(ar, br, alpha, beta, C, 0, 0);
-    oz_gemm(ai, bi, -sA * sB * alpha, 1.0, C, 0, 0);
-    oz_gemm(ar, bi, sB * alpha, beta, C, 0, 1);
-    oz_gemm(ai, br, sA * alpha, 1.0, C, 0, 1);
+    oz_gemm(ar, br, alpha, beta, C, herm, 0);
+    oz_gemm(ai, bi, -sA * sB * alpha, 1.0, C, herm, 0);
+    oz_gemm(ar, bi, sB * alpha, beta, C, herm, 1);
+    oz_gemm(ai, br, sA * alpha, 1.0, C, herm, 1);
 }
 
 }  // namespace ommgpu
