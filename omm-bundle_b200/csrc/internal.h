@@ -305,6 +305,7 @@ unsigned gemm_bf16_errors();
 struct OzOperand {
     DevBuf planes, exps;
     int rows = 0, K = 0, ldk = 0, nmod = 0, bits = 0;
+    int zrow = 0;  // complex source: the imaginary parts' rows start here (0: a real source)
     size_t plane = 0;
     // optional k-blocked copy (the int8 SpMM's A operand): per modulus, blocks of 256 rows, each
     // ldk / 16 chunks of 256 rows x 16 B
@@ -316,16 +317,16 @@ constexpr int OZ_NMOD = 16;    // moduli of the FP64-accurate products (53-bit o
 // the residues kept between products (grow-only device buffers, released by oz_release_scratch,
 // which omm_gpu_finalize calls): the CG step's direction and [HC; SC], the two operands of
 // gemm_f64_emu, the operand of omm_gpu_spmm_f64
-enum { OZS_DIR = 0, OZS_X, OZS_GEMM_A, OZS_GEMM_B, OZS_GEMM_AI, OZS_GEMM_BI, OZS_SPMM_A, OZS_COUNT };
+enum { OZS_DIR = 0, OZS_X, OZS_GEMM_A, OZS_GEMM_B, OZS_SPMM_A, OZS_COUNT };
 OzOperand& oz_scratch(int slot);
 void oz_release_scratch();
 int oz_bits(int K, int nmod);  // bits each operand keeps for inner dimension K
 // src: FP64 column-major; kcontig: element (r, k) at src[k + r ld] (else at src[r + k ld])
-// part: -1 for a real source; 0 / 1 for the real / imaginary part of a complex one
+// a complex source gives its real and imaginary rows stacked (zrow), each with exponents of its own
 // exps_in: the operand's row exponents already formed (oz_axpby_exps), copied instead of recomputed
 // kb_halves: the k-blocked copy in the SM-pair SpMM's half-major layout (oz_spmm_kb_halves)
 void oz_prepare(const DView& src, bool kcontig, int rows, int K, int nmod, int bits, OzOperand& op,
-                bool with_kb = false, int part = -1, const int* exps_in = nullptr, bool kb_halves = false);
+                bool with_kb = false, const int* exps_in = nullptr, bool kb_halves = false);
 // the SpMM's form wants A's k-blocked copy half-major (the SM-pair form, for products with S)
 bool oz_spmm_kb_halves(bool with_s);
 // Y = beta Y + alpha X (real, R x K, rows contiguous) with the exponents oz_prepare would form of
@@ -333,9 +334,7 @@ bool oz_spmm_kb_halves(bool with_s);
 void oz_axpby_exps(int R, int K, double alpha, const DView& X, double beta, DView& Y, int* erow, int* ecol);
 // out (A.rows x B.rows) = alpha * A B^T + beta * out; herm > 0 (any divisor of A.rows): out is a stack of
 // Hermitian herm x herm blocks and only the tiles reaching their upper triangles are formed
-// out_part 0 / 1: C is complex and the product goes to its real / imaginary part
-void oz_gemm(const OzOperand& A, const OzOperand& B, double alpha, double beta, DView& C, int herm = 0,
-             int out_part = -1);
+void oz_gemm(const OzOperand& A, const OzOperand& B, double alpha, double beta, DView& C, int herm = 0);
 // Y = A [H, S] in FP64 on the int8 tensor cores (S's product n rows below H's; H's only when S is
 // null) for real CSC H (and S of H's pattern) with a column-group plan; A's residues must carry
 // the k-blocked copy.  False (nothing done) when the matrices do not fit.

@@ -134,7 +134,7 @@ __global__ void set_element_kernel(T* C, size_t idx, zdbl alpha, zdbl beta) {
     C[idx] = Sc<T>::add(Sc<T>::from(alpha), Sc<T>::mul(beta, C[idx]));
 }
 
-// C(j,i) = conj(C(i,j)) for j > i  (omm_ops.F90:483-487 / :590-594).  One 32 x 32 tile of the
+// C(j,i) = conj(C(i,j)) for j > i and a real diagonal  (omm_ops.F90:483-487 / :590-594).  One 32 x 32 tile of the
 // lower triangle per block, its source tile of the upper triangle staged through shared memory
 // so that both the reads and the writes run down columns (coalesced).
 template <typename T>
@@ -151,6 +151,8 @@ __global__ void fill_lower_kernel(int n, T* C, int ldc) {
     for (int yy = ty; yy < 32; yy += 8) {
         int r = 32 * bi + tx, c = 32 * bj + yy;  // destination C(r, c) = conj(C(c, r))
         if (r < n && c < n && r > c) C[r + (size_t)c * ldc] = Sc<T>::conj(tile[tx][yy]);
+        if constexpr (sizeof(T) == 16)
+            if (r < n && r == c) C[r + (size_t)c * ldc].y = 0.0;  // as herk leaves a Hermitian diagonal
     }
 }
 

@@ -487,6 +487,16 @@ bool hermitian_blocks_batched(const DView& A, const DView& B, DView& W, int n, i
         }
         return true;
     }
+    if (!A.is_real && fp64_emu_enabled() && fp64_emu_worth(halves * n, n, k)) {
+        gemm_z_emu('n', 'c', halves * n, n, k, 1.0, A, B, 0.0, W, n);  // as above, on the parts
+        for (int hf = 0; hf < halves; ++hf) {
+            DView Wh = W;
+            Wh.rows = Wh.cols = n;
+            Wh.p = (char*)W.p + (size_t)hf * n * 16;
+            k_fill_lower_from_upper(Wh);
+        }
+        return true;
+    }
     int nb = 0;
     for (int c : {8, 4, 2})
         if (n % c == 0 && n / c >= 128) {
@@ -611,8 +621,8 @@ void eval_direction(OmmCall& c, const DView& Dir, double coeff[5]) {
         const int* de = (s.de_ok && s.de_src == Dir.p) ? s.De.as<int>() : nullptr;
         const int* xe = s.xr_ok ? s.Xe_r.as<int>() : nullptr;
         s.de_ok = s.xr_ok = false;
-        oz_prepare(Dir, false, n, m, OZ_NMOD, bits, *od, false, -1, de);
-        oz_prepare(X, false, 2 * n, m, OZ_NMOD, bits, *oa, false, -1, xe);
+        oz_prepare(Dir, false, n, m, OZ_NMOD, bits, *od, false, de);
+        oz_prepare(X, false, 2 * n, m, OZ_NMOD, bits, *oa, false, xe);
         oz_gemm(*oa, *od, 1.0, 0.0, Wd);                   // [HWd; SWd] = [HC; SC] Dir^T
         // [HG; SG] = Dir [H, S] on the FP64 tensor cores: 1.89 ms at lattice_8x8x8.  The int8 SpMM
         // (omm_gpu_spmm_f64) takes 1.71 + 0.25 ms for its reconstructions and 0.07 for the k-blocked
@@ -866,6 +876,11 @@ void density_product(const DView& C, const DView& CD, DView& D) {
         // FP64-accurate D = C^T CD on the int8 tensor cores: only the tiles reaching the upper
         // triangle, then the mirror
         gemm_f64_emu('t', 'n', m, m, n, 1.0, C, CD, 0.0, D, m);
+        k_fill_lower_from_upper(D);
+        return;
+    }
+    if (!C.is_real && fp64_emu_enabled() && fp64_emu_worth(m, m, n)) {
+        gemm_z_emu('c', 'n', m, m, n, 1.0, C, CD, 0.0, D, m);
         k_fill_lower_from_upper(D);
         return;
     }

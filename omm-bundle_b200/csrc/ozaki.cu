@@ -133,52 +133,96 @@ struct ModB {
 };
 
 // ------------------------------------------------------------------ row exponents
-// rows contiguous in the source (element (r, k) at A[r + k lda]): one thread per row over a
-// 256-column slab, combined across slabs with atomicMax; the loads go out 16 at a time so that
-// enough bytes are in flight to cover the memory latency
-__global__ void __launch_bounds__(256) oz_exp_rows_kernel(int R, int K, const double* __restrict__ A, int rs,
-                                                          int lda, int* __restrict__ e) {
+// rows contiguous in the source (element (r, k) at A[r + k lda]): one thread per row over a slab of
+// columns, combined across slabs with atomicMax into e (preset to ZERO_EXP); the loads go out 16 at a
+// time so that enough bytes are in flight to cover the memory latency.  The slab's width is chosen so
+// that the grid has some 600 CTAs: with 256 columns throughout, 512 x 4,096 complex was 32 CTAs and
+// took 27 us per part.  Complex sources: a row's real part in e[r], its imaginary part in e[rim + r],
+// from one read of both.
+template <bool CPLX>
+__global__ void __launch_bounds__(256) oz_exp_rows_kernel(int R, int K, const double* __restrict__ A, long long lda,
+                                                          int* __restrict__ e, int rim, int slab) {
+    constexpr int U = CPLX ? 8 : 16;
     const int r = blockIdx.x * 256 + threadIdx.x;
-    const int k0 = blockIdx.y * 256, k1 = min(K, k0 + 256);
+    const int k0 = blockIdx.y * slab, k1 = min(K, k0 + slab);
     if (r >= R) return;
-    double mx = 0.0;
-    bool bad = false;
-    for (int kb = k0; kb < k1; kb += 16) {
-        double v[16];
+    double mx[2] = {0.0, 0.0};
+    bool bad[2] = {false, false};
+    auto take = [&](double v, int q) {
+        const double a = fabs(v);
+        bad[q] |= !(a <= 1.7976931348623157e308);
+        mx[q] = fmax(mx[q], a);
+    };
+    for (int kb = k0; kb < k1; kb += U) {
+        double2 v[U];
 #pragma unroll
-        for (int u = 0; u < 16; ++u) {
+        for (int u = 0; u < U; ++u) {
             const int k = kb + u;
-            v[u] = k < k1 ? A[(size_t)r * rs + (size_t)k * lda] : 0.0;
+            v[u] = make_double2(0.0, 0.0);
+            if (k < k1) {
+                if constexpr (CPLX) v[u] = reinterpret_cast<const double2*>(A)[(size_t)r + (size_t)k * lda];
+                else v[u].x = A[(size_t)r + (size_t)k * lda];
+            }
         }
 #pragma unroll
-        for (int u = 0; u < 16; ++u) {
-            const double a = fabs(v[u]);
-            bad |= !(a <= 1.7976931348623157e308);
-            mx = fmax(mx, a);
+        for (int u = 0; u < U; ++u) {
+            take(v[u].x, 0);
+            if constexpr (CPLX) take(v[u].y, 1);
         }
     }
-    if (bad) atomicMax(&e[r], BAD_EXP);
-    else if (mx > 0.0) atomicMax(&e[r], ilogb(mx));
+#pragma unroll
+    for (int q = 0; q < (CPLX ? 2 : 1); ++q) {
+        if (bad[q]) atomicMax(&e[r + q * rim], BAD_EXP);
+        else if (mx[q] > 0.0) atomicMax(&e[r + q * rim], ilogb(mx[q]));
+    }
 }
 
-// K contiguous in the source (element (r, k) at A[k + r lda]): one warp per row
-__global__ void __launch_bounds__(256) oz_exp_kc_kernel(int R, int K, const double* __restrict__ A, int rs, int lda,
-                                                        int* __restrict__ e) {
+// K contiguous in the source (element (r, k) at A[k + r lda]): a warp per row and slab of K, eight
+// loads of a lane in flight (one at a time took 18 us for 1,001 x 2,003), combined with atomicMax into
+// e (preset to ZERO_EXP).  Complex sources as above.
+template <bool CPLX>
+__global__ void __launch_bounds__(256) oz_exp_kc_kernel(int R, int K, const double* __restrict__ A, long long lda,
+                                                        int* __restrict__ e, int rim, int slab) {
+    constexpr int U = 8;
     const int r = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (r >= R) return;
-    const double* a = A + (size_t)r * lda;
-    double mx = 0.0;
-    bool bad = false;
-    for (int k = lane; k < K; k += 32) {
-        const double v = fabs(a[(size_t)k * rs]);
-        bad |= !(v <= 1.7976931348623157e308);
-        mx = fmax(mx, v);
+    const int k0 = blockIdx.y * slab, k1 = min(K, k0 + slab);
+    const double* a = A + (size_t)r * lda * (CPLX ? 2 : 1);
+    double mx[2] = {0.0, 0.0};
+    int bad[2] = {0, 0};
+    auto take = [&](double x, int q) {
+        const double v = fabs(x);
+        bad[q] |= !(v <= 1.7976931348623157e308);
+        mx[q] = fmax(mx[q], v);
+    };
+    for (int kb = k0 + lane; kb < k1; kb += 32 * U) {
+        double2 v[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int k = kb + 32 * u;
+            v[u] = make_double2(0.0, 0.0);
+            if (k < k1) {
+                if constexpr (CPLX) v[u] = reinterpret_cast<const double2*>(a)[k];
+                else v[u].x = a[k];
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            take(v[u].x, 0);
+            if constexpr (CPLX) take(v[u].y, 1);
+        }
     }
-    for (int o = 16; o > 0; o >>= 1) {
-        mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-        bad |= __shfl_xor_sync(0xffffffffu, (int)bad, o) != 0;
+#pragma unroll
+    for (int q = 0; q < (CPLX ? 2 : 1); ++q) {
+        for (int o = 16; o > 0; o >>= 1) {
+            mx[q] = fmax(mx[q], __shfl_xor_sync(0xffffffffu, mx[q], o));
+            bad[q] |= __shfl_xor_sync(0xffffffffu, bad[q], o);
+        }
+        if (lane == 0) {
+            if (bad[q]) atomicMax(&e[r + q * rim], BAD_EXP);
+            else if (mx[q] > 0.0) atomicMax(&e[r + q * rim], ilogb(mx[q]));
+        }
     }
-    if (lane == 0) e[r] = bad ? BAD_EXP : (mx > 0.0 ? ilogb(mx) : ZERO_EXP);
 }
 
 // y = beta y + alpha x over R x K (rows contiguous: element (r, k) at y[r + k ldy], x likewise;
@@ -331,98 +375,136 @@ __device__ __forceinline__ void oz_store_planes_b(uint32_t* dst, size_t plane_wo
 constexpr int RT_ROWS = 32, RT_K = 128, RT_LD = RT_K + RT_K / 4 + 1;  // 161
 // The k-blocked copy (the int8 SpMM's A operand): plane l at kb + l kb_plane holds, per block of
 // 256 rows, its nch16 chunks of 16 k, each 256 rows x 16 B.
-template <bool KB>
-__global__ void __launch_bounds__(256) oz_res_rows_kernel(int R, int K, const double* __restrict__ A, int rs, int lda,
-                                                          const int* __restrict__ e, int bits, int8_t* __restrict__ out,
-                                                          int ldk, size_t plane, const __grid_constant__ ModB mb,
-                                                          uint8_t* __restrict__ kb, size_t kb_plane, int nch16,
-                                                          int kbh) {
+// Complex sources (CPLX; never with KB): the imaginary part's tile follows the real one's from the same
+// loads, into the plane rows rim + r.
+template <bool KB, bool CPLX>
+__global__ void __launch_bounds__(256) oz_res_rows_kernel(int R, int K, const double* __restrict__ A, long long lda,
+                                                          const int* __restrict__ e, int rim, int bits,
+                                                          int8_t* __restrict__ out, int ldk, size_t plane,
+                                                          const __grid_constant__ ModB mb, uint8_t* __restrict__ kb,
+                                                          size_t kb_plane, int nch16, int kbh) {
     __shared__ long long tile[RT_ROWS * RT_LD];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int r0 = blockIdx.x * RT_ROWS, k0 = blockIdx.y * RT_K;
+    double v[16], vi[CPLX ? 16 : 1];
     {
         const int r = r0 + lane;
-        double v[16];
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
             const int k = k0 + 16 * warp + j;
-            v[j] = (r < R && k < K) ? A[(size_t)r * rs + (size_t)k * lda] : 0.0;
-        }
-        double f1 = 0.0, f2 = 0.0;
-        if (r < R) oz_scales(e[r], bits, f1, f2);
-#pragma unroll
-        for (int j = 0; j < 16; ++j) {
-            const int kk = 16 * warp + j;
-            tile[lane * RT_LD + kk + kk / 4] = __double2ll_rn(oz_integer(v[j], f1, f2)) + (1ll << 53);
+            const bool in = r < R && k < K;
+            if constexpr (CPLX) {
+                const double2 z = in ? reinterpret_cast<const double2*>(A)[(size_t)r + (size_t)k * lda]
+                                     : make_double2(0.0, 0.0);
+                v[j] = z.x;
+                vi[j] = z.y;
+            } else {
+                v[j] = in ? A[(size_t)r + (size_t)k * lda] : 0.0;
+            }
         }
     }
-    __syncthreads();
     const int kk = KB ? 64 * (warp & 1) + 4 * (lane & 15) : 4 * lane, k = k0 + kk;
-    if (k >= ldk) return;  // past the padded row (ldk is a multiple of 16)
-#pragma unroll 1
-    for (int i = 0; i < 4; ++i) {
-        const int rr = KB ? 8 * (warp >> 1) + (lane >> 4) + 2 * i : 4 * warp + i, r = r0 + rr;
-        if (r >= R) break;
-        uint32_t lo[4], hi[4];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const unsigned long long v = (unsigned long long)tile[rr * RT_LD + kk + kk / 4 + u];
-            lo[u] = (uint32_t)v;
-            hi[u] = (uint32_t)(v >> 32);
+    for (int part = 0; part < (CPLX ? 2 : 1); ++part) {
+        const int roff = part * rim;
+        {
+            const int r = r0 + lane;
+            double f1 = 0.0, f2 = 0.0;
+            if (r < R) oz_scales(e[roff + r], bits, f1, f2);
+            if (part) __syncthreads();  // the real part's tile has been read
+#pragma unroll
+            for (int j = 0; j < 16; ++j) {
+                const int q = 16 * warp + j;
+                tile[lane * RT_LD + q + q / 4] = __double2ll_rn(oz_integer(part ? vi[CPLX ? j : 0] : v[j], f1, f2)) + (1ll << 53);
+            }
         }
-        uint32_t* dst = reinterpret_cast<uint32_t*>(out + (size_t)r * ldk + k);
-        // chunk (k / 16) of the 256-row block r / 256: 256 rows x 16 B, or (kbh, the SM-pair form's
-        // half-major layout) per 128-row half of the block its chunks of 128 rows x 16 B
-        const size_t kbo = kbh ? ((((size_t)(r / 256) * 2 + (r % 256) / 128) * nch16 + (k >> 4)) * 128 + (r % 128)) * 16
-                               : (((size_t)(r / 256) * nch16 + (k >> 4)) * 256 + (r % 256)) * 16;
-        uint32_t* d2 = KB ? reinterpret_cast<uint32_t*>(kb + kbo + (k & 15)) : nullptr;
-        oz_store_planes_b(dst, plane / 4, d2, kb_plane / 4, lo, hi, mb);
+        __syncthreads();
+        if (k >= ldk) continue;  // past the padded row (ldk is a multiple of 16)
+#pragma unroll 1
+        for (int i = 0; i < 4; ++i) {
+            const int rr = KB ? 8 * (warp >> 1) + (lane >> 4) + 2 * i : 4 * warp + i, r = r0 + rr;
+            if (r >= R) break;
+            uint32_t lo[4], hi[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const unsigned long long x = (unsigned long long)tile[rr * RT_LD + kk + kk / 4 + u];
+                lo[u] = (uint32_t)x;
+                hi[u] = (uint32_t)(x >> 32);
+            }
+            uint32_t* dst = reinterpret_cast<uint32_t*>(out + (size_t)(roff + r) * ldk + k);
+            // chunk (k / 16) of the 256-row block r / 256: 256 rows x 16 B, or (kbh, the SM-pair form's
+            // half-major layout) per 128-row half of the block its chunks of 128 rows x 16 B
+            const size_t kbo =
+                kbh ? ((((size_t)(r / 256) * 2 + (r % 256) / 128) * nch16 + (k >> 4)) * 128 + (r % 128)) * 16
+                    : (((size_t)(r / 256) * nch16 + (k >> 4)) * 256 + (r % 256)) * 16;
+            uint32_t* d2 = KB ? reinterpret_cast<uint32_t*>(kb + kbo + (k & 15)) : nullptr;
+            oz_store_planes_b(dst, plane / 4, d2, kb_plane / 4, lo, hi, mb);
+        }
     }
 }
 
 // K contiguous in the source (element (r, k) at A[k + r lda]): warp w of a CTA takes row
-// 8 blockIdx.x + w, lane j the k 4 j .. 4 j + 3 of each 128-k slab of the CTA's 512
-__global__ void __launch_bounds__(256) oz_res_kc_kernel(int R, int K, const double* __restrict__ A, int rs, int lda,
-                                                        const int* __restrict__ e, int bits, int8_t* __restrict__ out,
-                                                        int ldk, size_t plane, const __grid_constant__ ModB mb) {
+// 8 blockIdx.x + w, lane j the k 4 j .. 4 j + 3 of each 128-k slab of the CTA's 512 (256 for complex
+// sources, both parts from one read; the imaginary part's planes in rows rim + r)
+template <bool CPLX>
+__global__ void __launch_bounds__(256) oz_res_kc_kernel(int R, int K, const double* __restrict__ A, long long lda,
+                                                        const int* __restrict__ e, int rim, int bits,
+                                                        int8_t* __restrict__ out, int ldk, size_t plane,
+                                                        const __grid_constant__ ModB mb) {
+    constexpr int NS = CPLX ? 2 : 4, NP = CPLX ? 2 : 1;
     const int r = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (r >= R) return;
-    double f1, f2;
-    oz_scales(e[r], bits, f1, f2);
-    const double* a = A + (size_t)r * lda;
-    const int kb = blockIdx.y * 512 + 4 * lane;
-    // all sixteen loads first (four slabs of 128 k), then the residues slab by slab; a lane's four
-    // consecutive k are two 16-byte loads where the row is contiguous and 16-byte aligned
-    double v[4][4];
-    const bool vec = rs == 1 && ((reinterpret_cast<uintptr_t>(a) & 15) == 0);
+    const double* a = A + (size_t)r * lda * NP;
+    const int kb = blockIdx.y * (128 * NS) + 4 * lane;
+    // all loads first, then the residues slab by slab; a lane's four consecutive k are 16-byte loads
+    // where the row is 16-byte aligned (complex rows always are)
+    double v[NP][NS][4];
+    const bool vec = (reinterpret_cast<uintptr_t>(a) & 15) == 0;
 #pragma unroll
-    for (int s = 0; s < 4; ++s) {
+    for (int s = 0; s < NS; ++s) {
         const int k = kb + 128 * s;
-        if (vec && k + 3 < K) {
+        if constexpr (CPLX) {
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                double2 z = make_double2(0.0, 0.0);
+                if (k + u < K) {
+                    if (vec) z = reinterpret_cast<const double2*>(a)[k + u];
+                    else z = make_double2(a[2 * (size_t)(k + u)], a[2 * (size_t)(k + u) + 1]);
+                }
+                v[0][s][u] = z.x;
+                v[NP - 1][s][u] = z.y;
+            }
+        } else if (vec && k + 3 < K) {
             const double2 x0 = *reinterpret_cast<const double2*>(a + k);
             const double2 x1 = *reinterpret_cast<const double2*>(a + k + 2);
-            v[s][0] = x0.x;
-            v[s][1] = x0.y;
-            v[s][2] = x1.x;
-            v[s][3] = x1.y;
+            v[0][s][0] = x0.x;
+            v[0][s][1] = x0.y;
+            v[0][s][2] = x1.x;
+            v[0][s][3] = x1.y;
         } else {
 #pragma unroll
-            for (int u = 0; u < 4; ++u) v[s][u] = k + u < K ? a[(size_t)(k + u) * rs] : 0.0;
+            for (int u = 0; u < 4; ++u) v[0][s][u] = k + u < K ? a[k + u] : 0.0;
         }
     }
 #pragma unroll
-    for (int s = 0; s < 4; ++s) {
-        const int k = kb + 128 * s;
-        if (k >= ldk) break;
-        uint32_t lo[4], hi[4];
+    for (int part = 0; part < NP; ++part) {
+        double f1, f2;
+        oz_scales(e[part * rim + r], bits, f1, f2);
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const unsigned long long x = (unsigned long long)(__double2ll_rn(oz_integer(v[s][u], f1, f2)) + (1ll << 53));
-            lo[u] = (uint32_t)x;
-            hi[u] = (uint32_t)(x >> 32);
+        for (int s = 0; s < NS; ++s) {
+            const int k = kb + 128 * s;
+            if (k >= ldk) break;
+            uint32_t lo[4], hi[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const unsigned long long x =
+                    (unsigned long long)(__double2ll_rn(oz_integer(v[part][s][u], f1, f2)) + (1ll << 53));
+                lo[u] = (uint32_t)x;
+                hi[u] = (uint32_t)(x >> 32);
+            }
+            uint32_t* dst = reinterpret_cast<uint32_t*>(out + (size_t)(part * rim + r) * ldk + k);
+            oz_store_planes_b(dst, plane / 4, nullptr, 0, lo, hi, mb);
         }
-        uint32_t* dst = reinterpret_cast<uint32_t*>(out + (size_t)r * ldk + k);
-        oz_store_planes_b(dst, plane / 4, nullptr, 0, lo, hi, mb);
     }
 }
 
@@ -435,7 +517,7 @@ constexpr int B_BYTES = BN * BK;                         // 32 KB
 constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
 constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 + 256;
 constexpr uint32_t TMEM_COLS = 512;  // two 256-column accumulators
-constexpr int GEMM_THREADS = 192;   // warp 0 copies, warp 1 MMAs and TMEM, warps 2-5 epilogue
+constexpr int GEMM_THREADS = 320;   // warp 0 copies, warp 1 MMAs and TMEM, warps 2-9 epilogue
 // kind::i8: s32 accumulator (dtype 2), s8 A and B (1), K-major both, N = 256, M = 128
 constexpr uint32_t IDESC_I8 = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
 
@@ -443,10 +525,12 @@ struct GemmParams {
     int M, N, K, nmod;
     int p[MAXMOD];
     uint32_t magic[MAXMOD];  // ceil(2^39 / p): u / p = umulhi(u, magic) >> 7, at most one too high
-    uint32_t off[MAXMOD];    // a multiple of p >= 2^31: a + off is non-negative for any int32 a
+    uint32_t off[MAXMOD];    // a multiple of p >= 2^31 (exact: 2^27): a + off is non-negative for any accumulator a
+    int exact;               // |accumulator| < 2^27: u = a + off < 2^28, whose quotient is not too high
     uint8_t* R;  // residue planes of the product: (i, j) of plane l at R[l rplane + i + j ldr]
     size_t rplane;
     int ldr;
+    int bn;             // columns of a tile (SM pairs: a multiple of 32 up to 256; single SMs: 256)
     int b_row0;         // first row of the B operand this launch reads (column panels)
     const int2* tiles;  // (m0, n0) of the output tiles to form (tiles below a Hermitian block's
     int ntiles;         // diagonal are left out); work item w = tile w % ntiles, modulus w / ntiles
@@ -481,12 +565,61 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 
+// 32 columns of an accumulator row per lane, reduced mod p (to [0, p), integer operations only) and
+// stored to a residue plane: column c of the warp's 32 rows at R + c ldr.  The bytes of four columns are
+// packed into a word, the words of four neighbouring lanes transposed (4 x 4 bytes, two exchanges), and
+// each lane stores four rows of one column, so that a store instruction covers four whole sectors.  One
+// byte store per column -- 32 instructions of one sector each, by four warps -- held an item's epilogue
+// to 1.7 residues per clock and SM, longer than its MMAs for K below about 4,700: 8,192 x 8,192 x 512
+// 2.29 -> 0.78 ms (0.65 on single SMs), 648 x 5,184 x 1,296 162 -> 97 us, 1,001 x 515 x 2,003 44 -> 29 us.
+// EXACT: |accumulator| < 2^27 (K < 8,192), where the multiply gives the quotient itself (oz_residue) and
+// the correction step falls away.
+template <bool EXACT>
+__device__ __forceinline__ void oz_store_residues(const uint32_t (&v)[32], int lane, int p, uint32_t magic, uint32_t off,
+                                                  uint8_t* R, int ldr, int cols) {
+    const uint32_t selA = (lane & 1) ? 0x3715u : 0x6240u, selB = (lane & 2) ? 0x3276u : 0x5410u;
+    uint8_t* dst = R + (size_t)(lane & 3) * ldr + (lane & ~3);
+    int left = cols - (lane & 3);  // columns from this lane's first on
+#pragma unroll
+    for (int t = 0; t < 8; ++t) {
+        uint32_t r[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const uint32_t u = v[4 * t + q] + off;
+            int x = (int)(u - (__umulhi(u, magic) >> 7) * (uint32_t)p);
+            if (!EXACT && x < 0) x += p;  // the quotient was one too high
+            r[q] = (uint32_t)x;
+        }
+        const uint32_t w = __byte_perm(__byte_perm(r[0], r[1], 0x0040), __byte_perm(r[2], r[3], 0x0040), 0x5410);
+        const uint32_t a = __byte_perm(w, __shfl_xor_sync(0xffffffffu, w, 1), selA);
+        const uint32_t b = __byte_perm(a, __shfl_xor_sync(0xffffffffu, a, 2), selB);
+        if (left > 0) *reinterpret_cast<uint32_t*>(dst) = b;
+        left -= 4;
+        dst += 4 * (size_t)ldr;
+    }
+}
+// one item's columns c0 = cfirst, cfirst + 64, ... below bn, from the TMEM columns at acc (the warp's lanes)
+template <bool EXACT>
+__device__ __forceinline__ void oz_epilogue_item(const GemmParams& p, uint32_t acc, int cfirst, int bn, int lane, int l,
+                                                 int row0, int col0) {
+    uint8_t* R = p.R + (size_t)l * p.rplane + row0 + (size_t)col0 * p.ldr;
+    const int pm = p.p[l];
+    const uint32_t magic = p.magic[l], off = p.off[l];
+#pragma unroll 1
+    for (int c0 = cfirst; c0 < bn; c0 += 64) {
+        uint32_t v[32];
+        tmem_ld32(acc + (uint32_t)c0, v);
+        if (row0 < p.ldr)
+            oz_store_residues<EXACT>(v, lane, pm, magic, off, R + (size_t)c0 * p.ldr, p.ldr, p.N - col0 - c0);
+    }
+}
+
 // Persistent: each CTA walks the work items blockIdx.x, blockIdx.x + gridDim.x, ... (an item is one
 // 128 x 256 output tile modulo one p_l; items are modulus-major, so the CTAs running at the same
 // time share one modulus' residue planes in L2).  Warp 0 lane 0 issues the TMA loads of 128-byte K
 // slabs of both operands into a 4-stage ring, continuing from one item straight into the next;
 // warp 1 lane 0 issues the M128 N256 K32 int8 MMAs (4 per slab) into one of two TMEM accumulators,
-// alternating per item, so that warps 2-5 reduce the previous item's accumulator mod p to bytes
+// alternating per item, so that warps 2-9 reduce the previous item's accumulator mod p to bytes
 // (each thread one row, 32 columns at a time) while the next item's MMAs run.
 __global__ void __launch_bounds__(GEMM_THREADS, 1) oz_gemm_kernel(const __grid_constant__ CUtensorMap tA,
                                                                   const __grid_constant__ CUtensorMap tB,
@@ -515,7 +648,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) oz_gemm_kernel(const __grid_c
         }
         for (int b = 0; b < 2; ++b) {
             mbar_init(smem_u32(&accf[b]), 1);
-            mbar_init(smem_u32(&acce[b]), 4);  // one arrival per epilogue warp
+            mbar_init(smem_u32(&acce[b]), 8);  // one arrival per epilogue warp
         }
         mbar_init(smem_u32(doneb), 1);
         *abort_flag = 0;
@@ -534,9 +667,11 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) oz_gemm_kernel(const __grid_c
             // ---------------- TMA producer (issues nothing under the withholding test switch)
             int it = 0;
             bool stop = false;
+            int2 next = p.tiles[blockIdx.x % p.ntiles];  // an item's tile is fetched during the one before
             for (int w = blockIdx.x; w < items && !stop && !p.wc.withhold; w += gridDim.x) {
-                const int2 t = p.tiles[w % p.ntiles];
+                const int2 t = next;
                 const int l = w / p.ntiles;
+                next = p.tiles[(w + gridDim.x) % p.ntiles];
                 for (int kt = 0; kt < KT; ++kt, ++it) {
                     const int s = it % STAGES, r = it / STAGES;
                     if (r > 0 && !mbar_wait(smem_u32(&empty[s]), (r - 1) & 1, p.wc.ns)) {
@@ -599,11 +734,14 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) oz_gemm_kernel(const __grid_c
             mma_commit(smem_u32(doneb));  // arrives once every MMA issued above has completed
         }
     } else {
-        // ---------------- epilogue: warp w reads TMEM lanes 32 (w % 4) .. + 31, one row per thread
-        const int quarter = warp & 3;
+        // ---------------- epilogue: warp w reads TMEM lanes 32 (w % 4) .. + 31, one row per thread; the two
+        // warps of a quarter take every second block of 32 columns
+        const int quarter = warp & 3, cfirst = 32 * ((warp - 2) >> 2);
         int tc = 0;
         for (int w = blockIdx.x; w < items; w += gridDim.x, ++tc) {
             const int b = tc & 1, use = tc >> 1;
+            const int2 t = p.tiles[w % p.ntiles];
+            const int l = w / p.ntiles;
             const bool ok = mbar_wait(smem_u32(&accf[b]), use & 1, p.wc.ns);
             if (!ok) atomicOr(p.err, 2048u);
             if (!__all_sync(0xffffffffu, ok && !*abort_flag)) {
@@ -611,30 +749,9 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) oz_gemm_kernel(const __grid_c
                 break;
             }
             fence_after();
-            const int2 t = p.tiles[w % p.ntiles];
-            const int l = w / p.ntiles;
-            const int row = t.x + quarter * 32 + lane;
-            const int pm = p.p[l];
-            const uint32_t mg = p.magic[l], off = p.off[l];
-            uint8_t* R = p.R + (size_t)l * p.rplane + row;
-#pragma unroll 1
-            for (int c0 = 0; c0 < BN; c0 += 32) {
-                uint32_t v[32];
-                tmem_ld32(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(b * BN + c0), v);
-                if (row < p.M) {
-#pragma unroll
-                    for (int q = 0; q < 32; ++q) {
-                        const int col = t.y + c0 + q;
-                        if (col < p.N) {
-                            // (int32 accumulator) mod p in [0, p), integer operations only
-                            const uint32_t u = v[q] + off;
-                            int r = (int)(u - (__umulhi(u, mg) >> 7) * (uint32_t)pm);
-                            if (r < 0) r += pm;
-                            R[(size_t)col * p.ldr] = (uint8_t)r;
-                        }
-                    }
-                }
-            }
+            const uint32_t acc = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(b * BN);
+            if (p.exact) oz_epilogue_item<true>(p, acc, cfirst, BN, lane, l, t.x + quarter * 32, t.y);
+            else oz_epilogue_item<false>(p, acc, cfirst, BN, lane, l, t.x + quarter * 32, t.y);
             fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(smem_u32(&acce[b]));
@@ -653,27 +770,29 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) oz_gemm_kernel(const __grid_c
 // ---- the same GEMM on SM pairs: a cluster of two CTAs forms 256 x 256 tiles with M256 N256 K32
 // MMAs (cta_group::2).  Each CTA stages its own 128 rows of A and 128 rows of B per slab (32 KB, so
 // six stages fit), which halves the B bytes each SM loads per MMA against the one-CTA kernel; the
-// accumulator of CTA r holds rows 128 r .. 128 r + 127 of the tile, all 256 columns.
+// accumulator of CTA r holds rows 128 r .. 128 r + 127 of the tile, all its columns.  The tile's width
+// is a launch parameter (oz_tile_width): a product of few tiles takes the width whose last wave over the
+// 74 pairs is fullest (1,001 x 515 x 2,003: 224 columns).
 //   rank 0 (leader) warp 1 lane 0: waits for both CTAs' slabs on its full[s] (which counts the
 //       copies of both), issues the MMAs, and commits to empty[s] / accf[b] / doneb of BOTH CTAs
 //   both CTAs warp 0 lane 0: wait on their own empty[s], copy their half of the slab; the
 //       completion goes to the leader's full[s] (the leader also posts the expected bytes)
-//   both CTAs warps 2-5: epilogue of their own TMEM rows, then arrive on the leader's acce[b]
-//       (8 arrivals: four warps in each CTA)
+//   both CTAs warps 2-9: epilogue of their own TMEM rows, then arrive on the leader's acce[b]
+//       (16 arrivals: eight warps in each CTA)
 // Every wait is bounded as in the one-CTA kernel; both CTAs meet at a cluster barrier before TMEM
 // is freed, so neither leaves while the other can still touch its shared memory.
 constexpr int BM2 = 256, BN2 = 256, STAGES2 = 6;
 constexpr int A2_BYTES = 128 * BK, B2_BYTES = 128 * BK;  // each CTA's half of a slab: 16 KB + 16 KB
 constexpr int STAGE2_BYTES = A2_BYTES + B2_BYTES;
 constexpr int SMEM2_BYTES = STAGES2 * STAGE2_BYTES + 1024 + 256;
-constexpr uint32_t IDESC_I8_PAIR =
-    (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN2 >> 3) << 17) | ((uint32_t)(BM2 >> 4) << 24);
+constexpr uint32_t IDESC_I8_PAIR =  // without N
+    (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BM2 >> 4) << 24);
 
-__device__ __forceinline__ void mma_i8_pair(uint32_t tmem, uint64_t a, uint64_t b, uint32_t accumulate) {
+__device__ __forceinline__ void mma_i8_pair(uint32_t tmem, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
         "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::2.kind::i8 [%0], %1, %2, %3, p;\n}\n" ::"r"(
             tmem),
-        "l"(a), "l"(b), "r"(IDESC_I8_PAIR), "r"(accumulate)
+        "l"(a), "l"(b), "r"(idesc), "r"(accumulate)
         : "memory");
 }
 
@@ -699,6 +818,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
     const int pair = blockIdx.x >> 1, npairs = gridDim.x >> 1;
     const int KT = (p.K + BK - 1) / BK;
     const int items = p.ntiles * p.nmod;
+    const int bhalf = p.bn / 2;  // rows of B per CTA
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES2; ++s) {
@@ -707,7 +827,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
         }
         for (int b = 0; b < 2; ++b) {
             mbar_init(smem_u32(&accf[b]), 1);
-            mbar_init(smem_u32(&acce[b]), 8);  // four epilogue warps in each CTA
+            mbar_init(smem_u32(&acce[b]), 16);  // eight epilogue warps in each CTA
         }
         mbar_init(smem_u32(doneb), 1);
         *abort_flag = 0;
@@ -727,9 +847,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
             const uint32_t lead_full0 = peer_addr(smem_u32(&full[0]), 0);
             int it = 0;
             bool stop = false;
+            int2 next = p.tiles[pair % p.ntiles];  // an item's tile is fetched during the one before
             for (int w = pair; w < items && !stop && !p.wc.withhold; w += npairs) {
-                const int2 t = p.tiles[w % p.ntiles];
+                const int2 t = next;
                 const int l = w / p.ntiles;
+                next = p.tiles[(w + npairs) % p.ntiles];
                 for (int kt = 0; kt < KT; ++kt, ++it) {
                     const int s = it % STAGES2, r = it / STAGES2;
                     if (r > 0 && !mbar_wait_cl(smem_u32(&empty[s]), (r - 1) & 1, p.wc.ns)) {
@@ -741,9 +863,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
                         break;
                     }
                     const uint32_t fb = lead_full0 + (uint32_t)(s * sizeof(uint64_t));
-                    if (leader) mbar_expect_tx(smem_u32(&full[s]), 2 * STAGE2_BYTES);
+                    if (leader) mbar_expect_tx(smem_u32(&full[s]), 2 * (A2_BYTES + bhalf * BK));
                     tma_load_3d_pair(smem_u32(sA + s * A2_BYTES), &tA, kt * BK, t.x + 128 * (int)rank, l, fb);
-                    tma_load_3d_pair(smem_u32(sB + s * B2_BYTES), &tB, kt * BK, p.b_row0 + t.y + 128 * (int)rank, l,
+                    tma_load_3d_pair(smem_u32(sB + s * B2_BYTES), &tB, kt * BK, p.b_row0 + t.y + bhalf * (int)rank, l,
                                      fb);
                 }
             }
@@ -763,6 +885,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
             // ---------------- MMA issuer (leader only)
             int it = 0, tc = 0;
             bool stop = false;
+            const uint32_t idesc = IDESC_I8_PAIR | ((uint32_t)(p.bn >> 3) << 17);
             for (int w = pair; w < items && !stop; w += npairs, ++tc) {
                 const int b = tc & 1, use = tc >> 1;
                 if (use > 0 && !mbar_wait_cl(smem_u32(&acce[b]), (use - 1) & 1, p.wc.ns)) {
@@ -786,7 +909,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
                     const uint32_t a0 = smem_u32(sA + s * A2_BYTES), b0 = smem_u32(sB + s * B2_BYTES);
 #pragma unroll
                     for (int kk = 0; kk < BK / 32; ++kk)
-                        mma_i8_pair(acc, make_desc_sw128(a0 + kk * 32), make_desc_sw128(b0 + kk * 32),
+                        mma_i8_pair(acc, make_desc_sw128(a0 + kk * 32), make_desc_sw128(b0 + kk * 32), idesc,
                                     (kt > 0 || kk > 0) ? 1u : 0u);
                     mma_commit_pair(smem_u32(&empty[s]), 3);
                 }
@@ -796,12 +919,15 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
             mma_commit_pair(smem_u32(doneb), 3);  // arrives in both CTAs once every MMA above completed
         }
     } else {
-        // ---------------- epilogue: this CTA's 128 rows of the tile, one row per thread
-        const int quarter = warp & 3;
+        // ---------------- epilogue: this CTA's 128 rows of the tile, one row per thread; the two warps of a
+        // quarter take every second block of 32 columns
+        const int quarter = warp & 3, cfirst = 32 * ((warp - 2) >> 2);
         const uint32_t lead_acce0 = peer_addr(smem_u32(&acce[0]), 0);
         int tc = 0;
         for (int w = pair; w < items; w += npairs, ++tc) {
             const int b = tc & 1, use = tc >> 1;
+            const int2 t = p.tiles[w % p.ntiles];
+            const int l = w / p.ntiles;
             const bool ok = mbar_wait_cl(smem_u32(&accf[b]), use & 1, p.wc.ns);
             if (!ok) atomicOr(p.err, 2048u);
             if (!__all_sync(0xffffffffu, ok && !*abort_flag)) {
@@ -809,29 +935,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
                 break;
             }
             fence_after();
-            const int2 t = p.tiles[w % p.ntiles];
-            const int l = w / p.ntiles;
-            const int row = t.x + 128 * (int)rank + quarter * 32 + lane;
-            const int pm = p.p[l];
-            const uint32_t mg = p.magic[l], off = p.off[l];
-            uint8_t* R = p.R + (size_t)l * p.rplane + row;
-#pragma unroll 1
-            for (int c0 = 0; c0 < BN2; c0 += 32) {
-                uint32_t v[32];
-                tmem_ld32(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(b * BN2 + c0), v);
-                if (row < p.M) {
-#pragma unroll
-                    for (int q = 0; q < 32; ++q) {
-                        const int col = t.y + c0 + q;
-                        if (col < p.N) {
-                            const uint32_t u = v[q] + off;
-                            int r = (int)(u - (__umulhi(u, mg) >> 7) * (uint32_t)pm);
-                            if (r < 0) r += pm;
-                            R[(size_t)col * p.ldr] = (uint8_t)r;
-                        }
-                    }
-                }
-            }
+            const uint32_t acc = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(b * BN2);
+            const int row0 = t.x + 128 * (int)rank + quarter * 32;
+            if (p.exact) oz_epilogue_item<true>(p, acc, cfirst, p.bn, lane, l, row0, t.y);
+            else oz_epilogue_item<false>(p, acc, cfirst, p.bn, lane, l, row0, t.y);
             fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive_cl(lead_acce0 + (uint32_t)(b * sizeof(uint64_t)));
@@ -866,9 +973,14 @@ struct RecParams {
     const int* eB;
     int shift;  // (bitsA - 1) + (bitsB - 1)
     double alpha, beta;
-    double* out;  // out(i, j) at out[i os + j ldo]: os = 1, or 2 for a part of a complex matrix
-    int ldo, os;
+    double* out;  // out(i, j) at out[i + j ldo] (complex: element i + j ldo of (re, im) pairs)
+    int ldo;
     int herm, n_off;
+    // complex products: the imaginary rows of A are zrow below the real ones, the imaginary columns of B
+    // zcol to the right; Re C = a_rr RR + a_ii II, Im C = a_ri RI + a_ir IR (+ beta C)
+    int zrow, zcol;
+    const int* eBi;
+    double a_rr, a_ii, a_ri, a_ir;
     uint32_t W[MAXMOD][4];
     float w[MAXMOD];  // W_l / P
     uint32_t P[4];
@@ -935,8 +1047,28 @@ __device__ __forceinline__ void oz_transpose4(uint32_t a, uint32_t b, uint32_t c
     o[3] = __byte_perm(t1, t3, 0x7632);
 }
 
-// thread: rows 4 t .. 4 t + 3 of 8 columns; one 4-byte load per plane gives the four rows'
-// residues (the planes' leading dimension ldr is a multiple of 128)
+// the residues of rows 4 t .. 4 t + 3 of one column (one 4-byte load per plane gives the four rows'; r is
+// a multiple of 4 bytes) as rows[u][g]: row u's residues of the moduli 4 g .. 4 g + 3
+__device__ __forceinline__ void oz_load_rows(const RecParams& p, const uint8_t* r, uint32_t (&rows)[4][MAXMOD / 4]) {
+    uint32_t res[MAXMOD];
+#pragma unroll
+    for (int l = 0; l < MAXMOD; ++l)
+        res[l] = l < p.nmod ? *reinterpret_cast<const uint32_t*>(r + (size_t)l * p.rplane) : 0u;
+#pragma unroll
+    for (int g = 0; g < MAXMOD / 4; ++g) {
+        uint32_t o[4];
+        oz_transpose4(res[4 * g], res[4 * g + 1], res[4 * g + 2], res[4 * g + 3], o);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) rows[u][g] = o[u];
+    }
+}
+// Whether all of rows i0 .. i0 + 3 lie below the diagonal of their Hermitian block at column c: those
+// outputs are mirrored from the upper triangle by the caller, and their tiles may not have been formed
+__device__ __forceinline__ bool oz_rows_below(int i0, int herm, int c) {
+    return herm > 0 && i0 % herm > c && i0 % herm + 3 < herm;
+}
+
+// thread: rows 4 t .. 4 t + 3 of 8 columns
 __global__ void __launch_bounds__(256) oz_reconstruct_kernel(const __grid_constant__ RecParams p) {
     const int i0 = 4 * (blockIdx.x * 256 + threadIdx.x);
     if (i0 >= p.M) return;
@@ -946,25 +1078,67 @@ __global__ void __launch_bounds__(256) oz_reconstruct_kernel(const __grid_consta
     for (int jj = 0; jj < 8; ++jj) {
         const int j = blockIdx.y * 8 + jj;
         if (j >= p.N) return;
-        if (!oz_tile_needed(i0 / BM * BM, BM, p.M, p.herm, ((p.n_off + j) / BN) * BN + BN - 1)) continue;
+        if (oz_rows_below(i0, p.herm, p.n_off + j)) continue;
         const int eb = p.eB[j];
-        const uint8_t* r = p.R + (size_t)i0 + (size_t)j * p.ldr;
-        uint32_t res[MAXMOD];
-#pragma unroll
-        for (int l = 0; l < MAXMOD; ++l)
-            res[l] = l < p.nmod ? *reinterpret_cast<const uint32_t*>(r + (size_t)l * p.rplane) : 0u;
-        uint32_t rows[MAXMOD / 4][4];  // rows[g][u]: row u's residues of moduli 4 g .. 4 g + 3
-#pragma unroll
-        for (int g = 0; g < MAXMOD / 4; ++g) oz_transpose4(res[4 * g], res[4 * g + 1], res[4 * g + 2], res[4 * g + 3], rows[g]);
-        double* o = p.out + (size_t)i0 * p.os + (size_t)j * p.ldo;
+        uint32_t rows[4][MAXMOD / 4];
+        oz_load_rows(p, p.R + (size_t)i0 + (size_t)j * p.ldr, rows);
+        double* o = p.out + (size_t)i0 + (size_t)j * p.ldo;
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
             if (i0 + u >= p.M) break;
-            const uint32_t rp[MAXMOD / 4] = {rows[0][u], rows[1][u], rows[2][u], rows[3][u]};
-            double val = oz_value(p, rp, ea[u], eb) * p.alpha;
-            if (p.beta != 0.0) val = fma(p.beta, o[u * p.os], val);
-            o[u * p.os] = val;
+            double val = oz_value(p, rows[u], ea[u], eb) * p.alpha;
+            if (p.beta != 0.0) val = fma(p.beta, o[u], val);
+            o[u] = val;
         }
+    }
+}
+
+// The same for a complex product: its four real ones (stacked operands, one GEMM) joined in one pass
+// over C, where a pass per real product read and wrote C's parts twice each (512 x 512: 61 us for the
+// four against 15).  thread: rows 4 t .. 4 t + 3 of 2 columns.
+__global__ void __launch_bounds__(128) oz_reconstruct_z_kernel(const __grid_constant__ RecParams p) {
+    const int i0 = 4 * (blockIdx.x * 128 + threadIdx.x);
+    if (i0 >= p.M) return;
+    int ear[4], eai[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        ear[u] = i0 + u < p.M ? p.eA[i0 + u] : ZERO_EXP;
+        eai[u] = i0 + u < p.M ? p.eA[p.zrow + i0 + u] : ZERO_EXP;
+    }
+    for (int jj = 0; jj < 2; ++jj) {
+        const int j = blockIdx.y * 2 + jj;
+        if (j >= p.N) return;
+        if (oz_rows_below(i0, p.herm, p.n_off + j)) continue;
+        const int ebr = p.eB[j], ebi = p.eBi[j];
+        const uint8_t* r0 = p.R + (size_t)i0 + (size_t)j * p.ldr;
+        const uint8_t* r1 = r0 + (size_t)p.zcol * p.ldr;
+        double2* o = reinterpret_cast<double2*>(p.out) + (size_t)i0 + (size_t)j * p.ldo;
+        double re[4], im[4];
+        uint32_t rows[4][MAXMOD / 4];
+        oz_load_rows(p, r0, rows);  // RR
+#pragma unroll
+        for (int u = 0; u < 4; ++u) re[u] = oz_value(p, rows[u], ear[u], ebr) * p.a_rr;
+        oz_load_rows(p, r1, rows);  // RI
+#pragma unroll
+        for (int u = 0; u < 4; ++u) im[u] = oz_value(p, rows[u], ear[u], ebi) * p.a_ri;
+        if (p.beta != 0.0) {
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (i0 + u < p.M) {
+                    const double2 c = o[u];
+                    re[u] = fma(p.beta, c.x, re[u]);
+                    im[u] = fma(p.beta, c.y, im[u]);
+                }
+        }
+        oz_load_rows(p, r1 + p.zrow, rows);  // II
+#pragma unroll
+        for (int u = 0; u < 4; ++u) re[u] += oz_value(p, rows[u], eai[u], ebi) * p.a_ii;
+        oz_load_rows(p, r0 + p.zrow, rows);  // IR
+#pragma unroll
+        for (int u = 0; u < 4; ++u) im[u] += oz_value(p, rows[u], eai[u], ebr) * p.a_ir;
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (i0 + u < p.M) o[u] = make_double2(re[u], im[u]);
     }
 }
 
@@ -1552,66 +1726,76 @@ void oz_axpby_exps(int R, int K, double alpha, const DView& X, double beta, DVie
 }
 
 // residues of one operand (rows x K of A_op, K-major int8 planes) and its row exponents (exps_in:
-// exponents already formed, e.g. by oz_axpby_exps, copied instead of recomputed)
+// exponents already formed, e.g. by oz_axpby_exps, copied instead of recomputed).  A complex source gives
+// stacked operands: the real parts' rows, then (from a multiple of 4 on) the imaginary parts'.
 void oz_prepare(const DView& src, bool kcontig, int rows, int K, int nmod, int bits, OzOperand& op, bool with_kb,
-                int part, const int* exps_in, bool kb_halves) {
+                const int* exps_in, bool kb_halves) {
     using namespace oz;
-    if (with_kb && kcontig) fail(OMM_ERR_ARG, "oz_prepare: k-blocked residues need a row-contiguous source");
-    op.rows = rows;
+    if (with_kb && (kcontig || !src.is_real)) fail(OMM_ERR_ARG, "oz_prepare: k-blocked residues need a real row-contiguous source");
+    const bool cplx = !src.is_real;
+    op.zrow = cplx ? (rows + 3) / 4 * 4 : 0;
+    op.rows = op.zrow + rows;
     op.K = K;
     op.ldk = (K + 15) / 16 * 16;
     op.nmod = nmod;
     op.bits = bits;
-    op.plane = (size_t)op.ldk * rows;
+    op.plane = (size_t)op.ldk * op.rows;
     op.planes.ensure(op.plane * nmod);
     op.kb_plane = with_kb ? (size_t)(rows + 255) / 256 * 256 * op.ldk : 0;
     op.kb_halves = with_kb && kb_halves;
     if (with_kb) op.kb.ensure(op.kb_plane * nmod);
-    op.exps.ensure((size_t)rows * sizeof(int));
+    op.exps.ensure((size_t)op.rows * sizeof(int));
+    if (rows == 0 || K == 0) return;
     cudaStream_t st = rt().stream;
-    // a real matrix, or the real (part 0) / imaginary (part 1) part of a complex one: element
-    // (i, k) at a[i rs + k ld] with rs = 2 and ld twice the complex leading dimension
-    if ((part >= 0) == src.is_real) fail(OMM_ERR_ARG, "oz_prepare: part given for a real source or missing");
-    const double* a = src.as<double>() + (part > 0 ? 1 : 0);
-    const int rs = part >= 0 ? 2 : 1, ld = part >= 0 ? 2 * src.ld : src.ld;
+    const double* a = src.as<double>();
+    const long long ld = src.ld;
     // algorithmic bytes: the FP64 operand read once per pass, the residue planes written once
-    const double src_bytes = 8.0 * rows * (double)K;
+    const double src_bytes = (cplx ? 16.0 : 8.0) * rows * (double)K;
     if (exps_in) {
         OMM_CK(cudaMemcpyAsync(op.exps.p, exps_in, (size_t)rows * sizeof(int), cudaMemcpyDeviceToDevice, st));
     } else {
-        OMM_CK(cudaMemsetAsync(op.exps.p, 0x80, (size_t)rows * sizeof(int), st));
+        OMM_CK(cudaMemsetAsync(op.exps.p, 0x80, (size_t)op.rows * sizeof(int), st));
         ktime_begin();
-        if (kcontig) {
-            oz_exp_kc_kernel<<<(rows + 7) / 8, 256, 0, st>>>(rows, K, a, rs, ld, op.exps.as<int>());
-        } else {
-            dim3 g((rows + 255) / 256, (K + 255) / 256);
-            oz_exp_rows_kernel<<<g, 256, 0, st>>>(rows, K, a, rs, ld, op.exps.as<int>());
-        }
+        // slabs of K so that some 600 CTAs share the rows, at least 32 columns (256 entries of a row)
+        const int rb = kcontig ? (rows + 7) / 8 : (rows + 255) / 256;
+        const int unit = kcontig ? 256 : 32;
+        const int want = std::max(1, 600 / rb);
+        const int slab = std::max(unit, ((K + want - 1) / want + unit - 1) / unit * unit);
+        const dim3 g(rb, std::max(1, (K + slab - 1) / slab));
+        int* e = op.exps.as<int>();
+        if (kcontig && cplx) oz_exp_kc_kernel<true><<<g, 256, 0, st>>>(rows, K, a, ld, e, op.zrow, slab);
+        else if (kcontig) oz_exp_kc_kernel<false><<<g, 256, 0, st>>>(rows, K, a, ld, e, 0, slab);
+        else if (cplx) oz_exp_rows_kernel<true><<<g, 256, 0, st>>>(rows, K, a, ld, e, op.zrow, slab);
+        else oz_exp_rows_kernel<false><<<g, 256, 0, st>>>(rows, K, a, ld, e, 0, slab);
         OMM_KCHECK();
         ktime_end("oz_exp_kernel", src_bytes);
     }
     if (nmod != MAXMOD) fail(OMM_ERR_ARG, "oz_prepare: the residue kernels form all 16 moduli");
     static const ModB mb = mod_b();
     ktime_begin();
+    const int* e = op.exps.as<int>();
+    int8_t* out = op.planes.as<int8_t>();
     if (kcontig) {
-        dim3 g((rows + 7) / 8, (K + 511) / 512);
-        oz_res_kc_kernel<<<g, 256, 0, st>>>(rows, K, a, rs, ld, op.exps.as<int>(), bits, op.planes.as<int8_t>(),
-                                            op.ldk, op.plane, mb);
+        const int per = cplx ? 256 : 512;
+        dim3 g((rows + 7) / 8, (K + per - 1) / per);
+        if (cplx) oz_res_kc_kernel<true><<<g, 256, 0, st>>>(rows, K, a, ld, e, op.zrow, bits, out, op.ldk, op.plane, mb);
+        else oz_res_kc_kernel<false><<<g, 256, 0, st>>>(rows, K, a, ld, e, 0, bits, out, op.ldk, op.plane, mb);
     } else {
         dim3 g((rows + 31) / 32, (K + 127) / 128);
         if (with_kb)
-            oz_res_rows_kernel<true><<<g, 256, 0, st>>>(rows, K, a, rs, ld, op.exps.as<int>(), bits,
-                                                        op.planes.as<int8_t>(), op.ldk, op.plane, mb,
-                                                        op.kb.as<uint8_t>(), op.kb_plane, op.ldk / 16,
-                                                        op.kb_halves ? 1 : 0);
+            oz_res_rows_kernel<true, false><<<g, 256, 0, st>>>(rows, K, a, ld, e, 0, bits, out, op.ldk, op.plane, mb,
+                                                               op.kb.as<uint8_t>(), op.kb_plane, op.ldk / 16,
+                                                               op.kb_halves ? 1 : 0);
+        else if (cplx)
+            oz_res_rows_kernel<false, true><<<g, 256, 0, st>>>(rows, K, a, ld, e, op.zrow, bits, out, op.ldk, op.plane,
+                                                               mb, nullptr, 0, op.ldk / 16, 0);
         else
-            oz_res_rows_kernel<false><<<g, 256, 0, st>>>(rows, K, a, rs, ld, op.exps.as<int>(), bits,
-                                                         op.planes.as<int8_t>(), op.ldk, op.plane, mb, nullptr, 0,
-                                                         op.ldk / 16, 0);
+            oz_res_rows_kernel<false, false><<<g, 256, 0, st>>>(rows, K, a, ld, e, 0, bits, out, op.ldk, op.plane, mb,
+                                                                nullptr, 0, op.ldk / 16, 0);
     }
     OMM_KCHECK();
     ktime_end(kcontig ? "oz_res_kc_kernel" : "oz_res_rows_kernel",
-              src_bytes + (double)nmod * rows * K * (with_kb ? 2.0 : 1.0));
+              src_bytes + (cplx ? 2.0 : 1.0) * nmod * rows * (double)K * (with_kb ? 2.0 : 1.0));
 }
 
 namespace {
@@ -1621,7 +1805,8 @@ size_t g_panel_bytes = (size_t)4 << 30;  // cap on the product's residue planes 
 // output written (and read when beta != 0); a Hermitian product (herm > 0) forms the upper
 // tiles only, about half
 double recon_bytes(const oz::RecParams& rp, int M, int nc) {
-    const double per = rp.nmod + 8.0 + (rp.beta != 0.0 ? 8.0 : 0.0);
+    const double per = (rp.nmod + 8.0 + (rp.beta != 0.0 ? 8.0 : 0.0)) * (rp.zrow > 0 ? 2.0 : 1.0) +
+                       (rp.zrow > 0 ? 2.0 * rp.nmod : 0.0);
     return per * M * (double)nc * (rp.herm > 0 ? 0.5 : 1.0);
 }
 }
@@ -1654,11 +1839,12 @@ void oz_release_scratch() {
 }
 
 // (m0, n0) of the bm x bn tiles of an M x nc panel starting at global column c0 that reach the
-// upper triangle of their Hermitian block (all tiles when herm == 0); kept per shape
-const DevBuf& tile_list(int M, int nc, int herm, int c0, int bm, int bn) {
-    static std::map<std::tuple<int, int, int, int, int, int>, std::unique_ptr<DevBuf>>* cache =
-        new std::map<std::tuple<int, int, int, int, int, int>, std::unique_ptr<DevBuf>>();
-    auto key = std::make_tuple(M, nc, herm, c0, bm, bn);
+// upper triangle of their Hermitian block (all tiles when herm == 0); with hcols > 0 the panel's columns
+// are stacks of hcols columns too (the real and imaginary parts of a complex product).  Kept per shape.
+const DevBuf& tile_list(int M, int nc, int herm, int hcols, int c0, int bm, int bn) {
+    static std::map<std::tuple<int, int, int, int, int, int, int>, std::unique_ptr<DevBuf>>* cache =
+        new std::map<std::tuple<int, int, int, int, int, int, int>, std::unique_ptr<DevBuf>>();
+    auto key = std::make_tuple(M, nc, herm, hcols, c0, bm, bn);
     auto it = cache->find(key);
     if (it != cache->end()) return *it->second;
     // in groups of 8 tile rows walked column by column, so that the tiles in flight at one time
@@ -1668,7 +1854,13 @@ const DevBuf& tile_list(int M, int nc, int herm, int c0, int bm, int bn) {
     for (int L = 0; L < nM * nN; ++L) {
         const int per = GROUP * nN, g = L / per, first = g * GROUP, size = std::min(GROUP, nM - first), r = L - g * per;
         const int m0 = (first + r % size) * bm, n0 = (r / size) * bn;
-        if (oz::oz_tile_needed(m0, bm, M, herm, c0 + n0 + bn - 1)) v.push_back(make_int2(m0, n0));
+        int cmax = c0 + n0 + bn - 1;  // the last column the tile reaches
+        if (hcols > 0) {
+            const int last = std::min(nc, n0 + bn) - 1;
+            cmax = n0 / hcols != last / hcols ? hcols - 1 : last % hcols;
+            cmax += c0;
+        }
+        if (oz::oz_tile_needed(m0, bm, M, herm, cmax)) v.push_back(make_int2(m0, n0));
     }
     auto b = std::make_unique<DevBuf>();
     b->alloc(std::max<size_t>(1, v.size()) * sizeof(int2));
@@ -1686,57 +1878,109 @@ int oz_bits(int K, int nmod) {
     return std::min(53, (int)std::floor(room / 2.0));
 }
 
-// out (M x N FP64, column-major, ldo) = alpha * A B^T + beta * out from prepared operands
-void oz_gemm(const OzOperand& A, const OzOperand& B, double alpha, double beta, DView& C, int herm, int out_part) {
+// Width of the 256-row tiles of an M x nc product on the SM pairs: 256 columns move the fewest operand
+// bytes per MMA, but a product of few tiles may fill its last wave of (tile, modulus) items badly or
+// multiply columns past nc, so the width is the one with the smallest waves x (columns + 384): an
+// item's time falls by less than half of its columns (256 -> 128 columns: 16.0 -> 12.9 us at K = 4,096).
+static int oz_tile_width(int M, int nc, int pairs, int nmod) {
+    int best = 256;
+    double cost = 1e300;
+    for (int w = 256; w >= 96; w -= 32) {
+        const double items = (double)((M + 255) / 256) * ((nc + w - 1) / w) * nmod;
+        const double c = std::ceil(items / pairs) * (w + 384);
+        if (c < 0.97 * cost) {
+            cost = c;
+            best = w;
+        }
+    }
+    return best;
+}
+
+// the residue planes R (column-major bytes, ldr) of A B^T's columns b0 .. b0 + nc - 1, modulo every p_l
+static void oz_gemm_planes(const OzOperand& A, const OzOperand& B, int b0, int nc, uint8_t* R, size_t rplane, int ldr,
+                           int herm, int hcols, int c0) {
     using namespace oz;
-    const int M = A.rows, N = B.rows, K = A.K;
+    const int M = A.rows, K = A.K;
+    static bool attr = false;
+    static int sms = 0;
+    if (!attr) {
+        OMM_CK(cudaFuncSetAttribute(oz_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
+        OMM_CK(cudaFuncSetAttribute(oz_gemm_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM2_BYTES));
+        OMM_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, rt().device));
+        attr = true;
+    }
+    // 256-row tiles on SM pairs; for short K, where an item's epilogue is longer than its MMAs, 128-row ones
+    // on single SMs (8,192 x 8,192 x 512: 0.65 ms against 0.78; at K = 1,296 the pairs lead, 97 us to 111)
+    const bool pairs = tc_pairs_enabled() && M > BM && K > 640;
+    const int bm = pairs ? BM2 : BM, bn = pairs ? oz_tile_width(M, nc, sms / 2, A.nmod) : BN;
+    const CUtensorMap ta = map_planes(A.planes.p, M, K, A.ldk, A.nmod, BM);
+    const CUtensorMap tb = map_planes(B.planes.p, B.rows, K, B.ldk, B.nmod, pairs ? bn / 2 : BN);
+    const Table& t = table(A.nmod);
+    GemmParams gp{};
+    gp.M = M;
+    gp.N = nc;
+    gp.K = K;
+    gp.nmod = A.nmod;
+    gp.bn = bn;
+    gp.exact = K < 8192;
+    gp.b_row0 = b0;
+    for (int l = 0; l < A.nmod; ++l) {
+        const uint32_t pl = (uint32_t)t.p[l];
+        gp.p[l] = t.p[l];
+        gp.magic[l] = (uint32_t)(((1ull << 39) + pl - 1) / pl);
+        gp.off[l] = (uint32_t)(((gp.exact ? 1ull << 27 : 1ull << 31) + pl - 1) / pl * pl);
+    }
+    gp.R = R;
+    gp.rplane = rplane;
+    gp.ldr = ldr;
+    gp.err = tc_error_flag();
+    gp.wc = tc_wait_cfg();
+    const DevBuf& tl = tile_list(M, nc, herm, hcols, c0, bm, bn);
+    gp.tiles = tl.as<int2>();
+    gp.ntiles = (int)(tl.bytes / sizeof(int2));
+    const int items = gp.ntiles * A.nmod;
+    if (items == 0) return;
+    ktime_begin();
+    if (pairs) oz_gemm_pair_kernel<<<2 * std::min(items, sms / 2), GEMM_THREADS, SMEM2_BYTES, rt().stream>>>(ta, tb, gp);
+    else oz_gemm_kernel<<<std::min(items, sms), GEMM_THREADS, SMEM_BYTES, rt().stream>>>(ta, tb, gp);
+    OMM_KCHECK();
+    // int8 ops of the tiles formed (their useful part where all are), all moduli
+    const double cells = herm == 0 ? (double)M * nc : std::min((double)M * nc, (double)gp.ntiles * bm * bn);
+    ktime_end(pairs ? "oz_gemm_pair_kernel" : "oz_gemm_kernel", 2.0 * K * cells * A.nmod);
+}
+
+// out (FP64 or complex, column-major, ldo) = alpha * A B^T + beta * out from prepared operands.  Complex
+// (stacked operands of real and imaginary rows): with conjugation signs sA, sB of the operands,
+// Re C = RR - sA sB II, Im C = sB RI + sA IR.
+static void oz_gemm_any(const OzOperand& A, const OzOperand& B, double alpha, double beta, DView& C, int herm, double sA,
+                        double sB) {
+    using namespace oz;
+    const bool cplx = A.zrow > 0 || !C.is_real;
+    const int M = C.rows, N = C.cols, K = A.K;
     if (B.K != K || A.nmod != B.nmod) fail(OMM_ERR_ARG, "oz_gemm: operands differ in K or moduli");
     if (K > MAX_K) fail(OMM_ERR_ARG, "oz_gemm: K must be below 2^17");
+    if (A.rows != A.zrow + M || B.rows != B.zrow + N || (A.zrow > 0) != cplx || (B.zrow > 0) != cplx || C.is_real == cplx)
+        fail(OMM_ERR_ARG, "oz_gemm: operands do not match the result");
     if (herm < 0 || (herm > 0 && M % herm)) fail(OMM_ERR_ARG, "oz_gemm: bad Hermitian block size");
+    // the blocks' period in A's stacked rows: one block spans a part's rows with their padding; several
+    // blocks repeat over both parts when there is no padding (else every tile is formed)
+    const int hrow = !cplx || herm == 0 ? herm : herm == M ? A.zrow : A.zrow == M ? herm : 0;
     const Table& tb = table(A.nmod);
     if ((double)(A.bits + B.bits) > tb.log2P - 2.0 - std::log2((double)std::max(K, 1)))
         fail(OMM_ERR_ARG, "oz_gemm: operand bits exceed the moduli's range");
     if (M == 0 || N == 0) return;
     if (K == 0) {
-        if (out_part >= 0) fail(OMM_ERR_ARG, "oz_gemm: empty inner dimension for a complex part");
         const double b2[2] = {beta, 0.0};
         if (beta != 1.0) k_scale(C, b2);
         return;
     }
-    static bool attr = false;
-    if (!attr) {
-        OMM_CK(cudaFuncSetAttribute(oz_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
-        OMM_CK(cudaFuncSetAttribute(oz_gemm_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM2_BYTES));
-        attr = true;
-    }
-    const bool pairs = tc_pairs_enabled() && M > BM;  // 256 x 256 tiles on SM pairs
-    const int tbm_ = pairs ? BM2 : BM, tbn_ = pairs ? BN2 : BN;
-    const CUtensorMap ta = map_planes(A.planes.p, M, K, A.ldk, A.nmod, BM);
-    const CUtensorMap tbm = map_planes(B.planes.p, N, K, B.ldk, B.nmod, pairs ? 128 : BN);
     // the product's residue planes, for at most ~4 GB of them at a time: panels of columns
-    const int ldr = (M + 127) / 128 * 128;
-    const size_t cap = oz_panel_bytes();
-    int np = (int)std::min<size_t>((size_t)N, std::max<size_t>(BN, cap / ((size_t)A.nmod * ldr) / BN * BN));
+    const int ldr = (A.rows + 127) / 128 * 128, parts = cplx ? 2 : 1;
+    const size_t cap = oz_panel_bytes() / parts;
+    const int np = (int)std::min<size_t>((size_t)N, std::max<size_t>(BN, cap / ((size_t)A.nmod * ldr) / BN * BN));
     DevBuf& Rb = product_planes();
-    const size_t rplane = (size_t)ldr * np;
+    const size_t rplane = (size_t)ldr * (cplx ? 2 * (size_t)np + 3 : (size_t)np);  // B's parts start 4 rows apart
     Rb.ensure(rplane * A.nmod);
-    GemmParams gp{};
-    gp.M = M;
-    gp.K = K;
-    gp.nmod = A.nmod;
-    for (int l = 0; l < A.nmod; ++l) {
-        const uint32_t pl = (uint32_t)tb.p[l];
-        gp.p[l] = tb.p[l];
-        gp.magic[l] = (uint32_t)(((1ull << 39) + pl - 1) / pl);
-        gp.off[l] = (uint32_t)(((1ull << 31) + pl - 1) / pl * pl);
-    }
-    gp.R = Rb.as<uint8_t>();
-    gp.rplane = rplane;
-    gp.ldr = ldr;
-    gp.err = tc_error_flag();
-    gp.wc = tc_wait_cfg();
-    static int sms = 0;
-    if (!sms) OMM_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, rt().device));
     RecParams rp{};
     rp.M = M;
     rp.nmod = A.nmod;
@@ -1747,47 +1991,45 @@ void oz_gemm(const OzOperand& A, const OzOperand& B, double alpha, double beta, 
     rp.shift = (A.bits - 1) + (B.bits - 1);
     rp.alpha = alpha;
     rp.beta = beta;
-    if ((out_part >= 0) == C.is_real) fail(OMM_ERR_ARG, "oz_gemm: output part given for a real result or missing");
-    rp.ldo = out_part >= 0 ? 2 * C.ld : C.ld;
-    rp.os = out_part >= 0 ? 2 : 1;
+    rp.ldo = C.ld;
     rp.herm = herm;
+    rp.zrow = A.zrow;
+    rp.a_rr = alpha;
+    rp.a_ii = -sA * sB * alpha;
+    rp.a_ri = sB * alpha;
+    rp.a_ir = sA * alpha;
     fill_rec_tables(rp, tb, A.nmod);
     for (int c0 = 0; c0 < N; c0 += np) {
         const int nc = std::min(np, N - c0);
         // the panel's columns are rows c0 .. c0 + nc - 1 of the B operand
-        const DevBuf& tl = tile_list(M, nc, herm, c0, tbm_, tbn_);
-        gp.N = nc;
-        gp.b_row0 = c0;
-        gp.tiles = tl.as<int2>();
-        gp.ntiles = (int)(tl.bytes / sizeof(int2));
-        const int items = gp.ntiles * A.nmod;
-        if (items > 0) {
-            ktime_begin();
-            if (pairs) {
-                oz_gemm_pair_kernel<<<2 * std::min(items, sms / 2), GEMM_THREADS, SMEM2_BYTES, rt().stream>>>(ta, tbm,
-                                                                                                             gp);
-            } else {
-                oz_gemm_kernel<<<std::min(items, sms), GEMM_THREADS, SMEM_BYTES, rt().stream>>>(ta, tbm, gp);
-            }
-            OMM_KCHECK();
-            // int8 ops of the tiles formed (the useful rows x columns of each, all moduli)
-            double cells = 0.0;
-            for (int m0 = 0; m0 < M; m0 += tbm_)
-                for (int n0 = 0; n0 < nc; n0 += tbn_)
-                    if (oz_tile_needed(m0, tbm_, M, herm, c0 + n0 + tbn_ - 1))
-                        cells += (double)std::min(tbm_, M - m0) * std::min(tbn_, nc - n0);
-            ktime_end(pairs ? "oz_gemm_pair_kernel" : "oz_gemm_kernel", 2.0 * K * cells * A.nmod);
+        if (!cplx) {
+            oz_gemm_planes(A, B, c0, nc, Rb.as<uint8_t>(), rplane, ldr, herm, 0, c0);
+        } else if (nc == N) {
+            // both parts in one launch: B's rows run on from the real ones to the imaginary ones
+            oz_gemm_planes(A, B, 0, B.rows, Rb.as<uint8_t>(), rplane, ldr, hrow, B.zrow, 0);
+        } else {
+            oz_gemm_planes(A, B, c0, nc, Rb.as<uint8_t>(), rplane, ldr, hrow, nc, c0);
+            oz_gemm_planes(A, B, B.zrow + c0, nc, Rb.as<uint8_t>() + (size_t)nc * ldr, rplane, ldr,
+                           hrow, nc, c0);
         }
         rp.N = nc;
         rp.n_off = c0;
         rp.eB = B.exps.as<int>() + c0;
-        rp.out = C.as<double>() + (size_t)c0 * rp.ldo + (out_part > 0 ? 1 : 0);
-        dim3 rg((M + 1023) / 1024, (nc + 7) / 8);
+        rp.out = C.as<double>() + (size_t)c0 * C.ld * (cplx ? 2 : 1);
         ktime_begin();
-        oz_reconstruct_kernel<<<rg, 256, 0, rt().stream>>>(rp);
+        if (cplx) {
+            rp.zcol = nc == N ? B.zrow : nc;
+            rp.eBi = B.exps.as<int>() + B.zrow + c0;
+            oz_reconstruct_z_kernel<<<dim3((M + 511) / 512, (nc + 1) / 2), 128, 0, rt().stream>>>(rp);
+        } else {
+            oz_reconstruct_kernel<<<dim3((M + 1023) / 1024, (nc + 7) / 8), 256, 0, rt().stream>>>(rp);
+        }
         OMM_KCHECK();
         ktime_end("oz_reconstruct_kernel", recon_bytes(rp, M, nc));
     }
+}
+void oz_gemm(const OzOperand& A, const OzOperand& B, double alpha, double beta, DView& C, int herm) {
+    oz_gemm_any(A, B, alpha, beta, C, herm, 1.0, 1.0);
 }
 
 // ------------------------------------------------------------------ FP64 SpMM on the int8 tensor cores (host)
@@ -2080,7 +2322,6 @@ bool oz_spmm(const msw_matrix* H, const msw_matrix* S, const OzOperand& A, DView
     rp.alpha = 1.0;
     rp.beta = 0.0;
     rp.ldo = Y.ld;
-    rp.os = 1;
     rp.herm = 0;
     rp.n_off = 0;
     fill_rec_tables(rp, tb, OZ_NMOD);
@@ -2131,29 +2372,45 @@ void gemm_f64_emu(char opA, char opB, int M, int N, int K, double alpha, const D
     // A_op (M x K): A itself ('n', rows contiguous) or A^T ('t', K contiguous)
     oz_prepare(A, opA != 'n', M, K, OZ_NMOD, bits, *oa);
     // B_op (N x K) = op(B)^T: B^T when op(B) = B ('n': K contiguous), B when op(B) = B^T ('t')
-    oz_prepare(B, opB == 'n', N, K, OZ_NMOD, bits, *ob, false, -1, b_exps);
-    oz_gemm(*oa, *ob, alpha, beta, C, herm);
+    oz_prepare(B, opB == 'n', N, K, OZ_NMOD, bits, *ob, false, b_exps);
+    DView Cv = C;
+    Cv.rows = M;
+    Cv.cols = N;
+    oz_gemm(*oa, *ob, alpha, beta, Cv, herm);
 }
 
 // complex C = alpha op(A) op(B) + beta C (alpha, beta real; ops 'n', 't', 'c') as four real
-// FP64-accurate products of the parts: with op(A) = Ar + i sA Ai and op(B) = Br + i sB Bi
-// (s = -1 for 'c'),  Re C = Ar Br - sA sB Ai Bi,  Im C = sB Ar Bi + sA Ai Br
+// FP64-accurate products of the parts, formed as one: the operands' real and imaginary rows are stacked,
+// each part with exponents of its own.  With op(A) = Ar + i sA Ai and op(B) = Br + i sB Bi (s = -1 for
+// 'c'),  Re C = Ar Br - sA sB Ai Bi,  Im C = sB Ar Bi + sA Ai Br.
 void gemm_z_emu(char opA, char opB, int M, int N, int K, double alpha, const DView& A, const DView& B, double beta,
                 DView& C, int herm) {
     const int bits = oz_bits(K, OZ_NMOD);
-    const double sA = opA == 'c' ? -1.0 : 1.0, sB = opB == 'c' ? -1.0 : 1.0;
-    OzOperand& ar = oz_scratch(OZS_GEMM_A);
-    OzOperand& ai = oz_scratch(OZS_GEMM_AI);
-    OzOperand& br = oz_scratch(OZS_GEMM_B);
-    OzOperand& bi = oz_scratch(OZS_GEMM_BI);
-    oz_prepare(A, opA != 'n', M, K, OZ_NMOD, bits, ar, false, 0);
-    oz_prepare(A, opA != 'n', M, K, OZ_NMOD, bits, ai, false, 1);
-    oz_prepare(B, opB == 'n', N, K, OZ_NMOD, bits, br, false, 0);
-    oz_prepare(B, opB == 'n', N, K, OZ_NMOD, bits, bi, false, 1);
-    oz_gemm(ar, br, alpha, beta, C, herm, 0);
-    oz_gemm(ai, bi, -sA * sB * alpha, 1.0, C, herm, 0);
-    oz_gemm(ar, bi, sB * alpha, beta, C, herm, 1);
-    oz_gemm(ai, br, sA * alpha, 1.0, C, herm, 1);
+    OzOperand& oa = oz_scratch(OZS_GEMM_A);
+    OzOperand& ob = oz_scratch(OZS_GEMM_B);
+    // the kernels read and write (re, im) pairs as 16 bytes; a matrix on an 8-byte address goes through a copy
+    auto bytes16 = [](const DView& v) { return (reinterpret_cast<uintptr_t>(v.p) & 15) == 0; };
+    DevBuf tA, tB, tC;
+    auto aligned = [&](const DView& v, DevBuf& t) {
+        if (bytes16(v) || v.rows == 0 || v.cols == 0) return v;
+        t.alloc((size_t)v.rows * v.cols * 16);
+        DView o = v;
+        o.p = t.p;
+        o.ld = v.rows;
+        OMM_CK(cudaMemcpy2DAsync(o.p, (size_t)o.ld * 16, v.p, (size_t)v.ld * 16, (size_t)v.rows * 16, v.cols,
+                                 cudaMemcpyDeviceToDevice, rt().stream));
+        return o;
+    };
+    DView Cu = C;
+    Cu.rows = M;
+    Cu.cols = N;
+    DView Cv = aligned(Cu, tC);
+    oz_prepare(aligned(A, tA), opA != 'n', M, K, OZ_NMOD, bits, oa);
+    oz_prepare(aligned(B, tB), opB == 'n', N, K, OZ_NMOD, bits, ob);
+    oz_gemm_any(oa, ob, alpha, beta, Cv, herm, opA == 'c' ? -1.0 : 1.0, opB == 'c' ? -1.0 : 1.0);
+    if (Cv.p != C.p)
+        OMM_CK(cudaMemcpy2DAsync(C.p, (size_t)C.ld * 16, Cv.p, (size_t)Cv.ld * 16, (size_t)M * 16, N,
+                                 cudaMemcpyDeviceToDevice, rt().stream));
 }
 
 }  // namespace ommgpu
@@ -2248,7 +2505,7 @@ extern "C" int omm_gpu_spmm_f64(const double* A, int lda, int n, const msw_matri
         y.cols = m;
         y.ld = ldy;
         OzOperand* op = &oz_scratch(OZS_SPMM_A);
-        oz_prepare(a, false, n, m, OZ_NMOD, oz_bits(m, OZ_NMOD), *op, true, -1, nullptr, oz_spmm_kb_halves(S != nullptr));
+        oz_prepare(a, false, n, m, OZ_NMOD, oz_bits(m, OZ_NMOD), *op, true, nullptr, oz_spmm_kb_halves(S != nullptr));
         if (!oz_spmm(H, S, *op, y)) fail(OMM_ERR_UNSUPPORTED, "spmm_f64: n must be a multiple of 4");
         sync();
         unsigned e = gemm_bf16_errors();
