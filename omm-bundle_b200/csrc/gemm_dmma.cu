@@ -1,0 +1,397 @@
+// FP64 (real and complex) matrix products on the FP64 tensor cores (mma.sync m8n8k4 f64; tcgen05 has no
+// FP64 kind), for the products too small for the int8 emulation of ozaki.cu to pay: MatrixSwitch products
+// of a few hundred rows, and every product of the CG step of a small problem.
+//
+//   C_z = alpha * op(A_z) op(B_z) + beta * C_z,  op in {n, t, c},  z = 0 .. nz - 1 (nz <= 2)
+//
+// A CTA of four warps forms one 32 x 32 tile; its K runs in 16-k (complex: 8-k) chunks through a ring of
+// four stages filled by cp.async three chunks ahead, one barrier per chunk.  The warps share the chunk's k,
+// not the tile: each multiplies the whole tile by its own four k (16 independent DMMAs on 8 fragment
+// loads; complex: two warps by k, two by rows, 32 DMMAs on 6 loads), and the four partial tiles are added at
+// the end.  What bounds such products is latency -- one or two CTAs per SM, each a serial chain over K -- so
+//   * a chunk is few instructions: copies from pointers formed once, stages as immediate offsets of an
+//     unrolled turn (with addresses formed per chunk it was 200 instructions a warp, at five clocks each,
+//     for 16 DMMAs: 128 x 832 x 832 twice 31 us, now 21);
+//   * K is split over the CTAs of a cluster (up to 8): the partial tiles are added through distributed
+//     shared memory in rank order (the same bits every time), and each CTA writes its part of the tile;
+//   * two products of one shape run in one launch (D [H, S] and [X; Y] D^H of a CG step);
+//   * a Hermitian product forms its upper tiles only and writes both triangles.
+// Operands keep their global order in shared memory (rows or k contiguous, whichever the op makes of
+// them), padded so that the 16 lanes of a half-warp's fragment load (8 lanes for complex elements) fall
+// in distinct banks.  Complex products take four DMMAs per fragment pair.
+// Against cuBLAS (launches back to back): 256 x 128 x 832 twice 12.5 us (27 in two calls), 64 x 64 x 6,000
+// 17 (25), 1,024^3 76 (83), 2,049 x 1,999 x 4,001 1,086 (1,000), 260 x 130 x 600 complex twice 26 (51).
+// 64 x 64 tiles of eight warps were slower at every size up to 2,049 x 1,999 x 4,001 (1,157 us).
+#include "internal.h"
+
+#include <cooperative_groups.h>
+
+#include <algorithm>
+#include <cmath>
+
+namespace cg = cooperative_groups;
+
+namespace ommgpu {
+
+namespace {
+
+
+struct DgArgs {
+    int M, N, K;
+    const double *A[2], *B[2];
+    double* C[2];
+    long long lda, ldb, ldc;  // elements
+    zdbl alpha, beta;
+    int beta_zero;
+    int conj_a, conj_b;
+    int vec;      // 16-byte copies of A and B (real: even leading dimensions and 16-byte addresses)
+    int herm[2];  // rows per Hermitian block of C_z (0: none): both triangles from the upper tiles
+    int kper;     // k per CTA of the cluster (a multiple of the chunk)
+};
+
+template <bool CPLX> struct El { using T = double; };
+template <> struct El<true> { using T = double2; };
+
+// copy of 16 (WIDE) or 8 bytes to shared memory, `bytes` of them from src and zeros beyond
+template <bool WIDE>
+__device__ __forceinline__ void cp(uint32_t dst, const void* src, int bytes) {
+    if constexpr (WIDE)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+    else
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void dmma(double (&d)[2], double a, double b) {
+    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+                 : "+d"(d[0]), "+d"(d[1])
+                 : "d"(a), "d"(b));
+}
+
+template <bool CPLX, int R>
+constexpr int stride_rows() { return CPLX ? R + 2 : R + 4; }  // [k][r]
+template <bool CPLX>
+constexpr int chunk() { return CPLX ? 8 : 16; }
+template <bool CPLX>
+constexpr int stride_k() { return chunk<CPLX>() + 4; }  // [r][k]
+template <bool CPLX, int R, bool KC>
+constexpr int tile_elems() { return KC ? R * stride_k<CPLX>() : chunk<CPLX>() * stride_rows<CPLX, R>(); }
+template <bool CPLX, int BM, int BN, int WK, int ST, bool TA, bool TB>
+constexpr int smem_bytes() {
+    const int es = CPLX ? 16 : 8;
+    const int ring = ST * (tile_elems<CPLX, BM, TA>() + tile_elems<CPLX, BN, !TB>()) * es;
+    const int part = WK * BM * BN * es;  // the partial tiles of a split K
+    return ring > part ? ring : part;
+}
+
+// A thread's copies of an operand's chunks into shared memory: R rows (of op(A), or columns of op(B)) from
+// row r0 (of n), k from k_lo on.  KC: k contiguous in memory, element (r, k) at S[k + r ld], kept as
+// [r][k]; else rows contiguous, at S[r + k ld], kept as [k][r].  Source, place and bytes of every copy are
+// formed once: a chunk then costs an add and a copy each -- forming them per chunk took a warp longer than
+// its DMMAs, which at one or two CTAs per SM nothing hides.
+template <bool CPLX, int R, bool KC, int NTHR, bool VEC>
+struct Loader {
+    using T = typename El<CPLX>::T;
+    static constexpr int BK = chunk<CPLX>(), W = CPLX ? 2 : 1, PER = VEC && !CPLX ? 2 : 1;  // elements per copy
+    static constexpr int NU = BK * R / PER / NTHR;
+    const double* src[NU];
+    uint32_t dst[NU];
+    int bytes[NU], kk[NU];
+    long long step;
+    __device__ __forceinline__ Loader(T* ring, const double* S, long long ld, int r0, int n, int k_lo) {
+        step = (KC ? (long long)BK : BK * ld) * W;
+#pragma unroll
+        for (int u = 0; u < NU; ++u) {
+            const int e = threadIdx.x + NTHR * u;
+            const int k = KC ? PER * (e % (BK / PER)) : e / (R / PER);
+            const int rr = KC ? e / (BK / PER) : PER * (e % (R / PER)), r = r0 + rr;
+            kk[u] = k;
+            const int rows = KC ? (r < n ? PER : 0) : max(0, min(PER, n - r));
+            bytes[u] = rows * 8 * W;
+            // a copy of no bytes reads nothing: any address does
+            src[u] = S + (bytes[u] ? (KC ? (long long)(k_lo + k) + r * ld : (long long)r + (k_lo + k) * ld) * W : 0);
+            dst[u] = (uint32_t)__cvta_generic_to_shared(ring + (KC ? rr * stride_k<CPLX>() + k : k * stride_rows<CPLX, R>() + rr));
+        }
+    }
+    // the next chunk into the stage at `off` bytes
+    __device__ __forceinline__ void copy(uint32_t off) {
+#pragma unroll
+        for (int u = 0; u < NU; ++u) {
+            cp<CPLX || VEC>(dst[u] + off, src[u], bytes[u]);
+            src[u] += step;
+        }
+    }
+    // the last chunk, of which only krem k are left
+    __device__ __forceinline__ void copy_tail(uint32_t off, int krem) {
+#pragma unroll
+        for (int u = 0; u < NU; ++u) {
+            const int left = KC ? max(0, min(PER, krem - kk[u])) * 8 * W : (kk[u] < krem ? bytes[u] : 0);
+            cp<CPLX || VEC>(dst[u] + off, src[u], bytes[u] ? left : 0);
+        }
+    }
+};
+
+// TA: A is K-contiguous (op 't' / 'c'); TB: B is column-contiguous (op 't' / 'c')
+template <bool CPLX, int BM, int BN, int WM, int WN, int WK, int ST, bool TA, bool TB, bool VEC>
+__global__ void __launch_bounds__(32 * WM * WN * WK) gemm_dmma_kernel(const __grid_constant__ DgArgs p) {
+    using T = typename El<CPLX>::T;
+    constexpr int BK = chunk<CPLX>(), MT = BM / (8 * WM), NT = BN / (8 * WN), NP = CPLX ? 2 : 1, NTHR = 32 * WM * WN * WK;
+    constexpr int AE = tile_elems<CPLX, BM, TA>(), BE = tile_elems<CPLX, BN, !TB>();
+    extern __shared__ __align__(16) unsigned char raw[];
+    T* ring = reinterpret_cast<T*>(raw);
+    const int tm = (p.M + BM - 1) / BM;
+    const int m0 = (blockIdx.x % tm) * BM, n0 = (blockIdx.x / tm) * BN, z = blockIdx.y;
+    const int S = gridDim.z, rank = blockIdx.z;  // the cluster is the z dimension
+    const int herm = p.herm[z];
+    if (herm > 0) {
+        const int last = min(m0 + BM, p.M) - 1;
+        if (m0 / herm == last / herm && m0 % herm > n0 + BN - 1) return;  // below the diagonal: the same for the cluster
+    }
+    const int k_lo = min(p.K, rank * p.kper), k_hi = min(p.K, k_lo + p.kper);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int wm = (warp % WM) * (BM / WM), wn = (warp / WM % WN) * (BN / WN), wk = warp / (WM * WN);
+    const double *A = p.A[z], *B = p.B[z];
+
+    double acc[NP][MT][NT][2];
+#pragma unroll
+    for (int s = 0; s < NP; ++s)
+#pragma unroll
+        for (int i = 0; i < MT; ++i)
+#pragma unroll
+            for (int j = 0; j < NT; ++j) acc[s][i][j][0] = acc[s][i][j][1] = 0.0;
+
+    constexpr uint32_t STAGE = (AE + BE) * sizeof(T);
+    Loader<CPLX, BM, TA, NTHR, VEC> la(ring, A, p.lda, m0, p.M, k_lo);
+    Loader<CPLX, BN, !TB, NTHR, VEC> lb(ring + AE, B, p.ldb, n0, p.N, k_lo);
+    const int kspan = k_hi - k_lo, nfull = kspan / BK, nk = (kspan + BK - 1) / BK;
+    auto load = [&](int t, uint32_t off) {
+        if (t < nfull) {
+            la.copy(off);
+            lb.copy(off);
+        } else if (t < nk) {
+            la.copy_tail(off, kspan - t * BK);
+            lb.copy_tail(off, kspan - t * BK);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+#pragma unroll
+    for (int t = 0; t < ST - 1; ++t) load(t, t * STAGE);
+    const double sa = p.conj_a ? -1.0 : 1.0, sb = p.conj_b ? -1.0 : 1.0;
+    // this lane's elements of a stage's fragments; the stages of an unrolled turn are immediate offsets
+    const int fk = 4 * wk + (lane & 3), fr = lane >> 2;
+    const T* fa = ring + (TA ? (wm + fr) * stride_k<CPLX>() + fk : fk * stride_rows<CPLX, BM>() + wm + fr);
+    const T* fb = ring + AE + (TB ? fk * stride_rows<CPLX, BN>() + wn + fr : (wn + fr) * stride_k<CPLX>() + fk);
+    auto multiply = [&](int stage) {
+#pragma unroll
+        for (int k4 = 0; k4 < BK / (4 * WK); ++k4) {
+            T a[MT], b[NT];
+#pragma unroll
+            for (int i = 0; i < MT; ++i)
+                a[i] = fa[stage * (AE + BE) + (TA ? 8 * i * stride_k<CPLX>() + 4 * WK * k4
+                                                  : 4 * WK * k4 * stride_rows<CPLX, BM>() + 8 * i)];
+#pragma unroll
+            for (int j = 0; j < NT; ++j)
+                b[j] = fb[stage * (AE + BE) + (TB ? 4 * WK * k4 * stride_rows<CPLX, BN>() + 8 * j
+                                                  : 8 * j * stride_k<CPLX>() + 4 * WK * k4)];
+            if constexpr (CPLX) {
+#pragma unroll
+                for (int i = 0; i < MT; ++i) {
+                    const double ai = sa * a[i].y, nai = -ai;
+#pragma unroll
+                    for (int j = 0; j < NT; ++j) {
+                        const double bi = sb * b[j].y;
+                        dmma(acc[0][i][j], a[i].x, b[j].x);
+                        dmma(acc[NP - 1][i][j], a[i].x, bi);
+                        dmma(acc[0][i][j], nai, bi);
+                        dmma(acc[NP - 1][i][j], ai, b[j].x);
+                    }
+                }
+            } else {
+#pragma unroll
+                for (int i = 0; i < MT; ++i)
+#pragma unroll
+                    for (int j = 0; j < NT; ++j) dmma(acc[0][i][j], a[i], b[j]);
+            }
+        }
+    };
+    for (int t0 = 0; t0 < nk; t0 += ST) {
+#pragma unroll
+        for (int s = 0; s < ST; ++s) {
+            const int t = t0 + s;
+            if (t < nk) {
+                asm volatile("cp.async.wait_group %0;" ::"n"(ST - 2) : "memory");  // chunk t, this thread's part
+                __syncthreads();  // everyone's part, and the stage of chunk t - 1 is free
+                load(t + ST - 1, ((s + ST - 1) % ST) * STAGE);
+                multiply(s);
+            }
+        }
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+
+    // C(i, j) = alpha v + beta C(i, j), and the mirrored element of a Hermitian block
+    auto emit = [&](int i, int j, T v) {
+        if (i >= p.M || j >= p.N) return;
+        int ii = i, base = 0;
+        if (herm > 0) {
+            base = i / herm * herm;
+            ii = i - base;
+            if (ii > j) return;  // written by its mirror
+        }
+        T* C = reinterpret_cast<T*>(p.C[z]);
+        T* c = C + i + (long long)j * p.ldc;
+        if constexpr (CPLX) {
+            double re = p.alpha.x * v.x - p.alpha.y * v.y, im = p.alpha.x * v.y + p.alpha.y * v.x;
+            if (!p.beta_zero) {
+                const T o = *c;
+                re += p.beta.x * o.x - p.beta.y * o.y;
+                im += p.beta.x * o.y + p.beta.y * o.x;
+            }
+            if (herm > 0 && ii == j) im = 0.0;
+            *c = make_double2(re, im);
+            if (herm > 0 && ii < j) C[base + j + (long long)ii * p.ldc] = make_double2(re, -im);
+        } else {
+            double o = p.alpha.x * v;
+            if (!p.beta_zero) o += p.beta.x * *c;
+            *c = o;
+            if (herm > 0 && ii < j) C[base + j + (long long)ii * p.ldc] = o;
+        }
+    };
+    auto value = [&](int i, int j, int h) -> T {
+        if constexpr (CPLX) return make_double2(acc[0][i][j][h], acc[NP - 1][i][j][h]);
+        else return acc[0][i][j][h];
+    };
+    // the warps' partial tiles, column-major, in the ring's memory (one per k share); then each CTA of the
+    // cluster adds up and writes its part of the tile
+    cg::cluster_group cl = cg::this_cluster();
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < MT; ++i)
+#pragma unroll
+        for (int j = 0; j < NT; ++j)
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+                ring[wk * BM * BN + wm + 8 * i + (lane >> 2) + (wn + 8 * j + 2 * (lane & 3) + h) * BM] = value(i, j, h);
+    if (S > 1) cl.sync();
+    else __syncthreads();
+    for (int e = rank * NTHR + threadIdx.x; e < BM * BN; e += S * NTHR) {
+        T sum{};
+        for (int s = 0; s < S; ++s) {
+            const T* part = S > 1 ? cl.map_shared_rank(ring, s) : ring;
+            T v[WK];
+#pragma unroll
+            for (int w = 0; w < WK; ++w) v[w] = part[w * BM * BN + e];
+#pragma unroll
+            for (int w = 0; w < WK; ++w) {
+                if constexpr (CPLX) {
+                    sum.x += v[w].x;
+                    sum.y += v[w].y;
+                } else {
+                    sum += v[w];
+                }
+            }
+        }
+        emit(m0 + e % BM, n0 + e / BM, sum);
+    }
+    if (S > 1) cl.sync();  // no CTA leaves while another reads its partial tiles
+}
+
+template <bool CPLX, int BM, int BN, int WM, int WN, int WK, int ST, bool TA, bool TB, bool VEC>
+void launch_t(const DgArgs& a, int nz, int split) {
+    constexpr int SM = smem_bytes<CPLX, BM, BN, WK, ST, TA, TB>();
+    auto kernel = gemm_dmma_kernel<CPLX, BM, BN, WM, WN, WK, ST, TA, TB, VEC>;
+    static bool attr = false;
+    if (!attr) {
+        OMM_CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SM));
+        attr = true;
+    }
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(((a.M + BM - 1) / BM) * ((a.N + BN - 1) / BN), nz, split);
+    cfg.blockDim = dim3(32 * WM * WN * WK);
+    cfg.dynamicSmemBytes = SM;
+    cfg.stream = rt().stream;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim = {1, 1, (unsigned)split};
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    OMM_CK(cudaLaunchKernelEx(&cfg, kernel, a));
+    OMM_KCHECK();
+}
+template <bool CPLX, int BM, int BN, int WM, int WN, int WK, int ST, bool VEC>
+void launch_ops(const DgArgs& a, bool ta, bool tb, int nz, int split) {
+    if (ta && tb) launch_t<CPLX, BM, BN, WM, WN, WK, ST, true, true, VEC>(a, nz, split);
+    else if (ta) launch_t<CPLX, BM, BN, WM, WN, WK, ST, true, false, VEC>(a, nz, split);
+    else if (tb) launch_t<CPLX, BM, BN, WM, WN, WK, ST, false, true, VEC>(a, nz, split);
+    else launch_t<CPLX, BM, BN, WM, WN, WK, ST, false, false, VEC>(a, nz, split);
+}
+
+// Split of K by an estimate of the time in SM clocks: the CTAs of the busiest SM in turn, each with a
+// fixed cost (start, filling of the ring, and for a split the exchange) and a cost per chunk, which is the
+// DMMAs' 256 (complex: 450) clocks and what they leave idle, or the chunk's own latency where a CTA has the
+// SM to itself.  Fitted to 15 shapes from 37 x 53 x 61 to 3,000 x 30 x 3,000 (within 15 %).
+struct Config {
+    int split;
+    double us;
+};
+Config pick(bool cplx, int M, int N, int K, int nz, bool herm) {
+    const double chunk_k = cplx ? 8.0 : 16.0, busy = cplx ? 550.0 : 300.0, alone = cplx ? 800.0 : 425.0;
+    const double tiles = (double)((M + 31) / 32) * ((N + 31) / 32) * nz * (herm ? 0.6 : 1.0);
+    Config best{1, 1e300};
+    for (int s = 1; s <= 8; s *= 2) {
+        if (s > 1 && K < 48 * s) break;
+        const double chunks = std::ceil(K / (s * chunk_k)), turns = std::ceil(tiles * s / 148.0);
+        const double fixed = s > 1 ? 2400.0 : 900.0;
+        const double clocks = std::max(turns * (fixed + chunks * busy), fixed + chunks * alone);
+        const double us = 4.0 + clocks / 1850.0;
+        if (us < 0.97 * best.us) best = Config{s, us};
+    }
+    return best;
+}
+
+}  // namespace
+
+double gemm_dmma_us(bool cplx, int M, int N, int K, int nz) { return pick(cplx, M, N, K, nz, false).us; }
+
+bool gemm_dmma_takes(const DView& v) { return v.is_real || (reinterpret_cast<uintptr_t>(v.p) & 15) == 0; }
+
+void gemm_dmma(char opA, char opB, int M, int N, int K, const double alpha[2], const DView* A, const DView* B,
+               const double beta[2], DView* C, int nz, const int* herm) {
+    if (M == 0 || N == 0) return;
+    const bool cplx = !C[0].is_real;
+    auto code = [](char o) { return o == 'n' || o == 'N' ? 0 : o == 't' || o == 'T' ? 1 : 2; };
+    const bool ta = code(opA) != 0, tb = code(opB) != 0;
+    DgArgs a{};
+    a.M = M;
+    a.N = N;
+    a.K = K;
+    a.lda = A[0].ld;
+    a.ldb = B[0].ld;
+    a.ldc = C[0].ld;
+    a.alpha = {alpha[0], cplx ? alpha[1] : 0.0};
+    a.beta = {beta[0], cplx ? beta[1] : 0.0};
+    a.beta_zero = a.beta.x == 0.0 && a.beta.y == 0.0;
+    a.conj_a = cplx && code(opA) == 2;
+    a.conj_b = cplx && code(opB) == 2;
+    a.vec = a.lda % 2 == 0 && a.ldb % 2 == 0;
+    bool any = false;
+    for (int z = 0; z < nz; ++z) {
+        a.A[z] = A[z].as<double>();
+        a.B[z] = B[z].as<double>();
+        a.C[z] = C[z].as<double>();
+        a.vec = a.vec && (reinterpret_cast<uintptr_t>(A[z].p) & 15) == 0 && (reinterpret_cast<uintptr_t>(B[z].p) & 15) == 0;
+        a.herm[z] = herm ? herm[z] : 0;
+        any = any || a.herm[z] > 0;
+        if (A[z].ld != A[0].ld || B[z].ld != B[0].ld || C[z].ld != C[0].ld)
+            fail(OMM_ERR_ARG, "gemm_dmma: the products of one launch share their leading dimensions");
+    }
+    const Config c = pick(cplx, M, N, K, nz, any && nz == 1);
+    const int bk = cplx ? 8 : 16;
+    a.kper = std::max(bk, ((K + c.split - 1) / c.split + bk - 1) / bk * bk);
+    if (cplx) {
+        launch_ops<true, 32, 32, 2, 1, 2, 4, true>(a, ta, tb, nz, c.split);
+    } else if (a.vec) {
+        launch_ops<false, 32, 32, 1, 1, 4, 4, true>(a, ta, tb, nz, c.split);
+    } else {
+        launch_ops<false, 32, 32, 1, 1, 4, 4, false>(a, ta, tb, nz, c.split);
+    }
+}
+
+}  // namespace ommgpu

@@ -185,7 +185,7 @@ __global__ void __launch_bounds__(256) sum_partials(const double* part, int n, d
 // 250,000 elements (four passes for complex).  m = 4,096, n = 512, 16 complex V_k of 2 %: 0.7 ms
 // against 4.6; one such V_k: 0.7 against 0.29.
 bool adjoint_by_panels(double m, double n, double nnz, bool real) {
-    if (!fp64_emu_enabled() || !fp64_emu_worth((int)m, (int)m, (int)n)) return false;
+    if (!fp64_emu_enabled() || !fp64_emu_worth((int)m, (int)m, (int)n, !real)) return false;
     const double z = real ? 1.0 : 4.0;
     const double panels = 0.55 * z * 2.0 * m * m * n / 90e12 + z * m * m / 250e9 + 30e-6;
     return nnz * n * (real ? 8.0 : 16.0) / 9.5e12 > panels;

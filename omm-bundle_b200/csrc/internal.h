@@ -266,6 +266,14 @@ void gemm(char opA, char opB, int M, int N, int K, const double alpha[2], const 
           const double beta[2], DView& C);
 void transpose_into(const DView& A, char op, DView& T);  // T = op(A)
 
+// ----------------------------------------------------------------- FP64 products on the FP64 tensor cores (gemm_dmma.cu)
+// C_z = alpha op(A_z) op(B_z) + beta C_z for nz <= 2 products of one shape and set of leading dimensions;
+// herm[z] > 0: C_z is a stack of Hermitian blocks of that many rows, formed from their upper tiles.
+void gemm_dmma(char opA, char opB, int M, int N, int K, const double alpha[2], const DView* A, const DView* B,
+               const double beta[2], DView* C, int nz = 1, const int* herm = nullptr);
+double gemm_dmma_us(bool cplx, int M, int N, int K, int nz = 1);  // its estimated time
+bool gemm_dmma_takes(const DView& v);  // complex operands must lie on 16-byte addresses
+
 // ----------------------------------------------------------------- SpMM (spmm.cu)
 // C = alpha * A * B + beta * C with A dense (op 'n'), B CSC (op 'n').
 // B2/C2 optional second matrix with the same sparsity pattern (fused H and S).
@@ -351,7 +359,8 @@ void gemm_z_emu(char opA, char opB, int M, int N, int K, double alpha, const DVi
 bool fp64_emu_enabled();  // real FP64 GEMMs of the solver on the int8 tensor cores (default on)
 void set_fp64_emu(int mode, long long panel_bytes);
 size_t oz_panel_bytes();
-bool fp64_emu_worth(int M, int N, int K);  // large enough for the emulation to pay
+bool fp64_emu_worth(int M, int N, int K, bool cplx = false);  // the emulation is faster than gemm_dmma
+bool fp64_emu_fits(int M, int N, int K);  // large enough for the emulation to pay against cuBLAS's FP64 kernels
 
 // ----------------------------------------------------------------- tensor-core SpMM (spmm_tc.cu)
 struct SpmmPlanView {

@@ -707,16 +707,22 @@ void gemm(char opA, char opB, int M, int N, int K, const double alpha[2], const 
         return CUBLAS_OP_C;
     };
     if (M == 0 || N == 0) return;
-    if (C.is_real && fp64_emu_enabled() && fp64_emu_worth(M, N, K)) {
-        // FP64-accurate product on the int8 tensor cores (ozaki.cu); 'c' is 't' for real data
-        gemm_f64_emu(op_code(opA) ? 't' : 'n', op_code(opB) ? 't' : 'n', M, N, K, alpha[0], A, B, beta[0], C);
-        return;
-    }
-    if (!C.is_real && alpha[1] == 0.0 && beta[1] == 0.0 && fp64_emu_enabled() && fp64_emu_worth(M, N, K)) {
-        // complex, as four real products of the parts
+    if (fp64_emu_enabled()) {
         const char ops[3] = {'n', 't', 'c'};
-        gemm_z_emu(ops[op_code(opA)], ops[op_code(opB)], M, N, K, alpha[0], A, B, beta[0], C);
-        return;
+        const bool cplx = !C.is_real, real_scalars = !cplx || (alpha[1] == 0.0 && beta[1] == 0.0);
+        // the emulation reads its operands before it writes the result, the FP64 kernel while it does
+        const bool in_place = C.p == A.p || C.p == B.p;
+        if (real_scalars && (in_place ? fp64_emu_fits(M, N, K) : fp64_emu_worth(M, N, K, cplx))) {
+            // FP64-accurate product on the int8 tensor cores (ozaki.cu); 'c' is 't' for real data, complex
+            // ones are four real products of the parts
+            if (cplx) gemm_z_emu(ops[op_code(opA)], ops[op_code(opB)], M, N, K, alpha[0], A, B, beta[0], C);
+            else gemm_f64_emu(op_code(opA) ? 't' : 'n', op_code(opB) ? 't' : 'n', M, N, K, alpha[0], A, B, beta[0], C);
+            return;
+        }
+        if (!in_place && gemm_dmma_takes(A) && gemm_dmma_takes(B) && gemm_dmma_takes(C)) {
+            gemm_dmma(ops[op_code(opA)], ops[op_code(opB)], M, N, K, alpha, &A, &B, beta, &C);
+            return;
+        }
     }
     OMM_CKB(cublasSetStream(rt().blas, rt().stream));
     if (C.is_real) {

@@ -144,8 +144,8 @@ void reduce_upper_blocked(const DView& U, DView& H, int nb) {
     // the block row's symmetric products on the int8 tensor cores when they are large enough and
     // the trailing block splits into whole 256-row tiles (the Hermitian-tile skip of A22)
     auto emu_update = [&](int kb_, int nr_) {
-        return H.is_real && fp64_emu_enabled() && nr_ % 256 == 0 && fp64_emu_worth(nr_, nr_, kb_) &&
-               fp64_emu_worth(kb_, nr_, kb_);
+        return H.is_real && fp64_emu_enabled() && nr_ % 256 == 0 && fp64_emu_fits(nr_, nr_, kb_) &&
+               fp64_emu_fits(kb_, nr_, kb_);
     };
     for (int k = 0; k < m; k += nb) {
         const int kb = std::min(nb, m - k), r = k + kb, nr = m - r;
@@ -415,6 +415,14 @@ void apply_HS(OmmCall& c, const DView& A, DevBuf& stack) {
         spmm_dense_csc(A, c.Hm, top, ONE, ZERO, c.Sm, &bot);
         return;
     }
+    if (!c.hcb && !c.H_csc && !c.S_csc && c.H.ld == c.S.ld && fp64_emu_enabled() &&
+        !fp64_emu_worth(n, m, m, !c.real) && gemm_dmma_takes(A) && gemm_dmma_takes(c.H) && gemm_dmma_takes(c.S)) {
+        // dense H and S in one launch
+        const DView a[2] = {A, A}, b[2] = {c.H, c.S};
+        DView out[2] = {top, bot};
+        gemm_dmma('n', 'n', n, m, m, ONE, a, b, ZERO, out, 2);
+        return;
+    }
     apply_op(c, A, true, top);
     apply_op(c, A, false, bot);
 }
@@ -487,7 +495,7 @@ bool hermitian_blocks_batched(const DView& A, const DView& B, DView& W, int n, i
         }
         return true;
     }
-    if (!A.is_real && fp64_emu_enabled() && fp64_emu_worth(halves * n, n, k)) {
+    if (!A.is_real && fp64_emu_enabled() && fp64_emu_worth(halves * n, n, k, true)) {
         gemm_z_emu('n', 'c', halves * n, n, k, 1.0, A, B, 0.0, W, n);  // as above, on the parts
         for (int hf = 0; hf < halves; ++hf) {
             DView Wh = W;
@@ -495,6 +503,10 @@ bool hermitian_blocks_batched(const DView& A, const DView& B, DView& W, int n, i
             Wh.p = (char*)W.p + (size_t)hf * n * 16;
             k_fill_lower_from_upper(Wh);
         }
+        return true;
+    }
+    if (fp64_emu_enabled() && gemm_dmma_takes(A) && gemm_dmma_takes(B)) {
+        gemm_dmma('n', 'c', halves * n, n, k, ONE, &A, &B, ZERO, &W, 1, &n);  // both triangles
         return true;
     }
     int nb = 0;
@@ -636,9 +648,17 @@ void eval_direction(OmmCall& c, const DView& Dir, double coeff[5]) {
         k_fill_lower_from_upper(bot);
     } else {
         s.de_ok = s.xr_ok = false;
-        gemm('n', 'c', 2 * n, n, m, ONE, X, Dir, ZERO, Wd);  // [HWd; SWd] = [HC; SC] Dir^H
         apply_HS(c, Dir, s.Y);                                 // [HG; SG] = Dir [H, S]
-        hermitian_pair_nt(Y, Dir, Wdd, n, m);                 // [HWdd; SWdd] = [HG; SG] Dir^H
+        if (fp64_emu_enabled() && !fp64_emu_worth(2 * n, n, m, !c.real) && gemm_dmma_takes(Dir)) {
+            // [HWd; SWd] = [HC; SC] Dir^H and [HWdd; SWdd] = [HG; SG] Dir^H in one launch
+            const DView a[2] = {X, Y}, b[2] = {Dir, Dir};
+            DView w[2] = {Wd, Wdd};
+            const int herm[2] = {0, n};
+            gemm_dmma('n', 'c', 2 * n, n, m, ONE, a, b, ZERO, w, 2, herm);
+        } else {
+            gemm('n', 'c', 2 * n, n, m, ONE, X, Dir, ZERO, Wd);
+            hermitian_pair_nt(Y, Dir, Wdd, n, m);
+        }
     }
     r_coeff(view(s.HW, n, n, n, c.real), view(s.SW, n, n, n, c.real), view(s.Wd, n, n, 2 * n, c.real),
             view(s.Wd, n, n, 2 * n, c.real, n), view(s.Wdd, n, n, 2 * n, c.real),
@@ -879,9 +899,13 @@ void density_product(const DView& C, const DView& CD, DView& D) {
         k_fill_lower_from_upper(D);
         return;
     }
-    if (!C.is_real && fp64_emu_enabled() && fp64_emu_worth(m, m, n)) {
+    if (!C.is_real && fp64_emu_enabled() && fp64_emu_worth(m, m, n, true)) {
         gemm_z_emu('c', 'n', m, m, n, 1.0, C, CD, 0.0, D, m);
         k_fill_lower_from_upper(D);
+        return;
+    }
+    if (fp64_emu_enabled() && gemm_dmma_takes(C) && gemm_dmma_takes(D)) {
+        gemm_dmma('c', 'n', m, m, n, ONE, &C, &CD, ZERO, &D, 1, &m);  // both triangles
         return;
     }
     const int nb = m >= 8192 ? 8 : (m >= 2048 ? 4 : 1);
@@ -932,7 +956,7 @@ void density_product(const DView& C, const DView& CD, DView& D) {
 void hermitian_product_nt(const DView& A, const DView& B, DView& W) {
     Runtime& R = rt();
     int n = A.rows, k = A.cols;
-    if (n >= 256 && hermitian_blocks_batched(A, B, W, n, k, 1)) return;
+    if ((n >= 256 || fp64_emu_enabled()) && hermitian_blocks_batched(A, B, W, n, k, 1)) return;
     const int nb = n >= 2048 ? 8 : (n >= 768 ? 4 : (n >= 256 ? 2 : 1));
     if (nb > 1) {
         const size_t es = A.is_real ? 8 : 16;

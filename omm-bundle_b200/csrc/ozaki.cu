@@ -2360,8 +2360,23 @@ bool fp64_emu_enabled() {
     return g_emu == 1;
 }
 
-bool fp64_emu_worth(int M, int N, int K) {
+bool fp64_emu_fits(int M, int N, int K) {
     return K >= 64 && K < (1 << 17) && M >= 128 && N >= 128 && (double)M * N * K >= (double)(1 << 27);
+}
+// The emulated product against the one on the FP64 tensor cores (gemm_dmma.cu) by their estimated times.
+// Emulated: 36 us for its seven launches, the waves of (256 x 256 tile, modulus) items over the 74 SM pairs
+// at 0.37 us per 128-k slab (3 us at least, an item's epilogue) and 0.5, and the bytes of residues,
+// exponents and reconstruction at 3.5 TB/s; complex operands are stacked parts.  Within 15 % of 32 measured
+// shapes: 1,024^3 76 us either way; 2,000 x 1,000 x 2,000 159 against 264; 130 x 1,611 x 3,000 103 against 61;
+// complex 800^3 141 against 146, 300 x 150 x 3,000 98 against 70.
+bool fp64_emu_worth(int M, int N, int K, bool cplx) {
+    if (K < 64 || K >= (1 << 17) || M < 1 || N < 1) return false;
+    const double w = cplx ? 2.0 : 1.0;
+    const double items = std::ceil(w * M / 256.0) * std::ceil(w * N / 256.0) * OZ_NMOD;
+    const double waves = std::ceil(items / 74.0);
+    const double in = ((double)M * K + (double)N * K) * 32.0 * w, out = (double)M * N * (cplx ? 144.0 : 40.0);
+    const double us = 36.0 + waves * (std::max(3.0, 0.37 * std::ceil(K / 128.0)) + 0.5) + (in + out) / 3.5e6;
+    return us < gemm_dmma_us(cplx, M, N, K);
 }
 
 void gemm_f64_emu(char opA, char opB, int M, int N, int K, double alpha, const DView& A, const DView& B, double beta,

@@ -1,0 +1,76 @@
+"""FP64 products on the FP64 tensor cores at the edges of their tiles, chunks and K splits (mm_multiply picks
+them for products too small for the int8 emulation), against torch's FP64 products of the same operands:
+both sides are within a few ulp of the sums of magnitudes, so 1e-13 |A||B| holds at K up to 10^4."""
+import pytest
+
+import ommgpu as G
+
+pytestmark = pytest.mark.gpu
+
+
+def _mat(t):
+    buf = t.t().contiguous()
+    return G.Matrix.register_gden(buf.data_ptr(), t.shape[0], t.shape[1], t.is_complex(), keep=buf), buf
+
+
+def _op(t, o):
+    return t if o == "n" else t.t() if o == "t" else t.mH
+
+
+def _check(M, N, K, opA, opB, cplx, alpha=1.0, beta=0.0):
+    import torch
+
+    g = torch.Generator(device="cuda").manual_seed(M + 3 * N + 7 * K)
+    dt = torch.complex128 if cplx else torch.float64
+    A = torch.randn(*((M, K) if opA == "n" else (K, M)), generator=g, device="cuda", dtype=dt)
+    B = torch.randn(*((K, N) if opB == "n" else (N, K)), generator=g, device="cuda", dtype=dt)
+    C0 = torch.randn(M, N, generator=g, device="cuda", dtype=dt)
+    (a, ka), (b, kb), (c, kc) = _mat(A), _mat(B), _mat(C0)
+    torch.cuda.synchronize()
+    G.mm_multiply(a, opA, b, opB, c, alpha, beta)
+    x, y = _op(A, opA), _op(B, opB)
+    ref = alpha * (x @ y) + beta * C0
+    mag = abs(alpha) * (x.abs() @ y.abs()) + abs(beta) * C0.abs()
+    assert float(((kc.t() - ref).abs() / mag.clamp_min(1e-300)).max()) <= 1e-13
+
+
+@pytest.mark.parametrize("cplx", [False, True])
+@pytest.mark.parametrize("opA", ["n", "t", "c"])
+@pytest.mark.parametrize("opB", ["n", "t", "c"])
+@pytest.mark.parametrize("M,N,K", [(33, 31, 17), (64, 96, 100), (37, 53, 61), (130, 257, 70)])
+def test_ops(M, N, K, opA, opB, cplx):
+    _check(M, N, K, opA, opB, cplx, (0.75 - 0.5j) if cplx else 0.75, (-1.25 + 0.25j) if cplx else -1.25)
+
+
+@pytest.mark.parametrize("cplx", [False, True])
+@pytest.mark.parametrize("K", [1, 3, 4, 15, 16, 17, 95, 96, 97, 200, 385, 4099])
+@pytest.mark.parametrize("M,N", [(1, 1), (32, 32), (35, 66)])
+def test_chunks_and_splits(M, N, K, cplx):
+    _check(M, N, K, "n", "t" if K % 2 else "n", cplx)
+
+
+@pytest.mark.parametrize("cplx", [False, True])
+@pytest.mark.parametrize("m,n", [(60, 30), (101, 33), (200, 65)])
+def test_small_solve(m, n, cplx):
+    """The pair launches of a small CG step (D [H, S], both Gram products) and the Hermitian products:
+    energy against the constructed spectrum, density Hermitian and a projector."""
+    import torch
+
+    g = torch.Generator(device="cuda").manual_seed(m)
+    dt = torch.complex128 if cplx else torch.float64
+    Q, _ = torch.linalg.qr(torch.randn(m, m, generator=g, device="cuda", dtype=dt))
+    L = torch.eye(m, device="cuda", dtype=dt) + 0.1 / m ** 0.5 * torch.randn(m, m, generator=g, device="cuda", dtype=dt)
+    lam = torch.linspace(-2.0, -1.0, m, device="cuda", dtype=torch.float64)
+    lam[n:] += 2.5
+    W = L @ Q
+    H, S = (W * lam) @ W.mH, L @ L.mH
+    (h, kh), (s, ks) = _mat(0.5 * (H + H.mH)), _mat(0.5 * (S + S.mH))
+    (c, kc), (d, kd) = _mat(H[:n] * 0), _mat(H * 0)
+    torch.cuda.synchronize()
+    G.set_log(None)
+    e, rc = G.omm(m, n, h, s, True, d, False, 0.0, c, False, cg_tol=1e-12, dealloc=True)
+    assert rc == 0 and abs(e - float(lam[:n].sum())) <= 1e-9 * abs(e)
+    D = kd.t()
+    assert float((D - D.mH).abs().max()) == 0.0
+    U = torch.linalg.solve(L.mH, Q[:, :n])
+    assert float((D - U @ U.mH).abs().max()) <= 1e-4
