@@ -247,7 +247,9 @@ const msw_matrix* csc_transpose(const msw_matrix* A);
 
 // ----------------------------------------------------------------- kernels (kernels.cu)
 // Elementwise on column-major views; 'op' in {'n','t','c'} applies to A.
-void k_axpby(const DView& A, char op, DView& C, const double alpha[2], const double beta[2]);
+// beta_at: a device scalar that takes beta's place (op 'n' only)
+void k_axpby(const DView& A, char op, DView& C, const double alpha[2], const double beta[2],
+             const double* beta_at = nullptr);
 void k_scale(DView& C, const double beta[2]);
 void k_set(DView& C, char seC, const double alpha[2], const double beta[2]);
 void k_set_element(DView& C, int i, int j, const double alpha[2], const double beta[2]);
@@ -260,7 +262,12 @@ void r_trace(const DView& A, double out[2]);                          // sum of 
 void r_dot(const DView& A, const DView& B, double out[2]);            // sum conj(A) B
 void r_coeff(const DView& HW, const DView& SW, const DView& HWd, const DView& SWd, const DView& HWdd,
              const DView& SWdd, double coeff[5]);                     // calc_coeff traces
-void r_lambda(const DView& PG, const DView& G, const DView& Gp, const DView& PGp, double out[2]);
+// lambda = mm_trace(PG, G - G_p) / mm_trace(PG_p, G_p), written to device memory without waiting
+void r_lambda(const DView& PG, const DView& G, const DView& Gp, const DView& PGp, double* lambda);
+// one CG step's C += x D, [X += x Y], HW and SW updates and [L = [4I - 2SW, -2HW]] in one launch (contiguous
+// C, D, X, Y; Wd, Wdd stacked with leading dimension 2n)
+void k_cg_update(int n, int m, double x, DView& C, const DView& D, DView* X, const DView* Y, DView& HW, DView& SW,
+                 const DView& Wd, const DView& Wdd, DView* L);
 // dense products on cuBLAS (FP64 / complex FP64)
 void gemm(char opA, char opB, int M, int N, int K, const double alpha[2], const DView& A, const DView& B,
           const double beta[2], DView& C);
@@ -339,7 +346,9 @@ void oz_prepare(const DView& src, bool kcontig, int rows, int K, int nmod, int b
 bool oz_spmm_kb_halves(bool with_s);
 // Y = beta Y + alpha X (real, R x K, rows contiguous) with the exponents oz_prepare would form of
 // Y's rows (erow, R ints) and of its columns (ecol, K ints: the rows of Y^T); either may be null
-void oz_axpby_exps(int R, int K, double alpha, const DView& X, double beta, DView& Y, int* erow, int* ecol);
+// (beta_at: a device scalar in beta's place)
+void oz_axpby_exps(int R, int K, double alpha, const DView& X, double beta, DView& Y, int* erow, int* ecol,
+                   const double* beta_at = nullptr);
 // out (A.rows x B.rows) = alpha * A B^T + beta * out; herm > 0 (any divisor of A.rows): out is a stack of
 // Hermitian herm x herm blocks and only the tiles reaching their upper triangles are formed
 void oz_gemm(const OzOperand& A, const OzOperand& B, double alpha, double beta, DView& C, int herm = 0);
@@ -413,8 +422,9 @@ void mx_shadow_kblock(const DView& src, DevBuf& khi, DevBuf& klo, int nseg);
 void dense_to_csc(const DView& A, int mode, double thr, double soft, msw_matrix* M);
 void threshold_dense(DView& A, double thr, double soft);
 void mx_shadow_colmajor(const DView& src, DevBuf& hi, DevBuf& lo, int nseg, int& ldd);
-// D = b*D + a*G in place, with the row-major (and k-blocked) shadows of the result (one pass; real)
-void mx_update_shadow_rowmajor(DView& D, const DView& G, double a, double b, DevBuf& hi, DevBuf& lo, int nseg,
+// D = b*D + a*G in place, with the row-major (and k-blocked) shadows of the result (one pass; real);
+// b_at: a device scalar, null for b = 0
+void mx_update_shadow_rowmajor(DView& D, const DView& G, double a, const double* b_at, DevBuf& hi, DevBuf& lo, int nseg,
                                int& ldd, DevBuf* khi, DevBuf* klo);
 // X += a*Y in place, with the row-major and column-major shadows of the result (one pass; real)
 void mx_update_shadows(DView& X, const DView& Y, double a, DevBuf& thi, DevBuf& tlo, int& ldt, DevBuf& chi,
@@ -455,6 +465,8 @@ struct IpState {
     // update and cleared by the product that uses it or by any other write of the matrix.
     DevBuf De, Xe_r, Xe_c;
     bool de_ok = false, xr_ok = false, xc_ok = false;
+    DevBuf lam;          // the CG step's lambda (r_lambda)
+    bool lg_ok = false;  // Lg holds calc_G's left factor of the current W matrices (k_cg_update)
     const void* de_src = nullptr;  // the direction matrix De belongs to
 };
 

@@ -50,7 +50,8 @@ constexpr int kAhead = 4;  // elements whose loads a thread issues before it use
 // Bound by memory: two reads and a write per element.
 template <typename T>
 __global__ void axpby_kernel(int rows, int cols, const T* __restrict__ A, int lda, T* __restrict__ C, int ldc,
-                             zdbl alpha, zdbl beta, int beta_zero) {
+                             zdbl alpha, zdbl beta, int beta_zero, const double* __restrict__ beta_at) {
+    if (beta_at) beta = zdbl{*beta_at, 0.0};
     Walk w(rows, cols);
     while (w.e < w.total) {
         T a[kAhead], cin[kAhead];
@@ -255,11 +256,11 @@ __device__ unsigned g_reduce_done;
 
 // Every block stores its K partial sums; the block that arrives last adds the nb records up with
 // compensation, in a fixed order (each thread a strided share, then a tree over the warp's lanes,
-// then the warps in turn), so the result does not depend on timing, and writes it to `out` in pinned
-// host memory.  (A second kernel for the sum and a copy of its result cost 4 + 3 us and their gaps
+// then the warps in turn), so the result does not depend on timing, and writes it to `out` (pinned
+// host memory, or device memory for sums the host does not need).  True in that block.  (A second kernel for the sum and a copy of its result cost 4 + 3 us and their gaps
 // in each of a CG step's two reductions.)
 template <int K>
-__device__ inline void block_reduce_finish(double (&v)[K], double* part, double* out) {
+__device__ inline bool block_reduce_finish(double (&v)[K], double* part, double* out) {
     __shared__ double sm[K][kThreads / 32], s_cmp[K][kThreads / 32];
     __shared__ bool last;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nb = (int)gridDim.x;
@@ -279,7 +280,7 @@ __device__ inline void block_reduce_finish(double (&v)[K], double* part, double*
     __syncthreads();
     if (threadIdx.x == 0) last = atomicInc(&g_reduce_done, (unsigned)nb - 1u) == (unsigned)nb - 1u;
     __syncthreads();
-    if (!last) return;
+    if (!last) return false;
     __threadfence();
     double s[K], c[K];
 #pragma unroll
@@ -305,6 +306,7 @@ __device__ inline void block_reduce_finish(double (&v)[K], double* part, double*
         for (int i = 0; i < (int)(blockDim.x / 32); ++i) comp_add(S, C, sm[k][i], s_cmp[k][i]);
         out[k] = S + C;
     }
+    return true;
 }
 
 template <typename T>
@@ -435,11 +437,13 @@ __global__ void coeff_kernel(int n, const T* __restrict__ HW, int l0, const T* _
     block_reduce_finish<13>(v, part, out);
 }
 
+// Polak-Ribiere lambda = v0 / v1 for the next direction, left in device memory: the host has no use for
+// it, and waiting for it cost a round trip per CG step.
 // SAME: no preconditioner, PG is G and PG_p is G_p (two reads per element instead of four)
 template <typename T, bool SAME>
 __global__ void lambda_kernel(int rows, int cols, const T* __restrict__ PG, int l0, const T* __restrict__ G, int l1,
                               const T* __restrict__ Gp, int l2, const T* __restrict__ PGp, int l3, double* part,
-                              double* out) {
+                              double* out, double* lambda) {
     double v[2] = {0.0, 0.0};
     Walk w(rows, cols);
     while (w.e < w.total) {
@@ -472,7 +476,88 @@ __global__ void lambda_kernel(int rows, int cols, const T* __restrict__ PG, int 
                 }
             }
     }
-    block_reduce_finish<2>(v, part, out);
+    if (block_reduce_finish<2>(v, part, out)) {
+        __syncthreads();
+        if (threadIdx.x == 0) *lambda = out[0] / out[1];
+    }
+}
+
+// The updates of a CG step that do not wait for anything of it but x, in one launch (a small solve spent
+// five launches of 2 to 3 us and their gaps on them): C += x D, X += x Y (flat arrays; bX = 0: X is
+// updated elsewhere), both W updates of w_update_kernel, and with L the left factor of calc_G from the new
+// W matrices.  Blocks [0, bC) take C, [bC, bC + bX) X, the rest 32 x 32 tiles of the W matrices.
+template <typename T>
+struct CgUpdate {
+    size_t nc, nx;
+    T* C;
+    const T* D;
+    T* X;
+    const T* Y;
+    T *HW, *SW, *L;      // n x n, n x n, n x 2n
+    const T *Wd, *Wdd;   // [HWd; SWd], [HWdd; SWdd], leading dimension 2n
+    int n, bC, bX;
+    double x;
+};
+template <typename T>
+__global__ void __launch_bounds__(kThreads) cg_update_kernel(const __grid_constant__ CgUpdate<T> p) {
+    const zdbl xz{p.x, 0.0}, x2{p.x * p.x, 0.0};
+    int b = blockIdx.x;
+    if (b < p.bC + p.bX) {
+        const bool c = b < p.bC;
+        T* __restrict__ y = c ? p.C : p.X;
+        const T* __restrict__ a = c ? p.D : p.Y;
+        const size_t total = c ? p.nc : p.nx, step = (size_t)(c ? p.bC : p.bX) * blockDim.x;
+        for (size_t e = (size_t)(c ? b : b - p.bC) * blockDim.x + threadIdx.x; e < total; e += kAhead * step) {
+            T av[kAhead], yv[kAhead];
+#pragma unroll
+            for (int u = 0; u < kAhead; ++u)
+                if (e + u * step < total) {
+                    av[u] = a[e + u * step];
+                    yv[u] = y[e + u * step];
+                }
+#pragma unroll
+            for (int u = 0; u < kAhead; ++u)
+                if (e + u * step < total) y[e + u * step] = Sc<T>::add(yv[u], Sc<T>::mul(xz, av[u]));
+        }
+        return;
+    }
+    b -= p.bC + p.bX;
+    __shared__ T tile[2][32][33];
+    const int n = p.n, tx = threadIdx.x & 31, ty = threadIdx.x >> 5;  // 32 x 8
+    const int tiles = (n + 31) / 32, nb = gridDim.x - p.bC - p.bX;
+    for (long long t = b; t < (long long)tiles * tiles; t += nb) {
+        const int r0 = (int)(t % tiles) * 32, c0 = (int)(t / tiles) * 32;
+        __syncthreads();
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int yy = ty + 8 * q;
+            if (c0 + tx < n && r0 + yy < n) {
+                tile[0][yy][tx] = p.Wd[c0 + tx + (size_t)(r0 + yy) * 2 * n];
+                tile[1][yy][tx] = p.Wd[n + c0 + tx + (size_t)(r0 + yy) * 2 * n];
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int yy = ty + 8 * q, i = r0 + tx, j = c0 + yy;
+            if (i >= n || j >= n) continue;
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                T* W = h ? p.SW : p.HW;
+                const size_t at = (size_t)h * n + i + (size_t)j * 2 * n;
+                T v = W[i + (size_t)j * n];
+                v = Sc<T>::add(v, Sc<T>::mul(xz, Sc<T>::conj(tile[h][tx][yy])));
+                v = Sc<T>::add(v, Sc<T>::mul(xz, p.Wd[at]));
+                v = Sc<T>::add(v, Sc<T>::mul(x2, p.Wdd[at]));
+                W[i + (size_t)j * n] = v;
+                if (p.L) {
+                    T l = Sc<T>::mul(zdbl{-2.0, 0.0}, v);
+                    if (h && i == j) l = Sc<T>::add(Sc<T>::from(zdbl{4.0, 0.0}), l);
+                    p.L[i + (size_t)(h ? j : n + j) * n] = l;
+                }
+            }
+        }
+    }
 }
 
 // L = [4I - 2 SW, -2 HW] (n x 2n), the left factor of calc_G as one product
@@ -535,7 +620,7 @@ inline int tile_grid(int rows, int cols) {
 }  // namespace
 
 // ------------------------------------------------------------------ host wrappers
-void k_axpby(const DView& A, char op, DView& C, const double alpha[2], const double beta[2]) {
+void k_axpby(const DView& A, char op, DView& C, const double alpha[2], const double beta[2], const double* beta_at) {
     int oc = op_code(op);
     if (A.is_real && oc == 2) oc = 1;
     size_t tot = (size_t)C.rows * C.cols;
@@ -545,11 +630,12 @@ void k_axpby(const DView& A, char op, DView& C, const double alpha[2], const dou
     if (oc == 0) {
         if (C.is_real)
             axpby_kernel<double><<<grid_for(tot), kThreads, 0, rt().stream>>>(C.rows, C.cols, A.as<double>(), A.ld,
-                                                                                C.as<double>(), C.ld, a, b, bz);
+                                                                                C.as<double>(), C.ld, a, b, bz, beta_at);
         else
             axpby_kernel<zdbl><<<grid_for(tot), kThreads, 0, rt().stream>>>(C.rows, C.cols, A.as<zdbl>(), A.ld,
-                                                                              C.as<zdbl>(), C.ld, a, b, bz);
+                                                                              C.as<zdbl>(), C.ld, a, b, bz, beta_at);
     } else {
+        if (beta_at) fail(OMM_ERR_ARG, "axpby: a device scalar with a transposed operand");
         const int grid = tile_grid(C.rows, C.cols);
         if (C.is_real)
             axpby_trans_kernel<double><<<grid, kThreads, 0, rt().stream>>>(C.rows, C.cols, A.as<double>(), A.ld, 0,
@@ -682,7 +768,7 @@ void r_coeff(const DView& HW, const DView& SW, const DView& HWd, const DView& SW
     coeff[4] = -t[12];
 }
 
-void r_lambda(const DView& PG, const DView& G, const DView& Gp, const DView& PGp, double out[2]) {
+void r_lambda(const DView& PG, const DView& G, const DView& Gp, const DView& PGp, double* lambda) {
     size_t tot = (size_t)G.rows * G.cols;
     int nb = grid_for(tot, 8);
     double* part = scratch_partials(nb + 1, 2);
@@ -690,12 +776,40 @@ void r_lambda(const DView& PG, const DView& G, const DView& Gp, const DView& PGp
     auto launch = [&](auto tag, auto kernel) {
         using T = decltype(tag);
         kernel<<<nb, kThreads, 0, rt().stream>>>(G.rows, G.cols, PG.as<T>(), PG.ld, G.as<T>(), G.ld, Gp.as<T>(), Gp.ld,
-                                                 PGp.as<T>(), PGp.ld, part, rt().host_pinned);
+                                                 PGp.as<T>(), PGp.ld, part, part + (size_t)nb * 2, lambda);
     };
     if (G.is_real) launch(double{}, same ? lambda_kernel<double, true> : lambda_kernel<double, false>);
     else launch(zdbl{}, same ? lambda_kernel<zdbl, true> : lambda_kernel<zdbl, false>);
     OMM_KCHECK();
-    finish_reduce(2, out);
+}
+
+void k_cg_update(int n, int m, double x, DView& C, const DView& D, DView* X, const DView* Y, DView& HW, DView& SW,
+                 const DView& Wd, const DView& Wdd, DView* L) {
+    auto launch = [&](auto tag) {
+        using T = decltype(tag);
+        CgUpdate<T> p{};
+        p.n = n;
+        p.x = x;
+        p.C = C.as<T>();
+        p.D = D.as<T>();
+        p.nc = (size_t)n * m;
+        p.bC = grid_for(p.nc);
+        if (X) {
+            p.X = X->as<T>();
+            p.Y = Y->as<T>();
+            p.nx = (size_t)2 * n * m;
+            p.bX = grid_for(p.nx);
+        }
+        p.HW = HW.as<T>();
+        p.SW = SW.as<T>();
+        p.Wd = Wd.as<T>();
+        p.Wdd = Wdd.as<T>();
+        p.L = L ? L->as<T>() : nullptr;
+        cg_update_kernel<T><<<p.bC + p.bX + tile_grid(n, n), kThreads, 0, rt().stream>>>(p);
+    };
+    if (C.is_real) launch(double{});
+    else launch(zdbl{});
+    OMM_KCHECK();
 }
 
 void gemm(char opA, char opB, int M, int N, int K, const double alpha[2], const DView& A, const DView& B,

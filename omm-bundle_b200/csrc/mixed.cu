@@ -49,8 +49,10 @@ __global__ void shadow_rowmajor_kernel(int rows, int cols, double* __restrict__ 
                                        const TA* __restrict__ add, int ldadd, double a, double b,
                                        __nv_bfloat16* __restrict__ hi, __nv_bfloat16* __restrict__ lo, int ldd,
                                        __nv_bfloat16* __restrict__ khi, __nv_bfloat16* __restrict__ klo,
-                                       __nv_bfloat16* __restrict__ chi, __nv_bfloat16* __restrict__ clo, int ldc) {
+                                       __nv_bfloat16* __restrict__ chi, __nv_bfloat16* __restrict__ clo, int ldc,
+                                       const double* __restrict__ b_at = nullptr) {
     __shared__ double tile[32][33];
+    if (b_at) b = *b_at;
     int i0 = blockIdx.x * 32, k0 = blockIdx.y * 32;
     int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;  // 32 x 8
     for (int yy = ty; yy < 32; yy += 8) {
@@ -284,7 +286,7 @@ void mx_shadow_rowmajor(const DView& src, DevBuf& hi, DevBuf& lo, int nseg, int&
 
 // D = b*D + a*G (FP64, in place) and the row-major and (when khi is given) k-blocked bf16 shadows
 // of the result, in one pass: the real CG step's new direction and the operands of its products.
-void mx_update_shadow_rowmajor(DView& D, const DView& G, double a, double b, DevBuf& hi, DevBuf& lo, int nseg,
+void mx_update_shadow_rowmajor(DView& D, const DView& G, double a, const double* b_at, DevBuf& hi, DevBuf& lo, int nseg,
                                int& ldd, DevBuf* khi, DevBuf* klo) {
     if (!D.is_real || !G.is_real || D.rows != G.rows || D.cols != G.cols)
         fail(OMM_ERR_ARG, "mx_update_shadow_rowmajor: real operands of equal shape");
@@ -298,9 +300,9 @@ void mx_update_shadow_rowmajor(DView& D, const DView& G, double a, double b, Dev
     }
     dim3 grid((D.rows + 31) / 32, (D.cols + 31) / 32);
     shadow_rowmajor_kernel<double><<<grid, 256, 0, rt().stream>>>(
-        D.rows, D.cols, D.as<double>(), D.ld, G.as<double>(), G.ld, a, b, hi.as<__nv_bfloat16>(),
+        D.rows, D.cols, D.as<double>(), D.ld, G.as<double>(), G.ld, a, 0.0, hi.as<__nv_bfloat16>(),
         nseg == 3 ? lo.as<__nv_bfloat16>() : nullptr, ldd, khi ? khi->as<__nv_bfloat16>() : nullptr,
-        (khi && nseg == 3) ? klo->as<__nv_bfloat16>() : nullptr, nullptr, nullptr, 0);
+        (khi && nseg == 3) ? klo->as<__nv_bfloat16>() : nullptr, nullptr, nullptr, 0, b_at);
     OMM_KCHECK();
 }
 

@@ -580,39 +580,34 @@ bool fp64_step_emu(const OmmCall& c) {
     return c.real && fp64_emu_enabled() && fp64_emu_worth(2 * c.n, c.n, c.m);
 }
 
-// D = G + lambda D (omm.F90:444-446) for the FP64 step; on the int8 path the same pass forms the
+// D = G + lambda D (omm.F90:444-446; lambda in device memory, null for 0) for the FP64 step; on the
+// int8 path the same pass forms the
 // exponents of D's rows for eval_direction's residues of D
-void fp64_dir_update(OmmCall& c, const DView& G, DView& D, double lambda) {
+void fp64_dir_update(OmmCall& c, const DView& G, DView& D, const double* lam) {
     IpState& s = *c.s;
     if (fp64_step_emu(c)) {
         s.De.ensure((size_t)c.n * sizeof(int));
-        oz_axpby_exps(c.n, c.m, 1.0, G, lambda, D, s.De.as<int>(), nullptr);
+        oz_axpby_exps(c.n, c.m, 1.0, G, 0.0, D, s.De.as<int>(), nullptr, lam);
         s.de_ok = true;
         s.de_src = D.p;
     } else {
-        double lam[2] = {lambda, 0.0};
-        k_axpby(G, 'n', D, ONE, lam);
+        k_axpby(G, 'n', D, ONE, ZERO, lam);
         s.de_ok = false;
     }
 }
 
-// [HC; SC] += x [HG; SG] (omm.F90:503-504, both halves at once) for the FP64 step; on the int8
-// path the same pass forms the exponents of X's rows (eval_direction's Gram products) and columns
-// (calc_G's product)
+// [HC; SC] += x [HG; SG] (omm.F90:503-504, both halves at once) for the FP64 step on the int8 path
+// (fp64_x_exps; else it is part of k_cg_update): the same pass forms the exponents of X's rows
+// (eval_direction's Gram products) and columns (calc_G's product)
+bool fp64_x_exps(const OmmCall& c) { return fp64_step_emu(c) && fp64_emu_worth(c.n, c.m, 2 * c.n); }
 void fp64_x_update(OmmCall& c, double x) {
     IpState& s = *c.s;
     const int n = c.n, m = c.m;
     DView X2 = view(s.X, 2 * n, m, 2 * n, c.real), Y2 = view(s.Y, 2 * n, m, 2 * n, c.real);
-    if (fp64_step_emu(c) && fp64_emu_worth(n, m, 2 * n)) {
-        s.Xe_r.ensure((size_t)2 * n * sizeof(int));
-        s.Xe_c.ensure((size_t)m * sizeof(int));
-        oz_axpby_exps(2 * n, m, x, Y2, 1.0, X2, s.Xe_r.as<int>(), s.Xe_c.as<int>());
-        s.xr_ok = s.xc_ok = true;
-    } else {
-        double xz[2] = {x, 0.0};
-        k_axpby(Y2, 'n', X2, xz, ONE);
-        s.xr_ok = s.xc_ok = false;
-    }
+    s.Xe_r.ensure((size_t)2 * n * sizeof(int));
+    s.Xe_c.ensure((size_t)m * sizeof(int));
+    oz_axpby_exps(2 * n, m, x, Y2, 1.0, X2, s.Xe_r.as<int>(), s.Xe_c.as<int>());
+    s.xr_ok = s.xc_ok = true;
 }
 
 // HWd/SWd, HG/SG, HWdd/SWdd for direction Dir and the quartic coefficients
@@ -670,7 +665,8 @@ void calc_G(OmmCall& c, DView& G) {
     IpState& s = *c.s;
     int n = c.n, m = c.m;
     DView L = view(s.Lg, n, 2 * n, n, c.real);
-    k_calcG_left(view(s.SW, n, n, n, c.real), view(s.HW, n, n, n, c.real), L);
+    if (!s.lg_ok) k_calcG_left(view(s.SW, n, n, n, c.real), view(s.HW, n, n, n, c.real), L);
+    s.lg_ok = false;
     DView X = view(s.X, 2 * n, m, 2 * n, c.real);
     if (s.xc_ok && c.real && fp64_emu_enabled() && fp64_emu_worth(n, m, 2 * n)) {
         // X's column exponents from the update that just wrote X (fp64_x_update)
@@ -716,15 +712,14 @@ void mx_shadow_dir(OmmCall& c, MixedCtx& mc, const DView& A, int nseg) {
 
 // D = lambda D + G (the CG direction, omm.F90:437-441) and, for a real problem, D's shadows in the
 // same pass, for the mx_eval_direction of D that follows
-void mx_update_dir(OmmCall& c, MixedCtx& mc, DView& D, const DView& G, double lambda, int nseg) {
+void mx_update_dir(OmmCall& c, MixedCtx& mc, DView& D, const DView& G, const double* lam, int nseg) {
     IpState& s = *c.s;
     if (!c.real) {
-        double lam[2] = {lambda, 0.0};
-        k_axpby(G, 'n', D, ONE, lam);
+        k_axpby(G, 'n', D, ONE, ZERO, lam);
         return;
     }
     const bool kblock = dir_kblock(c);
-    mx_update_shadow_rowmajor(D, G, 1.0, lambda, s.Dt_h, s.Dt_l, nseg, mc.ldDt, kblock ? &s.Dk_h : nullptr,
+    mx_update_shadow_rowmajor(D, G, 1.0, lam, s.Dt_h, s.Dt_l, nseg, mc.ldDt, kblock ? &s.Dk_h : nullptr,
                               kblock ? &s.Dk_l : nullptr);
     mc.dir_src = D.p;
     mc.dir_nseg = nseg;
@@ -1323,7 +1318,8 @@ int omm_run(int m, int n, msw_matrix* H, msw_matrix* S, bool new_S, double* e_mi
     // if stage 2 does not converge).  Each switch is a CG restart from C.  Convergence
     // is tested (e_diff <= cg_tol, omm.F90:506) only in stages 2 and 3.
     MixedCtx mc;
-    s.de_ok = s.xr_ok = s.xc_ok = false;  // no exponents carried over from an earlier call
+    s.de_ok = s.xr_ok = s.xc_ok = s.lg_ok = false;  // nothing carried over from an earlier call
+    s.lam.ensure(sizeof(double));
     // complex problems take the reduced-precision stages with dense H and S (the tensor-core
     // SpMM is real only)
     const bool lowp_ok = c.real || (!c.H_csc && (c.s_identity || !c.S_csc));
@@ -1399,13 +1395,12 @@ int omm_run(int m, int n, msw_matrix* H, msw_matrix* S, bool new_S, double* e_mi
     double e_diff = 0.0;
     int outer_i = 0;
     for (outer_i = 1; outer_i <= n_step_max_outer; ++outer_i) {
-        double lambda = 0.0;
+        const double* lam = nullptr;  // lambda in device memory; null: 0
         for (long j = 1; j <= n_step_max_inner; ++j) {
-            double lam[2] = {lambda, 0.0};
             s.de_ok = false;
-            if (c.use_precon) k_axpby(PG, 'n', D, ONE, lam);
-            else if (stage < 3) mx_update_dir(c, mc, D, G, lambda, nseg_of(stage));
-            else fp64_dir_update(c, G, D, lambda);
+            if (c.use_precon) k_axpby(PG, 'n', D, ONE, ZERO, lam);
+            else if (stage < 3) mx_update_dir(c, mc, D, G, lam, nseg_of(stage));
+            else fp64_dir_update(c, G, D, lam);
             std::swap(G, Gp);  // G_p = G; G is recomputed before it is read again
             if (c.use_precon) std::swap(PG, PGp);
             double e_min_old = e_min;
@@ -1416,26 +1411,15 @@ int omm_run(int m, int n, msw_matrix* H, msw_matrix* S, bool new_S, double* e_mi
             double x;
             solve_quartic(coeff, &x, &ls_fail);
             g_cur->x_min[ip] = x;
-            double xz[2] = {x, 0.0}, x2[2] = {x * x, 0.0};
+            double xz[2] = {x, 0.0};
             if (ls_fail) {
                 if (log.f) log.line("| WARNING: Rescaling coefficients!            |");
                 e_min = 3.0 * e_min;
-                double h[2] = {0.5, 0.0};
-                k_scale(Cw, h);
-                if (c.s_identity) k_scale(SC, h);  // the S half mirrors C
-                s.xr_ok = s.xc_ok = false;
                 ls_conv = false;
                 g_stats.ls_fail++;
             } else {
                 e_min = coeff[4] * (x * x) * (x * x) + coeff[3] * x * x * x + coeff[2] * x * x + coeff[1] * x + coeff[0];
-                k_axpby(D, 'n', Cw, xz, ONE);
                 ls_conv = true;
-            }
-            if (ls_fail) {
-                double q[2] = {0.25, 0.0};
-                k_scale(SW, q);
-            } else {
-                k_w_update(SW, view(s.Wd, n, n, 2 * n, c.real, n), view(s.Wdd, n, n, 2 * n, c.real, n), x);
             }
             e_diff = 2.0 * std::fabs((e_min - e_min_old) / (e_min + e_min_old));
             if (log.f && long_out) {
@@ -1444,50 +1428,68 @@ int omm_run(int m, int n, msw_matrix* H, msw_matrix* S, bool new_S, double* e_mi
                 log.line(b);
             }
             ++icg;
+            // end of a stage: converged to its tolerance, reached its noise floor (the
+            // energy rose), a failed line search, or a step cap
+            bool next = false;
             if (stage < 3) {
                 if (stage < 2) g_stats.icg_low++;
                 else g_stats.icg_fp64++;
                 ++stage_steps;
-                // end of a stage: converged to its tolerance, reached its noise floor (the
-                // energy rose), a failed line search, or a step cap
                 bool rose = (e_min > e_min_old) && !ls_fail;
                 bool done2 = (stage == 2) && e_diff <= refine_tol;
-                bool next = (stage < 2) ? (e_diff <= stage_tol[stage] || rose || ls_fail || stage_steps >= 400)
-                                        : (!done2 && (rose || ls_fail || stage_steps >= 8));
-                if (next) {
-                    stage = ls_fail ? 3 : stage + 1;
-                    stage_steps = 0;
-                    if (stage == 2) {
-                        // FP64 state, the refinement gradient, and the split X shadows for the
-                        // split-bf16 Gram products
-                        refresh_from_C(c, mc, Cw, G, -1, true);
-                    }
-                    else if (stage == 3) refresh_from_C(c, mc, Cw, G, 0, true);
-                    else refresh_from_C(c, mc, Cw, G, nseg_of(stage), false);
-                    e_min = energy_c0(c);
-                    if (log.f) {
-                        char b[128];
-                        snprintf(b, sizeof b, "| precision stage %d from step %5d, e_min %s |", stage, icg,
-                                 es15(e_min).c_str());
-                        log.line(b);
-                    }
-                    lambda = 0.0;  // CG restarts from the refreshed gradient
-                    continue;
-                }
+                next = (stage < 2) ? (e_diff <= stage_tol[stage] || rose || ls_fail || stage_steps >= 400)
+                                   : (!done2 && (rose || ls_fail || stage_steps >= 8));
             } else {
                 g_stats.icg_fp64++;
             }
-            if (stage == 2 ? e_diff <= refine_tol : (stage == 3 && e_diff <= cg_tol_internal)) {
+            const bool done = !next && (stage == 2 ? e_diff <= refine_tol : (stage == 3 && e_diff <= cg_tol_internal));
+            // C and the W matrices; a last step of a stage or of the solve leaves HW (and [HC; SC]) as they are
+            DView Wd2 = view(s.Wd, 2 * n, n, 2 * n, c.real), Wdd2 = view(s.Wdd, 2 * n, n, 2 * n, c.real);
+            const bool x_here = stage == 3 && !fp64_x_exps(c);  // [HC; SC] += x [HG; SG] in the same launch
+            if (ls_fail) {
+                double h[2] = {0.5, 0.0}, q[2] = {0.25, 0.0};
+                k_scale(Cw, h);
+                if (c.s_identity) k_scale(SC, h);  // the S half mirrors C
+                s.xr_ok = s.xc_ok = false;
+                k_scale(SW, q);
+            } else if (next || done) {
+                k_axpby(D, 'n', Cw, xz, ONE);
+                k_w_update(SW, view(s.Wd, n, n, 2 * n, c.real, n), view(s.Wdd, n, n, 2 * n, c.real, n), x);
+            } else {
+                DView X2 = view(s.X, 2 * n, m, 2 * n, c.real), Y2 = view(s.Y, 2 * n, m, 2 * n, c.real);
+                DView L = view(s.Lg, n, 2 * n, n, c.real);
+                k_cg_update(n, m, x, Cw, D, x_here ? &X2 : nullptr, x_here ? &Y2 : nullptr, HW, SW, Wd2, Wdd2,
+                            stage == 3 ? &L : nullptr);
+                s.lg_ok = stage == 3;
+                if (x_here) s.xr_ok = s.xc_ok = false;
+            }
+            if (next) {
+                stage = ls_fail ? 3 : stage + 1;
+                stage_steps = 0;
+                if (stage == 2) {
+                    // FP64 state, the refinement gradient, and the split X shadows for the
+                    // split-bf16 Gram products
+                    refresh_from_C(c, mc, Cw, G, -1, true);
+                }
+                else if (stage == 3) refresh_from_C(c, mc, Cw, G, 0, true);
+                else refresh_from_C(c, mc, Cw, G, nseg_of(stage), false);
+                e_min = energy_c0(c);
+                if (log.f) {
+                    char b[128];
+                    snprintf(b, sizeof b, "| precision stage %d from step %5d, e_min %s |", stage, icg,
+                             es15(e_min).c_str());
+                    log.line(b);
+                }
+                lam = nullptr;  // CG restarts from the refreshed gradient
+                continue;
+            }
+            if (done) {
                 conv = true;
                 break;
             }
             if (ls_fail) {
                 double q[2] = {0.25, 0.0};
                 k_scale(HW, q);
-            } else {
-                k_w_update(HW, view(s.Wd, n, n, 2 * n, c.real), view(s.Wdd, n, n, 2 * n, c.real), x);
-            }
-            if (ls_fail) {
                 double h[2] = {0.5, 0.0}, f15[2] = {1.5, 0.0};
                 k_scale(HC, h);
                 if (!c.s_identity) k_scale(SC, h);  // with S = I the S half was halved with C
@@ -1514,16 +1516,15 @@ int omm_run(int m, int n, msw_matrix* H, msw_matrix* S, bool new_S, double* e_mi
                     if (stage < 2) mx_calc_G(c, mc, G, ns);
                     else calc_G_refine(c, mc, G);
                 } else {
-                    fp64_x_update(c, x);  // with the exponents of X's rows and columns
+                    if (!x_here) fp64_x_update(c, x);  // with the exponents of X's rows and columns
                     calc_G(c, G);
                 }
             }
             if (c.use_precon) apply_precon(c, G, PG);  // omm.F90:535
             if (ls_conv) {
-                double tr[2];
-                if (c.use_precon) r_lambda(PG, G, Gp, PGp, tr);
-                else r_lambda(G, G, Gp, Gp, tr);
-                lambda = tr[0] / tr[1];
+                if (c.use_precon) r_lambda(PG, G, Gp, PGp, s.lam.as<double>());
+                else r_lambda(G, G, Gp, Gp, s.lam.as<double>());
+                lam = s.lam.as<double>();
             } else {
                 break;
             }

@@ -243,7 +243,9 @@ __device__ __forceinline__ int oz_exp_of_bits(unsigned long long b) {
 }
 __global__ void __launch_bounds__(256) oz_axpby_exps_kernel(int R, int K, double alpha, const double* __restrict__ x,
                                                             int ldx, double beta, double* __restrict__ y, int ldy,
-                                                            int W, int* __restrict__ erow, int* __restrict__ ecol) {
+                                                            int W, int* __restrict__ erow, int* __restrict__ ecol,
+                                                            const double* __restrict__ beta_at) {
+    if (beta_at) beta = *beta_at;
     const int lane = threadIdx.x & 31;
     const int gw = blockIdx.x * 8 + (threadIdx.x >> 5);
     if (gw >= W) return;
@@ -1706,7 +1708,8 @@ ModParams mod_params(int nmod) {
 
 }  // namespace oz
 
-void oz_axpby_exps(int R, int K, double alpha, const DView& X, double beta, DView& Y, int* erow, int* ecol) {
+void oz_axpby_exps(int R, int K, double alpha, const DView& X, double beta, DView& Y, int* erow, int* ecol,
+                   const double* beta_at) {
     using namespace oz;
     if (!X.is_real || !Y.is_real) fail(OMM_ERR_ARG, "oz_axpby_exps: real operands only");
     if (R == 0 || K == 0) return;
@@ -1720,7 +1723,7 @@ void oz_axpby_exps(int R, int K, double alpha, const DView& X, double beta, DVie
     const int W = std::max(nrb, sms * 64 / nrb * nrb);
     ktime_begin();
     oz_axpby_exps_kernel<<<(W + 7) / 8, 256, 0, st>>>(R, K, alpha, X.as<double>(), X.ld, beta, Y.as<double>(), Y.ld,
-                                                      W, erow, ecol);
+                                                      W, erow, ecol, beta_at);
     OMM_KCHECK();
     ktime_end("oz_axpby_exps_kernel", 24.0 * R * (double)K);
 }
