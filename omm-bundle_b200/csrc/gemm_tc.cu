@@ -8,14 +8,14 @@
 // operands) give a product accurate to ~2^-16 relative at three times the cost,
 // accumulated in the same TMEM tile.
 //
-// CTA = one 128 x 256 output tile, 4 warps:
-//   warp 0 lane 0   TMA producer: 64-wide K chunks of A (128 rows) and B (256
-//                   rows) into a 4-stage ring of 128B-swizzled shared buffers,
+// CTA = one 128 x BN output tile (BN = 256, 128 or 64, tile_form), 4 warps:
+//   warp 0 lane 0   TMA producer: 64-wide K chunks of A (128 rows) and B (BN
+//                   rows) into a ring of 4, 6 or 8 stages of 128B-swizzled buffers,
 //                   completion counted on full[s]
-//   warp 1 lane 0   MMA issuer: 4 x tcgen05.mma (M128 N256 K16) per chunk into
+//   warp 1 lane 0   MMA issuer: 4 x tcgen05.mma (M128 NBN K16) per chunk into
 //                   TMEM, tcgen05.commit frees the stage (empty[s]); a last
 //                   commit signals the accumulator (acc)
-//   warp 2          allocates / frees the 256 TMEM columns
+//   warp 2          allocates / frees the BN TMEM columns
 //   warps 0-3       epilogue: tcgen05.ld 32 lanes x 32 columns at a time, each
 //                   thread one row, coalesced column-major FP64 stores
 // Every mbarrier wait gives up after ~2 s of global time, sets the error flag
@@ -24,6 +24,7 @@
 #include "internal.h"
 
 #include <cuda.h>
+#include <cmath>
 #include <cudaTypedefs.h>
 
 #include <cstdint>
@@ -56,12 +57,15 @@ unsigned* tc_error_flag() {
 
 namespace tc {
 
-constexpr int BM = 128, BN = 256, BK = 64, STAGES = 4;
+constexpr int BM = 128, BK = 64;
 constexpr int A_BYTES = BM * BK * 2;  // 16 KB
-constexpr int B_BYTES = BN * BK * 2;  // 32 KB
-constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 /*alignment slack*/ + 256 /*barriers*/;
-constexpr uint32_t TMEM_COLS = 256;
+// The one-SM kernel's tiles are 128 x BN with BN = 256, 128 or 64 columns, each with as many stages as fit
+template <int BN>
+constexpr int stages() { return BN == 256 ? 4 : BN == 128 ? 6 : 8; }
+template <int BN>
+constexpr int stage_bytes() { return A_BYTES + BN * BK * 2; }
+template <int BN>
+constexpr int smem_bytes() { return stages<BN>() * stage_bytes<BN>() + 1024 /*alignment slack*/ + 256 /*barriers*/; }
 
 
 struct Params {
@@ -97,21 +101,25 @@ __device__ __forceinline__ uint64_t make_desc(uint32_t saddr) {
     d |= (uint64_t)2 << 61;                            // SWIZZLE_128B
     return d;
 }
-// instruction descriptor: kind::f16, A/B bf16, FP32 accumulate, both K-major, M=128, N=256
-constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
+// instruction descriptor: kind::f16, A/B bf16, FP32 accumulate, both K-major, M=128, N=BN
+template <int BN>
+constexpr uint32_t idesc() { return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24); }
 
-__device__ __forceinline__ void mma_f16(uint32_t tmem, uint64_t a, uint64_t b, uint32_t accumulate) {
+__device__ __forceinline__ void mma_f16(uint32_t tmem, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
         "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(
             tmem),
-        "l"(a), "l"(b), "r"(IDESC), "r"(accumulate)
+        "l"(a), "l"(b), "r"(idesc), "r"(accumulate)
         : "memory");
 }
 
+template <int BN>
 __global__ void __launch_bounds__(128, 1) gemm_bf16_kernel(const __grid_constant__ CUtensorMap tA0,
                                                            const __grid_constant__ CUtensorMap tA1,
                                                            const __grid_constant__ CUtensorMap tB0,
                                                            const __grid_constant__ CUtensorMap tB1, Params p) {
+    constexpr int STAGES = stages<BN>(), STAGE_BYTES = stage_bytes<BN>(), B_BYTES = BN * BK * 2;
+    constexpr uint32_t TMEM_COLS = BN;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     uint8_t* sA = smem;
@@ -197,7 +205,7 @@ __global__ void __launch_bounds__(128, 1) gemm_bf16_kernel(const __grid_constant
             const uint32_t a0 = smem_u32(sA + s * A_BYTES), b0 = smem_u32(sB + s * B_BYTES);
 #pragma unroll
             for (int kk = 0; kk < BK / 16; ++kk)
-                mma_f16(tmem, make_desc(a0 + kk * 32), make_desc(b0 + kk * 32), (t > 0 || kk > 0) ? 1u : 0u);
+                mma_f16(tmem, make_desc(a0 + kk * 32), make_desc(b0 + kk * 32), idesc<BN>(), (t > 0 || kk > 0) ? 1u : 0u);
             mma_commit(smem_u32(&empty[s]));
         }
         mma_commit(smem_u32(accb));  // arrives once every MMA issued above has completed
@@ -256,6 +264,7 @@ __global__ void __launch_bounds__(128, 1) gemm_bf16_kernel(const __grid_constant
 // the leader's full[s]) and run the epilogue of their own rows.  Waits are bounded as above; the
 // pair meets at a cluster barrier before TMEM is freed.
 constexpr int BM2 = 256, BN2 = 256, STAGES2 = 6;
+constexpr uint32_t TMEM_COLS = 256;
 constexpr int HALF_BYTES = 128 * BK * 2;            // 16 KB: 128 rows of a 64-wide bf16 K chunk
 constexpr int STAGE2_BYTES = 2 * HALF_BYTES;        // this CTA's A half + B half
 constexpr int SMEM2_BYTES = STAGES2 * STAGE2_BYTES + 1024 + 256;
@@ -440,6 +449,33 @@ CUtensorMap tma_map_bf16(const void* base, int rows, int cols, int ld, int box_c
     return m;
 }
 
+namespace tc {
+// Tiles of an M x N product over `slabs` 64-wide K slabs: 0 = 256 x 256 on SM pairs, else 128 x (256, 128 or
+// 64) on single SMs -- the one with the smallest estimated time.  A slab costs a CTA 0.45 us in a pair and
+// 0.48, 0.39, 0.33 us alone (the copies' rate into one SM, not the MMAs, decides below 256 columns), a tile
+// its FP64 epilogue besides; narrow tiles win where wide ones leave most SMs idle (1,296 x 648 x 5,184: 36 us
+// against 45; 750 x 375 x 3,000: 24 against 37), wide ones beyond a wave (3,072 x 1,536 x 12,288: 88 us, 265
+// with 64 columns).  All forms add up K in the same order: the results are the same bits.
+int tile_form(int M, int N, int slabs, int herm) {
+    static int sms = 0;
+    if (!sms) OMM_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, rt().device));
+    auto time = [&](int bm, int bn, int units, double slab, double tail) {
+        double tiles = std::ceil((double)M / bm) * std::ceil((double)N / bn);
+        if (herm > 0) tiles *= 0.55;
+        return std::ceil(tiles / units) * (slabs * slab + tail);
+    };
+    int best = 256;
+    double us = time(BM, 256, sms, 0.48, 10.4);
+    const double t128 = time(BM, 128, sms, 0.39, 7.7), t64 = time(BM, 64, sms, 0.33, 6.3);
+    if (t128 < us) best = 128, us = t128;
+    if (t64 < us) best = 64, us = t64;
+    if (tc_pairs_enabled() && M > BM && (herm == 0 || herm % BM2 == 0) &&
+        time(BM2, BN2, sms / 2, 0.45, 12.0) < 1.03 * us)
+        best = 0;
+    return best;
+}
+}  // namespace tc
+
 // out (FP64, M x N, column-major, ldo) = alpha * sum_seg A_seg B_seg^T + beta * out.
 // nseg = 1: A_hi B_hi^T.  nseg = 3: A_hi B_hi^T + A_hi B_lo^T + A_lo B_hi^T.
 void gemm_bf16_tn(int M, int N, int K, const __nv_bfloat16* A_hi, const __nv_bfloat16* A_lo, int lda,
@@ -454,16 +490,21 @@ void gemm_bf16_tn(int M, int N, int K, const __nv_bfloat16* A_hi, const __nv_bfl
     if (nseg != 1 && nseg != 3) fail(OMM_ERR_ARG, "gemm_bf16: nseg must be 1 or 3");
     if (nseg == 3 && (!A_lo || !B_lo || (((uintptr_t)A_lo | (uintptr_t)B_lo) & 15)))
         fail(OMM_ERR_ARG, "gemm_bf16: split operands missing or misaligned");
-    // SM pairs (256 x 256 tiles) unless a Hermitian block would split a pair's rows
-    const bool pairs = tc_pairs_enabled() && M > BM && (herm == 0 || herm % BM2 == 0);
-    const int brows = pairs ? 128 : BN;
+    const int form = tile_form(M, N, (K + BK - 1) / BK * nseg, herm);
+    const bool pairs = form == 0;
+    const int brows = pairs ? 128 : form;
     CUtensorMap a0 = make_map(A_hi, M, K, lda, BM), b0 = make_map(B_hi, N, K, ldb, brows);
     CUtensorMap a1 = nseg == 3 ? make_map(A_lo, M, K, lda, BM) : a0;
     CUtensorMap b1 = nseg == 3 ? make_map(B_lo, N, K, ldb, brows) : b0;
     static bool attr = false;
     if (!attr) {
-        OMM_CK(cudaFuncSetAttribute(gemm_bf16_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
-        OMM_CK(cudaFuncSetAttribute(gemm_bf16_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM2_BYTES));
+        auto set = [](const void* f, int bytes) {
+            OMM_CK(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+        };
+        set((const void*)gemm_bf16_kernel<256>, smem_bytes<256>());
+        set((const void*)gemm_bf16_kernel<128>, smem_bytes<128>());
+        set((const void*)gemm_bf16_kernel<64>, smem_bytes<64>());
+        set((const void*)gemm_bf16_pair_kernel, SMEM2_BYTES);
         attr = true;
     }
     Params p{M, N, K, nseg, alpha, beta, out, ldo, err_flag(), herm, tc_wait_cfg()};
@@ -472,8 +513,10 @@ void gemm_bf16_tn(int M, int N, int K, const __nv_bfloat16* A_hi, const __nv_bfl
         dim3 grid(2 * ((M + BM2 - 1) / BM2), (N + BN2 - 1) / BN2);
         gemm_bf16_pair_kernel<<<grid, 128, SMEM2_BYTES, rt().stream>>>(a0, a1, b0, b1, p);
     } else {
-        dim3 grid((M + BM - 1) / BM, (N + BN - 1) / BN);
-        gemm_bf16_kernel<<<grid, 128, SMEM_BYTES, rt().stream>>>(a0, a1, b0, b1, p);
+        dim3 grid((M + BM - 1) / BM, (N + form - 1) / form);
+        if (form == 256) gemm_bf16_kernel<256><<<grid, 128, smem_bytes<256>(), rt().stream>>>(a0, a1, b0, b1, p);
+        else if (form == 128) gemm_bf16_kernel<128><<<grid, 128, smem_bytes<128>(), rt().stream>>>(a0, a1, b0, b1, p);
+        else gemm_bf16_kernel<64><<<grid, 128, smem_bytes<64>(), rt().stream>>>(a0, a1, b0, b1, p);
     }
     OMM_KCHECK();
     ktime_end(pairs ? "gemm_bf16_pair_kernel" : "gemm_bf16_kernel",
