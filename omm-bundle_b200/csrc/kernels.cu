@@ -255,13 +255,14 @@ __device__ inline void comp_add(double& s, double& c, double s2, double c2) {
 __device__ unsigned g_reduce_done;
 
 // Every block stores its K partial sums; the block that arrives last adds the nb records up with
-// compensation, in a fixed order (each thread a strided share, then a tree over the warp's lanes,
-// then the warps in turn), so the result does not depend on timing, and writes it to `out` (pinned
-// host memory, or device memory for sums the host does not need).  True in that block.  (A second kernel for the sum and a copy of its result cost 4 + 3 us and their gaps
-// in each of a CG step's two reductions.)
+// compensation, in a fixed order (a warp per value: each lane strided shares, then a tree over the
+// lanes), so the result does not depend on timing, and writes it to `out` (pinned
+// host memory, or device memory for sums the host does not need).  True in that block.  (A second kernel
+// for the sum and a copy of its result cost 4 + 3 us and their gaps in each of a CG step's two
+// reductions; all 13 values in every thread's registers, 4 us of the coefficients' last block.)
 template <int K>
 __device__ inline bool block_reduce_finish(double (&v)[K], double* part, double* out) {
-    __shared__ double sm[K][kThreads / 32], s_cmp[K][kThreads / 32];
+    __shared__ double sm[K][kThreads / 32];
     __shared__ bool last;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nb = (int)gridDim.x;
 #pragma unroll
@@ -282,29 +283,25 @@ __device__ inline bool block_reduce_finish(double (&v)[K], double* part, double*
     __syncthreads();
     if (!last) return false;
     __threadfence();
-    double s[K], c[K];
+    // warp w takes the values w, w + 8: its lanes strided shares of the records, four in flight, then a tree
 #pragma unroll
-    for (int k = 0; k < K; ++k) s[k] = c[k] = 0.0;
-    for (int b = threadIdx.x; b < nb; b += blockDim.x)
+    for (int k = w; k < K; k += kThreads / 32) {
+        double s[4] = {0.0, 0.0, 0.0, 0.0}, c[4] = {0.0, 0.0, 0.0, 0.0};
+        for (int b0 = lane; b0 < nb; b0 += 128) {
+            double x[4];
 #pragma unroll
-        for (int k = 0; k < K; ++k) comp_add(s[k], c[k], __ldcg(part + (size_t)b * K + k), 0.0);
+            for (int u = 0; u < 4; ++u) x[u] = b0 + 32 * u < nb ? __ldcg(part + (size_t)(b0 + 32 * u) * K + k) : 0.0;
 #pragma unroll
-    for (int k = 0; k < K; ++k) {
+            for (int u = 0; u < 4; ++u) comp_add(s[u], c[u], x[u], 0.0);
+        }
+        comp_add(s[0], c[0], s[1], c[1]);
+        comp_add(s[2], c[2], s[3], c[3]);
+        comp_add(s[0], c[0], s[2], c[2]);
         for (int o = 16; o > 0; o >>= 1) {
-            const double s2 = __shfl_down_sync(0xffffffffu, s[k], o), c2 = __shfl_down_sync(0xffffffffu, c[k], o);
-            comp_add(s[k], c[k], s2, c2);
+            const double s2 = __shfl_down_sync(0xffffffffu, s[0], o), c2 = __shfl_down_sync(0xffffffffu, c[0], o);
+            comp_add(s[0], c[0], s2, c2);
         }
-        if (lane == 0) {
-            sm[k][w] = s[k];
-            s_cmp[k][w] = c[k];
-        }
-    }
-    __syncthreads();
-    if (threadIdx.x < K) {
-        const int k = threadIdx.x;
-        double S = 0.0, C = 0.0;
-        for (int i = 0; i < (int)(blockDim.x / 32); ++i) comp_add(S, C, sm[k][i], s_cmp[k][i]);
-        out[k] = S + C;
+        if (lane == 0) out[k] = s[0] + c[0];
     }
     return true;
 }
@@ -611,6 +608,10 @@ void finish_reduce(int K, double* out) {
     for (int k = 0; k < K; ++k) out[k] = rt().host_pinned[k];
 }
 
+// blocks of a reduction: eight elements per thread, at most six blocks per SM (a block's own sums, its
+// fence and its record cost as much as some 30 elements per thread)
+inline int reduce_grid(size_t elems) { return std::min(grid_for(elems, 8), 148 * 6); }
+
 // blocks of a kernel that takes 32 x 32 tiles in turn
 inline int tile_grid(int rows, int cols) {
     const long long t = (long long)((rows + 31) / 32) * ((cols + 31) / 32);
@@ -728,7 +729,7 @@ void r_trace(const DView& A, double out[2]) {
 
 void r_dot(const DView& A, const DView& B, double out[2]) {
     size_t tot = (size_t)A.rows * A.cols;
-    int nb = grid_for(tot, 8);
+    int nb = reduce_grid(tot);
     double* part = scratch_partials(nb + 1, 2);
     if (A.is_real)
         dot_kernel<double><<<nb, kThreads, 0, rt().stream>>>(A.rows, A.cols, A.as<double>(), A.ld, B.as<double>(), B.ld, part,
@@ -770,7 +771,7 @@ void r_coeff(const DView& HW, const DView& SW, const DView& HWd, const DView& SW
 
 void r_lambda(const DView& PG, const DView& G, const DView& Gp, const DView& PGp, double* lambda) {
     size_t tot = (size_t)G.rows * G.cols;
-    int nb = grid_for(tot, 8);
+    int nb = reduce_grid(tot);
     double* part = scratch_partials(nb + 1, 2);
     const bool same = PG.p == G.p && PG.ld == G.ld && PGp.p == Gp.p && PGp.ld == Gp.ld;
     auto launch = [&](auto tag, auto kernel) {

@@ -44,58 +44,99 @@ __device__ __forceinline__ void split_bf16(double x, __nv_bfloat16& hi, __nv_bfl
 // lo / klo / clo (when given) receive the low bf16 parts of the hi/lo split.
 // With add != nullptr, src is first updated in place, src = b*src + a*add (the expression of
 // axpby_kernel), and the shadows are those of the updated values.
+// One 64 x 64 tile per CTA: a lane takes two rows of four columns at a time, all their loads first; the
+// hi/lo parts are formed once, packed as a word per element in shared memory, and every store of a warp
+// covers whole 128-byte lines of the row- and column-major shadows (32 x 32 tiles of FP64 values with one
+// load at a time and 64-byte stores took 40 us where this takes 27: [HC; SC] of 1,296 x 5,184; all eight
+// columns of a lane at once needed 110 registers and 53 us).
+constexpr int SH_T = 64, SH_LD = SH_T + 1;
 template <typename TA>
-__global__ void shadow_rowmajor_kernel(int rows, int cols, double* __restrict__ src, int lds,
-                                       const TA* __restrict__ add, int ldadd, double a, double b,
-                                       __nv_bfloat16* __restrict__ hi, __nv_bfloat16* __restrict__ lo, int ldd,
-                                       __nv_bfloat16* __restrict__ khi, __nv_bfloat16* __restrict__ klo,
-                                       __nv_bfloat16* __restrict__ chi, __nv_bfloat16* __restrict__ clo, int ldc,
-                                       const double* __restrict__ b_at = nullptr) {
-    __shared__ double tile[32][33];
+__global__ void __launch_bounds__(256, 4) shadow_rowmajor_kernel(
+    int rows, int cols, double* __restrict__ src, int lds, const TA* __restrict__ add, int ldadd, double a, double b,
+    __nv_bfloat16* __restrict__ hi, __nv_bfloat16* __restrict__ lo, int ldd, __nv_bfloat16* __restrict__ khi,
+    __nv_bfloat16* __restrict__ klo, __nv_bfloat16* __restrict__ chi, __nv_bfloat16* __restrict__ clo, int ldc,
+    const double* __restrict__ b_at = nullptr) {
+    __shared__ uint32_t tile[SH_T * SH_LD];  // element (row, k) at k SH_LD + row: hi | lo << 16
     if (b_at) b = *b_at;
-    int i0 = blockIdx.x * 32, k0 = blockIdx.y * 32;
-    int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;  // 32 x 8
-    for (int yy = ty; yy < 32; yy += 8) {
-        int i = i0 + tx, k = k0 + yy;
-        double v = 0.0;
-        if (i < rows && k < cols) {
-            v = src[(size_t)i + (size_t)k * lds];
-            if (add) {
-                const double c = b * v;
-                v = c + a * (double)add[(size_t)i + (size_t)k * ldadd];
-                src[(size_t)i + (size_t)k * lds] = v;
-            }
-            if (chi) {
-                __nv_bfloat16 h, l;
-                split_bf16(v, h, l);
-                chi[(size_t)i + (size_t)k * ldc] = h;
-                if (clo) clo[(size_t)i + (size_t)k * ldc] = l;
+    const int i0 = blockIdx.x * SH_T, k0 = blockIdx.y * SH_T;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int i = i0 + lane;  // and i + 32
+#pragma unroll 1
+    for (int q0 = 0; q0 < 8; q0 += 4) {
+        double v[4][2];
+        TA w[4][2];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int k = k0 + warp + 8 * (q0 + q);
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                v[q][h] = 0.0;
+                if (i + 32 * h < rows && k < cols) {
+                    v[q][h] = src[(size_t)(i + 32 * h) + (size_t)k * lds];
+                    if (add) w[q][h] = add[(size_t)(i + 32 * h) + (size_t)k * ldadd];
+                }
             }
         }
-        tile[yy][tx] = v;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int kk = warp + 8 * (q0 + q), k = k0 + kk;
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                if (add && i + 32 * h < rows && k < cols) {
+                    const double c = b * v[q][h];
+                    v[q][h] = c + a * (double)w[q][h];
+                    src[(size_t)(i + 32 * h) + (size_t)k * lds] = v[q][h];
+                }
+                __nv_bfloat16 x, y;
+                split_bf16(v[q][h], x, y);
+                tile[kk * SH_LD + lane + 32 * h] =
+                    (uint32_t)__bfloat16_as_ushort(x) | (uint32_t)__bfloat16_as_ushort(y) << 16;
+            }
+        }
     }
     __syncthreads();
-    if (hi) {
-        for (int yy = ty; yy < 32; yy += 8) {
-            int i = i0 + yy, k = k0 + tx;
-            if (i < rows && k < cols) {
-                __nv_bfloat16 h, l;
-                split_bf16(tile[tx][yy], h, l);
-                hi[(size_t)i * ldd + k] = h;
-                if (lo) lo[(size_t)i * ldd + k] = l;
+    if (chi) {
+        const int r = 2 * lane;  // ldc is a multiple of 8: the pair's second row is at worst padding
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            const int kk = warp + 8 * q, k = k0 + kk;
+            if (i0 + r < rows && k < cols) {
+                const uint32_t x = tile[kk * SH_LD + r], y = tile[kk * SH_LD + r + 1];
+                *reinterpret_cast<uint32_t*>(chi + (size_t)(i0 + r) + (size_t)k * ldc) = __byte_perm(x, y, 0x5410);
+                if (clo) *reinterpret_cast<uint32_t*>(clo + (size_t)(i0 + r) + (size_t)k * ldc) = __byte_perm(x, y, 0x7632);
             }
         }
     }
-    if (khi && threadIdx.x < 128) {
-        const int r = threadIdx.x & 31, q = threadIdx.x >> 5;  // row of the tile, 8-k block of the tile
-        const int i = i0 + r, kb = (k0 >> 3) + q;
-        if (i < rows && 8 * kb < cols) {
-            __align__(16) __nv_bfloat16 h[8], l[8];
+    if (hi) {
+        const int k = k0 + 2 * lane;
 #pragma unroll
-            for (int e = 0; e < 8; ++e) split_bf16(tile[8 * q + e][r], h[e], l[e]);
-            const size_t off = kblock_offset(i, 8 * kb, cols);
-            *reinterpret_cast<uint4*>(khi + off) = *reinterpret_cast<const uint4*>(h);
-            if (klo) *reinterpret_cast<uint4*>(klo + off) = *reinterpret_cast<const uint4*>(l);
+        for (int q = 0; q < 8; ++q) {
+            const int r = warp + 8 * q;
+            if (i0 + r < rows && k < cols) {
+                const uint32_t x = tile[2 * lane * SH_LD + r], y = tile[(2 * lane + 1) * SH_LD + r];
+                *reinterpret_cast<uint32_t*>(hi + (size_t)(i0 + r) * ldd + k) = __byte_perm(x, y, 0x5410);
+                if (lo) *reinterpret_cast<uint32_t*>(lo + (size_t)(i0 + r) * ldd + k) = __byte_perm(x, y, 0x7632);
+            }
+        }
+    }
+    if (khi) {
+        const int kb = (k0 >> 3) + warp;  // 8-k block of the matrix
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int r = lane + 32 * h, row = i0 + r;
+            if (row < rows && 8 * kb < cols) {
+                uint32_t x[8], p[4], q[4];
+#pragma unroll
+                for (int e = 0; e < 8; ++e) x[e] = tile[(8 * warp + e) * SH_LD + r];
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    p[e] = __byte_perm(x[2 * e], x[2 * e + 1], 0x5410);
+                    q[e] = __byte_perm(x[2 * e], x[2 * e + 1], 0x7632);
+                }
+                const size_t off = kblock_offset(row, 8 * kb, cols);
+                *reinterpret_cast<uint4*>(khi + off) = make_uint4(p[0], p[1], p[2], p[3]);
+                if (klo) *reinterpret_cast<uint4*>(klo + off) = make_uint4(q[0], q[1], q[2], q[3]);
+            }
         }
     }
 }
@@ -122,19 +163,34 @@ __global__ void to_f32_kernel(int rows, int cols, const double* __restrict__ src
     }
 }
 
-// Lt (row-major n x 2n, row stride ldl): row i = [4I - 2 SW, -2 HW](i, :)  (calc_G's left factor)
-__global__ void calcG_left_bf16_kernel(int n, const double* __restrict__ SW, const double* __restrict__ HW,
-                                       __nv_bfloat16* __restrict__ hi, __nv_bfloat16* __restrict__ lo, int ldl) {
-    size_t tot = (size_t)n * 2 * n;
-    for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < tot; e += (size_t)gridDim.x * blockDim.x) {
-        int k = (int)(e % (2 * n)), i = (int)(e / (2 * n));  // consecutive threads along a row of Lt
-        double v;
-        if (k < n) v = (i == k ? 4.0 : 0.0) - 2.0 * SW[i + (size_t)k * n];
-        else v = -2.0 * HW[i + (size_t)(k - n) * n];
+// Lt (row-major n x 2n, row stride ldl): row i = [4I - 2 SW, -2 HW](i, :)  (calc_G's left factor), a 32 x 32
+// tile at a time through shared memory (SW and HW are column-major)
+__global__ void __launch_bounds__(256) calcG_left_bf16_kernel(int n, const double* __restrict__ SW,
+                                                              const double* __restrict__ HW, __nv_bfloat16* __restrict__ hi,
+                                                              __nv_bfloat16* __restrict__ lo, int ldl) {
+    __shared__ uint32_t tile[32][33];
+    const int i0 = blockIdx.x * 32, k0 = blockIdx.y * 32, tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const int i = i0 + tx, k = k0 + ty + 8 * q;
+        double v = 0.0;
+        if (i < n && k < 2 * n) {
+            if (k < n) v = (i == k ? 4.0 : 0.0) - 2.0 * SW[i + (size_t)k * n];
+            else v = -2.0 * HW[i + (size_t)(k - n) * n];
+        }
         __nv_bfloat16 h, l;
         split_bf16(v, h, l);
-        hi[(size_t)i * ldl + k] = h;
-        if (lo) lo[(size_t)i * ldl + k] = l;
+        tile[ty + 8 * q][tx] = (uint32_t)__bfloat16_as_ushort(h) | (uint32_t)__bfloat16_as_ushort(l) << 16;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const int i = i0 + ty + 8 * q, k = k0 + tx;
+        if (i < n && k < 2 * n) {
+            const uint32_t x = tile[tx][ty + 8 * q];
+            hi[(size_t)i * ldl + k] = __ushort_as_bfloat16((unsigned short)x);
+            if (lo) lo[(size_t)i * ldl + k] = __ushort_as_bfloat16((unsigned short)(x >> 16));
+        }
     }
 }
 
@@ -276,7 +332,7 @@ void mx_shadow_rowmajor(const DView& src, DevBuf& hi, DevBuf& lo, int nseg, int&
         ensure_kblock(*khi, src.rows, src.cols);
         if (nseg == 3) ensure_kblock(*klo, src.rows, src.cols);
     }
-    dim3 grid((src.rows + 31) / 32, (src.cols + 31) / 32);
+    dim3 grid((src.rows + SH_T - 1) / SH_T, (src.cols + SH_T - 1) / SH_T);
     shadow_rowmajor_kernel<double><<<grid, 256, 0, rt().stream>>>(
         src.rows, src.cols, src.as<double>(), src.ld, nullptr, 0, 0.0, 1.0, hi.as<__nv_bfloat16>(),
         nseg == 3 ? lo.as<__nv_bfloat16>() : nullptr, ldd, khi ? khi->as<__nv_bfloat16>() : nullptr,
@@ -298,7 +354,7 @@ void mx_update_shadow_rowmajor(DView& D, const DView& G, double a, const double*
         ensure_kblock(*khi, D.rows, D.cols);
         if (nseg == 3) ensure_kblock(*klo, D.rows, D.cols);
     }
-    dim3 grid((D.rows + 31) / 32, (D.cols + 31) / 32);
+    dim3 grid((D.rows + SH_T - 1) / SH_T, (D.cols + SH_T - 1) / SH_T);
     shadow_rowmajor_kernel<double><<<grid, 256, 0, rt().stream>>>(
         D.rows, D.cols, D.as<double>(), D.ld, G.as<double>(), G.ld, a, 0.0, hi.as<__nv_bfloat16>(),
         nseg == 3 ? lo.as<__nv_bfloat16>() : nullptr, ldd, khi ? khi->as<__nv_bfloat16>() : nullptr,
@@ -322,7 +378,7 @@ void mx_update_shadows(DView& X, const DView& Y, double a, DevBuf& thi, DevBuf& 
         ensure(tlo, tb);
         ensure(clo, cb);
     }
-    dim3 grid((X.rows + 31) / 32, (X.cols + 31) / 32);
+    dim3 grid((X.rows + SH_T - 1) / SH_T, (X.cols + SH_T - 1) / SH_T);
     if (Y32)
         shadow_rowmajor_kernel<float><<<grid, 256, 0, rt().stream>>>(
             X.rows, X.cols, X.as<double>(), X.ld, Y32, ldy32, a, 1.0, thi.as<__nv_bfloat16>(),
@@ -339,7 +395,7 @@ void mx_update_shadows(DView& X, const DView& Y, double a, DevBuf& thi, DevBuf& 
 void mx_shadow_kblock(const DView& src, DevBuf& khi, DevBuf& klo, int nseg) {
     ensure_kblock(khi, src.rows, src.cols);
     if (nseg == 3) ensure_kblock(klo, src.rows, src.cols);
-    dim3 grid((src.rows + 31) / 32, (src.cols + 31) / 32);
+    dim3 grid((src.rows + SH_T - 1) / SH_T, (src.cols + SH_T - 1) / SH_T);
     shadow_rowmajor_kernel<double><<<grid, 256, 0, rt().stream>>>(src.rows, src.cols, src.as<double>(), src.ld, nullptr, 0,
                                                           0.0, 1.0, nullptr, nullptr, 0, khi.as<__nv_bfloat16>(),
                                                           nseg == 3 ? klo.as<__nv_bfloat16>() : nullptr, nullptr,
@@ -419,7 +475,7 @@ void mx_calcG_left(int n, const DView& SW, const DView& HW, DevBuf& hi, DevBuf& 
     size_t bytes = (size_t)n * ldl * sizeof(__nv_bfloat16);
     ensure(hi, bytes);
     if (nseg == 3) ensure(lo, bytes);
-    calcG_left_bf16_kernel<<<grid1d((size_t)n * 2 * n), 256, 0, rt().stream>>>(
+    calcG_left_bf16_kernel<<<dim3((n + 31) / 32, (2 * n + 31) / 32), 256, 0, rt().stream>>>(
         n, SW.as<double>(), HW.as<double>(), hi.as<__nv_bfloat16>(), nseg == 3 ? lo.as<__nv_bfloat16>() : nullptr,
         ldl);
     OMM_KCHECK();
