@@ -311,7 +311,7 @@ void launch_t(const DgArgs& a, int nz, int split) {
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim = {1, 1, (unsigned)split};
     cfg.attrs = at;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = split > 1 ? 1 : 0;
     OMM_CK(cudaLaunchKernelEx(&cfg, kernel, a));
     OMM_KCHECK();
 }

@@ -150,6 +150,7 @@ class Matrix:
         self.h = ct.c_void_p(handle)
         self._keep = keep  # host/device memory aliased by the handle
         self._owned = owned  # False for handles the library lends (omm_callback's C and HC)
+        self._dims = None
 
     def __del__(self):
         try:
@@ -253,9 +254,12 @@ class Matrix:
 
     # ---------------------------------------------------------- accessors
     def dims(self):
-        d1, d2, z, s = ct.c_int(), ct.c_int(), ct.c_int(), ct.c_int()
-        _check(lib().msw_dims(self.h, ct.byref(d1), ct.byref(d2), ct.byref(z), ct.byref(s)))
-        return d1.value, d2.value, bool(z.value), bool(s.value)
+        """(rows, columns, complex, sparse); fixed for a handle's life, so asked of the library once."""
+        if self._dims is None:
+            d1, d2, z, s = ct.c_int(), ct.c_int(), ct.c_int(), ct.c_int()
+            _check(lib().msw_dims(self.h, ct.byref(d1), ct.byref(d2), ct.byref(z), ct.byref(s)))
+            self._dims = d1.value, d2.value, bool(z.value), bool(s.value)
+        return self._dims
 
     @property
     def shape(self):
