@@ -177,7 +177,7 @@ Runtime& rt() {
         OMM_CKB(cublasSetStream(g_rt->blas, g_rt->stream));
         OMM_CKS(cusolverDnCreate(&g_rt->solver));
         OMM_CKS(cusolverDnSetStream(g_rt->solver, g_rt->stream));
-        OMM_CK(cudaMallocHost((void**)&g_rt->host_pinned, 64 * sizeof(double)));
+        OMM_CK(cudaMallocHost((void**)&g_rt->host_pinned, (64 + 16 * kStepRecords) * sizeof(double)));
     }
     return *g_rt;
 }
@@ -187,6 +187,7 @@ bool runtime_bound() {
 }
 static double g_sync_wait = 0.0;
 double sync_wait_seconds() { return g_sync_wait; }
+void add_sync_wait(double seconds) { g_sync_wait += seconds; }
 void sync() {
     auto t0 = std::chrono::steady_clock::now();
     OMM_CK(cudaStreamSynchronize(rt().stream));

@@ -47,6 +47,7 @@ struct DgArgs {
     int vec;      // 16-byte copies of A and B (real: even leading dimensions and 16-byte addresses)
     int herm[2];  // rows per Hermitian block of C_z (0: none): both triangles from the upper tiles
     int kper;     // k per CTA of the cluster (a multiple of the chunk)
+    const int* stop;
 };
 
 template <bool CPLX> struct El { using T = double; };
@@ -135,6 +136,7 @@ __global__ void __launch_bounds__(32 * WM * WN * WK) gemm_dmma_kernel(const __gr
     using T = typename El<CPLX>::T;
     constexpr int BK = chunk<CPLX>(), MT = BM / (8 * WM), NT = BN / (8 * WN), NP = CPLX ? 2 : 1, NTHR = 32 * WM * WN * WK;
     constexpr int AE = tile_elems<CPLX, BM, TA>(), BE = tile_elems<CPLX, BN, !TB>();
+    if (p.stop && *p.stop) return;
     extern __shared__ __align__(16) unsigned char raw[];
     T* ring = reinterpret_cast<T*>(raw);
     const int tm = (p.M + BM - 1) / BM;
@@ -353,7 +355,7 @@ double gemm_dmma_us(bool cplx, int M, int N, int K, int nz) { return pick(cplx, 
 bool gemm_dmma_takes(const DView& v) { return v.is_real || (reinterpret_cast<uintptr_t>(v.p) & 15) == 0; }
 
 void gemm_dmma(char opA, char opB, int M, int N, int K, const double alpha[2], const DView* A, const DView* B,
-               const double beta[2], DView* C, int nz, const int* herm) {
+               const double beta[2], DView* C, int nz, const int* herm, const int* stop) {
     if (M == 0 || N == 0) return;
     const bool cplx = !C[0].is_real;
     auto code = [](char o) { return o == 'n' || o == 'N' ? 0 : o == 't' || o == 'T' ? 1 : 2; };
@@ -362,6 +364,7 @@ void gemm_dmma(char opA, char opB, int M, int N, int K, const double alpha[2], c
     a.M = M;
     a.N = N;
     a.K = K;
+    a.stop = stop;
     a.lda = A[0].ld;
     a.ldb = B[0].ld;
     a.ldc = C[0].ld;

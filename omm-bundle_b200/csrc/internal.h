@@ -127,11 +127,14 @@ struct Runtime {
     DevBuf scratch;   // reduction partials and small temporaries
     DevBuf scratch2;  // transposes / staging
     double* host_pinned = nullptr;  // small pinned host buffer for scalar read-back
+    cudaGraphExec_t steps = nullptr;  // run_ahead's executable graph (omm.cu), updated by each call
+    long long steps_key[6] = {};      // the launches it was made for
 };
 Runtime& rt();
 bool runtime_bound();  // rt() has been set up on a device (no CUDA call is made to find out)
 void sync();
 double sync_wait_seconds();  // host time spent in sync() so far
+void add_sync_wait(double seconds);
 void pool_trim();  // return cached device blocks to the driver
 
 // ----------------------------------------------------------------- host memory
@@ -247,9 +250,20 @@ const msw_matrix* csc_transpose(const msw_matrix* A);
 
 // ----------------------------------------------------------------- kernels (kernels.cu)
 // Elementwise on column-major views; 'op' in {'n','t','c'} applies to A.
+// A line search solved in the coefficients' kernel.  state (device): [0] lambda, [1] x, [2] the energy, [3] the
+// steps evaluated; *stop is set when the host has to take over (at `most` steps at the latest).  record (pinned
+// host, kStepRecords of 16 doubles taken in turn): coeff[5], x, energy, e_diff, flag, the step's number from 1.
+constexpr int kStepRecords = 8;
+struct LineSearch {
+    double* state = nullptr;
+    int* stop = nullptr;
+    double tol = 0.0, most = 0.0;
+    double* record = nullptr;
+};
+// Kernels that take a `stop` flag do nothing once it is set.
 // beta_at: a device scalar that takes beta's place (op 'n' only)
 void k_axpby(const DView& A, char op, DView& C, const double alpha[2], const double beta[2],
-             const double* beta_at = nullptr);
+             const double* beta_at = nullptr, const int* stop = nullptr);
 void k_scale(DView& C, const double beta[2]);
 void k_set(DView& C, char seC, const double alpha[2], const double beta[2]);
 void k_set_element(DView& C, int i, int j, const double alpha[2], const double beta[2]);
@@ -261,13 +275,14 @@ void k_lcg_init(DView& C);                   // reference C0 (NORAND LCG), unsca
 void r_trace(const DView& A, double out[2]);                          // sum of diagonal
 void r_dot(const DView& A, const DView& B, double out[2]);            // sum conj(A) B
 void r_coeff(const DView& HW, const DView& SW, const DView& HWd, const DView& SWd, const DView& HWdd,
-             const DView& SWdd, double coeff[5]);                     // calc_coeff traces
+             const DView& SWdd, double coeff[5], const LineSearch* ls = nullptr);  // calc_coeff traces
 // lambda = mm_trace(PG, G - G_p) / mm_trace(PG_p, G_p), written to device memory without waiting
-void r_lambda(const DView& PG, const DView& G, const DView& Gp, const DView& PGp, double* lambda);
+void r_lambda(const DView& PG, const DView& G, const DView& Gp, const DView& PGp, double* lambda,
+              const int* stop = nullptr);
 // one CG step's C += x D, [X += x Y], HW and SW updates and [L = [4I - 2SW, -2HW]] in one launch (contiguous
-// C, D, X, Y; Wd, Wdd stacked with leading dimension 2n)
+// C, D, X, Y; Wd, Wdd stacked with leading dimension 2n); x_at: x in device memory
 void k_cg_update(int n, int m, double x, DView& C, const DView& D, DView* X, const DView* Y, DView& HW, DView& SW,
-                 const DView& Wd, const DView& Wdd, DView* L);
+                 const DView& Wd, const DView& Wdd, DView* L, const double* x_at = nullptr, const int* stop = nullptr);
 // dense products on cuBLAS (FP64 / complex FP64)
 void gemm(char opA, char opB, int M, int N, int K, const double alpha[2], const DView& A, const DView& B,
           const double beta[2], DView& C);
@@ -276,8 +291,9 @@ void transpose_into(const DView& A, char op, DView& T);  // T = op(A)
 // ----------------------------------------------------------------- FP64 products on the FP64 tensor cores (gemm_dmma.cu)
 // C_z = alpha op(A_z) op(B_z) + beta C_z for nz <= 2 products of one shape and set of leading dimensions;
 // herm[z] > 0: C_z is a stack of Hermitian blocks of that many rows, formed from their upper tiles.
+// Nothing is done when *stop (device memory, may be null) is set.
 void gemm_dmma(char opA, char opB, int M, int N, int K, const double alpha[2], const DView* A, const DView* B,
-               const double beta[2], DView* C, int nz = 1, const int* herm = nullptr);
+               const double beta[2], DView* C, int nz = 1, const int* herm = nullptr, const int* stop = nullptr);
 double gemm_dmma_us(bool cplx, int M, int N, int K, int nz = 1);  // its estimated time
 bool gemm_dmma_takes(const DView& v);  // complex operands must lie on 16-byte addresses
 

@@ -4,6 +4,7 @@
 // All matrices are column-major views (pointer, rows, cols, leading dimension).
 // Real matrices are double, complex ones zdbl (interleaved re, im).
 #include "internal.h"
+#include "line_search.h"
 
 #include <algorithm>
 #include <cmath>
@@ -50,7 +51,9 @@ constexpr int kAhead = 4;  // elements whose loads a thread issues before it use
 // Bound by memory: two reads and a write per element.
 template <typename T>
 __global__ void axpby_kernel(int rows, int cols, const T* __restrict__ A, int lda, T* __restrict__ C, int ldc,
-                             zdbl alpha, zdbl beta, int beta_zero, const double* __restrict__ beta_at) {
+                             zdbl alpha, zdbl beta, int beta_zero, const double* __restrict__ beta_at,
+                             const int* __restrict__ stop) {
+    if (stop && *stop) return;
     if (beta_at) beta = zdbl{*beta_at, 0.0};
     Walk w(rows, cols);
     while (w.e < w.total) {
@@ -369,11 +372,19 @@ __device__ inline double re_of(T a) {
     if constexpr (sizeof(T) == 8) return *(const double*)&a;
     else return ((const zdbl*)&a)->x;
 }
+__host__ __device__ inline void coeff_of_traces(const double t[13], double coeff[5]) {  // omm_ops.F90:213-217
+    coeff[0] = 2.0 * t[0] - t[1];
+    coeff[1] = 2.0 * (2.0 * t[2] - t[3] - t[4]);
+    coeff[2] = 2.0 * (t[5] - t[8] - t[9]) - t[6] - t[7];
+    coeff[3] = -2.0 * (t[10] + t[11]);
+    coeff[4] = -t[12];
+}
 template <typename T>
 __global__ void coeff_kernel(int n, const T* __restrict__ HW, int l0, const T* __restrict__ SW, int l1,
                              const T* __restrict__ HWd, int l2, const T* __restrict__ SWd, int l3,
                              const T* __restrict__ HWdd, int l4, const T* __restrict__ SWdd, int l5, double* part,
-                             double* out) {
+                             double* out, const LineSearch ls) {
+    if (ls.stop && *ls.stop) return;
     __shared__ T tileT[32][33];
     double v[13];
 #pragma unroll
@@ -431,7 +442,31 @@ __global__ void coeff_kernel(int n, const T* __restrict__ HW, int l0, const T* _
             }
         }
     }
-    block_reduce_finish<13>(v, part, out);
+    const bool last = block_reduce_finish<13>(v, part, out);
+    if (!last || !ls.record) return;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double c[5], x = 0.0;
+        coeff_of_traces(out, c);
+        bool fail = false, finite = true;
+        for (int k = 0; k < 5; ++k) finite = finite && isfinite(c[k]);
+        if (finite) solve_quartic(c, &x, &fail);
+        const double old = ls.state[2], e = quartic_energy(c, x), number = ls.state[3] + 1.0;
+        const double diff = 2.0 * fabs((e - old) / (e + old));
+        const bool stop = !finite || fail || diff <= ls.tol || number >= ls.most;
+        volatile double* q = ls.record + 16 * ((long long)ls.state[3] % kStepRecords);
+        for (int k = 0; k < 5; ++k) q[k] = c[k];
+        q[5] = x;
+        q[6] = e;
+        q[7] = diff;
+        q[8] = stop ? 1.0 : 0.0;
+        __threadfence_system();
+        q[9] = number;  // the host polls it: last
+        ls.state[1] = x;
+        ls.state[2] = e;
+        ls.state[3] = number;
+        if (stop) *ls.stop = 1;
+    }
 }
 
 // Polak-Ribiere lambda = v0 / v1 for the next direction, left in device memory: the host has no use for
@@ -440,7 +475,8 @@ __global__ void coeff_kernel(int n, const T* __restrict__ HW, int l0, const T* _
 template <typename T, bool SAME>
 __global__ void lambda_kernel(int rows, int cols, const T* __restrict__ PG, int l0, const T* __restrict__ G, int l1,
                               const T* __restrict__ Gp, int l2, const T* __restrict__ PGp, int l3, double* part,
-                              double* out, double* lambda) {
+                              double* out, double* lambda, const int* __restrict__ stop) {
+    if (stop && *stop) return;
     double v[2] = {0.0, 0.0};
     Walk w(rows, cols);
     while (w.e < w.total) {
@@ -494,10 +530,14 @@ struct CgUpdate {
     const T *Wd, *Wdd;   // [HWd; SWd], [HWdd; SWdd], leading dimension 2n
     int n, bC, bX;
     double x;
+    const double* x_at;
+    const int* stop;
 };
 template <typename T>
 __global__ void __launch_bounds__(kThreads) cg_update_kernel(const __grid_constant__ CgUpdate<T> p) {
-    const zdbl xz{p.x, 0.0}, x2{p.x * p.x, 0.0};
+    if (p.stop && *p.stop) return;
+    const double x = p.x_at ? *p.x_at : p.x;
+    const zdbl xz{x, 0.0}, x2{x * x, 0.0};
     int b = blockIdx.x;
     if (b < p.bC + p.bX) {
         const bool c = b < p.bC;
@@ -621,7 +661,8 @@ inline int tile_grid(int rows, int cols) {
 }  // namespace
 
 // ------------------------------------------------------------------ host wrappers
-void k_axpby(const DView& A, char op, DView& C, const double alpha[2], const double beta[2], const double* beta_at) {
+void k_axpby(const DView& A, char op, DView& C, const double alpha[2], const double beta[2], const double* beta_at,
+             const int* stop) {
     int oc = op_code(op);
     if (A.is_real && oc == 2) oc = 1;
     size_t tot = (size_t)C.rows * C.cols;
@@ -631,12 +672,12 @@ void k_axpby(const DView& A, char op, DView& C, const double alpha[2], const dou
     if (oc == 0) {
         if (C.is_real)
             axpby_kernel<double><<<grid_for(tot), kThreads, 0, rt().stream>>>(C.rows, C.cols, A.as<double>(), A.ld,
-                                                                                C.as<double>(), C.ld, a, b, bz, beta_at);
+                                                                                C.as<double>(), C.ld, a, b, bz, beta_at, stop);
         else
             axpby_kernel<zdbl><<<grid_for(tot), kThreads, 0, rt().stream>>>(C.rows, C.cols, A.as<zdbl>(), A.ld,
-                                                                              C.as<zdbl>(), C.ld, a, b, bz, beta_at);
+                                                                              C.as<zdbl>(), C.ld, a, b, bz, beta_at, stop);
     } else {
-        if (beta_at) fail(OMM_ERR_ARG, "axpby: a device scalar with a transposed operand");
+        if (beta_at || stop) fail(OMM_ERR_ARG, "axpby: a device scalar with a transposed operand");
         const int grid = tile_grid(C.rows, C.cols);
         if (C.is_real)
             axpby_trans_kernel<double><<<grid, kThreads, 0, rt().stream>>>(C.rows, C.cols, A.as<double>(), A.ld, 0,
@@ -742,34 +783,33 @@ void r_dot(const DView& A, const DView& B, double out[2]) {
 }
 
 void r_coeff(const DView& HW, const DView& SW, const DView& HWd, const DView& SWd, const DView& HWdd, const DView& SWdd,
-             double coeff[5]) {
+             double coeff[5], const LineSearch* lsp) {
     int n = HW.rows;
+    const LineSearch ls = lsp ? *lsp : LineSearch{};
     int tiles = (n + 31) / 32;
     int nb = tiles * tiles;
     if (nb > 148 * 8) nb = 148 * 8;
     double* part = scratch_partials(nb + 1, 13);
+    double* out = lsp ? part + (size_t)nb * 13 : rt().host_pinned;
     if (HW.is_real)
         coeff_kernel<double><<<nb, kThreads, 0, rt().stream>>>(n, HW.as<double>(), HW.ld, SW.as<double>(), SW.ld,
                                                                  HWd.as<double>(), HWd.ld, SWd.as<double>(), SWd.ld,
                                                                  HWdd.as<double>(), HWdd.ld, SWdd.as<double>(),
-                                                                 SWdd.ld, part, rt().host_pinned);
+                                                                 SWdd.ld, part, out, ls);
     else
         coeff_kernel<zdbl><<<nb, kThreads, 0, rt().stream>>>(n, HW.as<zdbl>(), HW.ld, SW.as<zdbl>(), SW.ld,
                                                                HWd.as<zdbl>(), HWd.ld, SWd.as<zdbl>(), SWd.ld,
                                                                HWdd.as<zdbl>(), HWdd.ld, SWdd.as<zdbl>(), SWdd.ld,
-                                                               part, rt().host_pinned);
+                                                               part, out, ls);
     OMM_KCHECK();
+    if (lsp) return;
     double t[13];
     finish_reduce(13, t);
-    // omm_ops.F90:213-217
-    coeff[0] = 2.0 * t[0] - t[1];
-    coeff[1] = 2.0 * (2.0 * t[2] - t[3] - t[4]);
-    coeff[2] = 2.0 * (t[5] - t[8] - t[9]) - t[6] - t[7];
-    coeff[3] = -2.0 * (t[10] + t[11]);
-    coeff[4] = -t[12];
+    coeff_of_traces(t, coeff);
 }
 
-void r_lambda(const DView& PG, const DView& G, const DView& Gp, const DView& PGp, double* lambda) {
+void r_lambda(const DView& PG, const DView& G, const DView& Gp, const DView& PGp, double* lambda,
+              const int* stop) {
     size_t tot = (size_t)G.rows * G.cols;
     int nb = reduce_grid(tot);
     double* part = scratch_partials(nb + 1, 2);
@@ -777,7 +817,7 @@ void r_lambda(const DView& PG, const DView& G, const DView& Gp, const DView& PGp
     auto launch = [&](auto tag, auto kernel) {
         using T = decltype(tag);
         kernel<<<nb, kThreads, 0, rt().stream>>>(G.rows, G.cols, PG.as<T>(), PG.ld, G.as<T>(), G.ld, Gp.as<T>(), Gp.ld,
-                                                 PGp.as<T>(), PGp.ld, part, part + (size_t)nb * 2, lambda);
+                                                 PGp.as<T>(), PGp.ld, part, part + (size_t)nb * 2, lambda, stop);
     };
     if (G.is_real) launch(double{}, same ? lambda_kernel<double, true> : lambda_kernel<double, false>);
     else launch(zdbl{}, same ? lambda_kernel<zdbl, true> : lambda_kernel<zdbl, false>);
@@ -785,12 +825,14 @@ void r_lambda(const DView& PG, const DView& G, const DView& Gp, const DView& PGp
 }
 
 void k_cg_update(int n, int m, double x, DView& C, const DView& D, DView* X, const DView* Y, DView& HW, DView& SW,
-                 const DView& Wd, const DView& Wdd, DView* L) {
+                 const DView& Wd, const DView& Wdd, DView* L, const double* x_at, const int* stop) {
     auto launch = [&](auto tag) {
         using T = decltype(tag);
         CgUpdate<T> p{};
         p.n = n;
         p.x = x;
+        p.x_at = x_at;
+        p.stop = stop;
         p.C = C.as<T>();
         p.D = D.as<T>();
         p.nc = (size_t)n * m;

@@ -17,6 +17,7 @@
 //     and Y holds copies of C and D, updated with the same operations, so the
 //     stacked products stay uniform.
 #include "internal.h"
+#include "line_search.h"
 
 #include <chrono>
 #include <cmath>
@@ -661,7 +662,7 @@ void eval_direction(OmmCall& c, const DView& Dir, double coeff[5]) {
 }
 
 // calc_G (omm_ops.F90:17-39): G = 4 HC - 2 SW HC - 2 HW SC = [4I - 2SW, -2HW] [HC; SC]
-void calc_G(OmmCall& c, DView& G) {
+void calc_G(OmmCall& c, DView& G, const int* stop = nullptr) {
     IpState& s = *c.s;
     int n = c.n, m = c.m;
     DView L = view(s.Lg, n, 2 * n, n, c.real);
@@ -675,7 +676,139 @@ void calc_G(OmmCall& c, DView& G) {
         return;
     }
     s.xc_ok = false;
-    gemm('n', 'n', n, m, 2 * n, ONE, L, X, ZERO, G);
+    if (stop) gemm_dmma('n', 'n', n, m, 2 * n, ONE, &L, &X, ZERO, &G, 1, nullptr, stop);
+    else gemm('n', 'n', n, m, 2 * n, ONE, L, X, ZERO, G);
+}
+
+// Whether the step's Gram products and calc_G both take gemm_dmma: the CG loop of such a problem runs
+// ahead of the host (run_ahead)
+bool step_runs_ahead(const OmmCall& c, const DView& Cw) {
+    const int n = c.n, m = c.m;
+    return !c.hcb && !c.use_precon && fp64_emu_enabled() && !fp64_emu_worth(2 * n, n, m, !c.real) &&
+           !fp64_emu_worth(n, m, 2 * n, !c.real) && gemm_dmma_takes(Cw);
+}
+
+// CG steps of a small problem without waiting for the host.  A step's line search is solved in the last
+// block of its coefficients' kernel (the host's own routine), which leaves x for the updates that follow
+// and a numbered record in pinned memory (at most four steps are out at a time); two steps (the gradient's buffers alternate) are one CUDA graph, and
+// the host, which polls the records, launches the next two while one of them is still to run.  A step that
+// needs the host -- converged, a failed line search, non-finite coefficients, the last one allowed -- raises
+// a flag, and every later kernel that would change C, D, G, X, the W matrices or lambda finds it and returns
+// (those that only form [HG; SG] again from the same D may run).  On return that step is evaluated and not
+// applied: coeff, e_min and the loop's counters are as after eval_dir of it.
+// A step of m = 832, n = 128 with a wait for its coefficients took 84 us, of m = 200, n = 40 63 us, of which
+// the kernels ran 62 and 39: the rest was seven launches and the wait.
+int run_ahead(OmmCall& c, DView& G, DView& Gp, DView& D, DView& Cw, long most, double tol, double* e_min, double coeff[5],
+              const std::function<void(int, double, double)>& applied) {
+    IpState& s = *c.s;
+    const int n = c.n, m = c.m;
+    const bool r = c.real;
+    Runtime& R = rt();
+    DView X = view(s.X, 2 * n, m, 2 * n, r), Y = view(s.Y, 2 * n, m, 2 * n, r);
+    DView Wd = view(s.Wd, 2 * n, n, 2 * n, r), Wdd = view(s.Wdd, 2 * n, n, 2 * n, r);
+    DView HW = view(s.HW, n, n, n, r), SW = view(s.SW, n, n, n, r), L = view(s.Lg, n, 2 * n, n, r);
+    LineSearch ls;
+    ls.state = s.lam.as<double>();
+    ls.stop = reinterpret_cast<int*>(ls.state + 4);
+    ls.tol = tol;
+    ls.most = (double)most;
+    ls.record = R.host_pinned + 64;
+    s.de_ok = s.xr_ok = s.xc_ok = false;
+    // state: [0] lambda (kept), [1] x, [2] the energy, [3] steps evaluated, [4] the flag
+    R.host_pinned[48] = 0.0;
+    R.host_pinned[49] = *e_min;
+    R.host_pinned[50] = R.host_pinned[51] = 0.0;
+    OMM_CK(cudaMemcpyAsync(ls.state + 1, R.host_pinned + 48, 4 * sizeof(double), cudaMemcpyHostToDevice, R.stream));
+    volatile double* rec = R.host_pinned + 64;  // records of 16 doubles; [9] of each: its step's number
+    for (int k = 0; k < kStepRecords; ++k) rec[16 * k + 9] = 0.0;
+    auto step = [&](DView& g, DView& gp) {  // g: the gradient at the current C; it ends in gp
+        k_axpby(g, 'n', D, ONE, ZERO, ls.state, ls.stop);  // D = G + lambda D
+        apply_HS(c, D, s.Y);
+        const DView a[2] = {X, Y}, b[2] = {D, D};
+        DView w[2] = {Wd, Wdd};
+        const int herm[2] = {0, n};
+        gemm_dmma('n', 'c', 2 * n, n, m, ONE, a, b, ZERO, w, 2, herm, ls.stop);
+        r_coeff(HW, SW, view(s.Wd, n, n, 2 * n, r), view(s.Wd, n, n, 2 * n, r, n), view(s.Wdd, n, n, 2 * n, r),
+                view(s.Wdd, n, n, 2 * n, r, n), nullptr, &ls);
+        k_cg_update(n, m, 0.0, Cw, D, &X, &Y, HW, SW, Wd, Wdd, &L, ls.state + 1, ls.stop);
+        s.lg_ok = true;
+        calc_G(c, gp, ls.stop);
+        r_lambda(gp, gp, g, g, ls.state, ls.stop);
+    };
+    auto two_steps = [&] {
+        step(G, Gp);
+        step(Gp, G);
+    };
+    // the graph of this call's buffers, captured anew; the executable kept from the last call takes its
+    // parameters where it was made for the same launches (an update does not change cluster shapes), else a
+    // new one is made.  Without one (a stream that cannot be captured) the steps are launched one by one.
+    bool graph = false;
+    if (!ktime_on()) {
+        cudaGraph_t g = nullptr;
+        if (cudaStreamBeginCapture(R.stream, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
+            try {
+                two_steps();
+            } catch (...) {
+                cudaStreamEndCapture(R.stream, &g);
+                if (g) cudaGraphDestroy(g);
+                cudaGetLastError();
+                throw;
+            }
+            graph = cudaStreamEndCapture(R.stream, &g) == cudaSuccess && g;
+        }
+        auto align = [](const void* p) { return (long long)((uintptr_t)p % 16); };
+        const long long key[6] = {n, m, r, c.H_csc ? (long long)c.Hm->pattern_id : -1,
+                                  c.S_csc ? (long long)c.Sm->pattern_id : -1, align(Cw.p) + align(c.H.p) * 16 + align(c.S.p) * 256 +
+                                      (c.s_identity ? 4096 : 0)};
+        if (graph && R.steps) {
+            cudaGraphExecUpdateResultInfo info{};
+            if (!std::equal(key, key + 6, R.steps_key) || cudaGraphExecUpdate(R.steps, g, &info) != cudaSuccess) {
+                cudaGraphExecDestroy(R.steps);
+                R.steps = nullptr;
+            }
+        }
+        std::copy(key, key + 6, R.steps_key);
+        if (graph && !R.steps && cudaGraphInstantiate(&R.steps, g, 0) != cudaSuccess) {
+            R.steps = nullptr;
+            graph = false;
+        }
+        if (g) cudaGraphDestroy(g);
+        cudaGetLastError();
+    }
+    auto launch = [&] {
+        if (graph) OMM_CK(cudaGraphLaunch(R.steps, R.stream));
+        else two_steps();
+    };
+    auto wait = [&](long t) {  // for the record of step t
+        auto t0 = std::chrono::steady_clock::now();
+        volatile double* q = rec + 16 * (t % kStepRecords);
+        for (long polls = 1; q[9] != (double)(t + 1); ++polls)
+            if (polls % 4096 == 0) {
+                const cudaError_t e = cudaStreamQuery(R.stream);
+                if (e != cudaErrorNotReady && q[9] != (double)(t + 1)) {
+                    OMM_CK(e);
+                    fail(OMM_ERR_CUDA, "omm: a CG step left no record");
+                }
+            }
+        std::atomic_thread_fence(std::memory_order_acquire);
+        add_sync_wait(std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count());
+    };
+    long launched = 0, t = 0;
+    for (;; ++t) {
+        if (launched - t < 2) {
+            launch();
+            launched += 2;
+        }
+        wait(t);
+        const volatile double* q = rec + 16 * (t % kStepRecords);
+        for (int i = 0; i < 5; ++i) coeff[i] = q[i];
+        if (q[8] != 0.0) break;
+        *e_min = q[6];
+        applied((int)t, q[6], q[7]);
+    }
+    if (t % 2 == 0) std::swap(G, Gp);  // step t's gradient is in Gp, as after its swap
+    s.lg_ok = false;
+    return (int)t;  // steps applied
 }
 
 // ---- reduced-precision stages of the "gmx" solver (products only; the state stays FP64)
@@ -1058,49 +1191,6 @@ void refresh_from_C(OmmCall& c, MixedCtx& mc, const DView& Cw, DView& G, int nse
     mx_calc_G(c, mc, G, nseg);
 }
 
-// quartic line search (omm_quartic.F90:60-153)
-void solve_quartic(const double c[5], double* x_min, bool* fail) {
-    const double Pi = 3.141592653589793238462643383279502884197;
-    *fail = false;
-    double a = 3.0 * c[3] / (4.0 * c[4]);
-    double b = 2.0 * c[2] / (4.0 * c[4]);
-    if ((std::fabs(b) >= 1.0e11) || (std::fabs(c[4]) <= 1.0e-11)) {
-        *x_min = -0.5 * c[1] / c[2];
-        return;
-    }
-    double d = c[1] / (4.0 * c[4]);
-    double Q = (a * a - 3.0 * b) / 9.0;
-    double R = (2.0 * a * a * a - 9.0 * a * b + 27.0 * d) / 54.0;
-    if (R * R < Q * Q * Q) {
-        double theta = std::acos(R / std::sqrt(Q * Q * Q));
-        double t[3], z[3];
-        t[0] = -2.0 * std::sqrt(Q) * std::cos(theta / 3.0) - a / 3.0;
-        t[1] = -2.0 * std::sqrt(Q) * std::cos((theta + 2.0 * Pi) / 3.0) - a / 3.0;
-        t[2] = -2.0 * std::sqrt(Q) * std::cos((theta - 2.0 * Pi) / 3.0) - a / 3.0;
-        for (int i = 0; i < 3; ++i) {
-            double tt = t[i];
-            z[i] = c[4] * (tt * tt) * (tt * tt) + c[3] * tt * tt * tt + c[2] * tt * tt + c[1] * tt + c[0];
-        }
-        if (c[4] > 0.0) {
-            int o[3];
-            if (z[0] >= z[1] && z[0] >= z[2]) { o[0] = 0; o[1] = 1; o[2] = 2; }
-            else if (z[1] > z[2]) { o[0] = 1; o[1] = 2; o[2] = 0; }
-            else { o[0] = 2; o[1] = 0; o[2] = 1; }
-            if ((0.0 <= t[o[0]]) && (t[o[1]] <= t[o[0]])) *x_min = t[o[1]];
-            else *x_min = t[o[2]];
-        } else {
-            if (z[0] <= z[1] && z[0] <= z[2]) *x_min = t[0];
-            else if (z[1] < z[2]) *x_min = t[1];
-            else *x_min = t[2];
-        }
-    } else {
-        double S = -(R >= 0.0 ? 1.0 : -1.0) * std::pow(std::fabs(R) + std::sqrt(R * R - Q * Q * Q), 1.0 / 3.0);
-        double U = (S == 0.0) ? 0.0 : Q / S;
-        *x_min = (S + U) - (a / 3.0);
-        if (c[4] < 0.0) *fail = true;
-    }
-}
-
 void alloc_nm(DevBuf& b, int rows, int cols, size_t es) {
     if (!b.p) b.alloc_zero(std::max<size_t>(1, (size_t)rows * cols) * es);
 }
@@ -1319,7 +1409,7 @@ int omm_run(int m, int n, msw_matrix* H, msw_matrix* S, bool new_S, double* e_mi
     // is tested (e_diff <= cg_tol, omm.F90:506) only in stages 2 and 3.
     MixedCtx mc;
     s.de_ok = s.xr_ok = s.xc_ok = s.lg_ok = false;  // nothing carried over from an earlier call
-    s.lam.ensure(sizeof(double));
+    s.lam.ensure(8 * sizeof(double));  // lambda, and run_ahead's x, energy, count and flag
     // complex problems take the reduced-precision stages with dense H and S (the tensor-core
     // SpMM is real only)
     const bool lowp_ok = c.real || (!c.H_csc && (c.s_identity || !c.S_csc));
@@ -1391,6 +1481,7 @@ int omm_run(int m, int n, msw_matrix* H, msw_matrix* S, bool new_S, double* e_mi
     int icg = 0;
     bool conv = false, ls_conv = false, ls_fail = false;
     const int n_step_max_outer = 100;
+    const bool ahead = step_runs_ahead(c, Cw);
     long n_step_max_inner = (m < 10000) ? (long)m * n - 1 : 10000000L;
     double e_diff = 0.0;
     int outer_i = 0;
@@ -1398,13 +1489,33 @@ int omm_run(int m, int n, msw_matrix* H, msw_matrix* S, bool new_S, double* e_mi
         const double* lam = nullptr;  // lambda in device memory; null: 0
         for (long j = 1; j <= n_step_max_inner; ++j) {
             s.de_ok = false;
+            bool evaluated = false;
+            if (ahead && stage == 3 && lam) {
+                // several steps at once; the last of them comes back evaluated
+                const int done_steps =
+                    run_ahead(c, G, Gp, D, Cw, n_step_max_inner - j + 1, cg_tol_internal, &e_min, coeff,
+                              [&](int k, double e, double diff) {
+                                  if (log.f && long_out) {
+                                      char b[128];
+                                      snprintf(b, sizeof b, "| %5d %5ld %s %s |", outer_i, j + k, es15(e).c_str(),
+                                               es15(diff).c_str());
+                                      log.line(b);
+                                  }
+                                  ++icg;
+                                  g_stats.icg_fp64++;
+                              });
+                j += done_steps;
+                evaluated = true;
+            }
+            if (!evaluated) {
             if (c.use_precon) k_axpby(PG, 'n', D, ONE, ZERO, lam);
             else if (stage < 3) mx_update_dir(c, mc, D, G, lam, nseg_of(stage));
             else fp64_dir_update(c, G, D, lam);
             std::swap(G, Gp);  // G_p = G; G is recomputed before it is read again
             if (c.use_precon) std::swap(PG, PGp);
-            double e_min_old = e_min;
             if (icg > 0) eval_dir(D, coeff, Gp);  // G_p holds the gradient at the current C
+            }
+            double e_min_old = e_min;
             if (!std::isfinite(coeff[0]) || !std::isfinite(coeff[1]) || !std::isfinite(coeff[2]) ||
                 !std::isfinite(coeff[3]) || !std::isfinite(coeff[4]))
                 fail(OMM_ERR_NONFINITE, "omm: non-finite line-search coefficients");
@@ -1418,7 +1529,7 @@ int omm_run(int m, int n, msw_matrix* H, msw_matrix* S, bool new_S, double* e_mi
                 ls_conv = false;
                 g_stats.ls_fail++;
             } else {
-                e_min = coeff[4] * (x * x) * (x * x) + coeff[3] * x * x * x + coeff[2] * x * x + coeff[1] * x + coeff[0];
+                e_min = quartic_energy(coeff, x);
                 ls_conv = true;
             }
             e_diff = 2.0 * std::fabs((e_min - e_min_old) / (e_min + e_min_old));
@@ -1673,6 +1784,11 @@ int omm_gpu_set_mixed(double bf16_tol, double split_tol, double refine_factor) {
 
 int omm_gpu_finalize(void) {
     try {
+        if (rt().steps) {
+            sync();
+            cudaGraphExecDestroy(rt().steps);
+            rt().steps = nullptr;
+        }
         g_state = OmmState();
         g_state_cb = OmmState();
         if (rt().stream) sync();

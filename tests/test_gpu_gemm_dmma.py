@@ -74,3 +74,32 @@ def test_small_solve(m, n, cplx):
     assert float((D - D.mH).abs().max()) == 0.0
     U = torch.linalg.solve(L.mH, Q[:, :n])
     assert float((D - U @ U.mH).abs().max()) <= 1e-4
+
+
+def test_solves_in_turn():
+    """Solves of different shapes and types one after another (the CG loop's graph is made anew or takes the
+    next call's parameters): each gives the same bits as it did alone."""
+    import torch
+
+    G.set_log(None)
+    cases = []
+    for m, n, dt in ((60, 30, torch.float64), (101, 33, torch.float64), (60, 30, torch.complex128),
+                     (200, 65, torch.float64)):
+        g = torch.Generator(device="cuda").manual_seed(m + n)
+        Q, _ = torch.linalg.qr(torch.randn(m, m, generator=g, device="cuda", dtype=dt))
+        lam = torch.linspace(-2.0, -1.0, m, device="cuda", dtype=torch.float64)
+        lam[n:] += 2.5
+        H = (Q * lam) @ Q.mH
+        cases.append((m, n, _mat(0.5 * (H + H.mH)), _mat(H[:n] * 0), _mat(H * 0)))
+    torch.cuda.synchronize()
+
+    def solve(m, n, h, c, d):
+        e, rc = G.omm(m, n, h[0], None, True, d[0], False, 0.0, c[0], False, dealloc=True)
+        assert rc == 0
+        return e, d[1].clone(), G.stats()["icg"]
+
+    first = [solve(*c) for c in cases]
+    for order in ((0, 0, 1, 2, 3), (3, 1, 3, 2, 0, 2)):
+        for k in order:
+            e, d, steps = solve(*cases[k])
+            assert e == first[k][0] and steps == first[k][2] and torch.equal(d, first[k][1])
