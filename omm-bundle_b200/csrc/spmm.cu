@@ -160,15 +160,11 @@ __global__ void __launch_bounds__(kGatherThreads) gather_kernel(int n, const T* 
 // Complex matrices (CPLX) take the same kernel: A, interleaved, is a real matrix of 2n rows; B_re
 // and B_im are the two value sets; and with P = A [B_re | B_im], Re C(r, c) = P(2r, c) - P(2r+1, G+c),
 // Im C(r, c) = P(2r, G+c) + P(2r+1, c): one lane exchange in the epilogue.
-__device__ __forceinline__ void cp_async8(double* dst, const double* src, int bytes) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)),
-                 "l"(src), "r"(bytes)
-                 : "memory");
+__device__ __forceinline__ void cp_async8(uint32_t dst, const double* src, int bytes) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
 }
-__device__ __forceinline__ void cp_async16(double* dst, const double* src, int bytes) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)),
-                 "l"(src), "r"(bytes)
-                 : "memory");
+__device__ __forceinline__ void cp_async16(uint32_t dst, const double* src, int bytes) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
@@ -224,76 +220,99 @@ __global__ void __launch_bounds__(128) cgu_dmma_kernel(const __grid_constant__ D
 #pragma unroll
             for (int nt = 0; nt < NT; ++nt) acc[s][mt][nt][0] = acc[s][mt][nt][1] = 0.0;
 
-    auto load = [&](int t) {
-        double* as = dsm + (t % ST) * STAGE;
+    // A thread's copies of a chunk: places and bytes are formed once, the rows' column comes from the union.
+    // Of A, with 16-byte copies, two rows (place mm) of the k kk0, kk0 + KS, ...; with 8-byte ones one row.
+    // Of B, a vector per turn of the value sets' contiguous chunk (complex: an element, re and im apart).
+    const int nk = (K + BK - 1) / BK, nfull = K / BK;
+    constexpr int VR = BM / 2, KS = 128 / VR, NV = BK / KS;                       // 16-byte copies
+    constexpr int KS1 = BM >= 128 ? 1 : 128 / BM, NV1 = BK * BM / 128;            // 8-byte copies
+    const int kk0 = p.vec ? (int)threadIdx.x / VR : (int)threadIdx.x / BM;
+    const int mm = p.vec ? 2 * ((int)threadIdx.x % VR) : (int)threadIdx.x % BM;
+    const int abytes = 8 * max(0, min(p.vec ? 2 : 1, p.n - (r0 + mm)));
+    const double* acol = abytes ? p.A + r0 + mm : p.A;
+    const long long alda = abytes ? p.lda : 0;
+    const uint32_t ad = (uint32_t)__cvta_generic_to_shared(dsm + kk0 * AS + mm);
+    constexpr int BV = CPLX ? 2 * BK * G : BK * G / 2, NB = (BV + 127) / 128;     // copies of B's chunk (per set)
+    uint32_t bd[NB];
+    int bk[NB];
+#pragma unroll
+    for (int u = 0; u < NB; ++u) {
+        const int e = threadIdx.x + 128 * u;
+        const int kk = CPLX ? e / (2 * G) : e / (G / 2), c = CPLX ? e % (2 * G) / 2 : 2 * (e % (G / 2));
+        bk[u] = e < BV ? kk : 1 << 30;
+        bd[u] = (uint32_t)__cvta_generic_to_shared(dsm + BK * AS + ((CPLX ? (e & 1) * BK : 0) + kk) * GS + c);
+    }
+    const double* bsrc[NM] = {};
+    bsrc[0] = p.B0 + (size_t)kb * G * (CPLX ? 2 : 1) + (CPLX ? 1 : 2) * threadIdx.x;
+    if constexpr (NM == 2 && !CPLX) bsrc[NM - 1] = p.B1 + (size_t)kb * G + 2 * threadIdx.x;
+    auto load = [&](int t, uint32_t off) {
         const int k0 = t * BK;
+        const bool full = t < nfull;
         if (p.vec) {
-            constexpr int VR = BM / 2;  // 16-byte vectors of a row of the tile
 #pragma unroll
-            for (int u = 0; u < BK * VR / 128; ++u) {
-                const int e = threadIdx.x + 128 * u;
-                const int kk = e / VR, mm = 2 * (e % VR), k = k0 + kk, r = r0 + mm;
-                const int bytes = k < K ? 8 * max(0, min(2, p.n - r)) : 0;
-                cp_async16(as + kk * AS + mm, bytes ? p.A + (size_t)ur[k] * p.lda + r : p.A, bytes);
+            for (int u = 0; u < NV; ++u) {
+                const int k = k0 + kk0 + KS * u;
+                const bool in = full || k < K;
+                cp_async16(ad + off + u * KS * AS * 8, acol + (in ? ur[k] * alda : 0), in ? abytes : 0);
             }
         } else {
 #pragma unroll
-            for (int u = 0; u < BK * BM / 128; ++u) {
-                const int e = threadIdx.x + 128 * u;
-                const int kk = e / BM, mm = e % BM, k = k0 + kk, r = r0 + mm;
-                const int bytes = k < K && r < p.n ? 8 : 0;
-                cp_async8(as + kk * AS + mm, bytes ? p.A + (size_t)ur[k] * p.lda + r : p.A, bytes);
+            for (int u = 0; u < NV1; ++u) {
+                const int kk = BM >= 128 ? u : kk0 + KS1 * u, k = k0 + kk;
+                const bool in = full || k < K;
+                cp_async8(ad + off + (BM >= 128 ? u : u * KS1) * AS * 8, acol + (in ? ur[k] * alda : 0), in ? abytes : 0);
             }
         }
-        double* bs = as + BK * AS;
-        if constexpr (CPLX) {
-            const double* B = p.B0 + (size_t)(kb + k0) * G * 2;
-            for (int e = threadIdx.x; e < 2 * BK * G; e += 128) {
-                const int kk = e / (2 * G), c = (e % (2 * G)) / 2, s = e & 1;
-                const int bytes = k0 + kk < K ? 8 : 0;
-                cp_async8(bs + (s * BK + kk) * GS + c, bytes ? B + e : p.B0, bytes);
-            }
-        } else {
 #pragma unroll
-            for (int s = 0; s < NM; ++s) {
-                const double* Bp = s == 0 ? p.B0 : p.B1;
-                const double* B = Bp + (size_t)(kb + k0) * G;
-                for (int e = threadIdx.x; e < BK * G / 2; e += 128) {
-                    const int kk = e / (G / 2), c = 2 * (e % (G / 2));
-                    const int bytes = k0 + kk < K ? 16 : 0;
-                    cp_async16(bs + (s * BK + kk) * GS + c, bytes ? B + 2 * e : Bp, bytes);
-                }
+        for (int u = 0; u < NB; ++u) {
+            if (NB * 128 != BV && bk[u] == 1 << 30) continue;  // no copy of this thread
+            const bool in = full || k0 + bk[u] < K;
+            if constexpr (CPLX) {
+                cp_async8(bd[u] + off, in ? bsrc[0] + 128 * u : p.B0, in ? 8 : 0);
+            } else {
+#pragma unroll
+                for (int s = 0; s < NM; ++s)
+                    cp_async16(bd[u] + off + s * BK * GS * 8, in ? bsrc[s] + 256 * u : p.B0, in ? 16 : 0);
             }
         }
+#pragma unroll
+        for (int s = 0; s < (CPLX ? 1 : NM); ++s) bsrc[s] += BK * G * (CPLX ? 2 : 1);
     };
 
-    const int nk = (K + BK - 1) / BK;
-#pragma unroll
-    for (int t = 0; t < ST - 1; ++t) {
-        if (t < nk) load(t);
-        cp_async_commit();
-    }
-    for (int t = 0; t < nk; ++t) {
-        cp_async_wait<ST - 2>();  // chunk t has landed (this thread's part)
-        __syncthreads();          // everyone's part, and the slot of chunk t - 1 is free
-        if (t + ST - 1 < nk) load(t + ST - 1);
-        cp_async_commit();
-        const double* as = dsm + (t % ST) * STAGE;
-        const double* bs = as + BK * AS;
+    const double* fa = dsm + (lane & 3) * AS + warp * 8 * MT + (lane >> 2);
+    const double* fb = dsm + BK * AS + (lane & 3) * GS + (lane >> 2);
+    auto multiply = [&](int stage) {
 #pragma unroll
         for (int k4 = 0; k4 < BK; k4 += 4) {
-            const int ka = k4 + (lane & 3);
             double af[MT];
 #pragma unroll
-            for (int mt = 0; mt < MT; ++mt) af[mt] = as[ka * AS + warp * 8 * MT + mt * 8 + (lane >> 2)];
+            for (int mt = 0; mt < MT; ++mt) af[mt] = fa[stage * STAGE + k4 * AS + mt * 8];
 #pragma unroll
             for (int s = 0; s < NM; ++s)
 #pragma unroll
                 for (int nt = 0; nt < NT; ++nt) {
-                    const double bf = bs[(s * BK + ka) * GS + nt * 8 + (lane >> 2)];
+                    const double bf = fb[stage * STAGE + (s * BK + k4) * GS + nt * 8];
 #pragma unroll
                     for (int mt = 0; mt < MT; ++mt) dmma(acc[s][mt][nt], af[mt], bf);
                 }
+        }
+    };
+#pragma unroll
+    for (int t = 0; t < ST - 1; ++t) {
+        if (t < nk) load(t, t * STAGE * 8);
+        cp_async_commit();
+    }
+    for (int t0 = 0; t0 < nk; t0 += ST) {
+#pragma unroll
+        for (int s = 0; s < ST; ++s) {
+            const int t = t0 + s;
+            if (t < nk) {
+                cp_async_wait<ST - 2>();  // chunk t has landed (this thread's part)
+                __syncthreads();          // everyone's part, and the slot of chunk t - 1 is free
+                if (t + ST - 1 < nk) load(t + ST - 1, (s + ST - 1) % ST * STAGE * 8);
+                cp_async_commit();
+                multiply(s);
+            }
         }
     }
     cp_async_wait<0>();
