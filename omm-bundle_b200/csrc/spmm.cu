@@ -152,10 +152,10 @@ __global__ void __launch_bounds__(kGatherThreads) gather_kernel(int n, const T* 
 // 16 lanes of a half-warp's fragment load (4 rows x 4 k) fall in 32 distinct banks.  With the padding
 // of 8 doubles used before, every fragment load took two passes and the L1 path (85 % busy)
 // held the DMMA pipe at 64 %.
-// lattice_8x8x8 (n = 1,536): H alone 1.30 -> 1.10 ms (27 TFLOP/s; the gathers then move about
-// 5.5 TB/s from L2), H and S fused 2.21 -> 1.89 ms (31.7 TFLOP/s, near cuBLAS DGEMM's 36).  Within 3 %:
-// three or five stages, 16-row chunks in two stages, 64-row tiles; 16-row chunks in four stages
-// (two CTAs per SM) 17 % slower.
+// lattice_8x8x8 (n = 1,536): H alone 1.30 -> 1.10 ms with that, 0.98 with the copies' addresses formed once
+// and five CTAs per SM (30.6 TFLOP/s; the gathers then move about 6 TB/s from L2), H and S fused
+// 2.21 -> 1.82 ms (32.8 TFLOP/s, near cuBLAS DGEMM's 36).  Within 3 %: three or five stages, 16-row chunks in
+// two or three stages.
 //
 // Complex matrices (CPLX) take the same kernel: A, interleaved, is a real matrix of 2n rows; B_re
 // and B_im are the two value sets; and with P = A [B_re | B_im], Re C(r, c) = P(2r, c) - P(2r+1, G+c),
@@ -197,8 +197,15 @@ struct DmmaArgs {
     int vec;      // A's column segments are 16-byte aligned
 };
 
+// CTAs per SM the registers are held to (0: no bound).  One value set, 128 rows: five CTAs 978 us, four 1,020;
+// 64 rows: eight 992, six 1,076; two value sets, 64 rows: five 1,820, four 1,936; 128 rows: three of 154
+// registers 1,822, four of 128 1,927.
+constexpr int dmma_ctas(int nm, int mt, bool cplx) {
+    return cplx ? 0 : nm == 1 ? (mt == 4 ? 5 : mt == 2 ? 8 : 0) : (mt == 2 ? 5 : 0);
+}
 template <int G, int NM, int MT, bool CPLX>
-__global__ void __launch_bounds__(128) cgu_dmma_kernel(const __grid_constant__ DmmaArgs p) {
+__global__ void __launch_bounds__(128, dmma_ctas(NM, MT, CPLX)) cgu_dmma_kernel(const __grid_constant__ DmmaArgs p) {
+    static_assert(MT <= 4, "the copies cover at most 128 rows");
     constexpr int BM = 32 * MT, BK = kDmmaBK, AS = BM + 4, GS = G + 4, NT = G / 8, ST = kDmmaStages;
     constexpr int STAGE = dmma_stage<G, NM, MT>();
     extern __shared__ __align__(16) double dsm[];  // [ST] stages: A [BK][AS], B [NM][BK][GS]
@@ -396,7 +403,7 @@ int dmma_row_tiles(int n, int ngroups) {
     for (int mt : {4, 2, 1}) {
         const long long blocks = (long long)((n + 32 * mt - 1) / (32 * mt)) * ngroups;
         const double waves = std::ceil((double)blocks / 148.0);
-        const double c = waves * mt * (mt == 4 ? 1.0 : mt == 2 ? 1.03 : 1.2);
+        const double c = waves * mt * (mt == 4 ? 1.0 : mt == 2 ? 1.01 : 1.15);
         if (mt == 4 || c < cost) {
             best = mt;
             cost = c;
