@@ -498,8 +498,9 @@ int omm_gpu_spmm_f64(const double* A, int lda, int n, const msw_matrix* H, const
  * the 256 rows; products without S take form 1).  All give the same bits.  OMM_ERR_ARG
  * otherwise.  No reference counterpart. */
 int omm_gpu_set_oz_spmm_form(int form);
-/* Which engine the real FP64 products of omm()/MatrixSwitch use: mode 1 = the
- * int8 tensor-core GEMM above (default), 0 = cuBLAS DGEMM.  panel_bytes caps
+/* Which engine the FP64 products of omm()/MatrixSwitch use: mode 1 (default) = the
+ * int8 tensor-core GEMM above or the FP64 tensor cores (mma.sync f64), whichever is
+ * estimated to be faster at the product's sizes, 0 = cuBLAS.  panel_bytes caps
  * the scratch of one int8 product's residues (0 = default 4 GiB; larger
  * products run in column panels).  No reference counterpart. */
 int omm_gpu_set_fp64_gemm(int mode, long long panel_bytes);

@@ -2,9 +2,10 @@
 //
 // MatrixSwitch's per-operation dispatch tables (MatrixSwitch.F90:1096-1351 and
 // siblings) choose an implementation from (storage format, serial, label).
-// Here every storage is served by the GPU: dense products go to cuBLAS
-// (FP64/complex FP64), dense x CSC and CSC x dense products to the SpMM kernels
-// of spmm.cu, and elementwise/trace operations to kernels.cu.  Host ('s')
+// Here every storage is served by the GPU: dense products go to the int8 emulation
+// (ozaki.cu) or the FP64 tensor cores (gemm_dmma.cu) by size, dense x CSC and CSC x
+// dense products to the SpMM kernels of spmm.cu, and elementwise/trace operations to
+// kernels.cu.  Host ('s')
 // matrices are staged to the device for the duration of one call.
 #include "internal.h"
 

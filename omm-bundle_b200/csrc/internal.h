@@ -283,7 +283,8 @@ void r_lambda(const DView& PG, const DView& G, const DView& Gp, const DView& PGp
 // C, D, X, Y; Wd, Wdd stacked with leading dimension 2n); x_at: x in device memory
 void k_cg_update(int n, int m, double x, DView& C, const DView& D, DView* X, const DView* Y, DView& HW, DView& SW,
                  const DView& Wd, const DView& Wdd, DView* L, const double* x_at = nullptr, const int* stop = nullptr);
-// dense products on cuBLAS (FP64 / complex FP64)
+// dense FP64 products: the int8 emulation or the FP64 tensor cores by their estimated times (cuBLAS where
+// neither takes the operands, and with omm_gpu_set_fp64_gemm(0, ...))
 void gemm(char opA, char opB, int M, int N, int K, const double alpha[2], const DView& A, const DView& B,
           const double beta[2], DView& C);
 void transpose_into(const DView& A, char op, DView& T);  // T = op(A)
@@ -385,7 +386,7 @@ bool fp64_emu_enabled();  // real FP64 GEMMs of the solver on the int8 tensor co
 void set_fp64_emu(int mode, long long panel_bytes);
 size_t oz_panel_bytes();
 bool fp64_emu_worth(int M, int N, int K, bool cplx = false);  // the emulation is faster than gemm_dmma
-bool fp64_emu_fits(int M, int N, int K);  // large enough for the emulation to pay against cuBLAS's FP64 kernels
+bool fp64_emu_fits(int M, int N, int K);  // in-place products: large enough for the emulation to pay against cuBLAS
 
 // ----------------------------------------------------------------- tensor-core SpMM (spmm_tc.cu)
 struct SpmmPlanView {

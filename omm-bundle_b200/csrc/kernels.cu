@@ -1,5 +1,5 @@
 // Elementwise, reduction and initialisation kernels of the libOMM CG loop, plus
-// the cuBLAS wrapper used for the FP64 dense products.
+// the dispatch of the FP64 dense products (gemm()).
 //
 // All matrices are column-major views (pointer, rows, cols, leading dimension).
 // Real matrices are double, complex ones zdbl (interleaved re, im).
@@ -871,7 +871,7 @@ void gemm(char opA, char opB, int M, int N, int K, const double alpha[2], const 
         const bool in_place = C.p == A.p || C.p == B.p;
         if (real_scalars && (in_place ? fp64_emu_fits(M, N, K) : fp64_emu_worth(M, N, K, cplx))) {
             // FP64-accurate product on the int8 tensor cores (ozaki.cu); 'c' is 't' for real data, complex
-            // ones are four real products of the parts
+            // ones are one product of the stacked parts
             if (cplx) gemm_z_emu(ops[op_code(opA)], ops[op_code(opB)], M, N, K, alpha[0], A, B, beta[0], C);
             else gemm_f64_emu(op_code(opA) ? 't' : 'n', op_code(opB) ? 't' : 'n', M, N, K, alpha[0], A, B, beta[0], C);
             return;

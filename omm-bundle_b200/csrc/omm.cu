@@ -3,9 +3,10 @@
 // Control flow, flavours, quirks and the per-ip SAVEd state follow omm.F90
 // line by line (citations inline).  What changes is where the data lives and
 // how the products are grouped:
-//   * all matrices stay in HBM for the whole call; only the five quartic
-//     coefficients and the two Polak-Ribiere traces come back to the host
-//     each CG step (two 8..104-byte reads);
+//   * all matrices stay in HBM for the whole call; a CG step is one wait on the
+//     host, for its line-search traces (lambda stays on the device), and the
+//     steps of a small problem are captured in graphs that run ahead of the
+//     host, the line search on the device (step_runs_ahead);
 //   * HC and SC are one stacked 2n x m matrix X = [HC; SC] and HG, SG one
 //     Y = [HG; SG] (column-major, leading dimension 2n).  The four Gram
 //     products of a step are then two GEMMs, [HWd; SWd] = X D^H and
@@ -1014,9 +1015,9 @@ double energy_c0(OmmCall& c) {
 }
 
 // D = C^H * CD for a Hermitian result (CD = QW C with QW Hermitian): only the blocks on and
-// above the diagonal are computed, then the lower triangle is mirrored.  For large m the blocks
-// are nb x nb plain GEMMs (cuBLAS's GEMM runs about 1.4x faster per flop than its syrkx at these
-// shapes; the diagonal blocks cost 1/nb extra flops); small m take syrkx / herkx.
+// above the diagonal are computed, then the lower triangle is mirrored: the emulation or the FP64 tensor cores by size.  Without the emulation
+// (omm_gpu_set_fp64_gemm(0, ...)) large m are nb x nb plain GEMMs (cuBLAS's GEMM runs about 1.4x faster per
+// flop than its syrkx at these shapes; the diagonal blocks cost 1/nb extra flops), small m take syrkx / herkx.
 void density_product(const DView& C, const DView& CD, DView& D) {
     Runtime& R = rt();
     int m = C.cols, n = C.rows;
@@ -1077,8 +1078,9 @@ void density_product(const DView& C, const DView& CD, DView& D) {
     k_fill_lower_from_upper(D);
 }
 
-// W (n x n) = A B^H for a Hermitian result (A = HC or SC, B = C: C H C^H, C S C^H): the upper
-// triangle as a staircase of row blocks (block i of A against rows i*bs.. of B, plain GEMMs,
+// W (n x n) = A B^H for a Hermitian result (A = HC or SC, B = C: C H C^H, C S C^H): the emulation's
+// or the FP64 tensor cores' Hermitian form (hermitian_blocks_batched), and where neither takes the operands
+// the upper triangle as a staircase of row blocks (block i of A against rows i*bs.. of B, plain GEMMs,
 // which run faster per flop than syrkx at these shapes), or syrkx / herkx for small n; the lower
 // triangle is mirrored.
 void hermitian_product_nt(const DView& A, const DView& B, DView& W) {

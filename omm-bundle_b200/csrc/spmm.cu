@@ -7,14 +7,15 @@
 //
 // Two kernels:
 //  * gather  : one CTA per (row chunk, output column); generic CSC.
-//  * cgu     : "column-group union", on the FP64 tensor cores (complex ones as two value sets).  Output columns are cut into groups of G
+//  * cgu     : "column-group union", on the FP64 tensor cores (complex ones as
+//              two value sets).  Output columns are cut into groups of G
 //              consecutive columns; a group's nonzeros live in the union U_g
 //              of their row indices, and the group is the dense product
 //              A(:, U_g) * B_g with B_g the |U_g| x G block of B (zero filled).
 //              For the block-sparse H and S of atom-centred bases (24 x 24
 //              atom blocks, all columns of an atom share one pattern) the
 //              union adds no fill at G = block size, and the product is a
-//              register-tiled dense GEMM with K = |U_g|.  A second value array
+//              tiled dense GEMM with K = |U_g|.  A second value array
 //              with the same pattern (S beside H) is multiplied in the same
 //              pass, so A is read once for both.
 // The plan (groups, union rows, dense blocks) is built once per matrix on the
@@ -1072,7 +1073,7 @@ void gemspm(char opA, const DView& A, char opB, const msw_matrix* B, DView& C, c
 // C^T = op(B)^T op(A)^T with the dense x CSC kernels.  op(A)^T is A^T's CSC for 'n' and A itself
 // otherwise; where 'c' asks for conj(A), the dense operand is conjugated instead and so is the
 // product: conj(conj(X) A) = X conj(A).  The column-group kernel writes the product transposed, in
-// place of a second matrix and a transposing add (5 x 5 x 5 atoms of 24 orbitals, 375 columns: 114 us
+// place of a second matrix and a transposing add (5 x 5 x 5 atoms of 24 orbitals, 375 columns: 100 us
 // with the transposed copy of B; the gather kernel, which took every pattern before, 500 us).
 void gespmm(char opA, const msw_matrix* A, char opB, const DView& B, DView& C, const double alpha[2],
             const double beta[2]) {
