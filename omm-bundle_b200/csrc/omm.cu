@@ -682,11 +682,13 @@ void calc_G(OmmCall& c, DView& G, const int* stop = nullptr) {
 }
 
 // Whether the step's Gram products and calc_G both take gemm_dmma: the CG loop of such a problem runs
-// ahead of the host (run_ahead)
+// ahead of the host (run_ahead).  Nothing in it may allocate while the steps are captured: complex operators
+// on 8-byte addresses, whose products go through copies, are left to the host's loop.
 bool step_runs_ahead(const OmmCall& c, const DView& Cw) {
     const int n = c.n, m = c.m;
     return !c.hcb && !c.use_precon && fp64_emu_enabled() && !fp64_emu_worth(2 * n, n, m, !c.real) &&
-           !fp64_emu_worth(n, m, 2 * n, !c.real) && gemm_dmma_takes(Cw);
+           !fp64_emu_worth(n, m, 2 * n, !c.real) && gemm_dmma_takes(Cw) && (c.H_csc || gemm_dmma_takes(c.H)) &&
+           (c.s_identity || c.S_csc || gemm_dmma_takes(c.S));
 }
 
 // CG steps of a small problem without waiting for the host.  A step's line search is solved in the last

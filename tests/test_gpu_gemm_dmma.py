@@ -103,3 +103,9 @@ def test_solves_in_turn():
         for k in order:
             e, d, steps = solve(*cases[k])
             assert e == first[k][0] and steps == first[k][2] and torch.equal(d, first[k][1])
+
+
+def test_solve_with_emulated_operator_products():
+    """m = 2,000, n = 400: the Gram products and calc_G stay on the FP64 tensor cores, so the steps run ahead
+    in a graph, while D H and D S are large enough for the int8 emulation: it is part of the graph."""
+    test_small_solve(2000, 400, False)
