@@ -4,11 +4,13 @@
 //
 //   C_z = alpha * op(A_z) op(B_z) + beta * C_z,  op in {n, t, c},  z = 0 .. nz - 1 (nz <= 2)
 //
-// A CTA of four warps forms one 32 x 32 tile; its K runs in 16-k (complex: 8-k) chunks through a ring of
-// four stages filled by cp.async three chunks ahead, one barrier per chunk.  The warps share the chunk's k,
-// not the tile: each multiplies the whole tile by its own four k (16 independent DMMAs on 8 fragment
-// loads; complex: two warps by k, two by rows, 32 DMMAs on 6 loads), and the four partial tiles are added at
-// the end.  What bounds such products is latency -- one or two CTAs per SM, each a serial chain over K -- so
+// A CTA of four warps forms one 32 x 32 tile, a 16 x 16 quarter each; its K runs in 16-k (complex: 8-k) chunks
+// through a ring of three (two) stages filled by cp.async ahead, one barrier per chunk, and an unsplit tile is
+// written from the accumulators.  Warps that share the chunk's k instead (each the whole tile by its own four
+// k, the partial tiles added at the end) load half as many fragments but were slower at every unsplit size
+// and most split ones: 3,000 x 3,000 x 16 74 us against 26, 1,895 x 415 x 160 19 against 12, 1,500 x 800 x 300
+// 33 against 26, 256 x 128 x 832 9.5 against 8.5.  Taller tiles (64 x 64, 64 x 32) were slower too.
+// What bounds small products is latency -- one or two CTAs per SM, each a serial chain over K -- so
 //   * a chunk is few instructions: copies from pointers formed once, stages as immediate offsets of an
 //     unrolled turn (with addresses formed per chunk it was 200 instructions a warp, at five clocks each,
 //     for 16 DMMAs: 128 x 832 x 832 twice 31 us, now 21);
@@ -19,9 +21,9 @@
 // Operands keep their global order in shared memory (rows or k contiguous, whichever the op makes of
 // them), padded so that the 16 lanes of a half-warp's fragment load (8 lanes for complex elements) fall
 // in distinct banks.  Complex products take four DMMAs per fragment pair.
-// Against cuBLAS (launches back to back): 256 x 128 x 832 twice 12.5 us (27 in two calls), 64 x 64 x 6,000
-// 17 (25), 1,024^3 76 (83), 2,049 x 1,999 x 4,001 1,086 (1,000), 260 x 130 x 600 complex twice 26 (51).
-// 64 x 64 tiles of eight warps were slower at every size up to 2,049 x 1,999 x 4,001 (1,157 us).
+// A call through the entry point against cuBLAS's (with its wait, microseconds): 256 x 128 x 832 21 (27), 1,895 x
+// 415 x 161 27 (29), 500^3 25 (28), 3,000 x 3,000 x 16 38 (41), 1,500 x 800 x 300 39 (151), complex 500^3 54
+// (57), 2,500 x 900 x 120 89 (556).
 #include "internal.h"
 
 #include <cooperative_groups.h>
@@ -67,6 +69,10 @@ __device__ __forceinline__ void dmma(double (&d)[2], double a, double b) {
                  : "d"(a), "d"(b));
 }
 
+__device__ __forceinline__ double flip(double v, int sign) {
+    return __hiloint2double(__double2hiint(v) ^ sign, __double2loint(v));
+}
+
 template <bool CPLX, int R>
 constexpr int stride_rows() { return CPLX ? R + 2 : R + 4; }  // [k][r]
 template <bool CPLX>
@@ -75,11 +81,11 @@ template <bool CPLX>
 constexpr int stride_k() { return chunk<CPLX>() + 4; }  // [r][k]
 template <bool CPLX, int R, bool KC>
 constexpr int tile_elems() { return KC ? R * stride_k<CPLX>() : chunk<CPLX>() * stride_rows<CPLX, R>(); }
-template <bool CPLX, int BM, int BN, int WK, int ST, bool TA, bool TB>
+template <bool CPLX, int BM, int BN, int ST, bool TA, bool TB>
 constexpr int smem_bytes() {
     const int es = CPLX ? 16 : 8;
     const int ring = ST * (tile_elems<CPLX, BM, TA>() + tile_elems<CPLX, BN, !TB>()) * es;
-    const int part = WK * BM * BN * es;  // the partial tiles of a split K
+    const int part = BM * BN * es;  // the partial tile of a split K
     return ring > part ? ring : part;
 }
 
@@ -131,10 +137,10 @@ struct Loader {
 };
 
 // TA: A is K-contiguous (op 't' / 'c'); TB: B is column-contiguous (op 't' / 'c')
-template <bool CPLX, int BM, int BN, int WM, int WN, int WK, int ST, bool TA, bool TB, bool VEC>
-__global__ void __launch_bounds__(32 * WM * WN * WK) gemm_dmma_kernel(const __grid_constant__ DgArgs p) {
+template <bool CPLX, int BM, int BN, int WM, int WN, int ST, bool TA, bool TB, bool VEC>
+__global__ void __launch_bounds__(32 * WM * WN) gemm_dmma_kernel(const __grid_constant__ DgArgs p) {
     using T = typename El<CPLX>::T;
-    constexpr int BK = chunk<CPLX>(), MT = BM / (8 * WM), NT = BN / (8 * WN), NP = CPLX ? 2 : 1, NTHR = 32 * WM * WN * WK;
+    constexpr int BK = chunk<CPLX>(), MT = BM / (8 * WM), NT = BN / (8 * WN), NP = CPLX ? 2 : 1, NTHR = 32 * WM * WN;
     constexpr int AE = tile_elems<CPLX, BM, TA>(), BE = tile_elems<CPLX, BN, !TB>();
     if (p.stop && *p.stop) return;
     extern __shared__ __align__(16) unsigned char raw[];
@@ -149,7 +155,7 @@ __global__ void __launch_bounds__(32 * WM * WN * WK) gemm_dmma_kernel(const __gr
     }
     const int k_lo = min(p.K, rank * p.kper), k_hi = min(p.K, k_lo + p.kper);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int wm = (warp % WM) * (BM / WM), wn = (warp / WM % WN) * (BN / WN), wk = warp / (WM * WN);
+    const int wm = (warp % WM) * (BM / WM), wn = (warp / WM) * (BN / WN);
     const double *A = p.A[z], *B = p.B[z];
 
     double acc[NP][MT][NT][2];
@@ -176,30 +182,31 @@ __global__ void __launch_bounds__(32 * WM * WN * WK) gemm_dmma_kernel(const __gr
     };
 #pragma unroll
     for (int t = 0; t < ST - 1; ++t) load(t, t * STAGE);
-    const double sa = p.conj_a ? -1.0 : 1.0, sb = p.conj_b ? -1.0 : 1.0;
+    // a conjugate's sign bit: integer work, which leaves the FP64 pipe to the DMMAs
+    const int sa = p.conj_a ? 0x80000000 : 0, sb = p.conj_b ? 0x80000000 : 0;
     // this lane's elements of a stage's fragments; the stages of an unrolled turn are immediate offsets
-    const int fk = 4 * wk + (lane & 3), fr = lane >> 2;
+    const int fk = lane & 3, fr = lane >> 2;
     const T* fa = ring + (TA ? (wm + fr) * stride_k<CPLX>() + fk : fk * stride_rows<CPLX, BM>() + wm + fr);
     const T* fb = ring + AE + (TB ? fk * stride_rows<CPLX, BN>() + wn + fr : (wn + fr) * stride_k<CPLX>() + fk);
     auto multiply = [&](int stage) {
 #pragma unroll
-        for (int k4 = 0; k4 < BK / (4 * WK); ++k4) {
+        for (int k4 = 0; k4 < BK / 4; ++k4) {
             T a[MT], b[NT];
 #pragma unroll
             for (int i = 0; i < MT; ++i)
-                a[i] = fa[stage * (AE + BE) + (TA ? 8 * i * stride_k<CPLX>() + 4 * WK * k4
-                                                  : 4 * WK * k4 * stride_rows<CPLX, BM>() + 8 * i)];
+                a[i] = fa[stage * (AE + BE) + (TA ? 8 * i * stride_k<CPLX>() + 4 * k4
+                                                  : 4 * k4 * stride_rows<CPLX, BM>() + 8 * i)];
 #pragma unroll
             for (int j = 0; j < NT; ++j)
-                b[j] = fb[stage * (AE + BE) + (TB ? 4 * WK * k4 * stride_rows<CPLX, BN>() + 8 * j
-                                                  : 8 * j * stride_k<CPLX>() + 4 * WK * k4)];
+                b[j] = fb[stage * (AE + BE) + (TB ? 4 * k4 * stride_rows<CPLX, BN>() + 8 * j
+                                                  : 8 * j * stride_k<CPLX>() + 4 * k4)];
             if constexpr (CPLX) {
 #pragma unroll
                 for (int i = 0; i < MT; ++i) {
-                    const double ai = sa * a[i].y, nai = -ai;
+                    const double ai = flip(a[i].y, sa), nai = flip(ai, 0x80000000);
 #pragma unroll
                     for (int j = 0; j < NT; ++j) {
-                        const double bi = sb * b[j].y;
+                        const double bi = flip(b[j].y, sb);
                         dmma(acc[0][i][j], a[i].x, b[j].x);
                         dmma(acc[NP - 1][i][j], a[i].x, bi);
                         dmma(acc[0][i][j], nai, bi);
@@ -260,8 +267,18 @@ __global__ void __launch_bounds__(32 * WM * WN * WK) gemm_dmma_kernel(const __gr
         if constexpr (CPLX) return make_double2(acc[0][i][j][h], acc[NP - 1][i][j][h]);
         else return acc[0][i][j][h];
     };
-    // the warps' partial tiles, column-major, in the ring's memory (one per k share); then each CTA of the
-    // cluster adds up and writes its part of the tile
+    if (S == 1) {
+#pragma unroll
+        for (int j = 0; j < NT; ++j)
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+#pragma unroll
+                for (int i = 0; i < MT; ++i)
+                    emit(m0 + wm + 8 * i + (lane >> 2), n0 + wn + 8 * j + 2 * (lane & 3) + h, value(i, j, h));
+        return;
+    }
+    // the CTA's partial tile, column-major, in the ring's memory; then each CTA of the cluster adds up and
+    // writes its part of the tile
     cg::cluster_group cl = cg::this_cluster();
     __syncthreads();
 #pragma unroll
@@ -270,35 +287,28 @@ __global__ void __launch_bounds__(32 * WM * WN * WK) gemm_dmma_kernel(const __gr
         for (int j = 0; j < NT; ++j)
 #pragma unroll
             for (int h = 0; h < 2; ++h)
-                ring[wk * BM * BN + wm + 8 * i + (lane >> 2) + (wn + 8 * j + 2 * (lane & 3) + h) * BM] = value(i, j, h);
-    if (S > 1) cl.sync();
-    else __syncthreads();
+                ring[wm + 8 * i + (lane >> 2) + (wn + 8 * j + 2 * (lane & 3) + h) * BM] = value(i, j, h);
+    cl.sync();
     for (int e = rank * NTHR + threadIdx.x; e < BM * BN; e += S * NTHR) {
         T sum{};
         for (int s = 0; s < S; ++s) {
-            const T* part = S > 1 ? cl.map_shared_rank(ring, s) : ring;
-            T v[WK];
-#pragma unroll
-            for (int w = 0; w < WK; ++w) v[w] = part[w * BM * BN + e];
-#pragma unroll
-            for (int w = 0; w < WK; ++w) {
-                if constexpr (CPLX) {
-                    sum.x += v[w].x;
-                    sum.y += v[w].y;
-                } else {
-                    sum += v[w];
-                }
+            const T v = cl.map_shared_rank(ring, s)[e];
+            if constexpr (CPLX) {
+                sum.x += v.x;
+                sum.y += v.y;
+            } else {
+                sum += v;
             }
         }
         emit(m0 + e % BM, n0 + e / BM, sum);
     }
-    if (S > 1) cl.sync();  // no CTA leaves while another reads its partial tiles
+    cl.sync();  // no CTA leaves while another reads its partial tile
 }
 
-template <bool CPLX, int BM, int BN, int WM, int WN, int WK, int ST, bool TA, bool TB, bool VEC>
+template <bool CPLX, int BM, int BN, int WM, int WN, int ST, bool TA, bool TB, bool VEC>
 void launch_t(const DgArgs& a, int nz, int split) {
-    constexpr int SM = smem_bytes<CPLX, BM, BN, WK, ST, TA, TB>();
-    auto kernel = gemm_dmma_kernel<CPLX, BM, BN, WM, WN, WK, ST, TA, TB, VEC>;
+    constexpr int SM = smem_bytes<CPLX, BM, BN, ST, TA, TB>();
+    auto kernel = gemm_dmma_kernel<CPLX, BM, BN, WM, WN, ST, TA, TB, VEC>;
     static bool attr = false;
     if (!attr) {
         OMM_CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SM));
@@ -306,7 +316,7 @@ void launch_t(const DgArgs& a, int nz, int split) {
     }
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(((a.M + BM - 1) / BM) * ((a.N + BN - 1) / BN), nz, split);
-    cfg.blockDim = dim3(32 * WM * WN * WK);
+    cfg.blockDim = dim3(32 * WM * WN);
     cfg.dynamicSmemBytes = SM;
     cfg.stream = rt().stream;
     cudaLaunchAttribute at[1];
@@ -317,12 +327,12 @@ void launch_t(const DgArgs& a, int nz, int split) {
     OMM_CK(cudaLaunchKernelEx(&cfg, kernel, a));
     OMM_KCHECK();
 }
-template <bool CPLX, int BM, int BN, int WM, int WN, int WK, int ST, bool VEC>
+template <bool CPLX, int BM, int BN, int WM, int WN, int ST, bool VEC>
 void launch_ops(const DgArgs& a, bool ta, bool tb, int nz, int split) {
-    if (ta && tb) launch_t<CPLX, BM, BN, WM, WN, WK, ST, true, true, VEC>(a, nz, split);
-    else if (ta) launch_t<CPLX, BM, BN, WM, WN, WK, ST, true, false, VEC>(a, nz, split);
-    else if (tb) launch_t<CPLX, BM, BN, WM, WN, WK, ST, false, true, VEC>(a, nz, split);
-    else launch_t<CPLX, BM, BN, WM, WN, WK, ST, false, false, VEC>(a, nz, split);
+    if (ta && tb) launch_t<CPLX, BM, BN, WM, WN, ST, true, true, VEC>(a, nz, split);
+    else if (ta) launch_t<CPLX, BM, BN, WM, WN, ST, true, false, VEC>(a, nz, split);
+    else if (tb) launch_t<CPLX, BM, BN, WM, WN, ST, false, true, VEC>(a, nz, split);
+    else launch_t<CPLX, BM, BN, WM, WN, ST, false, false, VEC>(a, nz, split);
 }
 
 // Split of K by an estimate of the time in SM clocks: the CTAs of the busiest SM in turn, each with a
@@ -333,8 +343,8 @@ struct Config {
     int split;
     double us;
 };
-Config pick(bool cplx, int M, int N, int K, int nz, bool herm) {
-    const double chunk_k = cplx ? 8.0 : 16.0, busy = cplx ? 550.0 : 300.0, alone = cplx ? 800.0 : 425.0;
+Config pick(bool cplx, int M, int N, int K, int nz, bool herm, bool wide = true) {
+    const double chunk_k = cplx ? 8.0 : 16.0, busy = cplx ? 550.0 : wide ? 300.0 : 390.0, alone = cplx ? 800.0 : 425.0;
     const double tiles = (double)((M + 31) / 32) * ((N + 31) / 32) * nz * (herm ? 0.6 : 1.0);
     Config best{1, 1e300};
     for (int s = 1; s <= 8; s *= 2) {
@@ -350,7 +360,16 @@ Config pick(bool cplx, int M, int N, int K, int nz, bool herm) {
 
 }  // namespace
 
-double gemm_dmma_us(bool cplx, int M, int N, int K, int nz) { return pick(cplx, M, N, K, nz, false).us; }
+// Products cuBLAS has the better split for, left to it (a call, microseconds, cuBLAS / this kernel): complex
+// ones with a long K (64 x 64 x 3,000 29 / 37, 100 x 1,000 x 3,000 115 / 131, 64 x 3,000 x 3,000 161 / 208; at
+// K = 1,000 or below this kernel leads, 257 x 259 x 1,001 45 / 43), and real ones of one or two rows of tiles
+// with a long K (64 x 3,000 x 3,000 61 / 64; 100 x 1,000 x 3,000 49 / 48, 130 x 260 x 3,000 34 / 30).
+bool gemm_dmma_slower(bool cplx, int M, int N, int K) {
+    if (cplx) return K >= 1500;
+    return K >= 2500 && std::min(M, N) <= 64 && std::max(M, N) >= 1500;
+}
+
+double gemm_dmma_us(bool cplx, int M, int N, int K, int nz, bool wide) { return pick(cplx, M, N, K, nz, false, wide).us; }
 
 bool gemm_dmma_takes(const DView& v) { return v.is_real || (reinterpret_cast<uintptr_t>(v.p) & 15) == 0; }
 
@@ -388,13 +407,9 @@ void gemm_dmma(char opA, char opB, int M, int N, int K, const double alpha[2], c
     const Config c = pick(cplx, M, N, K, nz, any && nz == 1);
     const int bk = cplx ? 8 : 16;
     a.kper = std::max(bk, ((K + c.split - 1) / c.split + bk - 1) / bk * bk);
-    if (cplx) {
-        launch_ops<true, 32, 32, 2, 1, 2, 4, true>(a, ta, tb, nz, c.split);
-    } else if (a.vec) {
-        launch_ops<false, 32, 32, 1, 1, 4, 4, true>(a, ta, tb, nz, c.split);
-    } else {
-        launch_ops<false, 32, 32, 1, 1, 4, 4, false>(a, ta, tb, nz, c.split);
-    }
+    if (cplx) launch_ops<true, 32, 32, 2, 2, 2, true>(a, ta, tb, nz, c.split);
+    else if (a.vec) launch_ops<false, 32, 32, 2, 2, 3, true>(a, ta, tb, nz, c.split);
+    else launch_ops<false, 32, 32, 2, 2, 3, false>(a, ta, tb, nz, c.split);
 }
 
 }  // namespace ommgpu

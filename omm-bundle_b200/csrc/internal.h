@@ -295,7 +295,8 @@ void transpose_into(const DView& A, char op, DView& T);  // T = op(A)
 // Nothing is done when *stop (device memory, may be null) is set.
 void gemm_dmma(char opA, char opB, int M, int N, int K, const double alpha[2], const DView* A, const DView* B,
                const double beta[2], DView* C, int nz = 1, const int* herm = nullptr, const int* stop = nullptr);
-double gemm_dmma_us(bool cplx, int M, int N, int K, int nz = 1);  // its estimated time
+bool gemm_dmma_slower(bool cplx, int M, int N, int K);  // than cuBLAS, for a single product
+double gemm_dmma_us(bool cplx, int M, int N, int K, int nz = 1, bool wide = true);  // its estimated time
 bool gemm_dmma_takes(const DView& v);  // complex operands must lie on 16-byte addresses
 
 // ----------------------------------------------------------------- SpMM (spmm.cu)
@@ -385,7 +386,8 @@ void gemm_z_emu(char opA, char opB, int M, int N, int K, double alpha, const DVi
 bool fp64_emu_enabled();  // real FP64 GEMMs of the solver on the int8 tensor cores (default on)
 void set_fp64_emu(int mode, long long panel_bytes);
 size_t oz_panel_bytes();
-bool fp64_emu_worth(int M, int N, int K, bool cplx = false);  // the emulation is faster than gemm_dmma
+// the emulation is faster than gemm_dmma (wide: operands it can copy 16 bytes at a time)
+bool fp64_emu_worth(int M, int N, int K, bool cplx = false, bool wide = true);
 bool fp64_emu_fits(int M, int N, int K);  // in-place products: large enough for the emulation to pay against cuBLAS
 
 // ----------------------------------------------------------------- tensor-core SpMM (spmm_tc.cu)

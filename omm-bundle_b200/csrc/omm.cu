@@ -399,7 +399,11 @@ void apply_op(OmmCall& c, const DView& A, bool isH, DView& out) {
         spmm_dense_csc(A, Mm, out, ONE, ZERO);
     } else {
         const DView& Md = isH ? c.H : c.S;
-        gemm('n', 'n', c.n, c.m, c.m, ONE, A, Md, ZERO, out);
+        // never cuBLAS here: the steps of a small problem may be under capture (run_ahead)
+        if (fp64_emu_enabled() && !fp64_emu_worth(c.n, c.m, c.m, !c.real) && gemm_dmma_takes(A) && gemm_dmma_takes(Md) &&
+            gemm_dmma_takes(out))
+            gemm_dmma('n', 'n', c.n, c.m, c.m, ONE, &A, &Md, ZERO, &out);
+        else gemm('n', 'n', c.n, c.m, c.m, ONE, A, Md, ZERO, out);
     }
 }
 

@@ -2372,14 +2372,14 @@ bool fp64_emu_fits(int M, int N, int K) {
 // exponents and reconstruction at 3.5 TB/s; complex operands are stacked parts.  Within 15 % of 32 measured
 // shapes: 1,024^3 76 us either way; 2,000 x 1,000 x 2,000 159 against 264; 130 x 1,611 x 3,000 103 against 61;
 // complex 800^3 141 against 146, 300 x 150 x 3,000 98 against 70.
-bool fp64_emu_worth(int M, int N, int K, bool cplx) {
+bool fp64_emu_worth(int M, int N, int K, bool cplx, bool wide) {
     if (K < 64 || K >= (1 << 17) || M < 1 || N < 1) return false;
     const double w = cplx ? 2.0 : 1.0;
     const double items = std::ceil(w * M / 256.0) * std::ceil(w * N / 256.0) * OZ_NMOD;
     const double waves = std::ceil(items / 74.0);
     const double in = ((double)M * K + (double)N * K) * 32.0 * w, out = (double)M * N * (cplx ? 144.0 : 40.0);
     const double us = 36.0 + waves * (std::max(3.0, 0.37 * std::ceil(K / 128.0)) + 0.5) + (in + out) / 3.5e6;
-    return us < gemm_dmma_us(cplx, M, N, K);
+    return us < gemm_dmma_us(cplx, M, N, K, 1, wide);
 }
 
 void gemm_f64_emu(char opA, char opB, int M, int N, int K, double alpha, const DView& A, const DView& B, double beta,

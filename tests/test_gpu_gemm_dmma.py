@@ -109,3 +109,12 @@ def test_solve_with_emulated_operator_products():
     """m = 2,000, n = 400: the Gram products and calc_G stay on the FP64 tensor cores, so the steps run ahead
     in a graph, while D H and D S are large enough for the int8 emulation: it is part of the graph."""
     test_small_solve(2000, 400, False)
+
+
+@pytest.mark.parametrize("cplx", [False, True])
+@pytest.mark.parametrize("M,N,K", [(515, 301, 16), (1025, 417, 33), (64, 1500, 2501), (40, 40, 1501), (301, 261, 401)])
+def test_short_and_long_k(M, N, K, cplx):
+    """Unsplit tiles written from the accumulators (short K, odd edges), and both sides of the rule that leaves
+    products with a long K to cuBLAS."""
+    _check(M, N, K, "t", "n", cplx, 0.75, -1.25)
+    _check(M, N, min(K, 1499), "n", "t", cplx)
