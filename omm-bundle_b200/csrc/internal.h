@@ -226,6 +226,15 @@ struct DView {
     bool is_real = true;
     template <typename T> T* as() const { return (T*)p; }
 };
+// Whether the memory that two views span has a byte in common (of views interleaved by their leading
+// dimensions too, where no element is shared)
+inline bool overlap(const DView& a, const DView& b) {
+    auto end = [](const DView& v) {
+        return (const char*)v.p + ((size_t)(v.cols - 1) * v.ld + v.rows) * (v.is_real ? 8 : 16);
+    };
+    if (a.rows <= 0 || a.cols <= 0 || b.rows <= 0 || b.cols <= 0) return false;
+    return (const char*)a.p < end(b) && (const char*)b.p < end(a);
+}
 
 // Parse/validate labels
 struct Label {

@@ -1110,7 +1110,9 @@ void gespmm(char opA, const msw_matrix* A, char opB, const DView& B, DView& C, c
     // every cell of the groups' blocks is a nonzero (atom blocks): nothing is multiplied that the sparse
     // product leaves out
     const bool full = P && P->efficiency == 1.0;
-    if (full && !aC) {
+    // the direct form writes C while it reads X, which is B itself for 't': where they share memory (C = op(A)
+    // B^T in place) the product goes through Z
+    if (full && !aC && !overlap(X, C)) {
         const int bz = (beta[0] == 0.0 && beta[1] == 0.0) ? 1 : 0;
         launch_cgu_dmma(X, *P, nullptr, C, nullptr, alpha, beta, bz, M, true);
         return;
