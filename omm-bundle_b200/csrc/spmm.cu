@@ -641,22 +641,8 @@ __global__ void __launch_bounds__(256) fill_blocks_kernel(int G, int N, const in
     }
 }
 
+// the dense blocks of the groups (which finish_plan has put on the device) with B's values
 void upload_blocks(const msw_matrix* B, SpmmPlan& P, DevBuf& dst) {
-    // the group structure on the device (cgu plans upload it in finish_plan; others need it here)
-    DevBuf gp, ur;
-    const int* d_gptr = P.gptr.as<int>();
-    const int* d_urows = P.urows.as<int>();
-    if (!P.gptr.p) {
-        gp.alloc(P.h_gptr.size() * sizeof(int));
-        ur.alloc(std::max<size_t>(1, P.h_urows.size()) * sizeof(int));
-        OMM_CK(cudaMemcpyAsync(gp.p, P.h_gptr.data(), P.h_gptr.size() * sizeof(int), cudaMemcpyHostToDevice,
-                               rt().stream));
-        if (!P.h_urows.empty())
-            OMM_CK(cudaMemcpyAsync(ur.p, P.h_urows.data(), P.h_urows.size() * sizeof(int), cudaMemcpyHostToDevice,
-                                   rt().stream));
-        d_gptr = gp.as<int>();
-        d_urows = ur.as<int>();
-    }
     ensure_csc_device(B);
     const size_t cells = std::max<size_t>(1, P.h_urows.size() * (size_t)P.G);
     const int smem = std::max(1, P.maxK) * (int)sizeof(int);
@@ -666,18 +652,18 @@ void upload_blocks(const msw_matrix* B, SpmmPlan& P, DevBuf& dst) {
         if (smem > 48 * 1024)
             OMM_CK(cudaFuncSetAttribute(fill_blocks_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
         fill_blocks_kernel<double><<<P.ngroups, 256, smem, rt().stream>>>(
-            P.G, B->dim2, d_gptr, d_urows, B->d_colptr.as<int>(), B->d_rowind.as<int>(), B->d_val.as<double>(),
-            dst.as<double>());
+            P.G, B->dim2, P.gptr.as<int>(), P.urows.as<int>(), B->d_colptr.as<int>(), B->d_rowind.as<int>(),
+            B->d_val.as<double>(), dst.as<double>());
     } else {
         dst.alloc_zero(cells * sizeof(zdbl));
         if (smem > 48 * 1024)
             OMM_CK(cudaFuncSetAttribute(fill_blocks_kernel<zdbl>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-        fill_blocks_kernel<zdbl><<<P.ngroups, 256, smem, rt().stream>>>(P.G, B->dim2, d_gptr, d_urows,
-                                                                       B->d_colptr.as<int>(), B->d_rowind.as<int>(),
-                                                                       B->d_val.as<zdbl>(), dst.as<zdbl>());
+        fill_blocks_kernel<zdbl><<<P.ngroups, 256, smem, rt().stream>>>(
+            P.G, B->dim2, P.gptr.as<int>(), P.urows.as<int>(), B->d_colptr.as<int>(), B->d_rowind.as<int>(),
+            B->d_val.as<zdbl>(), dst.as<zdbl>());
     }
     OMM_KCHECK();
-    OMM_CK(cudaStreamSynchronize(rt().stream));  // the temporary group structure goes out of scope
+    OMM_CK(cudaStreamSynchronize(rt().stream));  // the caller may change the plan's host arrays
 }
 
 // Column groups of recently planned patterns, by content: a caller that registers a matrix
@@ -810,6 +796,25 @@ void finish_plan(const msw_matrix* B, SpmmPlan& Pl) {
     }
 }
 
+// The plan of a matrix with P's pattern.  It is complete (groups on the device too): the matrix may be
+// multiplied by itself next.
+SpmmPlan& plan_of_pattern(const msw_matrix* B2, const SpmmPlan& P) {
+    msw_matrix* Bm = const_cast<msw_matrix*>(B2);
+    if (!Bm->plan) {
+        auto Q = std::make_shared<SpmmPlan>();
+        Q->G = P.G;
+        Q->ngroups = P.ngroups;
+        Q->efficiency = P.efficiency;
+        Q->cgu = P.cgu;
+        Q->h_gptr = P.h_gptr;
+        Q->h_urows = P.h_urows;
+        Q->owner = B2;
+        finish_plan(B2, *Q);
+        Bm->plan = Q;
+    }
+    return *Bm->plan;
+}
+
 }  // namespace
 
 void spmm_plan_cache_clear() { clear_kept_groups(); }
@@ -911,16 +916,7 @@ void spmm_dense_csc(const DView& A, const msw_matrix* B, DView& C, const double 
     }
     SpmmPlan* P2 = nullptr;
     if (fuse) {
-        msw_matrix* B2m = const_cast<msw_matrix*>(B2);
-        if (!B2m->plan) {
-            // same pattern: share the groups, fill the second value set
-            auto Q = std::make_shared<SpmmPlan>();
-            Q->G = P.G; Q->ngroups = P.ngroups; Q->efficiency = P.efficiency; Q->cgu = true; Q->maxK = P.maxK;
-            Q->h_gptr = P.h_gptr; Q->h_urows = P.h_urows; Q->owner = B2;
-            upload_blocks(B2, *Q, Q->bvals);
-            B2m->plan = Q;
-        }
-        P2 = B2m->plan.get();
+        P2 = &plan_of_pattern(B2, P);
         if (P2->G != P.G || P2->h_gptr != P.h_gptr) fuse = false, P2 = nullptr;
     }
     const int bz = (beta[0] == 0.0 && beta[1] == 0.0) ? 1 : 0;
@@ -966,16 +962,7 @@ void spmm32_dense_csc(const float* A, int lda, int n, const msw_matrix* B, DView
     ensure_f32_values(P);
     SpmmPlan* P2 = nullptr;
     if (B2 && C2 && same_pattern(B, B2)) {
-        // second value set sharing the groups (built like spmm_dense_csc does)
-        msw_matrix* B2m = const_cast<msw_matrix*>(B2);
-        if (!B2m->plan) {
-            auto Q = std::make_shared<SpmmPlan>();
-            Q->G = P.G; Q->ngroups = P.ngroups; Q->efficiency = P.efficiency; Q->cgu = true; Q->maxK = P.maxK;
-            Q->h_gptr = P.h_gptr; Q->h_urows = P.h_urows; Q->owner = B2;
-            upload_blocks(B2, *Q, Q->bvals);
-            B2m->plan = Q;
-        }
-        P2 = B2m->plan.get();
+        P2 = &plan_of_pattern(B2, P);  // the second value set
         if (P2->G != P.G || P2->h_gptr != P.h_gptr) P2 = nullptr;
         else ensure_f32_values(*P2);
     }
