@@ -867,8 +867,9 @@ void gemm(char opA, char opB, int M, int N, int K, const double alpha[2], const 
     if (fp64_emu_enabled()) {
         const char ops[3] = {'n', 't', 'c'};
         const bool cplx = !C.is_real, real_scalars = !cplx || (alpha[1] == 0.0 && beta[1] == 0.0);
-        // the emulation reads its operands before it writes the result, the FP64 kernel while it does
-        const bool in_place = C.p == A.p || C.p == B.p;
+        // the emulation reads its operands before it writes the result, the FP64 kernel while it does: products
+        // whose result shares any memory with an operand never take the latter
+        const bool in_place = overlap(C, A) || overlap(C, B);
         // real operands with odd leading dimensions are copied 8 bytes at a time: 1,001 x 515 x 2,003 109 us on the
         // FP64 tensor cores, 85 emulated
         const auto wide16 = [](const DView& v) { return v.ld % 2 == 0 && (reinterpret_cast<uintptr_t>(v.p) & 15) == 0; };

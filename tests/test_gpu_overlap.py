@@ -39,3 +39,27 @@ def test_csc_times_dense_in_place(norb, opA, opB, cplx):
         # eps of |alpha Z| + |beta C| <= |result| + 2 |beta C|
         bar = 4 * np.finfo(float).eps * (float(own.abs().max()) + 2 * float(X.abs().max()))
         assert float((both - own).abs().max()) <= bar
+
+
+@pytest.mark.parametrize("cplx", [False, True])
+@pytest.mark.parametrize("shift", [0, 1, 300 * 600, 600 * 600 - 1])
+@pytest.mark.parametrize("which", ["A", "B"])
+def test_dense_result_inside_an_operand(which, shift, cplx):
+    """C = A B with C registered `shift` elements into the memory of A or B, at a size where the int8 emulation
+    (which reads its operands first) is not the faster engine."""
+    import torch
+
+    m = 600
+    g = torch.Generator(device="cuda").manual_seed(shift)
+    A, B = _rnd(g, m, m, cplx=cplx), _rnd(g, m, m, cplx=cplx)
+    ref, mag = A.t() @ B.t(), A.abs().t() @ B.abs().t()  # the handles see the transposes
+    for _ in range(4):
+        store = torch.zeros(2 * m * m, dtype=A.dtype, device="cuda")
+        other = (B if which == "A" else A).clone()
+        store[:m * m] = (A if which == "A" else B).reshape(-1)
+        C = store[shift:shift + m * m]
+        hs, ho, hc = (G.Matrix.register_gden(t.data_ptr(), m, m, cplx, keep=t) for t in (store, other, C))
+        torch.cuda.synchronize()
+        G.mm_multiply(*((hs, "n", ho, "n") if which == "A" else (ho, "n", hs, "n")), hc)
+        # both products are within m eps |A||B| (complex: four real ones), the kept 53 bits included
+        assert float(((C.view(m, m).t() - ref).abs() / mag).max()) <= 8 * m * np.finfo(float).eps
