@@ -160,6 +160,7 @@ void DevBuf::release() {
 }
 
 // ------------------------------------------------------------------ runtime
+thread_local cudaStream_t LibraryStream::capture = nullptr;
 static Runtime* g_rt = nullptr;
 static std::mutex g_rt_mu;
 
@@ -172,7 +173,7 @@ Runtime& rt() {
         OMM_CK(cudaGetDevice(&dev));
         OMM_CK(cudaSetDevice(dev));
         g_rt->device = dev;
-        OMM_CK(cudaStreamCreateWithFlags(&g_rt->stream, cudaStreamNonBlocking));
+        OMM_CK(cudaStreamCreateWithFlags(&g_rt->stream.s, cudaStreamNonBlocking));
         g_rt->own_stream = true;
         OMM_CKB(cublasCreate(&g_rt->blas));
         OMM_CKB(cublasSetStream(g_rt->blas, g_rt->stream));
@@ -444,10 +445,10 @@ int omm_gpu_set_stream(void* s) {
     OMM_CK(cudaStreamSynchronize(r.stream));
     if (r.own_stream) OMM_CK(cudaStreamDestroy(r.stream));
     if (s) {
-        r.stream = (cudaStream_t)s;
+        r.stream.s = (cudaStream_t)s;
         r.own_stream = false;
     } else {
-        OMM_CK(cudaStreamCreateWithFlags(&r.stream, cudaStreamNonBlocking));
+        OMM_CK(cudaStreamCreateWithFlags(&r.stream.s, cudaStreamNonBlocking));
         r.own_stream = true;
     }
     OMM_CKB(cublasSetStream(r.blas, r.stream));

@@ -118,10 +118,18 @@ struct DevBuf {
 };
 
 // ----------------------------------------------------------------- runtime
+// The library's stream.  While a thread captures launches (run_ahead, omm.cu), that thread's work goes to the
+// private stream of the capture instead; every other thread, and the caller, keep the stream itself.
+struct LibraryStream {
+    cudaStream_t s = nullptr;
+    static thread_local cudaStream_t capture;
+    operator cudaStream_t() const { return capture ? capture : s; }
+};
 struct Runtime {
     int device = -1;
-    cudaStream_t stream = nullptr;
+    LibraryStream stream;
     bool own_stream = false;
+    cudaStream_t capture = nullptr;  // run_ahead's launches are captured here
     cublasHandle_t blas = nullptr;
     cusolverDnHandle_t solver = nullptr;
     DevBuf scratch;   // reduction partials and small temporaries

@@ -748,20 +748,26 @@ int run_ahead(OmmCall& c, DView& G, DView& Gp, DView& D, DView& Cw, long most, d
     };
     // the graph of this call's buffers, captured anew; the executable kept from the last call takes its
     // parameters where it was made for the same launches (an update does not change cluster shapes), else a
-    // new one is made.  Without one (a stream that cannot be captured) the steps are launched one by one.
+    // new one is made.  Captured on a stream of the library's own: R.stream may be the caller's, and what
+    // another thread queues there meanwhile is no part of a step.  Without a graph the steps are launched one
+    // by one.
     bool graph = false;
     if (!ktime_on()) {
         cudaGraph_t g = nullptr;
-        if (cudaStreamBeginCapture(R.stream, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
+        if (!R.capture) OMM_CK(cudaStreamCreateWithFlags(&R.capture, cudaStreamNonBlocking));
+        if (cudaStreamBeginCapture(R.capture, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
+            LibraryStream::capture = R.capture;
             try {
                 two_steps();
             } catch (...) {
-                cudaStreamEndCapture(R.stream, &g);
+                LibraryStream::capture = nullptr;
+                cudaStreamEndCapture(R.capture, &g);
                 if (g) cudaGraphDestroy(g);
                 cudaGetLastError();
                 throw;
             }
-            graph = cudaStreamEndCapture(R.stream, &g) == cudaSuccess && g;
+            LibraryStream::capture = nullptr;
+            graph = cudaStreamEndCapture(R.capture, &g) == cudaSuccess && g;
         }
         auto align = [](const void* p) { return (long long)((uintptr_t)p % 16); };
         const long long key[6] = {n, m, r, c.H_csc ? (long long)c.Hm->pattern_id : -1,
@@ -1796,6 +1802,10 @@ int omm_gpu_finalize(void) {
             sync();
             cudaGraphExecDestroy(rt().steps);
             rt().steps = nullptr;
+        }
+        if (rt().capture) {
+            cudaStreamDestroy(rt().capture);
+            rt().capture = nullptr;
         }
         g_state = OmmState();
         g_state_cb = OmmState();
