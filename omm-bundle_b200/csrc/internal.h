@@ -136,7 +136,7 @@ struct Runtime {
     DevBuf scratch2;  // transposes / staging
     double* host_pinned = nullptr;  // small pinned host buffer for scalar read-back
     cudaGraphExec_t steps = nullptr;  // run_ahead's executable graph (omm.cu), updated by each call
-    long long steps_key[6] = {};      // the launches it was made for
+    std::vector<unsigned long long> steps_shape;  // the launches it was made from (launch_shape)
 };
 Runtime& rt();
 bool runtime_bound();  // rt() has been set up on a device (no CUDA call is made to find out)

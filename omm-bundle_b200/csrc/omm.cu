@@ -695,6 +695,39 @@ bool step_runs_ahead(const OmmCall& c, const DView& Cw) {
            (c.s_identity || c.S_csc || gemm_dmma_takes(c.S));
 }
 
+// A graph's nodes as an executable made from it keeps them: kinds, kernels, grids, blocks and cluster shapes
+// (cudaGraphExecUpdate takes a kernel with another cluster shape and launches it with the old one).  Empty,
+// which stands for no executable, where a node does not tell.
+std::vector<unsigned long long> launch_shape(cudaGraph_t g) {
+    std::vector<unsigned long long> shape;
+    auto put = [&](unsigned x, unsigned y, unsigned z) { shape.insert(shape.end(), {x, y, z}); };
+    size_t count = 0;
+    bool told = cudaGraphGetNodes(g, nullptr, &count) == cudaSuccess;
+    std::vector<cudaGraphNode_t> nodes(count);
+    told = told && count > 0 && cudaGraphGetNodes(g, nodes.data(), &count) == cudaSuccess;
+    for (size_t i = 0; told && i < count; ++i) {
+        cudaGraphNodeType type;
+        told = cudaGraphNodeGetType(nodes[i], &type) == cudaSuccess;
+        if (!told) break;
+        shape.push_back((unsigned long long)type);
+        if (type != cudaGraphNodeTypeKernel) continue;
+        cudaKernelNodeParams k{};
+        cudaLaunchAttributeValue cluster{};
+        told = cudaGraphKernelNodeGetParams(nodes[i], &k) == cudaSuccess &&
+               cudaGraphKernelNodeGetAttribute(nodes[i], cudaLaunchAttributeClusterDimension, &cluster) == cudaSuccess;
+        shape.push_back((unsigned long long)(uintptr_t)k.func);
+        shape.push_back(k.sharedMemBytes);
+        put(k.gridDim.x, k.gridDim.y, k.gridDim.z);
+        put(k.blockDim.x, k.blockDim.y, k.blockDim.z);
+        put(cluster.clusterDim.x, cluster.clusterDim.y, cluster.clusterDim.z);
+    }
+    if (!told) {
+        cudaGetLastError();
+        shape.clear();
+    }
+    return shape;
+}
+
 // CG steps of a small problem without waiting for the host.  A step's line search is solved in the last
 // block of its coefficients' kernel (the host's own routine), which leaves x for the updates that follow
 // and a numbered record in pinned memory (at most four steps are out at a time); two steps (the gradient's buffers alternate) are one CUDA graph, and
@@ -769,21 +802,18 @@ int run_ahead(OmmCall& c, DView& G, DView& Gp, DView& D, DView& Cw, long most, d
             LibraryStream::capture = nullptr;
             graph = cudaStreamEndCapture(R.capture, &g) == cudaSuccess && g;
         }
-        auto align = [](const void* p) { return (long long)((uintptr_t)p % 16); };
-        const long long key[6] = {n, m, r, c.H_csc ? (long long)c.Hm->pattern_id : -1,
-                                  c.S_csc ? (long long)c.Sm->pattern_id : -1, align(Cw.p) + align(c.H.p) * 16 + align(c.S.p) * 256 +
-                                      (c.s_identity ? 4096 : 0)};
-        if (graph && R.steps) {
+        if (graph) {
+            const std::vector<unsigned long long> shape = launch_shape(g);
             cudaGraphExecUpdateResultInfo info{};
-            if (!std::equal(key, key + 6, R.steps_key) || cudaGraphExecUpdate(R.steps, g, &info) != cudaSuccess) {
+            if (R.steps && (shape.empty() || shape != R.steps_shape || cudaGraphExecUpdate(R.steps, g, &info) != cudaSuccess)) {
                 cudaGraphExecDestroy(R.steps);
                 R.steps = nullptr;
             }
-        }
-        std::copy(key, key + 6, R.steps_key);
-        if (graph && !R.steps && cudaGraphInstantiate(&R.steps, g, 0) != cudaSuccess) {
-            R.steps = nullptr;
-            graph = false;
+            if (!R.steps && cudaGraphInstantiate(&R.steps, g, 0) != cudaSuccess) {
+                R.steps = nullptr;
+                graph = false;
+            }
+            R.steps_shape = shape;
         }
         if (g) cudaGraphDestroy(g);
         cudaGetLastError();

@@ -118,3 +118,31 @@ def test_short_and_long_k(M, N, K, cplx):
     products with a long K to cuBLAS."""
     _check(M, N, K, "t", "n", cplx, 0.75, -1.25)
     _check(M, N, min(K, 1499), "n", "t", cplx)
+
+
+def test_kept_graph_follows_the_kernels_of_its_steps():
+    """The m = 2,000, n = 400 solve, whose steps hold emulated products, with those products on SM pairs (clusters
+    of two CTAs), on single SMs and on pairs again: a kept graph of the one form does not serve the other, and
+    all forms give the same bits."""
+    import torch
+
+    m, n = 2000, 400
+    g = torch.Generator(device="cuda").manual_seed(m)
+    Q, _ = torch.linalg.qr(torch.randn(m, m, generator=g, device="cuda", dtype=torch.float64))
+    lam = torch.linspace(-2.0, -1.0, m, device="cuda", dtype=torch.float64)
+    lam[n:] += 2.5
+    H = (Q * lam) @ Q.mH
+    (h, kh), (c, kc), (d, kd) = _mat(0.5 * (H + H.mH)), _mat(H[:n] * 0), _mat(H * 0)
+    torch.cuda.synchronize()
+    G.set_log(None)
+    got = []
+    try:
+        for pairs in (1, 1, 0, 0, 1):
+            assert G.lib().omm_gpu_tc_set_pairs(pairs) == 0
+            e, rc = G.omm(m, n, h, None, True, d, False, 0.0, c, False, dealloc=True)
+            assert rc == 0 and G.tc_errors() == 0
+            got.append((e, G.stats()["icg"], kd.clone()))
+    finally:
+        assert G.lib().omm_gpu_tc_set_pairs(1) == 0
+    for e, steps, dens in got[1:]:
+        assert e == got[0][0] and steps == got[0][1] and torch.equal(dens, got[0][2])
