@@ -1070,15 +1070,16 @@ __device__ __forceinline__ bool oz_rows_below(int i0, int herm, int c) {
     return herm > 0 && i0 % herm > c && i0 % herm + 3 < herm;
 }
 
-// thread: rows 4 t .. 4 t + 3 of 8 columns
+constexpr int REC_COLS = 8, REC_COLS_Z = 2;  // columns of a block's threads: real, complex
+// thread: rows 4 t .. 4 t + 3 of REC_COLS columns
 __global__ void __launch_bounds__(256) oz_reconstruct_kernel(const __grid_constant__ RecParams p) {
     const int i0 = 4 * (blockIdx.x * 256 + threadIdx.x);
     if (i0 >= p.M) return;
     int ea[4];
 #pragma unroll
     for (int u = 0; u < 4; ++u) ea[u] = i0 + u < p.M ? p.eA[i0 + u] : ZERO_EXP;
-    for (int jj = 0; jj < 8; ++jj) {
-        const int j = blockIdx.y * 8 + jj;
+    for (int jj = 0; jj < REC_COLS; ++jj) {
+        const int j = blockIdx.y * REC_COLS + jj;
         if (j >= p.N) return;
         if (oz_rows_below(i0, p.herm, p.n_off + j)) continue;
         const int eb = p.eB[j];
@@ -1097,7 +1098,7 @@ __global__ void __launch_bounds__(256) oz_reconstruct_kernel(const __grid_consta
 
 // The same for a complex product: its four real ones (stacked operands, one GEMM) joined in one pass
 // over C, where a pass per real product read and wrote C's parts twice each (512 x 512: 61 us for the
-// four against 15).  thread: rows 4 t .. 4 t + 3 of 2 columns.
+// four against 15).  thread: rows 4 t .. 4 t + 3 of REC_COLS_Z columns.
 __global__ void __launch_bounds__(128) oz_reconstruct_z_kernel(const __grid_constant__ RecParams p) {
     const int i0 = 4 * (blockIdx.x * 128 + threadIdx.x);
     if (i0 >= p.M) return;
@@ -1107,8 +1108,8 @@ __global__ void __launch_bounds__(128) oz_reconstruct_z_kernel(const __grid_cons
         ear[u] = i0 + u < p.M ? p.eA[i0 + u] : ZERO_EXP;
         eai[u] = i0 + u < p.M ? p.eA[p.zrow + i0 + u] : ZERO_EXP;
     }
-    for (int jj = 0; jj < 2; ++jj) {
-        const int j = blockIdx.y * 2 + jj;
+    for (int jj = 0; jj < REC_COLS_Z; ++jj) {
+        const int j = blockIdx.y * REC_COLS_Z + jj;
         if (j >= p.N) return;
         if (oz_rows_below(i0, p.herm, p.n_off + j)) continue;
         const int ebr = p.eB[j], ebi = p.eBi[j];
@@ -1980,7 +1981,10 @@ static void oz_gemm_any(const OzOperand& A, const OzOperand& B, double alpha, do
     // the product's residue planes, for at most ~4 GB of them at a time: panels of columns
     const int ldr = (A.rows + 127) / 128 * 128, parts = cplx ? 2 : 1;
     const size_t cap = oz_panel_bytes() / parts;
-    const int np = (int)std::min<size_t>((size_t)N, std::max<size_t>(BN, cap / ((size_t)A.nmod * ldr) / BN * BN));
+    // (and no more columns than the reconstruction's grid.y of 65,535 blocks covers)
+    const size_t most = (size_t)65535 * (cplx ? REC_COLS_Z : REC_COLS) / BN * BN;
+    const int np = (int)std::min<size_t>(
+        (size_t)N, std::max<size_t>(BN, std::min(most, cap / ((size_t)A.nmod * ldr) / BN * BN)));
     DevBuf& Rb = product_planes();
     const size_t rplane = (size_t)ldr * (cplx ? 2 * (size_t)np + 3 : (size_t)np);  // B's parts start 4 rows apart
     Rb.ensure(rplane * A.nmod);
@@ -2023,9 +2027,9 @@ static void oz_gemm_any(const OzOperand& A, const OzOperand& B, double alpha, do
         if (cplx) {
             rp.zcol = nc == N ? B.zrow : nc;
             rp.eBi = B.exps.as<int>() + B.zrow + c0;
-            oz_reconstruct_z_kernel<<<dim3((M + 511) / 512, (nc + 1) / 2), 128, 0, rt().stream>>>(rp);
+            oz_reconstruct_z_kernel<<<dim3((M + 511) / 512, (nc + REC_COLS_Z - 1) / REC_COLS_Z), 128, 0, rt().stream>>>(rp);
         } else {
-            oz_reconstruct_kernel<<<dim3((M + 1023) / 1024, (nc + 7) / 8), 256, 0, rt().stream>>>(rp);
+            oz_reconstruct_kernel<<<dim3((M + 1023) / 1024, (nc + REC_COLS - 1) / REC_COLS), 256, 0, rt().stream>>>(rp);
         }
         OMM_KCHECK();
         ktime_end("oz_reconstruct_kernel", recon_bytes(rp, M, nc));

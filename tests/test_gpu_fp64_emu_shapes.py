@@ -92,3 +92,26 @@ def test_hermitian_blocks_start_inside_tiles(m, n, cplx):
     assert float((D - D.mH).abs().max()) == 0.0
     P = Q[:, :n] @ Q[:, :n].mH
     assert float((D - P).abs().max()) <= 1e-4
+
+
+@pytest.mark.parametrize("cplx,N", [(True, 140001), (False, 530003)])
+def test_more_columns_than_one_reconstruction_grid(cplx, N):
+    """Emulated products of so many columns that one launch of the reconstruction could not number its blocks:
+    the columns before, at and behind the panels' ends."""
+    import torch
+
+    M, K = 256, 1000 if cplx else 512
+    g = torch.Generator(device="cuda").manual_seed(N)
+    dt = torch.complex128 if cplx else torch.float64
+    A = torch.randn(M, K, generator=g, device="cuda", dtype=dt)
+    B = torch.randn(N, K, generator=g, device="cuda", dtype=dt)  # column-major K x N
+    C = torch.zeros(N, M, device="cuda", dtype=dt)
+    a, ka = _mat(A)
+    b = G.Matrix.register_gden(B.data_ptr(), K, N, cplx, keep=B)
+    c = G.Matrix.register_gden(C.data_ptr(), M, N, cplx, keep=C)
+    torch.cuda.synchronize()
+    G.mm_multiply(a, "n", b, "n", c)
+    at = 130816 if cplx else 524032
+    for lo, hi in ((0, 300), (at - 300, at + 300), (N - 300, N)):
+        x = B[lo:hi].t()
+        assert float(((C[lo:hi].t() - A @ x).abs() / (A.abs() @ x.abs())).max()) <= 1e-13
