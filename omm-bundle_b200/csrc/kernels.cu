@@ -864,6 +864,12 @@ void gemm(char opA, char opB, int M, int N, int K, const double alpha[2], const 
         return CUBLAS_OP_C;
     };
     if (M == 0 || N == 0) return;
+    if (alpha[0] == 0.0 && alpha[1] == 0.0) {
+        // C = beta C, and 0 whatever C holds for beta = 0 (as BLAS has it): A and B are not read
+        if (beta[0] == 0.0 && beta[1] == 0.0) k_set(C, 'a', beta, beta);
+        else if (beta[0] != 1.0 || beta[1] != 0.0) k_scale(C, beta);
+        return;
+    }
     if (fp64_emu_enabled()) {
         const char ops[3] = {'n', 't', 'c'};
         const bool cplx = !C.is_real, real_scalars = !cplx || (alpha[1] == 0.0 && beta[1] == 0.0);

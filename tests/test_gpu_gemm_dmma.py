@@ -146,3 +146,22 @@ def test_kept_graph_follows_the_kernels_of_its_steps():
         assert G.lib().omm_gpu_tc_set_pairs(1) == 0
     for e, steps, dens in got[1:]:
         assert e == got[0][0] and steps == got[0][1] and torch.equal(dens, got[0][2])
+
+
+@pytest.mark.parametrize("cplx", [False, True])
+@pytest.mark.parametrize("beta", [0.0, 1.0, -0.5])
+@pytest.mark.parametrize("M,N,K", [(33, 31, 17), (700, 300, 90), (1100, 1000, 1200)])
+def test_zero_alpha_reads_no_operand(M, N, K, beta, cplx):
+    """alpha = 0 scales C alone: an Inf or NaN in A or B does not reach it, and beta = 0 clears what C held."""
+    import torch
+
+    dt = torch.complex128 if cplx else torch.float64
+    A = torch.full((M, K), float("nan"), device="cuda", dtype=dt)
+    B = torch.full((K, N), float("inf"), device="cuda", dtype=dt)
+    C0 = torch.randn(M, N, device="cuda", dtype=dt, generator=torch.Generator(device="cuda").manual_seed(M))
+    if beta == 0.0:
+        C0[0, 0] = float("nan")
+    (a, ka), (b, kb), (c, kc) = _mat(A), _mat(B), _mat(C0)
+    torch.cuda.synchronize()
+    G.mm_multiply(a, "n", b, "n", c, 0.0, beta)
+    assert torch.equal(kc.t(), torch.zeros_like(C0) if beta == 0.0 else beta * C0)
