@@ -41,6 +41,7 @@ struct SpmmPlan {
     std::vector<int> h_gptr;    // ngroups+1 offsets into union rows
     std::vector<int> h_urows;   // union rows
     int maxK = 0;               // the largest union
+    bool too_long = false;      // column groups that fill_blocks_kernel cannot form: maxK over kMaxUnion
     DevBuf gptr, urows;
     DevBuf bvals;               // sum(|U_g|*G) values, row-major per group (k, c)
     const msw_matrix* owner = nullptr;
@@ -615,6 +616,7 @@ __device__ __forceinline__ void add_to(zdbl* d, const zdbl* v, long long l) {
     atomicAdd(&d->x, v[l].x);
     atomicAdd(&d->y, v[l].y);
 }
+constexpr int kMaxUnion = 200 * 1024 / (int)sizeof(int);  // the union rows lie in its shared memory
 template <typename T>
 __global__ void __launch_bounds__(256) fill_blocks_kernel(int G, int N, const int* __restrict__ gptr,
                                                           const int* __restrict__ urows, const int* __restrict__ colptr,
@@ -646,7 +648,6 @@ void upload_blocks(const msw_matrix* B, SpmmPlan& P, DevBuf& dst) {
     ensure_csc_device(B);
     const size_t cells = std::max<size_t>(1, P.h_urows.size() * (size_t)P.G);
     const int smem = std::max(1, P.maxK) * (int)sizeof(int);
-    if (smem > 200 * 1024) fail(OMM_ERR_UNSUPPORTED, "spmm plan: a column group's row union is too long");
     if (B->is_real) {
         dst.alloc_zero(cells * sizeof(double));
         if (smem > 48 * 1024)
@@ -727,7 +728,8 @@ void keep_groups(const msw_matrix* B, const SpmmPlan& P) {
 
 void finish_plan(const msw_matrix* B, SpmmPlan& P);
 
-SpmmPlan& get_plan(const msw_matrix* B) {
+// The matrix's plan, whether its column groups can be formed or not (too_long)
+SpmmPlan& any_plan(const msw_matrix* B) {
     msw_matrix* Bm = const_cast<msw_matrix*>(B);
     if (Bm->plan) return *Bm->plan;
     auto P = std::make_shared<SpmmPlan>();
@@ -774,6 +776,13 @@ SpmmPlan& get_plan(const msw_matrix* B) {
     return *P;
 }
 
+// The plan for the paths that have no other way to a matrix with column groups
+SpmmPlan& get_plan(const msw_matrix* B) {
+    SpmmPlan& P = any_plan(B);
+    if (P.too_long) fail(OMM_ERR_UNSUPPORTED, "spmm plan: a column group's row union is too long");
+    return P;
+}
+
 void clear_kept_groups() {
     std::lock_guard<std::mutex> lk(g_groups_mu);
     g_groups.clear();
@@ -784,7 +793,8 @@ void finish_plan(const msw_matrix* B, SpmmPlan& Pl) {
     SpmmPlan* P = &Pl;
     P->maxK = 0;
     for (size_t g = 0; g + 1 < P->h_gptr.size(); ++g) P->maxK = std::max(P->maxK, P->h_gptr[g + 1] - P->h_gptr[g]);
-    if (P->cgu) {
+    P->too_long = P->cgu && P->maxK > kMaxUnion;
+    if (P->cgu && !P->too_long) {
         P->gptr.alloc(P->h_gptr.size() * sizeof(int));
         P->urows.alloc(std::max<size_t>(1, P->h_urows.size()) * sizeof(int));
         OMM_CK(cudaMemcpyAsync(P->gptr.p, P->h_gptr.data(), P->h_gptr.size() * sizeof(int), cudaMemcpyHostToDevice,
@@ -1092,8 +1102,8 @@ void gespmm(char opA, const msw_matrix* A, char opB, const DView& B, DView& C, c
     const msw_matrix* Y = aN ? csc_transpose(A) : A;
     if (N == 0 || M == 0) return;
     const double one[2] = {1.0, 0.0}, zero[2] = {0.0, 0.0};
-    const SpmmPlan* P = rules_out_groups(Y) ? nullptr : &get_plan(Y);
-    if (P && !P->cgu) P = nullptr;
+    const SpmmPlan* P = rules_out_groups(Y) ? nullptr : &any_plan(Y);
+    if (P && (!P->cgu || P->too_long)) P = nullptr;
     // every cell of the groups' blocks is a nonzero (atom blocks): nothing is multiplied that the sparse
     // product leaves out
     const bool full = P && P->efficiency == 1.0;

@@ -81,3 +81,27 @@ def test_gespmm_nonfinite_stays_in_its_rows(norb, bad):
     touched = np.zeros((m, n), bool)
     touched[:, 3] = H.to_dense()[:, k] != 0.0
     assert np.array_equal(~np.isfinite(got), touched)
+
+
+@pytest.mark.parametrize("opA", ["n", "t"])
+@pytest.mark.parametrize("cplx", [False, True])
+def test_gespmm_with_a_long_row_union(opA, cplx):
+    """A filled CSC whose column groups span more rows than the group kernel's plan can hold (51,200): the
+    product takes the gather kernel.  psp_gemspm, which has no other kernel for it, refuses it."""
+    rng = np.random.default_rng(8)
+    long, short, n = 52000, 40, 5
+    v = rng.standard_normal((long, short)) + (1j * rng.standard_normal((long, short)) if cplx else 0)
+    # 't': a long x short matrix; 'n': a short x long one, whose transpose is planned
+    d = v if opA == "t" else v.T
+    A = synth.CSCMatrix(d.shape[0], d.shape[1], (np.arange(d.shape[1] + 1) * d.shape[0]).astype(np.int32),
+                        np.tile(np.arange(d.shape[0], dtype=np.int32), d.shape[1]), d.T.reshape(-1).copy())
+    B, C0 = _rnd(rng, (long, n), cplx), _rnd(rng, (short, n), cplx)
+    h, C = G.Matrix.from_csc(A), G.Matrix.from_numpy(C0)
+    for _ in range(2):
+        C.upload(C0)
+        G.psp_gespmm(short, n, long, h, opA, G.Matrix.from_numpy(B), "n", C, 0.7, 0.3)
+        bar = 4 * long * np.finfo(float).eps * (np.abs(v.T) @ np.abs(B) + np.abs(C0))
+        assert np.all(np.abs(C.numpy() - (0.7 * (v.T @ B) + 0.3 * C0)) <= bar)
+    wide = G.Matrix.from_numpy(_rnd(rng, (n, long), cplx))
+    with pytest.raises(G.OmmError):
+        G.psp_gemspm(n, short, long, wide, "n", h, "n" if opA == "t" else "t", G.Matrix.from_numpy(_rnd(rng, (n, short), cplx)))
