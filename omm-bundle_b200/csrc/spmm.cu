@@ -1110,8 +1110,8 @@ void gespmm(char opA, const msw_matrix* A, char opB, const DView& B, DView& C, c
     // the direct form writes C while it reads X, which is B itself for 't': where they share memory (C = op(A)
     // B^T in place) the product goes through Z
     if (full && !aC && !overlap(X, C)) {
-        const int bz = (beta[0] == 0.0 && beta[1] == 0.0) ? 1 : 0;
-        launch_cgu_dmma(X, *P, nullptr, C, nullptr, alpha, beta, bz, M, true);
+        // beta multiplies C even when it is 0 (an Inf or NaN of C stays), as in the last pass of the other routes
+        launch_cgu_dmma(X, *P, nullptr, C, nullptr, alpha, beta, 0, M, true);
         return;
     }
     // Z = X * Y  (N x M), then C = alpha*Z^T (or Z^H) + beta*C

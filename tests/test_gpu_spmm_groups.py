@@ -105,3 +105,27 @@ def test_gespmm_with_a_long_row_union(opA, cplx):
     wide = G.Matrix.from_numpy(_rnd(rng, (n, long), cplx))
     with pytest.raises(G.OmmError):
         G.psp_gemspm(n, short, long, wide, "n", h, "n" if opA == "t" else "t", G.Matrix.from_numpy(_rnd(rng, (n, short), cplx)))
+
+
+@pytest.mark.parametrize("cplx", [False, True])
+@pytest.mark.parametrize("norb", [0, 13, 24])
+def test_gespmm_beta_zero_multiplies(norb, cplx):
+    """beta = 0 multiplies C: a NaN that C holds stays where it is, whatever kernel the pattern takes (column
+    groups with and without zero cells, norb = 0: no groups)."""
+    if norb:
+        H = _case(norb, cplx, 90)
+    else:
+        rng = np.random.default_rng(1)
+        d = np.where(rng.random((300, 300)) < 0.02, rng.standard_normal((300, 300)), 0.0) * (1j if cplx else 1.0)
+        at = np.nonzero(d.T)
+        colptr = np.concatenate([[0], np.cumsum(np.bincount(at[0], minlength=300))]).astype(np.int32)
+        H = synth.CSCMatrix(300, 300, colptr, at[1].astype(np.int32), d.T[at])
+    rng = np.random.default_rng(2)
+    m, n = H.dim1, 33
+    C0 = _rnd(rng, (m, n), cplx)
+    C0[5, 7] = np.nan
+    C = G.Matrix.from_numpy(C0)
+    G.psp_gespmm(m, n, m, G.Matrix.from_csc(H), "n", G.Matrix.from_numpy(_rnd(rng, (m, n), cplx)), "n", C, 1.0, 0.0)
+    held = np.zeros((m, n), bool)
+    held[5, 7] = True
+    assert np.array_equal(np.isnan(C.numpy()), held)
