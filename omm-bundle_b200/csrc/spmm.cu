@@ -38,6 +38,7 @@ struct SpmmPlan {
     int ngroups = 0;
     double efficiency = 0.0;  // nnz / sum(|U_g| * G)
     bool cgu = false;
+    bool full = false;  // no zero cell: every column of a group holds each of its union's rows once
     std::vector<int> h_gptr;    // ngroups+1 offsets into union rows
     std::vector<int> h_urows;   // union rows
     int maxK = 0;               // the largest union
@@ -675,7 +676,7 @@ struct GroupsOfPattern {
     HostVec<int> colptr, rowind;
     int G = 0;
     double efficiency = 0.0;
-    bool cgu = false;
+    bool cgu = false, full = false;
     std::vector<int> gptr, urows;
 };
 std::mutex g_groups_mu;
@@ -719,6 +720,7 @@ void keep_groups(const msw_matrix* B, const SpmmPlan& P) {
     e->G = P.G;
     e->efficiency = P.efficiency;
     e->cgu = P.cgu;
+    e->full = P.full;
     e->gptr = P.h_gptr;
     e->urows = P.h_urows;
     std::lock_guard<std::mutex> lk(g_groups_mu);
@@ -727,6 +729,28 @@ void keep_groups(const msw_matrix* B, const SpmmPlan& P) {
 }
 
 void finish_plan(const msw_matrix* B, SpmmPlan& P);
+
+// Whether every column of a group holds each row of its union exactly once.  As many nonzeros as cells do not
+// say so: duplicate entries (which add up) count several times and can make up for zero cells.
+bool no_zero_cell(const msw_matrix* B, const SpmmPlan& P) {
+    std::atomic<bool> all{true};
+    host_parallel(B->dim2, [&](long long j0, long long j1) {
+        std::vector<int> rows;
+        for (long long j = j0; j < j1 && all; ++j) {
+            const int* u = P.h_urows.data() + P.h_gptr[j / P.G];
+            const int nu = P.h_gptr[j / P.G + 1] - P.h_gptr[j / P.G];
+            const int* r = B->h_rowind.data() + B->h_colptr[j];
+            bool same = B->h_colptr[j + 1] - B->h_colptr[j] == nu;
+            if (same && !std::equal(r, r + nu, u)) {  // the same rows in another order, perhaps
+                rows.assign(r, r + nu);
+                std::sort(rows.begin(), rows.end());
+                same = std::equal(rows.begin(), rows.end(), u);
+            }
+            if (!same) all = false;
+        }
+    });
+    return all;
+}
 
 // The matrix's plan, whether its column groups can be formed or not (too_long)
 SpmmPlan& any_plan(const msw_matrix* B) {
@@ -739,6 +763,7 @@ SpmmPlan& any_plan(const msw_matrix* B) {
         P->ngroups = (int)hit->gptr.size() - 1;
         P->efficiency = hit->efficiency;
         P->cgu = hit->cgu;
+        P->full = hit->full;
         P->h_gptr = hit->gptr;
         P->h_urows = hit->urows;
         finish_plan(B, *P);
@@ -770,6 +795,7 @@ SpmmPlan& any_plan(const msw_matrix* B) {
     P->cgu = (P->efficiency >= 0.5) && (avg >= 16.0);
     P->h_gptr.swap(pick->gptr);
     P->h_urows.swap(pick->urows);
+    P->full = P->cgu && nnz == pick->cells && no_zero_cell(B, *P);
     finish_plan(B, *P);
     keep_groups(B, *P);
     Bm->plan = P;
@@ -816,6 +842,7 @@ SpmmPlan& plan_of_pattern(const msw_matrix* B2, const SpmmPlan& P) {
         Q->ngroups = P.ngroups;
         Q->efficiency = P.efficiency;
         Q->cgu = P.cgu;
+        Q->full = P.full;
         Q->h_gptr = P.h_gptr;
         Q->h_urows = P.h_urows;
         Q->owner = B2;
@@ -1106,7 +1133,7 @@ void gespmm(char opA, const msw_matrix* A, char opB, const DView& B, DView& C, c
     if (P && (!P->cgu || P->too_long)) P = nullptr;
     // every cell of the groups' blocks is a nonzero (atom blocks): nothing is multiplied that the sparse
     // product leaves out
-    const bool full = P && P->efficiency == 1.0;
+    const bool full = P && P->full;
     // the direct form writes C while it reads X, which is B itself for 't': where they share memory (C = op(A)
     // B^T in place) the product goes through Z
     if (full && !aC && !overlap(X, C)) {

@@ -129,3 +129,33 @@ def test_gespmm_beta_zero_multiplies(norb, cplx):
     held = np.zeros((m, n), bool)
     held[5, 7] = True
     assert np.array_equal(np.isnan(C.numpy()), held)
+
+
+@pytest.mark.parametrize("shuffled", [False, True])
+def test_gespmm_duplicates_do_not_hide_a_zero_cell(shuffled):
+    """An atom-block matrix with one entry of a column given twice (the two add up) and another one missing:
+    as many entries as cells, but an Inf of the dense operand at the missing entry's row does not reach that
+    column's result."""
+    H = _case(24, False, 33)
+    rng = np.random.default_rng(33)
+    j, m = 100, H.dim2
+    lo, hi = int(H.colptr[j]), int(H.colptr[j + 1])
+    rowind, val = H.rowind.copy(), H.val.copy()
+    hole = int(rowind[lo + 30])
+    rowind[lo + 30] = rowind[lo + 29]
+    if shuffled:
+        p = lo + rng.permutation(hi - lo)
+        rowind[lo:hi], val[lo:hi] = rowind[p], val[p]
+    A = synth.CSCMatrix(H.dim1, m, H.colptr, rowind, val)
+    dense = np.zeros((H.dim1, m))
+    np.add.at(dense, (rowind, np.repeat(np.arange(m), np.diff(H.colptr))), val)
+    B = _rnd(rng, (H.dim1, 40), False)
+    C = G.Matrix.allocate(m, 40)
+    G.psp_gespmm(m, 40, H.dim1, G.Matrix.from_csc(A), "t", G.Matrix.from_numpy(B), "n", C, 1.0, 0.0)
+    _check(C.numpy(), dense.T @ B, np.abs(dense).T @ np.abs(B))
+    B[hole, 3] = np.inf
+    C = G.Matrix.allocate(m, 40)
+    G.psp_gespmm(m, 40, H.dim1, G.Matrix.from_csc(A), "t", G.Matrix.from_numpy(B), "n", C, 1.0, 0.0)
+    touched = np.zeros((m, 40), bool)
+    touched[:, 3] = dense[hole] != 0.0
+    assert not touched[j, 3] and np.array_equal(~np.isfinite(C.numpy()), touched)
