@@ -294,11 +294,9 @@ const msw_matrix* csc_transpose(const msw_matrix* A) {
     T->h_val.resize((size_t)A->nnz * w);
     std::vector<std::vector<int>> pos(nt, std::vector<int>(rows, 0));
     auto run = [&](const std::function<void(int, int, int)>& f) {  // f(thread, first column, last column)
-        std::vector<std::thread> th;
-        for (int t = 1; t < nt; ++t)
-            th.emplace_back(f, t, (int)((long long)A->dim2 * t / nt), (int)((long long)A->dim2 * (t + 1) / nt));
-        f(0, 0, A->dim2 / nt);
-        for (auto& t : th) t.join();
+        host_shares(nt, [&](int t) {
+            f(t, (int)((long long)A->dim2 * t / nt), (int)((long long)A->dim2 * (t + 1) / nt));
+        });
     };
     run([&](int t, int c0, int c1) {
         for (int l = A->h_colptr[c0]; l < A->h_colptr[c1]; ++l) pos[t][A->h_rowind[l]]++;

@@ -8,6 +8,7 @@
 #include <mutex>
 #include <new>
 #include <set>
+#include <system_error>
 #include <thread>
 
 namespace ommgpu {
@@ -143,10 +144,19 @@ void host_parallel(long long count, const std::function<void(long long, long lon
         f(0, count);
         return;
     }
+    host_shares((int)nt, [&](int t) { f(count * t / nt, count * (t + 1) / nt); });
+}
+
+void host_shares(int n, const std::function<void(int)>& f) {
     std::vector<std::thread> th;
-    th.reserve((size_t)nt - 1);
-    for (long long t = 1; t < nt; ++t) th.emplace_back(f, count * t / nt, count * (t + 1) / nt);
-    f(0, count / nt);
+    th.reserve((size_t)std::max(0, n - 1));
+    int t = 1;
+    try {
+        for (; t < n; ++t) th.emplace_back(f, t);
+    } catch (const std::system_error&) {
+    }
+    if (n > 0) f(0);
+    for (; t < n; ++t) f(t);  // the system has no more threads to give
     for (auto& x : th) x.join();
 }
 

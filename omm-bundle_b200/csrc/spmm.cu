@@ -29,7 +29,6 @@
 #include <map>
 #include <mutex>
 #include <numeric>
-#include <thread>
 
 namespace ommgpu {
 
@@ -774,9 +773,7 @@ SpmmPlan& any_plan(const msw_matrix* B) {
     std::vector<Candidate> cands(4);
     {
         const int widths[4] = {8, 16, 24, 32};
-        std::vector<std::thread> th;
-        for (int i = 0; i < 4; ++i) th.emplace_back([&, i] { cands[i] = build_groups(B, widths[i]); });
-        for (auto& t : th) t.join();
+        host_shares(4, [&](int i) { cands[i] = build_groups(B, widths[i]); });
     }
     long long nnz = std::max(1, B->nnz);
     double best = 0.0;

@@ -82,3 +82,34 @@ def test_csc_element_insert_host():
     assert G.m_get_element(M, 3, 2) == 4.0
     assert G.m_get_element(M, 1, 1) == 2.0
     assert G.m_get_element(M, 2, 2) == 0.0
+
+
+def test_host_work_without_threads_to_be_had():
+    """A process that may map no more memory gets no thread (their stacks do not fit): the host-side loops run on
+    the calling thread then, and the call neither fails nor ends the process."""
+    import os
+    import subprocess
+    import sys
+
+    code = """
+import resource
+import numpy as np
+import ommgpu as G
+from ommgpu.synth import CSCMatrix
+m, per = 2000, 100
+rng = np.random.default_rng(0)
+colptr = (np.arange(m + 1) * per).astype(np.int32)
+rowind = np.concatenate([np.sort(rng.choice(m, per, replace=False)) for _ in range(m)]).astype(np.int32)
+A = CSCMatrix(m, m, colptr, rowind, rng.standard_normal(m * per))
+G.lib()
+kb = [int(x.split()[1]) for x in open("/proc/self/status") if x.startswith("VmSize")][0]
+resource.setrlimit(resource.RLIMIT_AS, ((kb << 10) + (7 << 20),) * 2)
+M = G.Matrix.from_csc(A, "sdcsc")
+B = M.csc()
+assert np.array_equal(B.rowind, A.rowind) and np.array_equal(B.val, A.val)
+print("registered")
+"""
+    pkg = os.path.dirname(os.path.dirname(os.path.abspath(G.__file__)))
+    env = dict(os.environ, PYTHONPATH=pkg, OPENBLAS_NUM_THREADS="1")
+    r = subprocess.run([sys.executable, "-c", code], env=env, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and "registered" in r.stdout, (r.returncode, r.stdout, r.stderr)
