@@ -467,7 +467,8 @@ int omm_gpu_tc_set_pairs(int on);
  * reference counterpart (the reference calls BLAS dgemm, e.g. omm_ops.F90:62,
  * MatrixSwitch.F90:1303).  C = alpha*op(A)*op(B) + beta*C, op 'n' or 't',
  * device FP64 column-major arrays.  Each row of op(A) and column of op(B) is
- * scaled by a power of two and rounded to a 53-bit integer; their exact
+ * scaled by a power of two and rounded to a 55-bit integer (54 bits for K
+ * above 10,628, 53 above 42,513); their exact
  * integer product is formed modulo 16 coprime moduli <= 256 by int8 tcgen05
  * GEMMs and rebuilt by the Chinese remainder theorem, then rounded once to
  * FP64 (the accuracy of an FP64 GEMM relative to the rows' and columns'
@@ -500,7 +501,16 @@ int omm_gpu_spmm_f64(const double* A, int lda, int n, const msw_matrix* H, const
 int omm_gpu_set_oz_spmm_form(int form);
 /* Which engine the FP64 products of omm()/MatrixSwitch use: mode 1 (default) = the
  * int8 tensor-core GEMM above or the FP64 tensor cores (mma.sync f64), whichever is
- * estimated to be faster at the product's sizes, 0 = cuBLAS.  panel_bytes caps
+ * estimated to be faster at the product's sizes, 0 = cuBLAS.  What mode 1 gives
+ * up where it takes the int8 GEMM: entries are kept to 53 to 55 bits of the largest
+ * entry of their row of op(A) or column of op(B) (omm_gpu_gemm_f64), not to 53 bits
+ * of their own, so a result that comes only from entries far below the largest
+ * (2^-54 and less of it) loses them, and one Inf or NaN makes its whole row or
+ * column of the result NaN.  This holds for large enough products of MatrixSwitch,
+ * the Gram products, gradients and densities of omm(), omm_gpu_functional_grad, and
+ * omm_gpu_energy_adjoint's density elements; at the solver's shapes the errors
+ * against the exact results are those of FP64 products or smaller.  Mode 0 keeps
+ * every bit of every entry.  panel_bytes caps
  * the scratch of one int8 product's residues (0 = default 4 GiB; larger
  * products run in column panels).  No reference counterpart. */
 int omm_gpu_set_fp64_gemm(int mode, long long panel_bytes);

@@ -366,7 +366,7 @@ struct OzOperand {
     size_t kb_plane = 0;
     bool kb_halves = false;  // kb per 128-row half of each block (the SM-pair SpMM's layout)
 };
-constexpr int OZ_NMOD = 16;    // moduli of the FP64-accurate products (53-bit operands for K < 2^17)
+constexpr int OZ_NMOD = 16;    // moduli of the FP64-accurate products (53- to 55-bit operands for K < 2^17)
 // the residues kept between products (grow-only device buffers, released by oz_release_scratch,
 // which omm_gpu_finalize calls): the CG step's direction and [HC; SC], the two operands of
 // gemm_f64_emu, the operand of omm_gpu_spmm_f64

@@ -18,9 +18,9 @@
 //      with q = round(sum_l r_l W_l / P) taken from FP64 sums of r_l (W_l / P) (exact, since
 //      C'/P is at most 1/4 away from an integer), and the sum formed modulo 2^128 in 32-bit
 //      limbs; C' (|C'| < 2^126) is converted to FP64 and scaled back by 2^(e_r + e_c - ...).
-// With 16 moduli (P ~ 2^125.4) both operands keep 53 bits for any K < 2^17: the result is
-// the exact product of the operands rounded to 53 bits relative to their row maxima, rounded
-// once to FP64 -- the accuracy class of an FP64 GEMM.  The int8 GEMMs run at the tensor
+// With 16 moduli (P ~ 2^125.4) both operands keep 55 bits up to K = 10,628, 54 up to 42,513 and 53 for any
+// K < 2^17 (oz_bits): the result is the exact product of the operands rounded to so many bits relative to
+// their row maxima, rounded once to FP64 -- the accuracy class of an FP64 GEMM.  The int8 GEMMs run at the tensor
 // cores' int8 rate (twice the bf16 rate), i.e. 16 of them cost about 8 bf16 GEMMs.
 //
 // Layouts: the int8 residue operands are K-major planes (plane l = rows x ldk bytes), read by
@@ -122,11 +122,15 @@ struct ModParams {
     uint32_t magic[MAXMOD];             // ceil(2^39 / p): u / p = umulhi(u, magic) >> 7 for u < 2^28
 };
 
-// The residue kernels' constants: x (|x| <= 2^53) is taken as x + 2^53 = hi 2^32 + lo (seven bytes),
-// and for p_l != 256
+// Most bits that an entry keeps: x + 2^MAX_BITS with |x| < 2^MAX_BITS has to fit the seven bytes below.
+// Two more than a double has cost nothing (the products are exact whatever the operands' bits) and leave the
+// entries down to a quarter of their row's largest unrounded, the others with a quarter of the error
+constexpr int MAX_BITS = 55;
+// The residue kernels' constants: x is taken as x + 2^MAX_BITS = hi 2^32 + lo (seven bytes), and for
+// p_l != 256
 struct ModB {
     uint32_t wlo[MAXMOD], whi[MAXMOD];  // the bytes 256^k mod p_l for k = 0..3 and k = 4..6
-    uint32_t e[MAXMOD];                 // p_l - (2^53 mod p_l)
+    uint32_t e[MAXMOD];                 // p_l - (2^MAX_BITS mod p_l)
     uint32_t negp[MAXMOD];              // -p_l (two's complement)
     uint32_t magic[MAXMOD];             // ceil(2^39 / p_l)
     unsigned long long mh[MAXMOD];      // magic * (p_l - 1) / 2
@@ -329,7 +333,7 @@ __device__ __forceinline__ int oz_residue(const Limbs& x, const ModParams& mp, i
     const uint32_t q = __umulhi(u + mp.half[l], mp.magic[l]) >> 7;
     return (int)(u - q * (uint32_t)mp.p[l]);
 }
-// The same residue from x + 2^53 = hi 2^32 + lo, in fewer operations: s = sum_k b_k (256^k mod p)
+// The same residue from x + 2^MAX_BITS = hi 2^32 + lo, in fewer operations: s = sum_k b_k (256^k mod p)
 // over its seven bytes b_k is two byte dot products (s < 7 * 255^2 < 2^19), u = s + e == x (mod p)
 // with u >= 0, q = floor((u + half) / p) = (u magic + half magic) >> 39 exactly (one 32 x 32 + 64
 // multiply-add; the quotient rule above, applied to u + half < 2^20), and r = u - q p in
@@ -340,7 +344,7 @@ __device__ __forceinline__ uint32_t oz_resb(uint32_t lo, uint32_t hi, const ModB
     const uint32_t q = (uint32_t)(((unsigned long long)u * mb.magic[l] + mb.mh[l]) >> 39);
     return u + q * mb.negp[l];
 }
-// the 16 moduli's words of four consecutive entries (x + 2^53 as lo / hi words), stored one plane
+// the 16 moduli's words of four consecutive entries (x + 2^MAX_BITS as lo / hi words), stored one plane
 // apart at dst and, when d2 is set, one kb plane apart at d2
 __device__ __forceinline__ void oz_store_planes_b(uint32_t* dst, size_t plane_words, uint32_t* d2, size_t kb_words,
                                                   const uint32_t (&lo)[4], const uint32_t (&hi)[4], const ModB& mb) {
@@ -365,7 +369,7 @@ __device__ __forceinline__ void oz_store_planes_b(uint32_t* dst, size_t plane_wo
 //
 // Rows contiguous in the source (element (r, k) at A[r + k lda]): a CTA transposes a tile of
 // 32 rows x 128 k through shared memory.  Loading, warp w reads k0 + 16 w .. + 15 for the 32 rows
-// (each read coalesced over the rows; all sixteen loads of a lane first) and stores x + 2^53 of
+// (each read coalesced over the rows; all sixteen loads of a lane first) and stores x + 2^MAX_BITS of
 // the rounded integers.  The tile keeps entry (row, k) at row * RT_LD + k + k / 4, so that the
 // loads' stores (one k, 32 rows: RT_LD odd) and the lanes' reads (one row, k = 4 j + u:
 // 5 j + u) fall in distinct banks.  Computing, without the k-blocked copy warp w takes rows
@@ -417,7 +421,8 @@ __global__ void __launch_bounds__(256) oz_res_rows_kernel(int R, int K, const do
 #pragma unroll
             for (int j = 0; j < 16; ++j) {
                 const int q = 16 * warp + j;
-                tile[lane * RT_LD + q + q / 4] = __double2ll_rn(oz_integer(part ? vi[CPLX ? j : 0] : v[j], f1, f2)) + (1ll << 53);
+                tile[lane * RT_LD + q + q / 4] =
+                    __double2ll_rn(oz_integer(part ? vi[CPLX ? j : 0] : v[j], f1, f2)) + (1ll << MAX_BITS);
             }
         }
         __syncthreads();
@@ -500,7 +505,7 @@ __global__ void __launch_bounds__(256) oz_res_kc_kernel(int R, int K, const doub
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
                 const unsigned long long x =
-                    (unsigned long long)(__double2ll_rn(oz_integer(v[part][s][u], f1, f2)) + (1ll << 53));
+                    (unsigned long long)(__double2ll_rn(oz_integer(v[part][s][u], f1, f2)) + (1ll << MAX_BITS));
                 lo[u] = (uint32_t)x;
                 hi[u] = (uint32_t)(x >> 32);
             }
@@ -1000,8 +1005,8 @@ struct RecParams {
 // q = round(sum_l r_l W_l / P) comes from the 16-bit fixed-point weights round(2^16 W_l / P)
 // (their error, below 16 * 255 * 2^-17, is far inside the 1/4 by which T / P stays off the
 // half-integers).  C' = T - q P = sum_i (S_i - q P[i]) 256^i is formed from i = 4 on: the bytes
-// below 2^32 change C' by less than 2^44, under 2^-60 of the bound 2^-52 max|A'| sum|B'| >= 2^52
-// that a 53-bit product is held to.  Each d_i = S_i - q P[i] is below 2^20 in magnitude (S_i and
+// below 2^32 change C' by less than 2^44, under 2^-60 of what rounding its operands does to C' (at least
+// 2^52, half a unit of A' times an entry of B' of 53 bits or more).  Each d_i = S_i - q P[i] is below 2^20 in magnitude (S_i and
 // q P[i] both lie in [0, 2^20)), so pairs d_i + 256 d_(i+1) stay below 2^29 in 32-bit integers;
 // the bytes 4..9 and 10..15 are summed exactly from three pairs each in two 64-bit integers and
 // joined by one fma, then scaled by 2^(ea + eb - shift + 32).
@@ -1682,7 +1687,7 @@ ModB mod_b() {
         }
         m.wlo[l] = (uint32_t)(w[0] | (w[1] << 8) | (w[2] << 16) | (w[3] << 24));
         m.whi[l] = (uint32_t)(w[4] | (w[5] << 8) | (w[6] << 16));
-        m.e[l] = (uint32_t)(p - (1ull << 53) % p);
+        m.e[l] = (uint32_t)(p - (1ull << MAX_BITS) % p);
         m.negp[l] = (uint32_t)(0u - (uint32_t)p);
         const uint64_t mg = ((1ull << 39) + p - 1) / p;
         m.magic[l] = (uint32_t)mg;
@@ -1877,9 +1882,11 @@ const DevBuf& tile_list(int M, int nc, int herm, int hcols, int c0, int bm, int 
     return ref;
 }
 
+// the int8 SpMM's operands: its column residues (oz_limbs) hold 53 bits
+static int oz_spmm_bits(int K) { return std::min(53, oz_bits(K, OZ_NMOD)); }
 int oz_bits(int K, int nmod) {
     const double room = oz::table(nmod).log2P - 2.0 - std::log2((double)std::max(K, 1));
-    return std::min(53, (int)std::floor(room / 2.0));
+    return std::min(oz::MAX_BITS, (int)std::floor(room / 2.0));
 }
 
 // Width of the 256-row tiles of an M x nc product on the SM pairs: 256 columns move the fewest operand
@@ -2231,8 +2238,8 @@ bool oz_spmm_available(const msw_matrix* H, const msw_matrix* S) {
     if (!H || H->fmt != Fmt::CSC || !H->is_real) return false;
     if (S && (S->fmt != Fmt::CSC || !S->is_real)) return false;
     if (H->dim1 >= (1 << 17) || H->dim1 != H->dim2) return false;
-    if (g_oz_spmm_form == 3 && S && oz_spmm_plan(H, S, oz_bits(H->dim1, OZ_NMOD), 2, true)) return true;
-    return oz_spmm_plan(H, S, oz_bits(H->dim1, OZ_NMOD), g_oz_spmm_form == 3 ? 1 : oz_spmm_sg(), false) != nullptr;
+    if (g_oz_spmm_form == 3 && S && oz_spmm_plan(H, S, oz_spmm_bits(H->dim1), 2, true)) return true;
+    return oz_spmm_plan(H, S, oz_spmm_bits(H->dim1), g_oz_spmm_form == 3 ? 1 : oz_spmm_sg(), false) != nullptr;
 }
 
 // Y (FP64, column-major, ld Y.ld) = A [H, S]: A's product with H in rows 0 .. n-1, with S in rows
@@ -2260,7 +2267,7 @@ bool oz_spmm(const msw_matrix* H, const msw_matrix* S, const OzOperand& A, DView
     // the layout of A's k-blocked copy decides: half-major goes to the SM-pair kernel
     const bool halves = A.kb_halves;
     if (halves && !S) return false;
-    OzSpmmPlan* T = oz_spmm_plan(H, S, oz_bits(H->dim1, OZ_NMOD), halves ? 2 : (g_oz_spmm_form == 3 ? 1 : oz_spmm_sg()),
+    OzSpmmPlan* T = oz_spmm_plan(H, S, oz_spmm_bits(H->dim1), halves ? 2 : (g_oz_spmm_form == 3 ? 1 : oz_spmm_sg()),
                                  halves);
     if (!T || T->bits != A.bits) return false;
     if (n % 4) return false;  // the reconstruction reads four rows' residues at a time
@@ -2527,7 +2534,7 @@ extern "C" int omm_gpu_spmm_f64(const double* A, int lda, int n, const msw_matri
         y.cols = m;
         y.ld = ldy;
         OzOperand* op = &oz_scratch(OZS_SPMM_A);
-        oz_prepare(a, false, n, m, OZ_NMOD, oz_bits(m, OZ_NMOD), *op, true, nullptr, oz_spmm_kb_halves(S != nullptr));
+        oz_prepare(a, false, n, m, OZ_NMOD, oz_spmm_bits(m), *op, true, nullptr, oz_spmm_kb_halves(S != nullptr));
         if (!oz_spmm(H, S, *op, y)) fail(OMM_ERR_UNSUPPORTED, "spmm_f64: n must be a multiple of 4");
         sync();
         unsigned e = gemm_bf16_errors();

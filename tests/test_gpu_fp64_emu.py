@@ -183,3 +183,36 @@ def test_complex_as_four_real_products(opA, opB):
     err_im = np.abs(got.imag - ref.imag.astype(np.float64))
     assert np.all(err_re <= TOL * mag_re + 1e-300), float(np.max(err_re / (mag_re + 1e-300)))
     assert np.all(err_im <= TOL * mag_im + 1e-300), float(np.max(err_im / (mag_im + 1e-300)))
+
+
+@pytest.mark.parametrize("K", [300, 2048, 10628])
+@pytest.mark.parametrize("opA,opB", [("n", "n"), ("t", "t")])
+def test_two_bits_more_than_a_double(opA, opB, K):
+    """Rows of A whose largest entry (1, the first) meets a zero of B and whose others are 2^-54: 55 bits of a
+    row hold them, so the product is theirs, as it is in FP64 arithmetic.  What C' loses below 2^32 units is
+    under 2^44 of its at least 0.5 (K - 1) 2^54 (2^-17 of it for K = 300)."""
+    rng = np.random.default_rng(K)
+    M, N = 150, 170
+    A = np.full((M, K), 2.0 ** -54)
+    A[:, 0] = 1.0
+    B = rng.uniform(0.5, 1.0, (K, N))
+    B[0] = 0.0
+    got, opa, opb, _ = _run(opA, opB, M, N, K, A=A if opA == "n" else np.ascontiguousarray(A.T),
+                            B=B if opB == "n" else np.ascontiguousarray(B.T), C0=np.zeros((M, N)))
+    want = 2.0 ** -54 * B.sum(axis=0)
+    assert np.all(np.abs(got - want) <= 2.0 ** -17 * want)
+
+
+def test_two_bits_more_than_a_double_complex():
+    """The same through the public product, whose complex form stacks the parts."""
+    rng = np.random.default_rng(4)
+    M, N, K = 512, 512, 2048
+    A = np.full((M, K), 2.0 ** -54 * (1 + 1j))
+    A[:, 0] = 1.0 + 1.0j
+    B = (rng.uniform(0.5, 1.0, (K, N)) + 1j * rng.uniform(0.5, 1.0, (K, N)))
+    B[0] = 0.0
+    C = G.Matrix.allocate(M, N, "gzden")
+    G.mm_multiply(G.Matrix.from_numpy(np.asfortranarray(A)), "n", G.Matrix.from_numpy(np.asfortranarray(B)), "n", C)
+    got, want = C.numpy(), 2.0 ** -54 * (1 + 1j) * B.sum(axis=0)
+    size = 2.0 ** -54 * np.abs(B).sum(axis=0)
+    assert np.all(np.abs(got - want) <= 2.0 ** -17 * size)
