@@ -159,3 +159,42 @@ def test_gespmm_duplicates_do_not_hide_a_zero_cell(shuffled):
     touched = np.zeros((m, 40), bool)
     touched[:, 3] = dense[hole] != 0.0
     assert not touched[j, 3] and np.array_equal(~np.isfinite(C.numpy()), touched)
+
+
+@pytest.mark.parametrize("cplx", [False, True])
+@pytest.mark.parametrize("identity", [False, True])
+def test_solve_with_operators_without_groups(identity, cplx):
+    """A small solve (its steps run as graphs) with CSC H and S of no column groups: the gather kernel's products
+    inside the graph give the energy and the density of the same operators held dense."""
+    m, n = 150, 30
+    rng = np.random.default_rng(6)
+
+    def hermitian(scale, diag):
+        x = np.where(rng.random((m, m)) < 0.01, _rnd(rng, (m, m), cplx), 0.0) * scale
+        x = x + x.conj().T
+        np.fill_diagonal(x, diag)
+        return np.asfortranarray(x)
+
+    H = hermitian(0.03, np.where(np.arange(m) < n, -1.0, 1.0))
+    S = None if identity else hermitian(0.01, 1.0)
+    lbl = "gzden" if cplx else "gdden"
+    got = []
+    G.set_log(None)
+    for sparse in (True, False):
+        def reg(x):
+            if x is None or not sparse:
+                return x if x is None else G.Matrix.from_numpy(x)
+            at = np.nonzero(x.T)
+            colptr = np.concatenate([[0], np.cumsum(np.bincount(at[0], minlength=m))]).astype(np.int32)
+            return G.Matrix.from_csc(synth.CSCMatrix(m, m, colptr, at[1].astype(np.int32), x.T[at]))
+
+        C, D = G.Matrix.allocate(n, m, lbl), G.Matrix.allocate(m, m, lbl)
+        e, rc = G.omm(m, n, reg(H), reg(S), True, D, False, 0.0, C, False, cg_tol=1e-12, dealloc=True)
+        assert rc == 0
+        got.append((e, D.numpy()))
+    lam, U = np.linalg.eigh(H if S is None else np.linalg.solve(np.linalg.cholesky(S), np.linalg.solve(
+        np.linalg.cholesky(S), H).conj().T))
+    want = float(lam[:n].sum())
+    for e, _ in got:  # the energies' relative steps fell to 1e-12: within 1e-9 of the eigenvalues' sum
+        assert abs(e - want) <= 1e-9 * abs(want)
+    assert np.abs(got[0][1] - got[1][1]).max() <= 1e-4  # the density's error is the energy's square root
