@@ -21,15 +21,17 @@
 // Operands keep their global order in shared memory (rows or k contiguous, whichever the op makes of
 // them), padded so that the 16 lanes of a half-warp's fragment load (8 lanes for complex elements) fall
 // in distinct banks.  Complex products take four DMMAs per fragment pair.
-// A call through the entry point against cuBLAS's (with its wait, microseconds): 256 x 128 x 832 21 (27), 1,895 x
-// 415 x 161 27 (29), 500^3 25 (28), 3,000 x 3,000 x 16 38 (41), 1,500 x 800 x 300 39 (151), complex 500^3 54
-// (57), 2,500 x 900 x 120 89 (556).
+// A call through the entry point, with cuBLAS's in brackets (with their waits, microseconds): 256 x 128 x 832 20
+// (22), 500^3 25 (26), 1,895 x 415 x 161 29 (26), 3,000 x 3,000 x 16 37 (39), 1,500 x 800 x 300 42 (42), 512 x
+// 512 x 4,096 99 (91), complex 500^3 57 (55), 2,500 x 900 x 120 96 (93); with a third of cuBLAS's rounding error
+// (Sums below), and in a launch that a graph can hold.
 #include "internal.h"
 
 #include <cooperative_groups.h>
 
 #include <algorithm>
 #include <cmath>
+#include <type_traits>
 
 namespace cg = cooperative_groups;
 
@@ -136,8 +138,41 @@ struct Loader {
     }
 };
 
+// A warp's part of the tile: NP parts (real; re and im) of MT x NT fragments.
+template <int NP, int MT, int NT>
+struct Sums {
+    double v[NP][MT][NT][2];
+    __device__ __forceinline__ void clear() {
+#pragma unroll
+        for (int s = 0; s < NP; ++s)
+#pragma unroll
+            for (int i = 0; i < MT; ++i)
+#pragma unroll
+                for (int j = 0; j < NT; ++j) v[s][i][j][0] = v[s][i][j][1] = 0.0;
+    }
+    // adds the sums o and sets them to zero
+    __device__ __forceinline__ void take(Sums& o) {
+#pragma unroll
+        for (int s = 0; s < NP; ++s)
+#pragma unroll
+            for (int i = 0; i < MT; ++i)
+#pragma unroll
+                for (int j = 0; j < NT; ++j) {
+                    v[s][i][j][0] += o.v[s][i][j][0];
+                    v[s][i][j][1] += o.v[s][i][j][1];
+                }
+        o.clear();
+    }
+};
+// LEVELS: K is added up in three levels -- runs of 32 products (two chunks) in the DMMAs' accumulators, eight
+// runs, and those -- because the rounding errors of one chain grow with its length: rms error over
+// sqrt(sum |a|^2 |b|^2) at 512 x 512 x 4,096 2.5e-16, in one chain 2.0e-15; 500^3 2.3e-16 and 7.1e-16 (complex
+// 2.4e-16 and 1.0e-15).  The emulation that larger products take keeps below 1e-16.  It costs 2 to 10 % (512 x 512 x
+// 4,096 94 -> 99 us, 256 x 128 x 832 18.1 -> 18.5); runs of one chunk wait for their DMMAs too often (137 us).
+constexpr int RUN = 2, RUNS = 8;  // chunks of a run, runs of the second level
+
 // TA: A is K-contiguous (op 't' / 'c'); TB: B is column-contiguous (op 't' / 'c')
-template <bool CPLX, int BM, int BN, int WM, int WN, int ST, bool TA, bool TB, bool VEC>
+template <bool CPLX, int BM, int BN, int WM, int WN, int ST, bool TA, bool TB, bool VEC, bool LEVELS>
 __global__ void __launch_bounds__(32 * WM * WN) gemm_dmma_kernel(const __grid_constant__ DgArgs p) {
     using T = typename El<CPLX>::T;
     constexpr int BK = chunk<CPLX>(), MT = BM / (8 * WM), NT = BN / (8 * WN), NP = CPLX ? 2 : 1, NTHR = 32 * WM * WN;
@@ -158,13 +193,10 @@ __global__ void __launch_bounds__(32 * WM * WN) gemm_dmma_kernel(const __grid_co
     const int wm = (warp % WM) * (BM / WM), wn = (warp / WM) * (BN / WN);
     const double *A = p.A[z], *B = p.B[z];
 
-    double acc[NP][MT][NT][2];
-#pragma unroll
-    for (int s = 0; s < NP; ++s)
-#pragma unroll
-        for (int i = 0; i < MT; ++i)
-#pragma unroll
-            for (int j = 0; j < NT; ++j) acc[s][i][j][0] = acc[s][i][j][1] = 0.0;
+    Sums<NP, MT, NT> acc, runs, total;  // the last two: LEVELS only
+    acc.clear();
+    runs.clear();
+    total.clear();
 
     constexpr uint32_t STAGE = (AE + BE) * sizeof(T);
     Loader<CPLX, BM, TA, NTHR, VEC> la(ring, A, p.lda, m0, p.M, k_lo);
@@ -207,17 +239,17 @@ __global__ void __launch_bounds__(32 * WM * WN) gemm_dmma_kernel(const __grid_co
 #pragma unroll
                     for (int j = 0; j < NT; ++j) {
                         const double bi = flip(b[j].y, sb);
-                        dmma(acc[0][i][j], a[i].x, b[j].x);
-                        dmma(acc[NP - 1][i][j], a[i].x, bi);
-                        dmma(acc[0][i][j], nai, bi);
-                        dmma(acc[NP - 1][i][j], ai, b[j].x);
+                        dmma(acc.v[0][i][j], a[i].x, b[j].x);
+                        dmma(acc.v[NP - 1][i][j], a[i].x, bi);
+                        dmma(acc.v[0][i][j], nai, bi);
+                        dmma(acc.v[NP - 1][i][j], ai, b[j].x);
                     }
                 }
             } else {
 #pragma unroll
                 for (int i = 0; i < MT; ++i)
 #pragma unroll
-                    for (int j = 0; j < NT; ++j) dmma(acc[0][i][j], a[i], b[j]);
+                    for (int j = 0; j < NT; ++j) dmma(acc.v[0][i][j], a[i], b[j]);
             }
         }
     };
@@ -230,10 +262,19 @@ __global__ void __launch_bounds__(32 * WM * WN) gemm_dmma_kernel(const __grid_co
                 __syncthreads();  // everyone's part, and the stage of chunk t - 1 is free
                 load(t + ST - 1, ((s + ST - 1) % ST) * STAGE);
                 multiply(s);
+                if (LEVELS && t % RUN == RUN - 1) {
+                    runs.take(acc);
+                    if (t % (RUN * RUNS) == RUN * RUNS - 1) total.take(runs);
+                }
             }
         }
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
+    if constexpr (LEVELS) {
+        runs.take(acc);
+        total.take(runs);
+        acc = total;
+    }
 
     // C(i, j) = alpha v + beta C(i, j), and the mirrored element of a Hermitian block
     auto emit = [&](int i, int j, T v) {
@@ -264,8 +305,8 @@ __global__ void __launch_bounds__(32 * WM * WN) gemm_dmma_kernel(const __grid_co
         }
     };
     auto value = [&](int i, int j, int h) -> T {
-        if constexpr (CPLX) return make_double2(acc[0][i][j][h], acc[NP - 1][i][j][h]);
-        else return acc[0][i][j][h];
+        if constexpr (CPLX) return make_double2(acc.v[0][i][j][h], acc.v[NP - 1][i][j][h]);
+        else return acc.v[0][i][j][h];
     };
     if (S == 1) {
 #pragma unroll
@@ -305,10 +346,10 @@ __global__ void __launch_bounds__(32 * WM * WN) gemm_dmma_kernel(const __grid_co
     cl.sync();  // no CTA leaves while another reads its partial tile
 }
 
-template <bool CPLX, int BM, int BN, int WM, int WN, int ST, bool TA, bool TB, bool VEC>
+template <bool CPLX, int BM, int BN, int WM, int WN, int ST, bool TA, bool TB, bool VEC, bool LEVELS>
 void launch_t(const DgArgs& a, int nz, int split) {
     constexpr int SM = smem_bytes<CPLX, BM, BN, ST, TA, TB>();
-    auto kernel = gemm_dmma_kernel<CPLX, BM, BN, WM, WN, ST, TA, TB, VEC>;
+    auto kernel = gemm_dmma_kernel<CPLX, BM, BN, WM, WN, ST, TA, TB, VEC, LEVELS>;
     static bool attr = false;
     if (!attr) {
         OMM_CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SM));
@@ -327,12 +368,12 @@ void launch_t(const DgArgs& a, int nz, int split) {
     OMM_CK(cudaLaunchKernelEx(&cfg, kernel, a));
     OMM_KCHECK();
 }
-template <bool CPLX, int BM, int BN, int WM, int WN, int ST, bool VEC>
+template <bool CPLX, int BM, int BN, int WM, int WN, int ST, bool VEC, bool LEVELS>
 void launch_ops(const DgArgs& a, bool ta, bool tb, int nz, int split) {
-    if (ta && tb) launch_t<CPLX, BM, BN, WM, WN, ST, true, true, VEC>(a, nz, split);
-    else if (ta) launch_t<CPLX, BM, BN, WM, WN, ST, true, false, VEC>(a, nz, split);
-    else if (tb) launch_t<CPLX, BM, BN, WM, WN, ST, false, true, VEC>(a, nz, split);
-    else launch_t<CPLX, BM, BN, WM, WN, ST, false, false, VEC>(a, nz, split);
+    if (ta && tb) launch_t<CPLX, BM, BN, WM, WN, ST, true, true, VEC, LEVELS>(a, nz, split);
+    else if (ta) launch_t<CPLX, BM, BN, WM, WN, ST, true, false, VEC, LEVELS>(a, nz, split);
+    else if (tb) launch_t<CPLX, BM, BN, WM, WN, ST, false, true, VEC, LEVELS>(a, nz, split);
+    else launch_t<CPLX, BM, BN, WM, WN, ST, false, false, VEC, LEVELS>(a, nz, split);
 }
 
 // Split of K by an estimate of the time in SM clocks: the CTAs of the busiest SM in turn, each with a
@@ -344,7 +385,7 @@ struct Config {
     double us;
 };
 Config pick(bool cplx, int M, int N, int K, int nz, bool herm, bool wide = true) {
-    const double chunk_k = cplx ? 8.0 : 16.0, busy = cplx ? 550.0 : wide ? 300.0 : 390.0, alone = cplx ? 800.0 : 425.0;
+    const double chunk_k = cplx ? 8.0 : 16.0, busy = cplx ? 590.0 : wide ? 315.0 : 405.0, alone = cplx ? 830.0 : 440.0;
     const double tiles = (double)((M + 31) / 32) * ((N + 31) / 32) * nz * (herm ? 0.6 : 1.0);
     Config best{1, 1e300};
     for (int s = 1; s <= 8; s *= 2) {
@@ -407,9 +448,16 @@ void gemm_dmma(char opA, char opB, int M, int N, int K, const double alpha[2], c
     const Config c = pick(cplx, M, N, K, nz, any && nz == 1);
     const int bk = cplx ? 8 : 16;
     a.kper = std::max(bk, ((K + c.split - 1) / c.split + bk - 1) / bk * bk);
-    if (cplx) launch_ops<true, 32, 32, 2, 2, 2, true>(a, ta, tb, nz, c.split);
-    else if (a.vec) launch_ops<false, 32, 32, 2, 2, 3, true>(a, ta, tb, nz, c.split);
-    else launch_ops<false, 32, 32, 2, 2, 3, false>(a, ta, tb, nz, c.split);
+    // at most 64 real products or 16 complex ones are one chain: as accurate as cuBLAS's, and the two sums more
+    // cost registers (3,000 x 3,000 x 16 38 us, 44 with them)
+    auto launch = [&](auto levels) {
+        constexpr bool LV = decltype(levels)::value;
+        if (cplx) launch_ops<true, 32, 32, 2, 2, 2, true, LV>(a, ta, tb, nz, c.split);
+        else if (a.vec) launch_ops<false, 32, 32, 2, 2, 3, true, LV>(a, ta, tb, nz, c.split);
+        else launch_ops<false, 32, 32, 2, 2, 3, false, LV>(a, ta, tb, nz, c.split);
+    };
+    if (a.kper <= (cplx ? 16 : 64)) launch(std::false_type{});
+    else launch(std::true_type{});
 }
 
 }  // namespace ommgpu

@@ -1,6 +1,7 @@
 """FP64 products on the FP64 tensor cores at the edges of their tiles, chunks and K splits (mm_multiply picks
 them for products too small for the int8 emulation), against torch's FP64 products of the same operands:
 both sides are within a few ulp of the sums of magnitudes, so 1e-13 |A||B| holds at K up to 10^4."""
+import numpy as np
 import pytest
 
 import ommgpu as G
@@ -165,3 +166,32 @@ def test_zero_alpha_reads_no_operand(M, N, K, beta, cplx):
     torch.cuda.synchronize()
     G.mm_multiply(a, "n", b, "n", c, 0.0, beta)
     assert torch.equal(kc.t(), torch.zeros_like(C0) if beta == 0.0 else beta * C0)
+
+
+@pytest.mark.parametrize("cplx,M,N,K", [(False, 512, 512, 4096), (False, 130, 1611, 3000), (False, 500, 500, 500),
+                                        (False, 45, 37, 260), (False, 256, 128, 832), (True, 500, 500, 500),
+                                        (True, 256, 128, 832), (True, 45, 37, 260)])
+@pytest.mark.parametrize("opA,opB", [("n", "n"), ("t", "c")])
+def test_errors_do_not_grow_with_k(M, N, K, opA, opB, cplx):
+    """K is added up in runs of 32 products, eights of runs and those: the rms error over sqrt(sum |a|^2 |b|^2).
+    A chain of L additions of terms of one variance rounds partial sums of variance j = 1 .. L; each rounding is
+    at most a half unit in the last place of its sum, of rms 2u / sqrt(12) of it, so the chain's relative variance
+    is at most (u^2 / 3) L / 2.  The levels' add: L = 32, 8 and K / 256 (complex: twice the products; and at most
+    eight parts of a split K).  One chain of K = 4,096 would be at 26 u.  A margin of 15 % for the sample."""
+    rng = np.random.default_rng(M + N + K)
+
+    def rnd(r, c):
+        a = rng.standard_normal((r, c))
+        return np.asfortranarray(a + 1j * rng.standard_normal((r, c)) if cplx else a)
+
+    A = rnd(*((M, K) if opA == "n" else (K, M)))
+    B = rnd(*((K, N) if opB == "n" else (N, K)))
+    C = G.Matrix.allocate(M, N, "gzden" if cplx else "gdden")
+    G.mm_multiply(G.Matrix.from_numpy(A), opA, G.Matrix.from_numpy(B), opB, C)
+    a = (A if opA == "n" else A.T)[:40]
+    b = (B if opB == "n" else B.conj().T)[:, :30]
+    long = np.clongdouble if cplx else np.longdouble
+    err = np.abs(C.numpy()[:40, :30] - a.astype(long) @ b.astype(long)).astype(float)
+    size = np.sqrt(np.abs(a) ** 2 @ np.abs(b) ** 2)
+    bar = 2.0 ** -53 * np.sqrt((32 + 8 + (2 if cplx else 1) * K / 256 + 8) / 6)
+    assert np.sqrt(np.mean((err / size) ** 2)) <= 1.15 * bar
