@@ -401,13 +401,17 @@ Config pick(bool cplx, int M, int N, int K, int nz, bool herm, bool wide = true)
 
 }  // namespace
 
-// Products cuBLAS has the better split for, left to it (a call, microseconds, cuBLAS / this kernel): complex
-// ones with a long K (64 x 64 x 3,000 29 / 37, 100 x 1,000 x 3,000 115 / 131, 64 x 3,000 x 3,000 161 / 208; at
-// K = 1,000 or below this kernel leads, 257 x 259 x 1,001 45 / 43), and real ones of one or two rows of tiles
-// with a long K (64 x 3,000 x 3,000 61 / 64; 100 x 1,000 x 3,000 49 / 48, 130 x 260 x 3,000 34 / 30).
+// Products cuBLAS has the better split for, left to it where the emulation never took them (a call, microseconds,
+// cuBLAS / this kernel): complex ones with a long K (64 x 64 x 3,000 27 / 37, 64 x 3,000 x 3,000 160 / 208; with
+// more than 32 tiles from K = 1,000 on: 300 x 150 x 1,000 34 / 40, 257 x 259 x 1,001 43 / 49; 64 x 200 x 1,300
+// leads with 24 / 25), and real ones of one or two rows of tiles with a long K (64 x 3,000 x 3,000 59 / 64; 100 x
+// 1,000 x 3,000 47 / 50, 130 x 260 x 3,000 32 / 29).  Complex ones large enough for the emulation to be had
+// (fp64_emu_fits) take it or this kernel although cuBLAS is faster (300 x 150 x 3,000 61 / 80, 130 x 700 x 2,000
+// 73 / 102): cuBLAS's rounding error there is 7.0e-16, this kernel's 2.5e-16, the emulation's below 1e-16.
 bool gemm_dmma_slower(bool cplx, int M, int N, int K) {
-    if (cplx) return K >= 1500;
-    return K >= 2500 && std::min(M, N) <= 64 && std::max(M, N) >= 1500;
+    if (!cplx) return K >= 2500 && std::min(M, N) <= 64 && std::max(M, N) >= 1500;
+    if (fp64_emu_fits(M, N, K)) return false;
+    return K >= 1500 || (K >= 1000 && ((M + 31) / 32) * (long long)((N + 31) / 32) > 32);
 }
 
 double gemm_dmma_us(bool cplx, int M, int N, int K, int nz, bool wide) { return pick(cplx, M, N, K, nz, false, wide).us; }

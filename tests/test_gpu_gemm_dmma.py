@@ -170,7 +170,7 @@ def test_zero_alpha_reads_no_operand(M, N, K, beta, cplx):
 
 @pytest.mark.parametrize("cplx,M,N,K", [(False, 512, 512, 4096), (False, 130, 1611, 3000), (False, 500, 500, 500),
                                         (False, 45, 37, 260), (False, 256, 128, 832), (True, 500, 500, 500),
-                                        (True, 256, 128, 832), (True, 45, 37, 260)])
+                                        (True, 256, 128, 832), (True, 45, 37, 260), (True, 300, 150, 3000)])
 @pytest.mark.parametrize("opA,opB", [("n", "n"), ("t", "c")])
 def test_errors_do_not_grow_with_k(M, N, K, opA, opB, cplx):
     """K is added up in runs of 32 products, eights of runs and those: the rms error over sqrt(sum |a|^2 |b|^2).
