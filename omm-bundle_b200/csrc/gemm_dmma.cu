@@ -164,15 +164,14 @@ struct Sums {
         o.clear();
     }
 };
-// LEVELS: K is added up in three levels -- runs of 32 products (two chunks) in the DMMAs' accumulators, eight
-// runs, and those -- because the rounding errors of one chain grow with its length: rms error over
-// sqrt(sum |a|^2 |b|^2) at 512 x 512 x 4,096 2.5e-16, in one chain 2.0e-15; 500^3 2.3e-16 and 7.1e-16 (complex
-// 2.4e-16 and 1.0e-15).  The emulation that larger products take keeps below 1e-16.  It costs 2 to 10 % (512 x 512 x
-// 4,096 94 -> 99 us, 256 x 128 x 832 18.1 -> 18.5); runs of one chunk wait for their DMMAs too often (137 us).
-constexpr int RUN = 2, RUNS = 8;  // chunks of a run, runs of the second level
+// RUN > 0: K is added up in runs of RUN chunks (16 products each) in the DMMAs' accumulators, and those -- with
+// THIRD in eights first -- because the rounding errors of one chain grow with its length.  Rms error over
+// sqrt(sum |a|^2 |b|^2), and time: 512 x 512 x 4,096 in one chain 2.0e-15 and 94 us, in runs of 32 products 2.4e-16
+// and 99 us (of 64: 3.8e-16 and 96; of 16, which wait for their DMMAs too often: 2.4e-16 and 137).
+constexpr int RUNS = 8;  // runs of the second level
 
 // TA: A is K-contiguous (op 't' / 'c'); TB: B is column-contiguous (op 't' / 'c')
-template <bool CPLX, int BM, int BN, int WM, int WN, int ST, bool TA, bool TB, bool VEC, bool LEVELS>
+template <bool CPLX, int BM, int BN, int WM, int WN, int ST, bool TA, bool TB, bool VEC, int RUN, bool THIRD>
 __global__ void __launch_bounds__(32 * WM * WN) gemm_dmma_kernel(const __grid_constant__ DgArgs p) {
     using T = typename El<CPLX>::T;
     constexpr int BK = chunk<CPLX>(), MT = BM / (8 * WM), NT = BN / (8 * WN), NP = CPLX ? 2 : 1, NTHR = 32 * WM * WN;
@@ -193,7 +192,7 @@ __global__ void __launch_bounds__(32 * WM * WN) gemm_dmma_kernel(const __grid_co
     const int wm = (warp % WM) * (BM / WM), wn = (warp / WM) * (BN / WN);
     const double *A = p.A[z], *B = p.B[z];
 
-    Sums<NP, MT, NT> acc, runs, total;  // the last two: LEVELS only
+    Sums<NP, MT, NT> acc, runs, total;  // runs: RUN > 0 only, total: THIRD only
     acc.clear();
     runs.clear();
     total.clear();
@@ -262,18 +261,25 @@ __global__ void __launch_bounds__(32 * WM * WN) gemm_dmma_kernel(const __grid_co
                 __syncthreads();  // everyone's part, and the stage of chunk t - 1 is free
                 load(t + ST - 1, ((s + ST - 1) % ST) * STAGE);
                 multiply(s);
-                if (LEVELS && t % RUN == RUN - 1) {
-                    runs.take(acc);
-                    if (t % (RUN * RUNS) == RUN * RUNS - 1) total.take(runs);
+                if constexpr (RUN > 0) {
+                    if (t % RUN == RUN - 1) {
+                        runs.take(acc);
+                        if constexpr (THIRD)
+                            if (t % (RUN * RUNS) == RUN * RUNS - 1) total.take(runs);
+                    }
                 }
             }
         }
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
-    if constexpr (LEVELS) {
+    if constexpr (RUN > 0) {
         runs.take(acc);
-        total.take(runs);
-        acc = total;
+        if constexpr (THIRD) {
+            total.take(runs);
+            acc = total;
+        } else {
+            acc = runs;
+        }
     }
 
     // C(i, j) = alpha v + beta C(i, j), and the mirrored element of a Hermitian block
@@ -346,10 +352,10 @@ __global__ void __launch_bounds__(32 * WM * WN) gemm_dmma_kernel(const __grid_co
     cl.sync();  // no CTA leaves while another reads its partial tile
 }
 
-template <bool CPLX, int BM, int BN, int WM, int WN, int ST, bool TA, bool TB, bool VEC, bool LEVELS>
+template <bool CPLX, int BM, int BN, int WM, int WN, int ST, bool TA, bool TB, bool VEC, int RUN, bool THIRD>
 void launch_t(const DgArgs& a, int nz, int split) {
     constexpr int SM = smem_bytes<CPLX, BM, BN, ST, TA, TB>();
-    auto kernel = gemm_dmma_kernel<CPLX, BM, BN, WM, WN, ST, TA, TB, VEC, LEVELS>;
+    auto kernel = gemm_dmma_kernel<CPLX, BM, BN, WM, WN, ST, TA, TB, VEC, RUN, THIRD>;
     static bool attr = false;
     if (!attr) {
         OMM_CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SM));
@@ -368,12 +374,12 @@ void launch_t(const DgArgs& a, int nz, int split) {
     OMM_CK(cudaLaunchKernelEx(&cfg, kernel, a));
     OMM_KCHECK();
 }
-template <bool CPLX, int BM, int BN, int WM, int WN, int ST, bool VEC, bool LEVELS>
+template <bool CPLX, int BM, int BN, int WM, int WN, int ST, bool VEC, int RUN, bool THIRD>
 void launch_ops(const DgArgs& a, bool ta, bool tb, int nz, int split) {
-    if (ta && tb) launch_t<CPLX, BM, BN, WM, WN, ST, true, true, VEC, LEVELS>(a, nz, split);
-    else if (ta) launch_t<CPLX, BM, BN, WM, WN, ST, true, false, VEC, LEVELS>(a, nz, split);
-    else if (tb) launch_t<CPLX, BM, BN, WM, WN, ST, false, true, VEC, LEVELS>(a, nz, split);
-    else launch_t<CPLX, BM, BN, WM, WN, ST, false, false, VEC, LEVELS>(a, nz, split);
+    if (ta && tb) launch_t<CPLX, BM, BN, WM, WN, ST, true, true, VEC, RUN, THIRD>(a, nz, split);
+    else if (ta) launch_t<CPLX, BM, BN, WM, WN, ST, true, false, VEC, RUN, THIRD>(a, nz, split);
+    else if (tb) launch_t<CPLX, BM, BN, WM, WN, ST, false, true, VEC, RUN, THIRD>(a, nz, split);
+    else launch_t<CPLX, BM, BN, WM, WN, ST, false, false, VEC, RUN, THIRD>(a, nz, split);
 }
 
 // Split of K by an estimate of the time in SM clocks: the CTAs of the busiest SM in turn, each with a
@@ -452,16 +458,28 @@ void gemm_dmma(char opA, char opB, int M, int N, int K, const double alpha[2], c
     const Config c = pick(cplx, M, N, K, nz, any && nz == 1);
     const int bk = cplx ? 8 : 16;
     a.kper = std::max(bk, ((K + c.split - 1) / c.split + bk - 1) / bk * bk);
-    // at most 64 real products or 16 complex ones are one chain: as accurate as cuBLAS's, and the two sums more
-    // cost registers (3,000 x 3,000 x 16 38 us, 44 with them)
-    auto launch = [&](auto levels) {
-        constexpr bool LV = decltype(levels)::value;
-        if (cplx) launch_ops<true, 32, 32, 2, 2, 2, true, LV>(a, ta, tb, nz, c.split);
-        else if (a.vec) launch_ops<false, 32, 32, 2, 2, 3, true, LV>(a, ta, tb, nz, c.split);
-        else launch_ops<false, 32, 32, 2, 2, 3, false, LV>(a, ta, tb, nz, c.split);
+    auto launch = [&](auto run, auto third) {
+        constexpr int RUN = decltype(run)::value;
+        constexpr bool THIRD = decltype(third)::value;
+        if (cplx) launch_ops<true, 32, 32, 2, 2, 2, true, RUN, (RUN > 0)>(a, ta, tb, nz, c.split);
+        else if (a.vec) launch_ops<false, 32, 32, 2, 2, 3, true, RUN, THIRD>(a, ta, tb, nz, c.split);
+        else launch_ops<false, 32, 32, 2, 2, 3, false, RUN, THIRD>(a, ta, tb, nz, c.split);
     };
-    if (a.kper <= (cplx ? 16 : 64)) launch(std::false_type{});
-    else launch(std::true_type{});
+    // At most 64 real products or 16 complex ones are one chain: as accurate as cuBLAS's, and the sums cost
+    // registers (3,000 x 3,000 x 16 38 us, 44 with all three).  Runs of 32 where the emulation was had before this
+    // kernel (fp64_emu_fits), whose 2.0e-16 to 2.5e-16 they keep, and for short complex products (37 x 53 x 61
+    // 2.1e-16 as cuBLAS, in runs of 64 2.6e-16); elsewhere cuBLAS's 3.4e-16 to 7e-16 are the measure, and runs of 64
+    // do: 500^3 24.0 -> 24.4 us, 7.1e-16 -> 2.8e-16; complex 51 -> 52, 1.0e-15 -> 2.9e-16; 256 x 128 x 832 18.3 us
+    // either way, 4.7e-16 -> 2.8e-16.  The third level's registers let five CTAs of a
+    // real product share an SM: where a few more are to be run, and at most 32 runs, two levels are faster (900^3,
+    // 841 CTAs, 72 us against 85, 65 in one chain; 1,100 x 900 x 700, 1,015, 67 against 72), elsewhere slower
+    // (1,500 x 800 x 300, 1,175, 47 against 41; 512 x 512 x 4,096 118 against 99).
+    const long long ctas = (long long)((M + 31) / 32) * ((N + 31) / 32) * nz;
+    const bool crowded = !cplx && c.split == 1 && ctas > 148 * 5 && ctas <= 148 * 7 && a.kper <= 1024;
+    if (a.kper <= (cplx ? 16 : 64)) launch(std::integral_constant<int, 0>{}, std::false_type{});
+    else if (!fp64_emu_fits(M, N, K) && !(cplx && K <= 128)) launch(std::integral_constant<int, 4>{}, std::true_type{});
+    else if (crowded) launch(std::integral_constant<int, 2>{}, std::false_type{});
+    else launch(std::integral_constant<int, 2>{}, std::true_type{});
 }
 
 }  // namespace ommgpu
