@@ -4,11 +4,11 @@
 #include <algorithm>
 #include <cstdlib>
 #include <deque>
+#include <exception>
 #include <map>
 #include <mutex>
 #include <new>
 #include <set>
-#include <system_error>
 #include <thread>
 
 namespace ommgpu {
@@ -148,16 +148,27 @@ void host_parallel(long long count, const std::function<void(long long, long lon
 }
 
 void host_shares(int n, const std::function<void(int)>& f) {
+    std::exception_ptr thrown;
+    std::mutex mu;
+    auto share = [&](int t) {  // nothing may leave a thread, or pass threads that run
+        try {
+            f(t);
+        } catch (...) {
+            std::lock_guard<std::mutex> lk(mu);
+            if (!thrown) thrown = std::current_exception();
+        }
+    };
     std::vector<std::thread> th;
     th.reserve((size_t)std::max(0, n - 1));
     int t = 1;
     try {
-        for (; t < n; ++t) th.emplace_back(f, t);
-    } catch (const std::system_error&) {
+        for (; t < n; ++t) th.emplace_back(share, t);
+    } catch (const std::exception&) {  // no thread to be had, or no memory for its state
     }
-    if (n > 0) f(0);
-    for (; t < n; ++t) f(t);  // the system has no more threads to give
+    if (n > 0) share(0);
+    for (; t < n; ++t) share(t);  // the system has no more threads to give
     for (auto& x : th) x.join();
+    if (thrown) std::rethrow_exception(thrown);
 }
 
 }  // namespace ommgpu

@@ -178,10 +178,10 @@ template <typename T>
 using HostVec = std::vector<T, HostAlloc<T>>;
 
 // f(begin, end) over [0, count) split across up to 16 host threads (one thread below
-// 64 items per thread).  f must not throw: record failures and report them after the call.
+// 64 items per thread), with exceptions as host_shares has them.
 void host_parallel(long long count, const std::function<void(long long, long long)>& f);
-// f(0) .. f(n - 1) on a host thread each; those that the system refuses a thread run on the caller's.  f must
-// not throw.
+// f(0) .. f(n - 1) on a host thread each; those that the system refuses a thread run on the caller's.  What a share
+// throws (the first of them) is thrown to the caller once all have ended.
 void host_shares(int n, const std::function<void(int)>& f);
 void spmm_plan_cache_clear();  // drop the column-group plans kept by pattern (spmm.cu)
 
