@@ -291,7 +291,8 @@ void k_fill_lower_from_upper(DView& C);      // C(j,i) = conj(C(i,j)) for j > i
 void k_w_update(DView& W, const DView& Wd, const DView& Wdd, double x);  // W += x (Wd^H + Wd) + x^2 Wdd
 void k_calcG_left(const DView& SW, const DView& HW, DView& L);  // L = [4I - 2 SW, -2 HW], n x 2n
 void k_lcg_init(DView& C);                   // reference C0 (NORAND LCG), unscaled
-// reductions (deterministic two-pass); results copied to host
+// reductions: the block that ends last adds up the others' sums in a fixed order and writes the result to pinned
+// memory (r_lambda, and r_coeff with a line search: to device memory)
 void r_trace(const DView& A, double out[2]);                          // sum of diagonal
 void r_dot(const DView& A, const DView& B, double out[2]);            // sum conj(A) B
 void r_coeff(const DView& HW, const DView& SW, const DView& HWd, const DView& SWd, const DView& HWdd,

@@ -1152,8 +1152,8 @@ __global__ void __launch_bounds__(128) oz_reconstruct_z_kernel(const __grid_cons
 
 // ------------------------------------------------------------------ FP64 SpMM on the int8 tensor cores
 // Y = A [H, S] for atom-block CSC H and S (omm_gpu_spmm_f64; the CG step's [HG; SG] = D [H, S] takes the
-// FP64 tensor-core kernel of spmm.cu) by the same modular method: A's rows and H's / S's columns are rounded to 53-bit integers, and every modulus
-// is one int8 SpMM over the column-group plan of spmm.cu -- output columns in groups of G whose
+// FP64 tensor-core kernel of spmm.cu) by the same modular method: A's rows and H's / S's columns are rounded to
+// 53-bit integers, and every modulus is one int8 SpMM over the column-group plan of spmm.cu -- output columns in groups of G whose
 // nonzero rows form a union U_g -- with U_g covered by 16-row chunks.  A's residues come
 // k-blocked (per block of 256 rows, chunk c holds A(:, 16 c .. 16 c + 15) as 256 rows x 16 B,
 // contiguous), so a chunk is one 4 KB bulk copy that lands in the K-major no-swizzle layout

@@ -199,9 +199,10 @@ struct DmmaArgs {
     int vec;      // A's column segments are 16-byte aligned
 };
 
-// CTAs per SM the registers are held to (0: no bound).  One value set, 128 rows: five CTAs 978 us, four 1,020;
-// 64 rows: eight 992, six 1,076; two value sets, 64 rows: five 1,820, four 1,936; 128 rows: three of 154
-// registers 1,822, four of 128 1,927.
+// CTAs per SM the registers are held to (0: no bound), from groups of 24 columns.  One value set, 128 rows: five
+// CTAs 978 us, four 1,020; 64 rows: eight 992, six 1,076; two value sets, 64 rows: five 1,820, four 1,936; 128 rows:
+// three of 154 registers 1,822, four of 128 1,927.  With groups of 32 the first bound spills 40 bytes (6 x 6 x 6
+// atoms, 1,536 rows: 783 us; the kernel without the bound and the copies' fixed addresses took 894).
 constexpr int dmma_ctas(int nm, int mt, bool cplx) {
     return cplx ? 0 : nm == 1 ? (mt == 4 ? 5 : mt == 2 ? 8 : 0) : (mt == 2 ? 5 : 0);
 }
@@ -1094,8 +1095,8 @@ void gemspm(char opA, const DView& A, char opB, const msw_matrix* B, DView& C, c
 // C^T = op(B)^T op(A)^T with the dense x CSC kernels.  op(A)^T is A^T's CSC for 'n' and A itself
 // otherwise; where 'c' asks for conj(A), the dense operand is conjugated instead and so is the
 // product: conj(conj(X) A) = X conj(A).  The column-group kernel writes the product transposed, in
-// place of a second matrix and a transposing add (5 x 5 x 5 atoms of 24 orbitals, 375 columns: 100 us
-// with the transposed copy of B; the gather kernel, which took every pattern before, 500 us).
+// place of a second matrix and a transposing add (5 x 5 x 5 atoms of 24 orbitals, 375 columns: 109 us
+// with the transposed copy of B and C's read; the gather kernel, which took every pattern before, 500 us).
 void gespmm(char opA, const msw_matrix* A, char opB, const DView& B, DView& C, const double alpha[2],
             const double beta[2]) {
     const bool real = B.is_real;
