@@ -424,7 +424,8 @@ void apply_HS(OmmCall& c, const DView& A, DevBuf& stack) {
     if (!c.hcb && !c.H_csc && !c.S_csc && c.H.ld == c.S.ld && fp64_emu_enabled() &&
         !fp64_emu_worth(n, m, m, !c.real) && gemm_dmma_takes(A) && gemm_dmma_takes(c.H) && gemm_dmma_takes(c.S)) {
         // dense H and S in one launch, also where a single product would be left to cuBLAS (gemm_dmma_slower):
-        // complex solves of m = 1,500 to 3,000, n = 24 to 100 were as fast or up to 1.7 times faster than with it
+        // complex solves of m = 1,500 to 3,000, n = 24 to 100 are as fast as their steps with cuBLAS were, or up to
+        // 1.7 times faster
         const DView a[2] = {A, A}, b[2] = {c.H, c.S};
         DView out[2] = {top, bot};
         gemm_dmma('n', 'n', n, m, m, ONE, a, b, ZERO, out, 2);
@@ -1060,8 +1061,9 @@ double energy_c0(OmmCall& c) {
 
 // D = C^H * CD for a Hermitian result (CD = QW C with QW Hermitian): only the blocks on and
 // above the diagonal are computed, then the lower triangle is mirrored: the emulation or the FP64 tensor cores
-// by size.  Without the emulation (omm_gpu_set_fp64_gemm(0, ...)) large m are nb x nb plain GEMMs (cuBLAS's GEMM runs about 1.4x faster per
-// flop than its syrkx at these shapes; the diagonal blocks cost 1/nb extra flops), small m take syrkx / herkx.
+// by size.  Without the emulation (omm_gpu_set_fp64_gemm(0, ...)) large m are nb x nb plain GEMMs (cuBLAS's GEMM
+// runs about 1.4x faster per flop than its syrkx at these shapes; the diagonal blocks cost 1/nb extra flops), small
+// m take syrkx / herkx.
 void density_product(const DView& C, const DView& CD, DView& D) {
     Runtime& R = rt();
     int m = C.cols, n = C.rows;
